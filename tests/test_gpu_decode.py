@@ -74,3 +74,23 @@ def test_evaluate_guesses(qcb, frames, k):
     # no guessed faults: a shot fails exactly when a measured logical bit is set
     z = qcb.evaluate_guesses(f, logical, np.zeros((frames, k), bool), faults)
     assert z == np.count_nonzero(om[:, logical - 1].any(axis=1)) / frames
+
+
+@pytest.mark.parametrize("frames,nsel,start", [(1, 1, 0), (511, 63, 3), (512, 64, 0), (513, 65, 1), (1025, 1023, 1),
+                                               (95, 1024, 0), (544, 1025, 0), (33, 2113, 0)])
+def test_syndrome_rows_tile_edges(qcb, frames, nsel, start):
+    """Edges of the transposing kernel's tiles (512 shots, 64..1024 bits): runs
+    of consecutive bits and index lists, into host and device memory."""
+    import torch
+
+    rng = np.random.default_rng(nsel)
+    nb = 2200
+    meas = rng.random((frames, nb)) < 0.5
+    f = qcb.PauliFrame(frames, 1, nb, init=False).set_measurements(meas)
+    for bits in (np.arange(start + 1, start + nsel + 1), rng.integers(1, nb + 1, nsel)):
+        want = pack_rows(meas[:, bits - 1])
+        assert np.array_equal(f.syndrome_rows(bits), want)
+        b = bits.astype(np.uint32)
+        out = torch.full(want.shape, -1, dtype=torch.int64, device="cuda")
+        qcb.check(qcb.lib().qcb_frame_syndrome_rows(f.handle, b.ctypes.data, len(b), out.data_ptr(), 1, None))
+        assert np.array_equal(out.cpu().numpy().view(np.uint64), want)
