@@ -207,20 +207,21 @@ __global__ void prodphase_comm_kernel(const uint64_t* l, uint8_t lph, const uint
 // ---------------------------------------------------------- symbolic gates
 // Bit-sliced truth tables with the phase flag (src/symbolic_cliffords.jl
 // :105-118 and :358-395).
-__device__ __forceinline__ uint64_t g1(uint32_t op, uint64_t& x, uint64_t& z) {
-  const uint64_t X = x, Z = z;
+template <class T>
+__device__ __forceinline__ T g1(uint32_t op, T& x, T& z) {
+  const T X = x, Z = z;
   if ((op & 0xFFu) == QCB_OP_SQO) {
     // SingleQubitOperator (src/symbolic_cliffords.jl:178-206), flags in bits
     // 8..13: +2 for px & x, for pz & z, and for x & z when the map sends Y to
     // minus the product of the images of X and Z
     const uint32_t f = op >> 8;
     const bool bxx = f & 1u, bxz = f & 2u, bzx = f & 4u, bzz = f & 8u;
-    const uint64_t xx = 0ull - (uint64_t)bxx, xz = 0ull - (uint64_t)bxz;
-    const uint64_t zx = 0ull - (uint64_t)bzx, zz = 0ull - (uint64_t)bzz;
+    const T xx = (T)0 - (T)bxx, xz = (T)0 - (T)bxz;
+    const T zx = (T)0 - (T)bzx, zz = (T)0 - (T)bzz;
     const bool anticom = (!bzz && bxz && !bxx && bzx) || (bzz && !bxz && bxx && bzx) || (bzz && bxz && bxx && !bzx);
     x = (X & xx) ^ (Z & zx);
     z = (X & xz) ^ (Z & zz);
-    return ((f & 16u) ? X : 0ull) ^ ((f & 32u) ? Z : 0ull) ^ (anticom ? (X & Z) : 0ull);
+    return ((f & 16u) ? X : (T)0) ^ ((f & 32u) ? Z : (T)0) ^ (anticom ? (X & Z) : (T)0);
   }
   switch (op) {
     case QCB_OP_H: x = Z; z = X; return X & Z;
@@ -241,9 +242,9 @@ __device__ __forceinline__ uint64_t g1(uint32_t op, uint64_t& x, uint64_t& z) {
   }
 }
 
-__device__ __forceinline__ uint64_t g2(uint32_t op, uint64_t& x1, uint64_t& z1, uint64_t& x2,
-                                       uint64_t& z2) {
-  const uint64_t a = x1, b = z1, c = x2, d = z2;
+template <class T>
+__device__ __forceinline__ T g2(uint32_t op, T& x1, T& z1, T& x2, T& z2) {
+  const T a = x1, b = z1, c = x2, d = z2;
   switch (op) {
     case QCB_OP_SWAP: x1 = c; z1 = d; x2 = a; z2 = b; return 0;
     case QCB_OP_CNOT: z1 = b ^ d; x2 = c ^ a; return (a & b & c & d) | (a & d & ~(b | c));
@@ -351,6 +352,111 @@ __global__ void apply_gates_kernel(uint64_t* xzs, uint8_t* ph, uint32_t rows, ui
     }
   }
   ph[r] = (uint8_t)p;
+}
+
+// Gate lists bit-sliced over rows (apply_layers_kernel).  A CTA takes 32 rows
+// and keeps them transposed in shared memory: one word holds the x bits of a
+// qubit in those rows, one its z bits, so a gate is a few 32-bit operations, gates on different qubits run on different threads, and a phase
+// flip is the XOR of the gates' flag words in any order.  The host sorts the
+// list into levels (a gate's level is one past the last level of a gate before
+// it on one of its qubits: levels hold disjoint qubits, and every qubit sees
+// its gates in list order); one barrier orders two levels.  The list comes by
+// value (kernel parameters, up to 32 KB): no allocation, no copy, nothing that
+// a graph capture of the call would have to keep alive.  Bound by a level's
+// latency (the parameter reads, the words, a barrier: 0.3-0.5 us) and, for few
+// gates, by the transposes.  400 gates on a 2000 x 1000-qubit tableau: 7.1 us;
+// a circuit of 2300 gates on 1000 x 500 qubits 25 us, with one row per thread
+// (every gate a read and a write of global words) 1.5 ms.
+//  list: per level a header (the level's gate count), then its gates
+//  (opcode and flags | q1 << 16 | q2 << 40, 0-based qubits below 2^24).
+template <uint32_t CAP>
+struct LayerList {
+  uint64_t e[CAP];
+};
+constexpr uint32_t LAYER_CAP_S = 480, LAYER_CAP_L = 4032;  // entries of a launch: 4 KB and 32 KB of parameters
+constexpr uint32_t LAYER_SLICE = 32;                       // rows of a CTA
+
+// 32 x 32 bits, lane i holding row i: afterwards lane i holds column i.  Round
+// j swaps the off-diagonal j x j blocks with the lane j away: keep the words'
+// own blocks (mask) and take the partner's, rotated into place.
+struct WarpTranspose {
+  uint32_t keep[5], rot[5];
+  __device__ __forceinline__ explicit WarpTranspose(uint32_t lane) {
+    const uint32_t m[5] = {0x0000FFFFu, 0x00FF00FFu, 0x0F0F0F0Fu, 0x33333333u, 0x55555555u};
+#pragma unroll
+    for (uint32_t k = 0; k < 5; k++) {
+      const bool up = lane & (16u >> k);
+      keep[k] = up ? ~m[k] : m[k];
+      rot[k] = up ? 32u - (16u >> k) : 16u >> k;
+    }
+  }
+  __device__ __forceinline__ uint32_t operator()(uint32_t v) const {
+#pragma unroll
+    for (uint32_t k = 0; k < 5; k++) {
+      const uint32_t o = __shfl_xor_sync(0xFFFFFFFFu, v, 16u >> k);
+      v = (v & keep[k]) | (__funnelshift_l(o, o, rot[k]) & ~keep[k]);
+    }
+    return v;
+  }
+};
+
+// The slice [32 rows][2 W words of 32 bits] at an odd row stride; a column of
+// words (word w of the 32 rows) is transposed in place, which leaves qubit q's
+// x word at row q % 32, word q / 32, and its z word W further on.
+template <uint32_t CAP>
+__global__ void __launch_bounds__(512) apply_layers_kernel(uint64_t* xzs, uint8_t* ph, uint32_t rows, uint32_t W,
+                                                           const __grid_constant__ LayerList<CAP> list,
+                                                           uint32_t nent, int phases) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  extern __shared__ __align__(16) uint32_t sl[];
+  __shared__ uint32_t flip;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  const uint32_t r0 = blockIdx.x * LAYER_SLICE, nr = min(LAYER_SLICE, rows - r0);
+  const uint32_t words = 2 * W, ST = words + 1;  // 32-bit words of a row, their stride
+  uint32_t* base = (uint32_t*)(xzs + (uint64_t)r0 * W);
+  const WarpTranspose transpose(lane);
+  if (tid == 0) flip = 0;
+  for (uint32_t r = warp; r < LAYER_SLICE; r += nw)
+#pragma unroll 4
+    for (uint32_t w = lane; w < words; w += 32) sl[r * ST + w] = r < nr ? base[(uint64_t)r * words + w] : 0u;
+  __syncthreads();
+#pragma unroll 2
+  for (uint32_t w = warp; w < words; w += nw) sl[lane * ST + w] = transpose(sl[lane * ST + w]);
+  __syncthreads();
+  uint32_t f = 0;
+#pragma unroll 1
+  for (uint32_t k = 0; k < nent;) {
+    const uint32_t cnt = (uint32_t)list.e[k++];
+#pragma unroll 1
+    for (uint32_t g = tid; g < cnt; g += blockDim.x) {
+      const uint64_t e = list.e[k + g];
+      const uint32_t op = (uint32_t)e & 0xFFFFu, q1 = (uint32_t)(e >> 16) & 0xFFFFFFu, q2 = (uint32_t)(e >> 40);
+      uint32_t* a = sl + (q1 & 31) * ST + (q1 >> 5);
+      uint32_t x1 = a[0], z1 = a[W];
+      if ((op & 0xFFu) < QCB_OP_CNOT) {
+        f ^= g1<uint32_t>(op, x1, z1);
+      } else {
+        uint32_t* b = sl + (q2 & 31) * ST + (q2 >> 5);
+        uint32_t x2 = b[0], z2 = b[W];
+        f ^= g2<uint32_t>(op, x1, z1, x2, z2);
+        b[0] = x2;
+        b[W] = z2;
+      }
+      a[0] = x1;
+      a[W] = z1;
+    }
+    k += cnt;
+    __syncthreads();
+  }
+  f = __reduce_xor_sync(0xFFFFFFFFu, f);
+  if (lane == 0 && f) atomicXor(&flip, f);
+#pragma unroll 2
+  for (uint32_t w = warp; w < words; w += nw) sl[lane * ST + w] = transpose(sl[lane * ST + w]);
+  __syncthreads();
+  for (uint32_t r = warp; r < nr; r += nw)
+    for (uint32_t w = lane; w < words; w += 32) base[(uint64_t)r * words + w] = sl[r * ST + w];
+  if (phases && warp == 0 && lane < nr && ((flip >> lane) & 1u)) ph[r0 + lane] = (uint8_t)((ph[r0 + lane] + 2u) & 3u);
 }
 
 // ---------------------------------------------------------- dense apply!
@@ -589,6 +695,97 @@ __global__ void mul_left_batch_finish_kernel(uint8_t* r_phase, const uint8_t* l_
 static uint32_t g_gates_pdl = 1;  // symbolic gate launches as programmatic dependents (0: plain)
 void set_gates_pdl(uint32_t v) { g_gates_pdl = v; }
 
+// A gate launch: a programmatic dependent of the previous launch on the
+// stream, so that in a stream of single-gate calls each launch is scheduled
+// while the one before it runs, instead of after it drains.
+template <class... P, class... A>
+static cudaError_t launch_gates(void (*k)(P...), uint32_t grid, uint32_t block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = g_gates_pdl ? 1 : 0;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, args...);
+}
+
+// Shortest gate list that runs bit-sliced.  The row-per-thread kernel takes
+// 1.6 us + 0.55..1.1 us a gate whatever the rows; the slices cost a read, two
+// transposes and a write of the tableau whatever the gates (2n rows, n = 100 /
+// 1000 / 4000: 5.5 / 4.4 / 17.5 us), so the lines cross at 8 gates for small
+// tableaux and one more per MB of a large one (8 MB: 16 gates, 17.5 us both).
+static size_t layer_min_gates(const qcb_tableau* t) { return 8 + (((size_t)t->rows * t->W * 8) >> 20); }
+
+static size_t layer_smem(const qcb_tableau* t) { return (size_t)LAYER_SLICE * (2 * t->W + 1) * 4; }
+
+template <uint32_t CAP>
+static int launch_layers(const qcb_tableau* t, const std::vector<uint64_t>& list, uint32_t threads, int phases,
+                         cudaStream_t st) {
+  LayerList<CAP> l;
+  std::copy(list.begin(), list.end(), l.e);
+  const size_t sm = layer_smem(t);
+  if (sm > 40 * 1024)
+    QCB_CUDA(cudaFuncSetAttribute(apply_layers_kernel<CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  QCB_CUDA(launch_gates(apply_layers_kernel<CAP>, (t->rows + LAYER_SLICE - 1) / LAYER_SLICE, threads, sm, st, t->xzs,
+                        t->phases, t->rows, t->W, (const LayerList<CAP>&)l, (uint32_t)list.size(), phases));
+  QCB_LAUNCHED();
+  return QCB_OK;
+}
+
+// The list as levels of disjoint gates, launch by launch.
+static int apply_layers(const qcb_tableau* t, const std::vector<GateOp>& g, int phases, cudaStream_t st) {
+  std::vector<uint32_t> qlev(t->nqubits), lev, start, at;
+  std::vector<uint64_t> list;
+  for (size_t k0 = 0; k0 < g.size();) {
+    // as many gates as fit with their level headers
+    std::fill(qlev.begin(), qlev.end(), 0u);
+    lev.clear();
+    uint32_t depth = 0;
+    size_t k = k0;
+    for (; k < g.size(); k++) {
+      const bool two = (g[k].op & 0xFFu) >= QCB_OP_CNOT;
+      const uint32_t l = std::max(qlev[g[k].q1], two ? qlev[g[k].q2] : 0u);
+      if (k - k0 + 1 + std::max(depth, l + 1) > LAYER_CAP_L) break;
+      depth = std::max(depth, l + 1);
+      qlev[g[k].q1] = l + 1;
+      if (two) qlev[g[k].q2] = l + 1;
+      lev.push_back(l);
+    }
+    // by opcode (a warp then runs one branch of the gate table), then by level
+    const size_t n = k - k0;
+    start.assign(257, 0);
+    for (size_t i = 0; i < n; i++) start[(g[k0 + i].op & 0xFFu) + 1]++;
+    for (uint32_t i = 0; i < 256; i++) start[i + 1] += start[i];
+    at.resize(n);
+    for (size_t i = 0; i < n; i++) at[start[g[k0 + i].op & 0xFFu]++] = (uint32_t)i;
+    start.assign(depth + 1, 0);
+    for (size_t i = 0; i < n; i++) start[lev[i] + 1]++;
+    uint32_t most = 0;
+    for (uint32_t i = 0; i < depth; i++) {
+      most = std::max(most, start[i + 1]);
+      start[i + 1] += start[i];
+    }
+    list.resize(n + depth);
+    for (uint32_t i = 0; i < depth; i++) list[start[i] + i] = start[i + 1] - start[i];
+    for (size_t i = 0; i < n; i++) {
+      const GateOp& o = g[k0 + at[i]];
+      const uint32_t l = lev[at[i]];
+      list[start[l]++ + l + 1] = (uint64_t)o.op | ((uint64_t)o.q1 << 16) | ((uint64_t)o.q2 << 40);
+    }
+    // threads for the widest level, and a warp per two transposes
+    const uint32_t threads = std::min<uint32_t>(512, std::max<uint32_t>(64, std::max((most + 31) / 32 * 32, 32 * t->W)));
+    if (int s = list.size() <= LAYER_CAP_S ? launch_layers<LAYER_CAP_S>(t, list, threads, phases, st)
+                                           : launch_layers<LAYER_CAP_L>(t, list, threads, phases, st))
+      return s;
+    k0 = k;
+  }
+  return QCB_OK;
+}
+
 }  // namespace qcb
 
 using namespace qcb;
@@ -782,23 +979,14 @@ int qcb_apply_gates(qcb_tableau* t, const qcb_op* ops, size_t n_ops, int phases,
   }
   if (g.empty() || !t->rows) return QCB_OK;
   cudaStream_t st = S(stream);
+  if (g.size() >= layer_min_gates(t) && layer_smem(t) <= (size_t)device_max_smem_optin() - 1024)
+    return apply_layers(t, g, phases, st);
   for (size_t k0 = 0; k0 < g.size(); k0 += GATE_BATCH) {
     const uint32_t n = (uint32_t)std::min<size_t>(GATE_BATCH, g.size() - k0);
     GateBatch b{};
     std::copy(g.begin() + k0, g.begin() + k0 + n, b.op);
-    // a programmatic dependent of the previous launch on the stream: in a
-    // stream of single-gate calls each launch is scheduled while the one
-    // before it runs, instead of after it drains
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((t->rows + 127) / 128);
-    cfg.blockDim = dim3(128);
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = g_gates_pdl ? 1 : 0;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    QCB_CUDA(cudaLaunchKernelEx(&cfg, apply_gates_kernel, t->xzs, t->phases, t->rows, t->W, (const GateBatch)b, n, phases));
+    QCB_CUDA(launch_gates(apply_gates_kernel, (t->rows + 127) / 128, 128, 0, st, t->xzs, t->phases, t->rows, t->W,
+                          (const GateBatch)b, n, phases));
     QCB_LAUNCHED();
   }
   return QCB_OK;

@@ -86,3 +86,45 @@ def test_single_gate_calls_replayed_from_a_graph(qcb):
     del graph
     g.to_cpu()
     assert np.array_equal(g.xzs, xz) and np.array_equal(g.phases, ph)
+
+
+@pytest.mark.parametrize("n,rows,count,local", [
+    (1, 1, 8, 1), (2, 33, 9, 2), (63, 31, 7, 63), (64, 64, 200, 64), (65, 65, 470, 65), (200, 32, 481, 3),
+    (130, 257, 4100, 130), (500, 1000, 9000, 500), (3000, 40, 700, 3000), (70, 5, 5000, 2)])
+def test_gate_lists_by_levels(qcb, n, rows, count, local):
+    """Gate lists of the bit-sliced kernel: around the shortest such list, the
+    two parameter sizes and several launches, wide levels and chains on few
+    qubits (`local`: the gates touch the first that many), ragged rows and
+    words; the row-per-thread kernel takes the shorter ones."""
+    rng = np.random.default_rng(n + count)
+    t = rand_tab(rows, n, rng)
+    arr = O.to_array(random_gates(local, count, rng) if local > 1 else
+                     [O.Op(O.OP[G1[rng.integers(len(G1))]], 1) for _ in range(count)])
+    for phases in (True, False):
+        g = t.copy().to_gpu()
+        qcb.apply_(g, arr, phases=phases)
+        g.to_cpu()
+        ph, xz = oracle.apply_gates(t.phases, t.xzs, n, arr, phases)
+        assert np.array_equal(g.xzs, xz) and np.array_equal(g.phases, ph)
+
+
+def test_gate_list_replayed_from_a_graph(qcb):
+    n, rng = 300, np.random.default_rng(5)
+    t = rand_tab(n, n, rng)
+    arr = O.to_array(random_gates(n, 900, rng))
+    want = arr.copy()
+    g = t.copy().to_gpu()
+    h = g._need_dev().handle
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        check(qcb.lib().qcb_apply_gates(h, ptr(arr), len(arr), 1, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    arr[:] = 0  # the list is borrowed for the call only
+    ph, xz = t.phases.copy(), t.xzs.copy()
+    for _ in range(2):
+        graph.replay()
+        ph, xz = oracle.apply_gates(ph, xz, n, want, True)
+    torch.cuda.synchronize()
+    del graph
+    g.to_cpu()
+    assert np.array_equal(g.xzs, xz) and np.array_equal(g.phases, ph)
