@@ -353,12 +353,10 @@ int qcb_pftrajectories_fresh(qcb_frame* f, const qcb_program* prog, uint64_t see
  * hit keeps results right).  Knob "server_fill" (read by qcb_server_create):
  * 1 (default) admits onto idle SMs only, 0 whenever a slot is free.
  * canonicalize! by panels over the whole GPU: "canon_grid" 0 (automatic:
- * stabilizer views of 640..8192 rows) / 1 always / 2 never; "canon_rpt"
- * rows per pivot-search thread (0: automatic, 1, 2, 4, 8, 16);
- * "canon_apply_rows" rows per apply CTA (0 or 8..32); "canon_pdl" 1
+ * stabilizer views of 64..8192 rows) / 1 always / 2 never; "canon_pdl" 1
  * (default) / 0: the panel launches as programmatic dependent launches or
- * plain; "canon_lookahead" 1 (default) / 0: each panel's pivot steps run
- * beside the previous panel's grid-wide apply, or the two in turn.  project! on the whole GPU: "project_grid" 0 (automatic: generic
+ * plain.  "canon_rpt" (0, 1, 2, 4, 8, 16), "canon_apply_rows" (0 or 8..32) and
+ * "canon_lookahead" (1 default, 0) are accepted without effect.  project! on the whole GPU: "project_grid" 0 (automatic: generic
  * Paulis on Stabilizer kinds too tall for one cluster's shared memory) / 1
  * always where it applies / 2 never.  Test knob "project_withhold" 1: one CTA
  * of that kernel leaves before the first grid barrier, the others' bounded

@@ -26,6 +26,7 @@
 #include <memory>
 #include <vector>
 
+#include "panel.cuh"
 #include "qcb_internal.h"
 
 namespace cg = cooperative_groups;
@@ -890,484 +891,498 @@ __global__ void __launch_bounds__(CANON_THREADS) canon_batch_kernel(const CanonB
 }
 
 // ---------------------------------------------------------------- panels over the whole GPU
-// canonicalize! by 64-column panels with the per-row work spread over every
-// SM: per panel two launches, (1) canon_search_kernel, one CTA: the panel's
-// pivot steps on the panel words of all rows (the same search as
-// blocked_body, positions kept in global memory between panels), the pivot
-// rows as they are at the panel start copied aside, and the panel's phase
-// data (C, D_t, the pivots' q); (2) canon_apply_kernel, a grid over the rows:
-// every row's mask, bits and phase from that record (the same bilinear-form
-// replay as blocked_body).  The launch boundary is the barrier between the
-// two; the rows live in global memory (L2-resident) throughout.
-struct PanelRec {
-  uint32_t T;        // pivots of the panel
-  uint32_t i;        // next pivot position after the panel
-  uint32_t rx;       // pivots of the X stage (kept from the last X-stage panel)
-  uint32_t done;     // every position has a pivot: later panels do nothing
-  uint32_t stp[PANEL];
-  uint8_t bt[PANEL];
-  uint8_t qp[PANEL];
-  uint64_t A[PANEL], PWP[PANEL], Dt[PANEL];
-};
-
-struct PanelArgs {
+// canonicalize! by 64-column panels over every SM (panel.cuh): the rows in
+// tiles, per panel p two launches,
+//   L1(p): CTA 0 runs panel p's pivot steps on the rows' panel words, while
+//          the other CTAs apply panel p - 1 to the rows (a CTA per tile of
+//          word columns and range of rows; a few CTAs their q);
+//   L2(p): a CTA per tile forms panel p's reduced pivots and the tile's share
+//          of the phase data; CTAs over the rows find every row's set U and
+//          its word of panel p + 1 (one word, from the reduced pivots').
+// So the serial chain of a panel is its steps and L2; the apply runs beside
+// the next panel's steps.  The launch boundaries are the only
+// synchronisation; records alternate between two buffers by panel parity.
+// Bound by that chain: L1 12 us and L2 6.3 us alone, 18 us a panel in
+// sequence (n = 4000), of which the steps are 7.5 us and the rest launch and
+// load latencies.  Random states, n = 1000 / 2000 / 4000: 706 / 1661 / 4643 ->
+// 281 / 595 / 1381 us (the search over all rows with a block barrier a step,
+// every pivot row XORed for itself and 64 dot products a row for the phases
+// before); sparse rows (weight 4), 863 / 2114 / 6027 -> 475 / 1050 / 2507 us.
+struct CanonPanelArgs {
+  PanelTiles p;
   uint64_t* xzs;
   uint8_t* ph;
-  uint32_t rows, n, W;
-  int phases;
-  uint32_t stage, c0;   // this panel: stage 0 (X) or 1 (Z), first column
-  uint32_t* pos;        // [rows] row -> position (persistent)
-  PanelRec* rec;        // this panel's record
-  uint64_t* po;         // [PANEL][W] the pivot rows at the panel start
+  uint32_t n;
+  uint32_t* inv;        // [rows] position -> row
+  PanelRecord* rec;     // this panel's record
+  PanelRecord* prev;    // the previous panel's
   int32_t* out;         // [0] X-stage pivots, [1] next pivot position
-  // look-ahead schedule only
-  PanelRec* prev;       // the previous panel's record (its i / rx / done start this panel)
-  uint64_t* po_prev;    // the previous panel's pivot rows
-  uint64_t* nw;         // [rows] each row's word of this panel (of the next one, once written)
-  uint32_t wj_prev;     // word index of the previous panel (UINT32_MAX: none)
-  uint32_t wj_next;     // word index of the next panel (UINT32_MAX: none)
-  uint32_t steps;       // 1: this launch runs this panel's pivot steps
+  uint32_t stage, c0;   // this panel: stage 0 (X) or 1 (Z), first column
+  uint32_t wn;          // the next panel's word (WORD_NONE: none)
+  uint32_t steps;       // L1: run this panel's steps
+  uint32_t apply;       // L1: apply the previous panel
+  uint32_t nq, groups, per;  // L1: CTAs for q, row ranges per tile and their rows
 };
+constexpr uint32_t WORD_NONE = 0xFFFFFFFFu;
 
 // The word index of a panel's columns in a row (X words, then Z words).
-__host__ __device__ inline uint32_t panel_word(uint32_t stage, uint32_t c0, uint32_t len) {
-  return stage * len + (c0 >> 6);
+inline uint32_t panel_word(uint32_t stage, uint32_t c0, uint32_t len) { return stage * len + (c0 >> 6); }
+
+// The pivot steps of a panel.  Only rows at positions >= i0 (the next pivot
+// position) with a nonzero panel word can become pivots, and the first of them
+// with the column's bit does: warp 0 keeps the first STEP_WINDOW of them in
+// registers and runs the steps on these alone, without a block barrier; the
+// pivot's word and mask go through its record in shared memory.  For dense
+// rows a pivot outside the window has probability 2^-33 a column.  When the
+// window has none, the other warps, which keep the remaining rows' words,
+// catch up with the pivots so far and look for the first of theirs.  Where the
+// first STEP_WINDOW positions hold many zero words (sparse rows), the rows
+// with a nonzero word are listed first, in order of position; all others are
+// inert.  A row swap only changes positions: every row's position is kept by
+// value, and the permutation is brought up to date afterwards
+// (canon_permute).  Bound by warp 0's chain: three tests, a warp minimum, a
+// store and a load, an XOR: 226 cycles a step whatever the rows (0.42 / 0.22
+// us a step at 4000 / 1000 rows with all rows in all warps and a block barrier
+// a step).
+constexpr uint32_t STEP_SLOTS = 3, STEP_WINDOW = 32 * STEP_SLOTS, STEP_DENSE = 80;
+constexpr uint32_t STEP_REST = 31 * 32;  // threads of the remaining rows
+
+// A slot of the window: (word, mask) ^= p where the slot's word `test` has the bit.
+__device__ __forceinline__ void xor_if(uint32_t (&v)[4], uint32_t test, uint32_t bit, const uint32_t (&p)[4]) {
+  asm("{.reg .pred y; .reg .u32 x; and.b32 x, %4, %5; setp.ne.u32 y, x, 0;"
+      "@y xor.b32 %0, %0, %6; @y xor.b32 %1, %1, %7; @y xor.b32 %2, %2, %8; @y xor.b32 %3, %3, %9;}"
+      : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3])
+      : "r"(test), "r"(bit), "r"(p[0]), "r"(p[1]), "r"(p[2]), "r"(p[3]));
 }
 
-// (1) The panel's pivot steps on the panel words of the candidate rows
-// (positions >= the next pivot position), word(r) = wsrc[r * wstride]; the
-// positions of those rows are updated in `pos`, and the record g gets the
-// pivot rows, their columns, masks and words (stp, bt, A, PWP) and T, i, rx,
-// done, starting from prev's i / rx / done (prev may be g itself).
 template <uint32_t RPT>
-__device__ __forceinline__ void panel_steps(const PanelArgs& a, const PanelRec& prev, PanelRec& g,
-                                            const uint64_t* wsrc, uint32_t wstride, uint32_t* cand) {
-  __shared__ uint32_t stp[PANEL];
-  __shared__ uint8_t bt[PANEL];
-  __shared__ uint64_t A[PANEL], PWP[PANEL];
-  __shared__ uint64_t red2[2][32][3];
-  __shared__ uint32_t shT, shI, ncand;
-  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-  const uint32_t R = a.rows, n = a.n;
-  const uint32_t c0 = a.c0, ncp = min(PANEL, n - c0);
-  uint32_t i = prev.i;
-  const uint32_t rx0 = prev.rx;
-  if (prev.done) {  // every position has its pivot: this panel applies nothing
-    __syncthreads();  // every thread has read prev before g (maybe prev) is written
-    if (tid == 0) { g.T = 0; g.i = i; g.rx = rx0; g.done = 1; }
-    __syncthreads();
+__device__ __forceinline__ void canon_steps(const CanonPanelArgs& a, uint8_t* dsm) {
+  constexpr uint32_t NONE = 0xFFFFFFFFu, KW = STEP_SLOTS, UNITS = KW + 31 * RPT;
+  __shared__ uint4 recA[PSTEPS];  // pivot t: (panel word, mask)
+  __shared__ uint4 recB[PSTEPS];  // (position before the step, bit, row)
+  __shared__ uint64_t rw[32], ra[32];
+  __shared__ uint32_t rpos[32], off[UNITS], shT, dense, rb, rT;
+  PanelRecord& g = *a.rec;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, R = a.p.rows;
+  const uint32_t i0 = a.prev->i, rx0 = a.prev->rx, ncp = min(PSTEPS, a.n - a.c0);
+  if (tid < PSTEPS) { g.G[tid] = 0; g.q0[tid] = 0; }
+  if (a.prev->done) {  // every position has its pivot
+    if (tid == 0) { g.T = 0; g.i = i0; g.i0 = i0; g.rx = rx0; g.done = 1; }
     return;
   }
-  // Only rows at positions >= i can become pivots; the search runs on them
-  // alone (the others' panel words do not matter to it), so it shrinks as
-  // the elimination proceeds.
-  if (tid == 0) ncand = 0;
-  __syncthreads();
-  for (uint32_t r = tid; r < R; r += blockDim.x)
-    if (a.pos[r] >= i) cand[atomicAdd(&ncand, 1u)] = r;
-  __syncthreads();
-  const uint32_t Rc = ncand;
-  const uint32_t NB = min(nwarps, max(1u, (Rc + 32 * RPT - 1) / (32 * RPT))), nbt = NB * 32;
-  uint32_t rrow[RPT], rpos[RPT];
-  uint64_t rpw[RPT], rcb[RPT];
-  uint32_t T = 0;
-  if (warp < NB) {
+  // warp 0: the window's slots, position i0 + 32 k + lane; the others: the
+  // rest, position i0 + STEP_WINDOW + STEP_REST k + tid - 32
+  uint32_t wd[KW][4], pos[KW], row[KW];  // wd: panel word, mask of pivots absorbed
+  uint64_t w[RPT], A[RPT];
+  uint32_t wp[RPT];
+  if (warp == 0) {
+    uint32_t cnt = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < KW; k++) {
+      const uint32_t p = i0 + 32 * k + lane;
+      row[k] = p < R ? a.inv[p] : NONE;
+      pos[k] = p;
+      const uint64_t v = p < R ? a.p.word[row[k]] : 0ull;
+      wd[k][0] = (uint32_t)v;
+      wd[k][1] = (uint32_t)(v >> 32);
+      wd[k][2] = wd[k][3] = 0;
+      cnt += __popc(__ballot_sync(0xFFFFFFFFu, v != 0));
+    }
+    if (lane == 0) dense = cnt >= STEP_DENSE;
+  } else {
 #pragma unroll
     for (uint32_t k = 0; k < RPT; k++) {
-      const uint32_t j = tid + k * nbt;
-      rrow[k] = j < Rc ? cand[j] : 0xFFFFFFFFu;
-      rpos[k] = j < Rc ? a.pos[rrow[k]] : 0xFFFFFFFFu;
-      rpw[k] = j < Rc ? wsrc[(size_t)rrow[k] * wstride] : 0ull;
-      rcb[k] = 0;
+      const uint32_t p = i0 + STEP_WINDOW + STEP_REST * k + tid - 32;
+      wp[k] = p;
+      w[k] = p < R ? a.p.word[a.inv[p]] : 0ull;
+      A[k] = 0;
     }
-    // the steps (as blocked_body): one named barrier among the search warps
-    // per column.  Kept short, as the search is instruction-bound on its SM:
-    // rows past the candidates hold a zero word (never a candidate, never
-    // updated); the previous step's pivot is applied lazily at the start of
-    // a step (pwprev = 0 after a column without one), which also zeroes the
-    // pivot row's own word, so it never competes again; positions i and kpos
-    // swap by value; the warp's best row travels with its position and the
-    // winning lane posts it.
-    uint32_t bprev = 0;
-    uint64_t pwprev = 0, aprev = 0;
-    for (uint32_t b = 0; b < ncp && i < R; b++) {
-      uint32_t bpos = 0xFFFFFFFFu, brow = 0;
-      uint64_t bpw = 0, bcb = 0;
-#pragma unroll
-      for (uint32_t k = 0; k < RPT; k++) {
-        if ((rpw[k] >> bprev) & 1ull) {
-          rpw[k] ^= pwprev;
-          rcb[k] ^= aprev;
-        }
-        if (((rpw[k] >> b) & 1ull) && rpos[k] < bpos) {
-          bpos = rpos[k];
-          brow = rrow[k];
-          bpw = rpw[k];
-          bcb = rcb[k];
-        }
-      }
-      {
-        const uint32_t m = __reduce_min_sync(0xFFFFFFFFu, bpos);
-        const uint32_t src = __ffs(__ballot_sync(0xFFFFFFFFu, bpos == m)) - 1;
-        if (lane == src) {
-          red2[b & 1][warp][0] = ((uint64_t)m << 32) | brow;
-          red2[b & 1][warp][1] = bpw;
-          red2[b & 1][warp][2] = bcb;
-        }
-      }
-      asm volatile("bar.sync 1, %0;" ::"r"(nbt) : "memory");
-      const uint64_t e = lane < NB ? red2[b & 1][lane][0] : ~0ull;
-      const uint32_t kpos = __reduce_min_sync(0xFFFFFFFFu, (uint32_t)(e >> 32));
-      if (kpos == 0xFFFFFFFFu) {
-        pwprev = 0;
-        aprev = 0;
-        continue;
-      }
-      const uint32_t kw = __ffs(__ballot_sync(0xFFFFFFFFu, (uint32_t)(e >> 32) == kpos)) - 1;
-      pwprev = red2[b & 1][kw][1];
-      aprev = red2[b & 1][kw][2] | (1ull << T);
-#pragma unroll
-      for (uint32_t k = 0; k < RPT; k++) rpos[k] = rpos[k] == kpos ? i : (rpos[k] == i ? kpos : rpos[k]);
-      if (tid == 0) {
-        stp[T] = (uint32_t)red2[b & 1][kw][0];
-        bt[T] = (uint8_t)b;
-        A[T] = aprev;
-        PWP[T] = pwprev;
-      }
-      bprev = b;
-      T++;
-      i++;
-    }
-#pragma unroll
-    for (uint32_t k = 0; k < RPT; k++)
-      if (rrow[k] != 0xFFFFFFFFu) a.pos[rrow[k]] = rpos[k];
-    if (tid == 0) { shT = T; shI = i; }
   }
   __syncthreads();
-  T = shT;
-  i = shI;
-  for (uint32_t t = tid; t < T; t += blockDim.x) {
-    g.stp[t] = stp[t];
-    g.bt[t] = bt[t];
-    g.A[t] = A[t];
-    g.PWP[t] = PWP[t];
+  uint32_t nrest = R - i0 > STEP_WINDOW ? R - i0 - STEP_WINDOW : 0u;
+  uint64_t* lw = (uint64_t*)dsm;               // sparse: the listed rows' words,
+  uint32_t* lp = (uint32_t*)(lw + R);          // positions
+  uint32_t* lr = lp + R;                       // and rows
+  const bool listed = !dense && nrest;
+  if (listed) {
+    // offsets of the units (32 positions each, in order) by their counts
+    if (warp == 0) {
+#pragma unroll
+      for (uint32_t k = 0; k < KW; k++) {
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, (wd[k][0] | wd[k][1]) != 0);
+        if (lane == 0) off[k] = __popc(m);
+      }
+    } else {
+#pragma unroll
+      for (uint32_t k = 0; k < RPT; k++) {
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, w[k] != 0);
+        if (lane == 0) off[KW + 31 * k + warp - 1] = __popc(m);
+      }
+    }
+    __syncthreads();
+    if (warp == 0) {
+      uint32_t sum = 0;
+      for (uint32_t u0 = 0; u0 < UNITS; u0 += 32) {
+        const uint32_t c = u0 + lane < UNITS ? off[u0 + lane] : 0u;
+        uint32_t inc = c;
+#pragma unroll
+        for (uint32_t d = 1; d < 32; d <<= 1) {
+          const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, inc, d);
+          if (lane >= d) inc += v;
+        }
+        if (u0 + lane < UNITS) off[u0 + lane] = sum + inc - c;
+        sum += __shfl_sync(0xFFFFFFFFu, inc, 31);
+      }
+      if (lane == 0) rT = sum;
+    }
+    __syncthreads();
+    const uint32_t below = (1u << lane) - 1u, total = rT;
+    if (warp == 0) {
+#pragma unroll
+      for (uint32_t k = 0; k < KW; k++) {
+        const bool in = (wd[k][0] | wd[k][1]) != 0;
+        const uint32_t o = off[k] + __popc(__ballot_sync(0xFFFFFFFFu, in) & below);
+        if (in) {
+          lw[o] = (uint64_t)wd[k][0] | ((uint64_t)wd[k][1] << 32);
+          lp[o] = pos[k];
+          lr[o] = row[k];
+        }
+      }
+    } else {
+#pragma unroll
+      for (uint32_t k = 0; k < RPT; k++) {
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, w[k] != 0);
+        if (w[k]) {
+          const uint32_t o = off[KW + 31 * k + warp - 1] + __popc(m & below);
+          lw[o] = w[k];
+          lp[o] = wp[k];
+          lr[o] = a.inv[wp[k]];
+        }
+      }
+    }
+    __syncthreads();
+    nrest = total > STEP_WINDOW ? total - STEP_WINDOW : 0u;
+    if (warp == 0) {
+#pragma unroll
+      for (uint32_t k = 0; k < KW; k++) {
+        const uint32_t o = 32 * k + lane;
+        const uint64_t v = o < total ? lw[o] : 0ull;
+        wd[k][0] = (uint32_t)v;
+        wd[k][1] = (uint32_t)(v >> 32);
+        pos[k] = o < total ? lp[o] : NONE;
+        row[k] = o < total ? lr[o] : NONE;
+      }
+    }
+  }
+  // the warps that hold remaining rows, and their rows' stride
+  const uint32_t nbw = min(31u, (nrest + 31) / 32), stride = listed ? 32 * nbw : STEP_REST, nbar = 32 * (nbw + 1);
+  if (warp == 0) {
+    const uint32_t tmax = min(PSTEPS, R - i0);
+    uint32_t T = 0, i = i0, t0 = 1, t1 = 0;  // t1:t0: bit T
+    uint32_t ad = (uint32_t)__cvta_generic_to_shared(recA);
+    const uint32_t bd = (uint32_t)__cvta_generic_to_shared(recB) - ad;
+#pragma unroll
+    for (uint32_t h = 0; h < 2; h++) {
+      const uint32_t ce = ncp > 32 * h ? min(32u, ncp - 32 * h) : 0u;
+      for (uint32_t c = 0; c < ce && T < tmax; c++) {
+        bool miss = false;
+        uint32_t cm = 1u << c;
+        // columns whose pivot is in the window
+#pragma unroll 1
+        for (; c < ce && T < tmax; c++, cm <<= 1) {
+          const uint32_t c0 = (wd[0][h] & cm) ? pos[0] : NONE, c1 = (wd[1][h] & cm) ? pos[1] : NONE,
+                         c2 = (wd[2][h] & cm) ? pos[2] : NONE;
+          const uint32_t best = min(min(c0, c1), c2), m = __reduce_min_sync(0xFFFFFFFFu, best);
+          const bool y1 = c1 == best, y2 = c2 == best;
+          uint32_t s[4];
+#pragma unroll
+          for (uint32_t q = 0; q < 4; q++) s[q] = y2 ? wd[2][q] : (y1 ? wd[1][q] : wd[0][q]);
+          const uint32_t sr = y2 ? row[2] : (y1 ? row[1] : row[0]);
+          if (m == NONE) { miss = true; break; }
+          // stored by the one lane with the least position
+          asm volatile("{.reg .pred p; setp.eq.u32 p, %0, %1; @p st.shared.v4.u32 [%2], {%3, %4, %5, %6};"
+                       "@p st.shared.v4.u32 [%7], {%1, %8, %9, %9};}" ::"r"(best), "r"(m), "r"(ad), "r"(s[0]), "r"(s[1]),
+                       "r"(s[2] | t0), "r"(s[3] | t1), "r"(ad + bd), "r"(32 * h + c), "r"(sr)
+                       : "memory");
+          __syncwarp();
+          uint32_t p[4];
+          asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(p[0]), "=r"(p[1]), "=r"(p[2]), "=r"(p[3]) : "r"(ad) : "memory");
+          ad += 16;
+#pragma unroll
+          for (uint32_t k = 0; k < KW; k++) {
+            const uint32_t q = pos[k], u = q == i ? m : q;  // rowswap!
+            pos[k] = q == m ? i : u;
+            xor_if(wd[k], wd[k][h], cm, p);  // the pivot's own word becomes zero: it never competes again
+          }
+          T++;
+          i++;
+          t1 = (t1 << 1) | (t0 >> 31);
+          t0 <<= 1;
+        }
+        if (!miss) break;
+        if (!nrest) continue;
+        if (lane == 0) { rb = 32 * h + c; rT = T; }
+        __syncwarp();
+        asm volatile("bar.sync 1, %0;" ::"r"(nbar) : "memory");
+        asm volatile("bar.sync 2, %0;" ::"r"(nbar) : "memory");
+        const uint32_t v = lane >= 1 && lane <= nbw ? rpos[lane] : NONE, m = __reduce_min_sync(0xFFFFFFFFu, v);
+        if (m == NONE) continue;  // no pivot in this column
+        if (v == m) {             // no row of the window has the bit
+          recA[T] = make_uint4((uint32_t)rw[lane], (uint32_t)(rw[lane] >> 32), (uint32_t)ra[lane] | t0,
+                               (uint32_t)(ra[lane] >> 32) | t1);
+          recB[T].x = m;
+          recB[T].y = 32 * h + c;
+        }
+        __syncwarp();
+#pragma unroll
+        for (uint32_t k = 0; k < KW; k++) pos[k] = pos[k] == i ? m : pos[k];
+        ad += 16;
+        T++;
+        i++;
+        t1 = (t1 << 1) | (t0 >> 31);
+        t0 <<= 1;
+      }
+    }
+    if (lane == 0) { shT = T; rb = NONE; }
+    __syncwarp();
+    if (nrest) asm volatile("bar.sync 1, %0;" ::"r"(nbar) : "memory");
+  } else if (warp <= nbw) {
+    const uint32_t o0 = STEP_WINDOW + tid - 32;  // first index in the list
+    if (listed) {
+#pragma unroll
+      for (uint32_t k = 0; k < RPT; k++) {
+        const bool in = o0 + k * stride < STEP_WINDOW + nrest;
+        w[k] = in ? lw[o0 + k * stride] : 0ull;
+        wp[k] = in ? lp[o0 + k * stride] : NONE;
+      }
+    }
+    uint32_t t = 0;
+    while (true) {
+      asm volatile("bar.sync 1, %0;" ::"r"(nbar) : "memory");
+      const uint32_t b = rb, T = rT;
+      if (b == NONE) break;
+      for (; t < T; t++) {
+        const uint4 e = recA[t];
+        const uint2 f = *(const uint2*)&recB[t];
+        const uint64_t pw = (uint64_t)e.x | ((uint64_t)e.y << 32), pA = (uint64_t)e.z | ((uint64_t)e.w << 32);
+        const uint32_t i = i0 + t;
+#pragma unroll
+        for (uint32_t k = 0; k < RPT; k++) {
+          if (k && k * stride >= nrest) break;
+          const uint64_t y = bitmask64(w[k], f.y);
+          w[k] ^= pw & y;
+          A[k] ^= pA & y;
+          wp[k] = wp[k] == f.x ? i : (wp[k] == i ? f.x : wp[k]);
+        }
+      }
+      uint32_t bp = NONE, bk = 0;
+      uint64_t bw = 0, bA = 0;
+#pragma unroll
+      for (uint32_t k = 0; k < RPT; k++) {
+        if (k && k * stride >= nrest) break;
+        if (((w[k] >> b) & 1ull) && wp[k] < bp) {
+          bp = wp[k];
+          bw = w[k];
+          bA = A[k];
+          bk = k;
+        }
+      }
+      const uint32_t m = __reduce_min_sync(0xFFFFFFFFu, bp);
+      if (lane == 0) rpos[warp] = m;
+      if (bp == m && m != NONE) { rw[warp] = bw; ra[warp] = bA; }
+      asm volatile("bar.sync 2, %0;" ::"r"(nbar) : "memory");
+      const uint32_t kp = __reduce_min_sync(0xFFFFFFFFu, lane >= 1 && lane <= nbw ? rpos[lane] : NONE);
+      if (kp != NONE && bp == kp)  // this thread's row is the pivot
+        recB[T].z = listed ? lr[o0 + bk * stride] : a.inv[i0 + o0 + bk * stride];
+    }
+  }
+  __syncthreads();
+  const uint32_t T = shT, i = i0 + T;
+  if (tid < T) {
+    const uint4 e = recA[tid], h = recB[tid];
+    g.stp[tid] = h.z;
+    g.bt[tid] = h.y;
+    g.m[tid] = h.x;
+    g.A[tid] = (uint64_t)e.z | ((uint64_t)e.w << 32);
+    g.PW[tid] = (uint64_t)e.x | ((uint64_t)e.y << 32);
   }
   if (tid == 0) {
     g.T = T;
+    g.i0 = i0;
     g.i = i;
     g.rx = a.stage == 0 ? i : rx0;
     g.done = i >= R ? 1u : 0u;
     a.out[0] = (int32_t)g.rx;
     a.out[1] = (int32_t)i;
   }
-  __syncthreads();  // the record is complete for the whole CTA
 }
 
-// (2) The pivot rows of the record g as they are at the panel start: copied
-// to po, their q = phase + |x & z|, and the panel's phase data (C, D_t and
-// the pivots' q, into g.Dt and g.qp).  wj: the panel's word index.
-__device__ __forceinline__ void panel_post(const PanelArgs& a, PanelRec& g, uint64_t* po, uint32_t wj,
-                                           uint64_t* XT) {
-  __shared__ uint32_t stp[PANEL];
-  __shared__ uint8_t bt[PANEL], qo[PANEL];
-  __shared__ uint64_t A[PANEL], PWP[PANEL], C[PANEL], Dt[PANEL], Us[PANEL];
-  __shared__ uint8_t bases[PANEL];
-  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-  const uint32_t W = a.W, len = W / 2;
-  const uint32_t T = g.T;
-  // XT[w * XS + t] / ZT[w * XS + t]: X / Z word w of pivot t; the odd stride
-  // keeps the transposing stores (lane = word) free of bank conflicts
-  constexpr uint32_t XS = PANEL + 1;
-  uint64_t* ZT = XT + (size_t)len * XS;
-  for (uint32_t t = tid; t < T; t += blockDim.x) {
-    stp[t] = g.stp[t];
-    bt[t] = g.bt[t];
-    A[t] = g.A[t];
-    PWP[t] = g.PWP[t];
+// The row swaps of a panel's record on the permutation inv: at step t the row
+// at position i0 + t goes to position m_t, whose row (the pivot) comes there.
+// One warp; positions past the panel's first PSTEPS are only written.
+__device__ __forceinline__ void canon_permute(const PanelRecord& g, uint32_t* inv, uint32_t rows) {
+  __shared__ uint32_t occ[PSTEPS], sm[PSTEPS], sp[PSTEPS];
+  const uint32_t lane = threadIdx.x, T = g.T, i0 = g.i0;
+  if (lane >= 32) return;
+  for (uint32_t k = lane; k < PSTEPS; k += 32) {
+    occ[k] = i0 + k < rows ? inv[i0 + k] : 0u;
+    sm[k] = g.m[k];
+    sp[k] = g.stp[k];
   }
-  __syncthreads();
-  // the pivot rows at the panel start, their q = phase + |x & z|, XT, ZT
-  for (uint32_t t = warp; t < T; t += nwarps) {
-    const uint32_t r = stp[t];
-    uint32_t s = 0;
-    for (uint32_t w = lane; w < len; w += 32) {
-      const uint64_t vx = a.xzs[(size_t)r * W + w], vz = a.xzs[(size_t)r * W + len + w];
-      po[(size_t)t * W + w] = vx;
-      po[(size_t)t * W + len + w] = vz;
-      XT[(size_t)w * XS + t] = vx;
-      ZT[(size_t)w * XS + t] = vz;
-      s += __popcll(vx & vz);
-    }
-    s = __reduce_add_sync(0xFFFFFFFFu, s);
-    if (lane == 0) qo[t] = (uint8_t)((a.ph[r] + s) & 3u);
-  }
-  __syncthreads();
-  if (a.phases && T) {
-    // C[a] bit b = z_a . x_b over the pivot rows (both transposed in shared
-    // memory); the parity of a sum of popcounts is the parity of the XOR of
-    // the words, so the words are XOR-accumulated and counted once
-    for (uint32_t t = warp; t < T; t += nwarps) {
-      uint64_t p0 = 0, p1 = 0;
-      for (uint32_t w = 0; w < len; w++) {
-        const uint64_t zw = ZT[(size_t)w * XS + t];
-        p0 ^= zw & XT[(size_t)w * XS + lane];
-        p1 ^= zw & XT[(size_t)w * XS + lane + 32];
-      }
-      const uint32_t lo = __ballot_sync(0xFFFFFFFFu, (__popcll(p0) & 1) && lane < T);
-      const uint32_t hi = __ballot_sync(0xFFFFFFFFu, (__popcll(p1) & 1) && lane + 32 < T);
-      if (lane == 0) C[t] = (uint64_t)lo | ((uint64_t)hi << 32);
-    }
-    __syncthreads();
-    if (tid < T) {
-      uint64_t d = 0;
-      for (uint32_t x = 0; x < T; x++)
-        if ((A[tid] >> x) & 1ull) d ^= C[x];
-      Dt[tid] = d;
-    }
-    __syncthreads();
-    if (tid < T) {
-      const uint32_t t = tid;
-      uint64_t u = 0;
-      for (uint32_t x = 0; x < T; x++) u |= ((C[x] >> t) & 1ull) << x;
-      uint64_t pw = po[(size_t)t * W + wj], cm = 0, ut = 0;
-      uint32_t cross = 0;
-      for (uint32_t t2 = 0; t2 < t; t2++) {
-        if ((pw >> bt[t2]) & 1ull) {
-          cross += (uint32_t)((__popcll(Dt[t2] & cm) + __popcll(u & A[t2])) & 1);
-          ut |= 1ull << t2;
-          cm ^= A[t2];
-          pw ^= PWP[t2];
-        }
-      }
-      Us[t] = ut;
-      bases[t] = (uint8_t)((qo[t] + 2u * cross) & 3u);
-    }
-    __syncthreads();
-    if (tid == 0) {
-      uint64_t Q1 = 0, Q2 = 0;
-      for (uint32_t t = 0; t < T; t++) {
-        const uint32_t q = (bases[t] + (uint32_t)__popcll(Us[t] & Q1) + 2u * (uint32_t)__popcll(Us[t] & Q2)) & 3u;
-        g.qp[t] = (uint8_t)q;
-        Q1 |= (uint64_t)(q & 1u) << t;
-        Q2 |= (uint64_t)(q >> 1) << t;
-      }
-    }
-  }
-  for (uint32_t t = tid; t < T; t += blockDim.x) g.Dt[t] = a.phases ? Dt[t] : 0ull;
-}
-
-// (3) Rows of block blk of nblk: apply the record g (pivot rows po at the
-// panel start, word index wj) to every row, as blocked_body's step 3 with
-// rows and phases in global memory.
-__device__ __forceinline__ void panel_apply(const PanelArgs& a, const PanelRec& g, const uint64_t* po,
-                                            uint32_t wj, uint32_t blk, uint32_t nblk, uint64_t* sm) {
-  const uint32_t T = g.T;
-  if (T == 0) return;
-  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5, bd = blockDim.x;
-  const uint32_t R = a.rows, W = a.W, len = W / 2;
-  const uint32_t per = (R + nblk - 1) / nblk, r0 = blk * per;
-  const uint32_t nloc = r0 < R ? min(per, R - r0) : 0u;
-  if (!nloc) return;
-  uint64_t* PO = sm;                      // [T][W]
-  uint64_t* cml = PO + (size_t)PANEL * W; // per local row: mask
-  uint8_t* ql = (uint8_t*)(cml + per);    // per local row: q
-  __shared__ uint32_t stp[PANEL];
-  __shared__ uint8_t bt[PANEL], qp[PANEL];
-  __shared__ uint64_t A[PANEL], PWP[PANEL], Dt[PANEL];
-  for (uint32_t t = tid; t < T; t += bd) {
-    stp[t] = g.stp[t]; bt[t] = g.bt[t]; qp[t] = g.qp[t];
-    A[t] = g.A[t]; PWP[t] = g.PWP[t]; Dt[t] = g.Dt[t];
-  }
-  for (size_t w = tid; w < (size_t)T * W; w += bd) PO[w] = po[w];
-  __syncthreads();
-  // (a) per row (warp per row): u[x] = z_x . x_row and q = phase + |x & z|;
-  // the lane's X words (up to four at a time) stay in registers, and for
-  // each pivot x their products with z_x are XOR-accumulated and counted
-  // once (parity of the XOR = parity of the popcounts)
-  if (a.phases) {
-    for (uint32_t lr = warp; lr < nloc; lr += nwarps) {
-      const uint64_t* row = a.xzs + (size_t)(r0 + lr) * W;
-      uint32_t lo = 0, hi = 0, s = 0;
-      for (uint32_t wb = 0; wb < len; wb += 128) {
-        const uint32_t kn = min(4u, (len - wb + 31) / 32);  // warp-uniform
-        if (kn == 1) row_parities<1>(PO, W, len, T, wb, lane, row, lo, hi, s);
-        else if (kn == 2) row_parities<2>(PO, W, len, T, wb, lane, row, lo, hi, s);
-        else if (kn == 3) row_parities<3>(PO, W, len, T, wb, lane, row, lo, hi, s);
-        else row_parities<4>(PO, W, len, T, wb, lane, row, lo, hi, s);
-      }
-      s = __reduce_add_sync(0xFFFFFFFFu, s);
-      lo = __reduce_xor_sync(0xFFFFFFFFu, lo);
-      hi = __reduce_xor_sync(0xFFFFFFFFu, hi);
-      if (lane == 0) {
-        cml[lr] = (uint64_t)lo | ((uint64_t)hi << 32);
-        ql[lr] = (uint8_t)((a.ph[r0 + lr] + s) & 3u);
-      }
-    }
-    __syncthreads();
-  }
-  // (b) the steps replayed, one thread per row
-  for (uint32_t lr = tid; lr < nloc; lr += bd) {
-    const uint32_t r = r0 + lr;
-    uint64_t pw = a.xzs[(size_t)r * W + wj], cm = 0;
-    const uint64_t u = a.phases ? cml[lr] : 0;
-    uint32_t q = a.phases ? ql[lr] : 0;
+  __syncwarp();
+  if (lane == 0)
     for (uint32_t t = 0; t < T; t++) {
-      if (r != stp[t] && ((pw >> bt[t]) & 1ull)) {
-        if (a.phases) q += qp[t] + 2u * (uint32_t)((__popcll(Dt[t] & cm) + __popcll(u & A[t])) & 1);
-        cm ^= A[t];
-        pw ^= PWP[t];
-      }
+      const uint32_t d = occ[t], m = sm[t];
+      occ[t] = sp[t];
+      if (m == i0 + t) continue;
+      if (m < i0 + PSTEPS) occ[m - i0] = d;
+      else inv[m] = d;
     }
-    cml[lr] = cm;
-    ql[lr] = (uint8_t)(q & 3u);
+  __syncwarp();
+  for (uint32_t k = lane; k < PSTEPS; k += 32)
+    if (i0 + k < rows) inv[i0 + k] = occ[k];
+}
+
+// L1.
+template <uint32_t RPT>
+__global__ void __launch_bounds__(CANON_THREADS) canon_steps_apply_kernel(const CanonPanelArgs a) {
+  extern __shared__ __align__(16) uint8_t dsm[];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+  const uint32_t blk = blockIdx.x;
+  if (blk == 0) {
+    if (a.steps) canon_steps<RPT>(a, dsm);
+    return;
+  }
+  const PanelRecord& g = *a.prev;
+  if (!a.apply || g.T == 0) return;
+  const PanelTiles& p = a.p;
+  if (blk <= a.nq) {  // q of every row
+    PhaseSmem& s = *(PhaseSmem*)dsm;
+    phase_data(p, g, s);
+    for (uint32_t r = (blk - 1) * blockDim.x + threadIdx.x; r < p.rows; r += a.nq * blockDim.x) {
+      const uint64_t U = p.U[r];
+      if (U) p.q[r] = (uint8_t)((p.q[r] + phase_of(s, U)) & 3u);
+    }
+    return;
+  }
+  const uint32_t u = blk - 1 - a.nq, tile = u / a.groups, grp = u - tile * a.groups;
+  ApplySmem& s = *(ApplySmem*)dsm;
+  apply_tables(p, tile, s);
+  const uint32_t r1 = min(p.rows, (grp + 1) * a.per);
+  for (uint32_t r = grp * a.per + threadIdx.x; r < r1; r += blockDim.x) {
+    const uint64_t U = p.U[r];
+    if (!U) continue;
+    ulonglong2* d = p.t + ((size_t)tile * p.rows + r) * 2;
+    const ulonglong2 x = d[0], z = d[1];
+    ulonglong2 mx, mz;
+    apply_lookup(s, U, mx, mz);
+    d[0] = xor128(x, mx);
+    d[1] = xor128(z, mz);
+    if (p.phases && parity64((mz.x & x.x) ^ (mz.y & x.y))) p.par[(size_t)tile * p.rows + r] ^= 1u;
+  }
+}
+
+// L2: blocks 0 .. ntile - 1 a tile each, block ntile the permutation, the
+// others MID_THREADS rows each.
+__global__ void __launch_bounds__(MID_THREADS) canon_mid_kernel(const CanonPanelArgs a) {
+  __shared__ union {
+    TileSmem t;
+    struct {
+      uint64_t start[PSTEPS];
+      ulonglong2 P[PSTEPS];   // (panel word, next word) of the reduced pivots
+      uint2 sb[PSTEPS];       // (pivot row, 31 - bit within its half word)
+    } r;
+  } s;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+  PanelRecord& g = *a.rec;
+  const PanelTiles& p = a.p;
+  const uint32_t tid = threadIdx.x, blk = blockIdx.x;
+  if (blk < p.ntile) {
+    tile_reduce(
+        p, g, blk, s.t, [&](uint32_t r) { return p.t + ((size_t)blk * p.rows + r) * 2; },
+        [&](uint32_t r) { return 2u * p.par[(size_t)blk * p.rows + r] + (blk == 0 ? p.q[r] : 0u); });
+    return;
+  }
+  if (blk == p.ntile) {
+    canon_permute(g, a.inv, p.rows);
+    return;
+  }
+  // the record's fields beyond its T steps are stale but readable (row 0 at
+  // the start): nothing here waits for T before loading
+  const uint32_t T = g.T, r = (blk - p.ntile - 1) * MID_THREADS + tid;
+  const bool next = a.wn != WORD_NONE, in = r < p.rows;
+  const uint32_t t4 = tid >> 2, x0 = (tid & 3) * 16;
+  uint64_t A = g.A[t4] >> x0, pw = in ? p.word[r] : 0ull, v = 0, st = 0;
+  uint32_t bt = 64, sp = 0;
+  if (tid < PSTEPS) {
+    bt = g.bt[tid];
+    sp = g.stp[tid];
+    s.r.P[tid].x = g.PW[tid];
+    s.r.sb[tid] = make_uint2(sp, 31u - (bt & 31u));
+    if (next) st = tile_word(p, sp, a.wn);
+    s.r.start[tid] = st;
+  }
+  if (in && next) v = tile_word(p, r, a.wn);
+  if (T == 0 && g.done) return;  // nothing to apply, and no later panel runs
+  const uint32_t T0 = __syncthreads_count(tid < T && bt < 32);  // steps in the word's low half
+  {  // the reduced pivots' next words: a thread per pivot and 16 start rows
+    uint64_t n = 0;
+#pragma unroll
+    for (uint32_t x = 0; x < 16; x++) n ^= s.r.start[x0 + x] & bitmask64(A, x);
+    n ^= __shfl_xor_sync(0xFFFFFFFFu, n, 1);
+    n ^= __shfl_xor_sync(0xFFFFFFFFu, n, 2);
+    if ((tid & 3) == 0) s.r.P[t4].y = n;
   }
   __syncthreads();
-  // (c) the rows: start bits XOR the pivot rows of the mask
-  for (uint32_t lr = warp; lr < nloc; lr += nwarps) {
-    const uint64_t cm = cml[lr];
-    if (!cm) continue;
-    uint64_t* row = a.xzs + (size_t)(r0 + lr) * W;
-    uint32_t s = 0;
-    for (uint32_t w = lane; w < len; w += 32) {
-      uint64_t vx = row[w], vz = row[len + w];
-      uint64_t m = cm;
-      while (m) {
-        const uint32_t x = __ffsll(m) - 1;
-        m &= m - 1;
-        vx ^= PO[(size_t)x * W + w];
-        vz ^= PO[(size_t)x * W + len + w];
-      }
-      row[w] = vx;
-      row[len + w] = vz;
-      s += __popcll(vx & vz);
-    }
-    if (a.phases) {
-      s = __reduce_add_sync(0xFFFFFFFFu, s);
-      if (lane == 0) a.ph[r0 + lr] = (uint8_t)((ql[lr] - s) & 3u);
-    }
-  }
+  uint32_t p0 = (uint32_t)pw, p1 = (uint32_t)(pw >> 32), u0 = 0, u1 = 0;
+  auto replay = [&](uint32_t t, uint32_t& half) {
+    const ulonglong2 P = s.r.P[t];
+    const uint2 sb = s.r.sb[t];
+    const uint32_t m = r == sb.x ? 0u : (uint32_t)((int32_t)(half << sb.y) >> 31);
+    const uint64_t mm = (uint64_t)m | ((uint64_t)m << 32), tb = 1ull << t;
+    p0 ^= (uint32_t)P.x & m;
+    p1 ^= (uint32_t)(P.x >> 32) & m;
+    v ^= P.y & mm;
+    u0 |= (uint32_t)tb & m;
+    u1 |= (uint32_t)(tb >> 32) & m;
+  };
+#pragma unroll 4
+  for (uint32_t t = 0; t < T0; t++) replay(t, p0);
+#pragma unroll 4
+  for (uint32_t t = T0; t < T; t++) replay(t, p1);
+  if (!in) return;
+  p.U[r] = (uint64_t)u0 | ((uint64_t)u1 << 32);
+  if (next) p.word[r] = v;
 }
 
-// (4) Look-ahead: every row's word wn (the next panel's) after this panel,
-// into a.nw, computed before the panel's apply has run: the row's mask by the
-// same replay as the apply's step (b) on its word wj, then its word wn XOR
-// the pivot rows' words wn of the mask (all read at the panel start).
-__device__ __forceinline__ void panel_next(const PanelArgs& a, const PanelRec& g, uint32_t wj, uint32_t wn,
-                                           uint32_t blk, uint32_t nblk) {
-  __shared__ uint32_t stp[PANEL];
-  __shared__ uint8_t bt[PANEL];
-  __shared__ uint64_t A[PANEL], PWP[PANEL], PN[PANEL];
-  const uint32_t T = g.T, tid = threadIdx.x, R = a.rows, W = a.W;
-  for (uint32_t t = tid; t < T; t += blockDim.x) {
-    stp[t] = g.stp[t]; bt[t] = g.bt[t]; A[t] = g.A[t]; PWP[t] = g.PWP[t];
-    PN[t] = a.xzs[(size_t)g.stp[t] * W + wn];
-  }
-  __syncthreads();
-  const uint32_t per = (R + nblk - 1) / nblk, r0 = blk * per, r1 = min(R, r0 + per);
-  for (uint32_t r = r0 + tid; r < r1; r += blockDim.x) {
-    uint64_t pw = a.xzs[(size_t)r * W + wj], cm = 0;
-    for (uint32_t t = 0; t < T; t++) {
-      if (r != stp[t] && ((pw >> bt[t]) & 1ull)) {
-        cm ^= A[t];
-        pw ^= PWP[t];
-      }
-    }
-    uint64_t v = a.xzs[(size_t)r * W + wn];
-    while (cm) {
-      const uint32_t x = __ffsll(cm) - 1;
-      cm &= cm - 1;
-      v ^= PN[x];
-    }
-    a.nw[r] = v;
-  }
-}
-
-// The plain schedule: per panel a one-CTA search launch (steps, then the
-// pivot rows and phase data) and a grid-wide apply launch.
-template <uint32_t RPT>
-__global__ void __launch_bounds__(CANON_THREADS) canon_search_kernel(const PanelArgs a) {
-  extern __shared__ __align__(16) uint64_t sm[];
-  // launched as a programmatic dependent of the previous panel's apply: wait
-  // for it (complete, its writes visible), then let the next launch in
+// The rows into the tiles (a warp a row): identity positions, empty records,
+// the first panel's words.
+__global__ void __launch_bounds__(256) canon_tiles_load_kernel(const CanonPanelArgs a) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;");
-  PanelRec& g = *a.rec;
-  const uint32_t len = a.W / 2, wj = panel_word(a.stage, a.c0, len);
-  uint64_t* XT = sm;                                                   // [len][PANEL + 1] X, then Z
-  uint32_t* cand = (uint32_t*)(XT + (size_t)2 * len * (PANEL + 1));    // the candidate rows
-  const bool was_done = g.done != 0;
-  panel_steps<RPT>(a, g, g, a.xzs + wj, a.W, cand);
-  if (!was_done) panel_post(a, g, a.po, wj, XT);
-}
-
-__global__ void __launch_bounds__(CANON_THREADS) canon_apply_kernel(const PanelArgs a) {
-  extern __shared__ __align__(16) uint64_t sm[];
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;");
-  panel_apply(a, *a.rec, a.po, panel_word(a.stage, a.c0, a.W / 2), blockIdx.x, gridDim.x, sm);
-}
-
-// The look-ahead schedule: per panel p two launches,
-//   L1(p): CTA 0 runs panel p's pivot steps on the words a.nw (panel p's
-//          word of every row as it is after panel p - 1), while CTAs 1..
-//          apply panel p - 1 to the rows;
-//   L2(p): CTA 0 copies panel p's pivot rows (the rows are complete through
-//          panel p - 1 now) and computes its phase data, while CTAs 1..
-//          compute every row's word of panel p + 1 after panel p into a.nw.
-// So the serial part of a panel is the steps and the post-processing; the
-// grid-wide apply runs beside the next panel's steps.  The records and pivot
-// copies alternate between two buffers by panel parity (L1(p)'s apply reads
-// panel p - 1's while its steps write panel p's).
-template <uint32_t RPT>
-__global__ void __launch_bounds__(CANON_THREADS) canon_steps_apply_kernel(const PanelArgs a) {
-  extern __shared__ __align__(16) uint64_t sm[];
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;");
-  if (blockIdx.x == 0) {
-    if (a.steps) panel_steps<RPT>(a, *a.prev, *a.rec, a.nw, 1u, (uint32_t*)sm);
-  } else if (a.wj_prev != 0xFFFFFFFFu) {
-    panel_apply(a, *a.prev, a.po_prev, a.wj_prev, blockIdx.x - 1, gridDim.x - 1, sm);
+  const uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (blockIdx.x == 0)
+    for (uint32_t k = threadIdx.x; k < 2 * sizeof(PanelRecord) / 4; k += blockDim.x) ((uint32_t*)a.rec)[k] = 0;
+  if (r >= a.p.rows) return;
+  const uint64_t* row = a.xzs + (size_t)r * a.p.W;
+  tiles_load_row(a.p, row, r, a.ph[r], lane);
+  if (lane == 0) {
+    a.inv[r] = r;
+    a.p.word[r] = row[0];
   }
 }
 
-__global__ void __launch_bounds__(CANON_THREADS) canon_post_next_kernel(const PanelArgs a) {
-  extern __shared__ __align__(16) uint64_t sm[];
+// The rows to their final positions.  Without phases the reference's row
+// swaps leave the phases in place.
+__global__ void __launch_bounds__(256) canon_tiles_store_kernel(const CanonPanelArgs a) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;");
-  const uint32_t wj = panel_word(a.stage, a.c0, a.W / 2);
-  if (blockIdx.x == 0) {
-    panel_post(a, *a.rec, a.po, wj, sm);
-  } else if (a.wj_next != 0xFFFFFFFFu) {
-    panel_next(a, *a.rec, wj, a.wj_next, blockIdx.x - 1, gridDim.x - 1);
-  }
-}
-
-// rows to their final positions: out[pos[r]] = row r
-__global__ void canon_place_kernel(const uint64_t* xzs, const uint8_t* ph, const uint32_t* pos, uint32_t rows,
-                                   uint32_t W, uint64_t* out, uint8_t* out_ph) {
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (warp >= rows) return;
-  const uint32_t p = pos[warp];
-  for (uint32_t w = lane; w < W; w += 32) out[(size_t)p * W + w] = xzs[(size_t)warp * W + w];
-  if (lane == 0) out_ph[p] = ph[warp];
-}
-
-__global__ void canon_grid_init_kernel(uint32_t* pos, uint32_t rows, PanelRec* rec) {
-  const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r < rows) pos[r] = r;
-  if (r == 0) { rec->T = 0; rec->i = 0; rec->rx = 0; rec->done = 0; }
-}
-
-// The look-ahead schedule's start: positions, both records empty, and every
-// row's word of the first panel (X word 0).
-__global__ void canon_look_init_kernel(uint32_t* pos, uint32_t rows, PanelRec* rec, const uint64_t* xzs,
-                                       uint32_t W, uint64_t* nw) {
-  const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r < rows) {
-    pos[r] = r;
-    nw[r] = xzs[(size_t)r * W];
-  }
-  if (r < 2) { rec[r].T = 0; rec[r].i = 0; rec[r].rx = 0; rec[r].done = 0; }
+  const uint32_t pos = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (pos >= a.p.rows) return;
+  const uint32_t ph = tiles_store_row(a.p, a.xzs + (size_t)pos * a.p.W, a.inv[pos], lane);
+  if (lane == 0 && a.p.phases) a.ph[pos] = (uint8_t)ph;
 }
 
 struct CanonPlan {
@@ -1481,21 +1496,28 @@ static int launch_blocked(const ElimSpec& e, cudaStream_t st) {
 }
 
 static uint32_t g_canon_grid = 0;  // 0: automatic, 1: always, 2: never (panels over the whole GPU)
-static uint32_t g_canon_rpt = 0;         // tuner: rows per search thread (0: automatic; 4, 8, 16)
-static uint32_t g_canon_apply_rows = 0;  // tuner: rows per apply CTA (0: automatic)
-static uint32_t g_canon_pdl = 1;         // panel launches as programmatic dependents (0: plain)
-static uint32_t g_canon_lookahead = 1;   // the next panel's steps beside this panel's apply (0: in turn)
-// Smallest stabilizer view that runs by panels over the whole GPU (below it,
-// one cluster holds the rows in shared memory).
-constexpr uint32_t CANON_GRID_MIN_ROWS = 640;
+static uint32_t g_canon_pdl = 1;   // panel launches as programmatic dependents (0: plain)
+// Stabilizer views that run by panels over the whole GPU.
+constexpr uint32_t CANON_GRID_MIN_ROWS = 16, CANON_GRID_MAX_ROWS = 8192;
+
+// Whether a view of automatic choice does.  A panel that finds pivots takes
+// about 18 us and one without 4 us (two launches); the one-cluster kernels
+// take about 75 us per 64 rows and next to nothing once every row has its
+// pivot, so views much wider than tall stay with them (rows x qubits, us, grid
+// / cluster: 12 x 12 36 / 34, 16 x 16 34 / 42, 64 x 64 40 / 87, 64 x 384 63 /
+// 80, 64 x 800 121 / 90, 100 x 2000 259 / 160, 300 x 1900 264 / 349).  From
+// 640 rows on always.
+static bool canon_grid_pays(uint32_t rows, uint32_t n) {
+  return rows >= 640 || (rows >= CANON_GRID_MIN_ROWS && (n + 63) / 64 <= 7 * ((rows + 63) / 64));
+}
 
 // A panel launch.  With g_canon_pdl it is a programmatic dependent of the
 // launch before it on the stream: its CTAs may be scheduled while that one
 // finishes (each kernel waits for its predecessor with griddepcontrol.wait
-// before touching memory), which hides the launch gap between the ~2 x 63
-// dependent launches of each stage.
-static cudaError_t launch_panel(void (*k)(const PanelArgs), uint32_t grid, uint32_t block, size_t smem,
-                                cudaStream_t st, const PanelArgs& a) {
+// before touching memory), which hides the launch gap between the dependent
+// launches.
+static cudaError_t launch_panel(void (*k)(const CanonPanelArgs), uint32_t grid, uint32_t block, size_t smem,
+                                cudaStream_t st, const CanonPanelArgs& a) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(block);
@@ -1506,144 +1528,63 @@ static cudaError_t launch_panel(void (*k)(const PanelArgs), uint32_t grid, uint3
   at[0].val.programmaticStreamSerializationAllowed = g_canon_pdl ? 1 : 0;
   cfg.attrs = at;
   cfg.numAttrs = 1;
+  g_launches.fetch_add(1, std::memory_order_relaxed);
   return cudaLaunchKernelEx(&cfg, k, a);
 }
 
-// canonicalize! by panels over the whole GPU with look-ahead
-// (canon_steps_apply_kernel + canon_post_next_kernel per panel, one more
-// canon_steps_apply_kernel for the last panel's apply); scratch from the
-// stream-ordered pool.
-static int launch_grid_lookahead(const ElimSpec& e, cudaStream_t st) {
-  const uint32_t R = e.rows, W = e.W, len = W / 2;
-  uint32_t* pos = nullptr;
-  PanelRec* rec = nullptr;
-  uint64_t *po = nullptr, *nw = nullptr, *gtmp = nullptr;
-  uint8_t* gtmp_ph = nullptr;
-  QCB_CUDA(cudaMallocAsync(&pos, (size_t)R * 4, st));
-  QCB_CUDA(cudaMallocAsync(&rec, 2 * sizeof(PanelRec), st));
-  QCB_CUDA(cudaMallocAsync(&po, (size_t)2 * PANEL * W * 8, st));
-  QCB_CUDA(cudaMallocAsync(&nw, (size_t)R * 8, st));
-  QCB_CUDA(cudaMallocAsync(&gtmp, (size_t)R * W * 8, st));
-  QCB_CUDA(cudaMallocAsync(&gtmp_ph, R, st));
-  canon_look_init_kernel<<<(R + 255) / 256, 256, 0, st>>>(pos, R, rec, e.xzs, W, nw);
-  QCB_LAUNCHED();
-  uint32_t rpt = g_canon_rpt ? g_canon_rpt : 4u;
-  while (rpt * CANON_THREADS < R) rpt *= 2;
-  void (*steps)(const PanelArgs) = rpt == 1 ? canon_steps_apply_kernel<1>
-                                 : rpt == 2 ? canon_steps_apply_kernel<2>
-                                 : rpt == 4 ? canon_steps_apply_kernel<4>
-                                 : rpt == 8 ? canon_steps_apply_kernel<8> : canon_steps_apply_kernel<16>;
-  // CTA 0 of each L1 launch runs the steps on an SM of its own (1024 threads
-  // of up to 64 registers fill an SM's register file); the apply takes the
-  // other SMs, one CTA each
+// canonicalize! by panels over the whole GPU; scratch (the tiles: the tableau
+// rounded up to two word columns, and small arrays) from the stream-ordered
+// pool in one piece.
+static int launch_grid(const ElimSpec& e, cudaStream_t st) {
+  const uint32_t R = e.rows, W = e.W, len = W / 2, ntile = (len + 1) / 2;
+  CanonPanelArgs a{};
+  size_t bytes = 0;
+  auto place = [&](size_t n) { const size_t o = bytes; bytes += (n + 127) / 128 * 128; return o; };
+  const size_t o_t = place((size_t)ntile * R * 32), o_po = place((size_t)ntile * PSTEPS * 32), o_w = place((size_t)R * 8),
+               o_u = place((size_t)R * 8), o_q = place(R), o_par = place((size_t)ntile * R), o_inv = place((size_t)R * 4), o_rec = place(2 * sizeof(PanelRecord));
+  uint8_t* m = nullptr;
+  QCB_CUDA(cudaMallocAsync(&m, bytes, st));
+  PanelRecord* rec = (PanelRecord*)(m + o_rec);
+  a.p = PanelTiles{R, W, len, ntile, e.phases, (ulonglong2*)(m + o_t), (ulonglong2*)(m + o_po), (uint64_t*)(m + o_w),
+                   (uint64_t*)(m + o_u), m + o_q, m + o_par};
+  a.xzs = e.xzs; a.ph = e.ph; a.n = e.n; a.inv = (uint32_t*)(m + o_inv);
+  a.rec = rec; a.out = e.d_out;
+  const uint32_t warps = 8, row_blocks = (R + warps - 1) / warps;
+  QCB_CUDA(launch_panel(canon_tiles_load_kernel, row_blocks, 32 * warps, 0, st, a));
+  // rows per thread of the search's other warps (registers)
+  const uint32_t rest = R > STEP_WINDOW ? R - STEP_WINDOW : 0;
+  void (*l1)(const CanonPanelArgs) = rest <= STEP_REST ? canon_steps_apply_kernel<1>
+                                   : rest <= 2 * STEP_REST ? canon_steps_apply_kernel<2>
+                                   : rest <= 5 * STEP_REST ? canon_steps_apply_kernel<5> : canon_steps_apply_kernel<9>;
+  static_assert(STEP_WINDOW + 9 * STEP_REST >= CANON_GRID_MAX_ROWS, "every row has a thread");
+  const size_t smem = std::max({sizeof(ApplySmem), sizeof(PhaseSmem), (size_t)R * 16});
+  QCB_CUDA(cudaFuncSetAttribute(l1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // L1: the steps' CTA has an SM of its own (1024 threads of up to 64
+  // registers fill its register file), the apply the other SMs: a CTA per
+  // tile and range of at least 256 rows (a CTA's tables cost about as much
+  // as 400 rows' lookups)
   const uint32_t nsm = (uint32_t)device_sm_count();
-  const uint32_t rows_per_cta = g_canon_apply_rows ? g_canon_apply_rows : 8u;
-  const uint32_t G = std::max<uint32_t>(1, std::min<uint32_t>((R + rows_per_cta - 1) / rows_per_cta, nsm - 1));
-  const uint32_t per = (R + G - 1) / G;
-  const size_t l1_smem = std::max<size_t>((size_t)R * 4, (size_t)PANEL * W * 8 + (size_t)per * 9 + 16);
-  const size_t l2_smem = (size_t)2 * len * (PANEL + 1) * 8;
-  // the next words: a share of the rows on every other SM (the replay is a
-  // serial loop over the panel's pivots per row, so the rows are spread thin)
-  const uint32_t G2 = std::max<uint32_t>(1, std::min<uint32_t>(R, nsm - 1));
-  QCB_CUDA(cudaFuncSetAttribute(steps, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l1_smem));
-  QCB_CUDA(cudaFuncSetAttribute(canon_post_next_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l2_smem));
+  a.nq = e.phases ? (R + CANON_THREADS - 1) / CANON_THREADS : 0;
+  const uint32_t room = nsm > 1 + a.nq ? nsm - 1 - a.nq : 1;
+  a.groups = std::max<uint32_t>(1, std::min<uint32_t>(room / ntile, (R + 255) / 256));
+  a.per = (R + a.groups - 1) / a.groups;
   std::vector<std::pair<uint32_t, uint32_t>> panels;  // (stage, first column)
   for (uint32_t stage = 0; stage < 2; stage++)
-    for (uint32_t c0 = 0; c0 < e.n; c0 += PANEL) panels.push_back({stage, c0});
+    for (uint32_t c0 = 0; c0 < e.n; c0 += PSTEPS) panels.push_back({stage, c0});
   const uint32_t P = (uint32_t)panels.size();
-  PanelArgs a{};
-  a.xzs = e.xzs; a.ph = e.ph; a.rows = R; a.n = e.n; a.W = W; a.phases = e.phases;
-  a.pos = pos; a.out = e.d_out; a.nw = nw;
-  for (uint32_t p = 0; p <= P; p++) {
-    // L1(p): panel p's steps (p < P) beside panel p - 1's apply (p > 0)
-    a.steps = p < P ? 1u : 0u;
-    if (p < P) { a.stage = panels[p].first; a.c0 = panels[p].second; }
-    a.rec = rec + (p & 1);
-    a.prev = rec + ((p + 1) & 1);
-    a.po_prev = po + (size_t)((p + 1) & 1) * PANEL * W;
-    a.wj_prev = p > 0 ? panel_word(panels[p - 1].first, panels[p - 1].second, len) : 0xFFFFFFFFu;
-    QCB_CUDA(launch_panel(steps, 1 + G, CANON_THREADS, l1_smem, st, a));
-    if (p == P) break;
-    // L2(p): panel p's pivot rows and phase data beside every row's next word
-    a.po = po + (size_t)(p & 1) * PANEL * W;
-    a.wj_next = p + 1 < P ? panel_word(panels[p + 1].first, panels[p + 1].second, len) : 0xFFFFFFFFu;
-    QCB_CUDA(launch_panel(canon_post_next_kernel, 1 + G2, CANON_THREADS, l2_smem, st, a));
+  for (uint32_t k = 0; k <= P; k++) {
+    a.steps = k < P;
+    a.apply = k > 0;
+    if (k < P) { a.stage = panels[k].first; a.c0 = panels[k].second; }
+    a.rec = rec + (k & 1);
+    a.prev = rec + ((k + 1) & 1);
+    QCB_CUDA(launch_panel(l1, 1 + (a.apply ? a.nq + ntile * a.groups : 0), CANON_THREADS, smem, st, a));
+    if (k == P) break;
+    a.wn = k + 1 < P ? panel_word(panels[k + 1].first, panels[k + 1].second, len) : WORD_NONE;
+    QCB_CUDA(launch_panel(canon_mid_kernel, ntile + 1 + (R + MID_THREADS - 1) / MID_THREADS, MID_THREADS, 0, st, a));
   }
-  canon_place_kernel<<<(R * 32 + 255) / 256, 256, 0, st>>>(e.xzs, e.ph, pos, R, W, gtmp, gtmp_ph);
-  QCB_LAUNCHED();
-  QCB_CUDA(cudaMemcpyAsync(e.xzs, gtmp, (size_t)R * W * 8, cudaMemcpyDeviceToDevice, st));
-  // without phases the reference's row swaps leave the phases in place
-  if (e.phases) QCB_CUDA(cudaMemcpyAsync(e.ph, gtmp_ph, R, cudaMemcpyDeviceToDevice, st));
-  QCB_CUDA(cudaFreeAsync(pos, st));
-  QCB_CUDA(cudaFreeAsync(rec, st));
-  QCB_CUDA(cudaFreeAsync(po, st));
-  QCB_CUDA(cudaFreeAsync(nw, st));
-  QCB_CUDA(cudaFreeAsync(gtmp, st));
-  QCB_CUDA(cudaFreeAsync(gtmp_ph, st));
-  return QCB_OK;
-}
-
-// canonicalize! by panels over the whole GPU (canon_search_kernel +
-// canon_apply_kernel per panel); scratch from the stream-ordered pool.
-static int launch_grid(const ElimSpec& e, cudaStream_t st) {
-  if (g_canon_lookahead) return launch_grid_lookahead(e, st);
-  const uint32_t R = e.rows, W = e.W, len = W / 2;
-  uint32_t* pos = nullptr;
-  PanelRec* rec = nullptr;
-  uint64_t *po = nullptr, *gtmp = nullptr;
-  uint8_t* gtmp_ph = nullptr;
-  QCB_CUDA(cudaMallocAsync(&pos, (size_t)R * 4, st));
-  QCB_CUDA(cudaMallocAsync(&rec, sizeof(PanelRec), st));
-  QCB_CUDA(cudaMallocAsync(&po, (size_t)PANEL * W * 8, st));
-  QCB_CUDA(cudaMallocAsync(&gtmp, (size_t)R * W * 8, st));
-  QCB_CUDA(cudaMallocAsync(&gtmp_ph, R, st));
-  canon_grid_init_kernel<<<(R + 255) / 256, 256, 0, st>>>(pos, R, rec);
-  QCB_LAUNCHED();
-  // rows per search thread: 4, or the fewest that fit the rows in 1024
-  // threads (n = 1000: 1 / 2 / 4 / 8 rows 1.225 / 1.233 / 1.223 / 1.333 ms;
-  // n = 2000: 2 / 4 / 8 rows 2.71 / 2.63 / 2.81 ms; n = 4000: 4 / 8 / 16
-  // rows 7.66 / 7.86 / 11.19 ms)
-  uint32_t rpt = g_canon_rpt ? g_canon_rpt : 4u;
-  while (rpt * CANON_THREADS < R) rpt *= 2;
-  void (*search)(const PanelArgs) = rpt == 1 ? canon_search_kernel<1>
-                                  : rpt == 2 ? canon_search_kernel<2>
-                                  : rpt == 4 ? canon_search_kernel<4>
-                                  : rpt == 8 ? canon_search_kernel<8> : canon_search_kernel<16>;
-  const size_t search_smem = (size_t)2 * len * (PANEL + 1) * 8 + (size_t)R * 4;
-  // opt in always: the static shared memory counts against the default 48 KB too
-  QCB_CUDA(cudaFuncSetAttribute(search, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)search_smem));
-  // rows per apply CTA: 8 while that still fits one CTA per SM, else 16
-  // (n = 1000: 8 / 16 rows 0.982 / 1.005 ms; n = 2000: 2.420 / 2.400 ms;
-  // n = 4000: 7.89 / 7.43 ms)
-  const uint32_t rows_per_cta =
-      g_canon_apply_rows ? g_canon_apply_rows : (R <= 8u * (uint32_t)device_sm_count() ? 8u : 16u);
-  const uint32_t G = std::max<uint32_t>(1, std::min<uint32_t>((R + rows_per_cta - 1) / rows_per_cta,
-                                                              2 * (uint32_t)device_sm_count()));
-  const uint32_t per = (R + G - 1) / G;
-  const uint32_t threads = std::min<uint32_t>(CANON_THREADS, std::max<uint32_t>(64, 32 * per));
-  const size_t apply_smem = (size_t)PANEL * W * 8 + (size_t)per * 9 + 16;
-  QCB_CUDA(cudaFuncSetAttribute(canon_apply_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)apply_smem));
-  PanelArgs a{};
-  a.xzs = e.xzs; a.ph = e.ph; a.rows = R; a.n = e.n; a.W = W; a.phases = e.phases;
-  a.pos = pos; a.rec = rec; a.po = po; a.out = e.d_out;
-  for (uint32_t stage = 0; stage < 2; stage++) {
-    for (uint32_t c0 = 0; c0 < e.n; c0 += PANEL) {
-      a.stage = stage;
-      a.c0 = c0;
-      QCB_CUDA(launch_panel(search, 1, CANON_THREADS, search_smem, st, a));
-      QCB_CUDA(launch_panel(canon_apply_kernel, G, threads, apply_smem, st, a));
-    }
-  }
-  canon_place_kernel<<<(R * 32 + 255) / 256, 256, 0, st>>>(e.xzs, e.ph, pos, R, W, gtmp, gtmp_ph);
-  QCB_LAUNCHED();
-  QCB_CUDA(cudaMemcpyAsync(e.xzs, gtmp, (size_t)R * W * 8, cudaMemcpyDeviceToDevice, st));
-  // without phases the reference's row swaps leave the phases in place
-  if (e.phases) QCB_CUDA(cudaMemcpyAsync(e.ph, gtmp_ph, R, cudaMemcpyDeviceToDevice, st));
-  QCB_CUDA(cudaFreeAsync(pos, st));
-  QCB_CUDA(cudaFreeAsync(rec, st));
-  QCB_CUDA(cudaFreeAsync(po, st));
-  QCB_CUDA(cudaFreeAsync(gtmp, st));
-  QCB_CUDA(cudaFreeAsync(gtmp_ph, st));
+  QCB_CUDA(launch_panel(canon_tiles_store_kernel, row_blocks, 32 * warps, 0, st, a));
+  QCB_CUDA(cudaFreeAsync(m, st));
   return QCB_OK;
 }
 
@@ -1655,9 +1596,8 @@ static int eliminate(const ElimSpec& e, cudaStream_t st) {
     return QCB_OK;
   }
   const bool D = e.dxzs != nullptr;
-  // by panels up to 8192 rows (the search keeps at most 8 rows per thread in registers)
-  if (e.mode == ELIM_BOTH && !D && e.rows <= 8192 && g_canon_grid != 2 &&
-      (g_canon_grid == 1 || e.rows >= CANON_GRID_MIN_ROWS) && g_canon_blocked != 2 && e.n > 0)
+  if (e.mode == ELIM_BOTH && !D && e.n > 0 && g_canon_blocked != 2 && g_canon_grid != 2 && e.rows <= CANON_GRID_MAX_ROWS &&
+      (g_canon_grid == 1 || canon_grid_pays(e.rows, e.n)))
     return launch_grid(e, st);
   if (e.mode == ELIM_BOTH && !D && e.rows <= 8192 && g_canon_blocked != 2 && (g_canon_blocked == 1 || e.rows >= 64))
     return launch_blocked(e, st);
@@ -1773,10 +1713,7 @@ void set_canon_cluster(uint32_t cs) { g_canon_cs = cs; }
 void set_canon_threads(uint32_t n) { g_canon_threads = n; }
 void set_canon_blocked(uint32_t v) { g_canon_blocked = v; }
 void set_canon_grid(uint32_t v) { g_canon_grid = v; }
-void set_canon_rpt(uint32_t v) { g_canon_rpt = v; }
 void set_canon_pdl(uint32_t v) { g_canon_pdl = v; }
-void set_canon_lookahead(uint32_t v) { g_canon_lookahead = v; }
-void set_canon_apply_rows(uint32_t v) { g_canon_apply_rows = v; }
 
 }  // namespace qcb
 

@@ -60,13 +60,10 @@ void set_project_withhold(uint32_t v);
 void set_canon_blocked(uint32_t v);
 void set_canon_grid(uint32_t v);
 void set_server_fill(uint32_t v);
-void set_canon_rpt(uint32_t v);
 void set_canon_pdl(uint32_t v);
 void set_gates_pdl(uint32_t v);
-void set_canon_lookahead(uint32_t v);
 void set_walker_pdl(uint32_t v);
 void set_walker_narrow(uint32_t v);
-void set_canon_apply_rows(uint32_t v);
 
 }  // namespace qcb
 
@@ -172,13 +169,12 @@ int qcb_tune_set(const char* key, int64_t value) {
     if (value > 2) return fail(QCB_EARG, "canon_blocked must be 0 (automatic), 1 (always) or 2 (never)");
     set_canon_blocked((uint32_t)value);
   } else if (k == "canon_grid") {
-    // canonicalize! by panels over the whole GPU: 0 from 640 rows, 1 always, 2 never
+    // canonicalize! by panels over the whole GPU: 0 from 64 rows, 1 always, 2 never
     if (value > 2) return fail(QCB_EARG, "canon_grid must be 0 (automatic), 1 (always) or 2 (never)");
     set_canon_grid((uint32_t)value);
   } else if (k == "canon_rpt") {
     if (value && value != 1 && value != 2 && value != 4 && value != 8 && value != 16)
       return fail(QCB_EARG, "canon_rpt must be 0, 1, 2, 4, 8 or 16");
-    set_canon_rpt((uint32_t)value);
   } else if (k == "walker_narrow") {
     // tall programs whose 16-column tile does not fit shared memory: 8..14-
     // column tiles (1, default) or the walker on the HBM planes (0)
@@ -193,17 +189,14 @@ int qcb_tune_set(const char* key, int64_t value) {
     if (value > 1) return fail(QCB_EARG, "canon_pdl must be 0 or 1");
     set_canon_pdl((uint32_t)value);
   } else if (k == "canon_lookahead") {
-    // canonicalize! by panels over the whole GPU: the next panel's pivot
-    // steps beside this panel's apply (1, default) or the two in turn (0)
+    // accepted without effect, as canon_rpt and canon_apply_rows
     if (value > 1) return fail(QCB_EARG, "canon_lookahead must be 0 or 1");
-    set_canon_lookahead((uint32_t)value);
   } else if (k == "gates_pdl") {
     // symbolic apply! launches (qcb_apply_gates) as programmatic dependents (1, default) or plain (0)
     if (value > 1) return fail(QCB_EARG, "gates_pdl must be 0 or 1");
     set_gates_pdl((uint32_t)value);
   } else if (k == "canon_apply_rows") {
     if (value && (value < 8 || value > 32)) return fail(QCB_EARG, "canon_apply_rows must be 0 or 8..32");
-    set_canon_apply_rows((uint32_t)value);
   } else if (k == "project_grid") {
     // project! of generic Paulis on Stabilizer / MixedStabilizer tableaux on
     // the whole GPU: 0 when the tableau does not fit one cluster's shared

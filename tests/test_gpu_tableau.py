@@ -387,3 +387,35 @@ def test_canonicalize_panels_rectangular_views(qcb, rows, n, lookahead):
         ph, xz, orx, orz = oracle.canonicalize(t.phases, t.xzs, n, phases)
         assert (rx, rz) == (orx, orz)
         assert np.array_equal(s.tab.xzs, xz) and np.array_equal(s.tab.phases, ph)
+
+
+@pytest.mark.parametrize("rows,n,density", [
+    (16, 20, 0.5), (95, 70, 0.5), (96, 64, 0.5), (97, 65, 0.5), (200, 130, 0.02), (1088, 70, 0.5), (1089, 130, 0.01),
+    (2080, 66, 0.004), (2081, 64, 0.5), (3000, 129, 0.0008), (5056, 65, 0.002), (5057, 130, 0.5), (8192, 70, 0.0005),
+    (300, 200, "late"), (1500, 190, "late")])
+@pytest.mark.parametrize("phases", [True, False])
+def test_canonicalize_panel_windows(qcb, rows, n, density, phases):
+    """The panels' pivot search at its edges: views around the window's 96 rows
+    and the rows per thread of the remaining ones, dense rows, rows sparse
+    enough to be listed, and ("late") pivots that lie far behind the window."""
+    rng = np.random.default_rng(rows + n)
+    if density == "late":
+        xs = np.zeros((rows, n), bool)
+        zs = np.zeros((rows, n), bool)
+        xs[:, 0] = zs[:, 1] = True                 # dense words, one live column
+        xs[rows - 90:, :] = rng.random((90, n)) < 0.5
+        zs[rows - 90:, :] = rng.random((90, n)) < 0.5
+    else:
+        xs = rng.random((rows, n)) < density
+        zs = rng.random((rows, n)) < density
+    t = Tableau.from_bits(rng.integers(0, 4, rows), xs, zs)
+    qcb.check(qcb.lib().qcb_tune_set(b"canon_grid", 1))
+    try:
+        s = qcb.Stabilizer(t.copy()).to_gpu()
+        _, rx, rz = qcb.canonicalize_(s, phases=phases, ranks=True)
+        s.to_cpu()
+    finally:
+        qcb.check(qcb.lib().qcb_tune_set(b"canon_grid", 0))
+    ph, xz, orx, orz = oracle.canonicalize(t.phases, t.xzs, n, phases)
+    assert (rx, rz) == (orx, orz)
+    assert np.array_equal(s.tab.xzs, xz) and np.array_equal(s.tab.phases, ph)
