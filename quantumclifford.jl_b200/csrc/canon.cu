@@ -905,9 +905,9 @@ __global__ void __launch_bounds__(CANON_THREADS) canon_batch_kernel(const CanonB
 // Bound by that chain: L1 12 us and L2 6.3 us alone, 18 us a panel in
 // sequence (n = 4000), of which the steps are 7.5 us and the rest launch and
 // load latencies.  Random states, n = 1000 / 2000 / 4000: 706 / 1661 / 4643 ->
-// 281 / 595 / 1381 us (the search over all rows with a block barrier a step,
+// 290 / 600 / 1410 us (the search over all rows with a block barrier a step,
 // every pivot row XORed for itself and 64 dot products a row for the phases
-// before); sparse rows (weight 4), 863 / 2114 / 6027 -> 475 / 1050 / 2507 us.
+// before); sparse rows (weight 4), 863 / 2114 / 6027 -> 500 / 1150 / 2770 us.
 struct CanonPanelArgs {
   PanelTiles p;
   uint64_t* xzs;
@@ -934,13 +934,13 @@ inline uint32_t panel_word(uint32_t stage, uint32_t c0, uint32_t len) { return s
 // registers and runs the steps on these alone, without a block barrier; the
 // pivot's word and mask go through its record in shared memory.  For dense
 // rows a pivot outside the window has probability 2^-33 a column.  When the
-// window has none, the other warps, which keep the remaining rows' words,
-// catch up with the pivots so far and look for the first of theirs.  Where the
-// first STEP_WINDOW positions hold many zero words (sparse rows), the rows
-// with a nonzero word are listed first, in order of position; all others are
-// inert.  A row swap only changes positions: every row's position is kept by
-// value, and the permutation is brought up to date afterwards
-// (canon_permute).  Bound by warp 0's chain: three tests, a warp minimum, a
+// window has none before the remaining rows' positions, the other warps, which
+// keep those rows' words, catch up with the pivots so far and look for the
+// first of theirs.  Where the first STEP_WINDOW positions hold many zero words
+// (sparse rows), the rows with a nonzero word are listed first, in order of
+// position; all others are inert.  A row swap only changes positions: every
+// row's position is kept by value, and the permutation is brought up to date
+// afterwards (canon_permute).  Bound by warp 0's chain: three tests, a warp minimum, a
 // store and a load, an XOR: 226 cycles a step whatever the rows (0.42 / 0.22
 // us a step at 4000 / 1000 rows with all rows in all warps and a block barrier
 // a step).
@@ -961,7 +961,7 @@ __device__ __forceinline__ void canon_steps(const CanonPanelArgs& a, uint8_t* ds
   __shared__ uint4 recA[PSTEPS];  // pivot t: (panel word, mask)
   __shared__ uint4 recB[PSTEPS];  // (position before the step, bit, row)
   __shared__ uint64_t rw[32], ra[32];
-  __shared__ uint32_t rpos[32], off[UNITS], shT, dense, rb, rT;
+  __shared__ uint32_t rpos[32], off[UNITS], shT, dense, rb, rT, rm;
   PanelRecord& g = *a.rec;
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, R = a.p.rows;
   const uint32_t i0 = a.prev->i, rx0 = a.prev->rx, ncp = min(PSTEPS, a.n - a.c0);
@@ -1078,6 +1078,8 @@ __device__ __forceinline__ void canon_steps(const CanonPanelArgs& a, uint8_t* ds
   const uint32_t nbw = min(31u, (nrest + 31) / 32), stride = listed ? 32 * nbw : STEP_REST, nbar = 32 * (nbw + 1);
   if (warp == 0) {
     const uint32_t tmax = min(PSTEPS, R - i0);
+    // positions below `bound` are the window's: a row there is the first
+    const uint32_t bound = !nrest ? NONE : (listed ? lp[STEP_WINDOW] : i0 + STEP_WINDOW);
     uint32_t T = 0, i = i0, t0 = 1, t1 = 0;  // t1:t0: bit T
     uint32_t ad = (uint32_t)__cvta_generic_to_shared(recA);
     const uint32_t bd = (uint32_t)__cvta_generic_to_shared(recB) - ad;
@@ -1098,7 +1100,7 @@ __device__ __forceinline__ void canon_steps(const CanonPanelArgs& a, uint8_t* ds
 #pragma unroll
           for (uint32_t q = 0; q < 4; q++) s[q] = y2 ? wd[2][q] : (y1 ? wd[1][q] : wd[0][q]);
           const uint32_t sr = y2 ? row[2] : (y1 ? row[1] : row[0]);
-          if (m == NONE) { miss = true; break; }
+          if (m >= bound) { miss = true; break; }
           // stored by the one lane with the least position
           asm volatile("{.reg .pred p; setp.eq.u32 p, %0, %1; @p st.shared.v4.u32 [%2], {%3, %4, %5, %6};"
                        "@p st.shared.v4.u32 [%7], {%1, %8, %9, %9};}" ::"r"(best), "r"(m), "r"(ad), "r"(s[0]), "r"(s[1]),
@@ -1120,22 +1122,51 @@ __device__ __forceinline__ void canon_steps(const CanonPanelArgs& a, uint8_t* ds
           t0 <<= 1;
         }
         if (!miss) break;
-        if (!nrest) continue;
-        if (lane == 0) { rb = 32 * h + c; rT = T; }
-        __syncwarp();
-        asm volatile("bar.sync 1, %0;" ::"r"(nbar) : "memory");
-        asm volatile("bar.sync 2, %0;" ::"r"(nbar) : "memory");
-        const uint32_t v = lane >= 1 && lane <= nbw ? rpos[lane] : NONE, m = __reduce_min_sync(0xFFFFFFFFu, v);
+        // the window's first row with the bit, if any, lies among the
+        // remaining rows (a swap took it there): the first of both
+        uint32_t cand[KW], best = NONE;
+#pragma unroll
+        for (uint32_t k = 0; k < KW; k++) {
+          cand[k] = (wd[k][h] & cm) ? pos[k] : NONE;
+          best = min(best, cand[k]);
+        }
+        uint32_t m = __reduce_min_sync(0xFFFFFFFFu, best);
+        bool outside = false;
+        if (nrest) {
+          if (lane == 0) { rb = 32 * h + c; rT = T; rm = m; }
+          __syncwarp();
+          asm volatile("bar.sync 1, %0;" ::"r"(nbar) : "memory");
+          asm volatile("bar.sync 2, %0;" ::"r"(nbar) : "memory");
+          const uint32_t v = lane >= 1 && lane <= nbw ? rpos[lane] : NONE, kr = __reduce_min_sync(0xFFFFFFFFu, v);
+          outside = kr < m;
+          if (outside) {
+            m = kr;
+            if (v == m) {  // its row comes from the thread that holds it
+              recA[T] = make_uint4((uint32_t)rw[lane], (uint32_t)(rw[lane] >> 32), (uint32_t)ra[lane] | t0,
+                                   (uint32_t)(ra[lane] >> 32) | t1);
+              recB[T].x = m;
+              recB[T].y = 32 * h + c;
+            }
+          }
+        }
         if (m == NONE) continue;  // no pivot in this column
-        if (v == m) {             // no row of the window has the bit
-          recA[T] = make_uint4((uint32_t)rw[lane], (uint32_t)(rw[lane] >> 32), (uint32_t)ra[lane] | t0,
-                               (uint32_t)(ra[lane] >> 32) | t1);
-          recB[T].x = m;
-          recB[T].y = 32 * h + c;
+        if (!outside && best == m) {
+#pragma unroll
+          for (uint32_t k = 0; k < KW; k++)
+            if (cand[k] == m) {
+              recA[T] = make_uint4(wd[k][0], wd[k][1], wd[k][2] | t0, wd[k][3] | t1);
+              recB[T] = make_uint4(m, 32 * h + c, row[k], 0);
+            }
         }
         __syncwarp();
+        const uint4 e = recA[T];
+        const uint32_t p[4] = {e.x, e.y, e.z, e.w};
 #pragma unroll
-        for (uint32_t k = 0; k < KW; k++) pos[k] = pos[k] == i ? m : pos[k];
+        for (uint32_t k = 0; k < KW; k++) {
+          const uint32_t q = pos[k], u = q == i ? m : q;
+          pos[k] = q == m ? i : u;
+          xor_if(wd[k], wd[k][h], cm, p);
+        }
         ad += 16;
         T++;
         i++;
@@ -1159,7 +1190,7 @@ __device__ __forceinline__ void canon_steps(const CanonPanelArgs& a, uint8_t* ds
     uint32_t t = 0;
     while (true) {
       asm volatile("bar.sync 1, %0;" ::"r"(nbar) : "memory");
-      const uint32_t b = rb, T = rT;
+      const uint32_t b = rb, T = rT, first = rm;
       if (b == NONE) break;
       for (; t < T; t++) {
         const uint4 e = recA[t];
@@ -1192,7 +1223,7 @@ __device__ __forceinline__ void canon_steps(const CanonPanelArgs& a, uint8_t* ds
       if (bp == m && m != NONE) { rw[warp] = bw; ra[warp] = bA; }
       asm volatile("bar.sync 2, %0;" ::"r"(nbar) : "memory");
       const uint32_t kp = __reduce_min_sync(0xFFFFFFFFu, lane >= 1 && lane <= nbw ? rpos[lane] : NONE);
-      if (kp != NONE && bp == kp)  // this thread's row is the pivot
+      if (kp < first && bp == kp)  // this thread's row is the pivot
         recB[T].z = listed ? lr[o0 + bk * stride] : a.inv[i0 + o0 + bk * stride];
     }
   }
