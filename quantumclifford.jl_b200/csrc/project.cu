@@ -517,6 +517,7 @@ __global__ void __launch_bounds__(PROJ_THREADS) project_smem_kernel(const ProjSm
           a.result[j] = a.phases ? (int32_t)((s + extra) & 3u) : (int32_t)(pphase & 3u);
         }
       }
+      cl.sync();  // the partial products and P are read until here
       continue;
     }
     // 3. MixedDestabilizer logical branch: the row swaps (rare), by CTA 0

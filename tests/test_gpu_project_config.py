@@ -67,3 +67,29 @@ def test_project_independent_stabilizer(qcb, n):
         if j % 50 == 0:
             work.to_cpu()
             assert np.array_equal(work.tab.xzs, xz) and np.array_equal(work.tab.phases, ph), j
+
+
+def test_project_after_a_commuting_pauli_in_the_cluster_kernel(qcb):
+    """A Pauli whose result is the product of stabilizer rows, followed by
+    others, on a tableau over several CTAs of one cluster: the partial
+    products of the CTAs are read before the next Pauli overwrites them."""
+    n, k = 1100, 70
+    rng = np.random.default_rng(1230)
+    d = randoms.random_destabilizer(n, rng)
+    ps = randoms.random_paulis(k, n, rng, phases=True)
+    for j in (0, 30, 64):
+        src = (ps.xzs[j - 1], ps.phases[j - 1]) if j else (d.tab.xzs[n], d.tab.phases[n])
+        ps.xzs[j], ps.phases[j] = src
+    st = qcb.Destabilizer(d.tab.copy()).to_gpu()
+    qcb.check(qcb.lib().qcb_tune_set(b"project_grid", 2))
+    try:
+        _, anti, res = qcb.project_(st, ps.copy().to_gpu())
+    finally:
+        qcb.check(qcb.lib().qcb_tune_set(b"project_grid", 0))
+    st.to_cpu()
+    ph, xz, outs = d.tab.phases.copy(), d.tab.xzs.copy(), []
+    for j in range(k):
+        code, ph, xz, _, a, v = oracle.project("Destabilizer", ph, xz, n, ps.xzs[j], ps.phases[j])
+        outs.append((a, None if v < 0 else v))
+    assert list(zip(anti, res)) == outs
+    assert np.array_equal(st.tab.xzs, xz) and np.array_equal(st.tab.phases, ph)
