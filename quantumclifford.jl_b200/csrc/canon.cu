@@ -947,14 +947,6 @@ inline uint32_t panel_word(uint32_t stage, uint32_t c0, uint32_t len) { return s
 constexpr uint32_t STEP_SLOTS = 3, STEP_WINDOW = 32 * STEP_SLOTS, STEP_DENSE = 80;
 constexpr uint32_t STEP_REST = 31 * 32;  // threads of the remaining rows
 
-// A slot of the window: (word, mask) ^= p where the slot's word `test` has the bit.
-__device__ __forceinline__ void xor_if(uint32_t (&v)[4], uint32_t test, uint32_t bit, const uint32_t (&p)[4]) {
-  asm("{.reg .pred y; .reg .u32 x; and.b32 x, %4, %5; setp.ne.u32 y, x, 0;"
-      "@y xor.b32 %0, %0, %6; @y xor.b32 %1, %1, %7; @y xor.b32 %2, %2, %8; @y xor.b32 %3, %3, %9;}"
-      : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3])
-      : "r"(test), "r"(bit), "r"(p[0]), "r"(p[1]), "r"(p[2]), "r"(p[3]));
-}
-
 template <uint32_t RPT>
 __device__ __forceinline__ void canon_steps(const CanonPanelArgs& a, uint8_t* dsm) {
   constexpr uint32_t NONE = 0xFFFFFFFFu, KW = STEP_SLOTS, UNITS = KW + 31 * RPT;
@@ -1290,7 +1282,7 @@ __global__ void __launch_bounds__(CANON_THREADS) canon_steps_apply_kernel(const 
   const PanelTiles& p = a.p;
   if (blk <= a.nq) {  // q of every row
     PhaseSmem& s = *(PhaseSmem*)dsm;
-    phase_data(p, g, s);
+    phase_data(g, s, [&](uint32_t t) { return p.U[g.stp[t]] & ((1ull << t) - 1ull); });
     for (uint32_t r = (blk - 1) * blockDim.x + threadIdx.x; r < p.rows; r += a.nq * blockDim.x) {
       const uint64_t U = p.U[r];
       if (U) p.q[r] = (uint8_t)((p.q[r] + phase_of(s, U)) & 3u);
@@ -1332,8 +1324,9 @@ __global__ void __launch_bounds__(MID_THREADS) canon_mid_kernel(const CanonPanel
   const uint32_t tid = threadIdx.x, blk = blockIdx.x;
   if (blk < p.ntile) {
     tile_reduce(
-        p, g, blk, s.t, [&](uint32_t r) { return p.t + ((size_t)blk * p.rows + r) * 2; },
-        [&](uint32_t r) { return 2u * p.par[(size_t)blk * p.rows + r] + (blk == 0 ? p.q[r] : 0u); });
+        p, g, blk, s.t, [&](uint32_t, uint32_t r) { return p.t + ((size_t)blk * p.rows + r) * 2; },
+        [&](uint32_t, uint32_t r) { return 2u * p.par[(size_t)blk * p.rows + r] + (blk == 0 ? p.q[r] : 0u); },
+        [](uint32_t, const uint64_t*) {});
     return;
   }
   if (blk == p.ntile) {

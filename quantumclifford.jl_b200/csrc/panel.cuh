@@ -45,6 +45,9 @@ struct PanelRecord {
   uint32_t m[PSTEPS];         // canonicalize!: its position before the step
   uint64_t A[PSTEPS];         // start rows in the reduced pivot t
   uint64_t PW[PSTEPS];        // the pivot's panel word at its step
+  uint32_t src[PSTEPS];       // project!: the step whose Pauli is pivot t's start row (PSTEPS: row stp)
+  uint64_t own[PSTEPS];       // project!: the steps that multiplied pivot t before its own
+  uint32_t s[PSTEPS];         // project!: |x & z| of the reduced pivot, summed over the tiles
   unsigned long long G[PSTEPS];  // z_{P_t} . x_{P_s} (bit s), summed over the tiles
   uint32_t q0[PSTEPS];        // q of the pivot's start row, summed over the tiles
 };
@@ -59,6 +62,14 @@ struct PanelTiles {
   uint8_t* q;         // [rows] q without the tiles' parities
   uint8_t* par;       // [ntile][rows]
 };
+
+// (word, mask) ^= p where `test` has the bit.
+__device__ __forceinline__ void xor_if(uint32_t (&v)[4], uint32_t test, uint32_t bit, const uint32_t (&p)[4]) {
+  asm("{.reg .pred y; .reg .u32 x; and.b32 x, %4, %5; setp.ne.u32 y, x, 0;"
+      "@y xor.b32 %0, %0, %6; @y xor.b32 %1, %1, %7; @y xor.b32 %2, %2, %8; @y xor.b32 %3, %3, %9;}"
+      : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3])
+      : "r"(test), "r"(bit), "r"(p[0]), "r"(p[1]), "r"(p[2]), "r"(p[3]));
+}
 
 __device__ __forceinline__ ulonglong2 xor128(ulonglong2 a, ulonglong2 b) { return make_ulonglong2(a.x ^ b.x, a.y ^ b.y); }
 __device__ __forceinline__ uint32_t parity64(uint64_t v) { return __popc((uint32_t)v ^ (uint32_t)(v >> 32)) & 1u; }
@@ -112,22 +123,23 @@ __device__ __forceinline__ uint32_t tiles_store_row(const PanelTiles& p, uint64_
 
 // ---------------------------------------------------------------- reduced pivots
 // A CTA of 256 threads on one tile: the pivots' start rows reduced by A into
-// po, and the tile's share of G and of the start rows' q.  base(r) is row r
-// of the tile (two ulonglong2), q0(r) its share of q.
+// po, and the tile's share of G and of the start rows' q.  base(t, r) are the
+// start words of pivot t, row r, on the tile (two ulonglong2, readable for
+// stale records too), q0(t, r) its share of q; red(t) sees the reduced pivot.
 constexpr uint32_t MID_THREADS = 256;
 
 struct __align__(16) TileSmem {
   uint64_t start[PSTEPS][4], red[PSTEPS][4];
 };
 
-template <class Base, class Q0>
+template <class Base, class Q0, class Red>
 __device__ __forceinline__ void tile_reduce(const PanelTiles& p, PanelRecord& g, uint32_t tile, TileSmem& s, Base base,
-                                            Q0 q0) {
+                                            Q0 q0, Red red) {
   // fields beyond the record's T steps are stale but readable
   const uint32_t tid = threadIdx.x, T = g.T;
   const uint32_t t = tid >> 2, w = tid & 3;
   const uint32_t r = g.stp[t];
-  const uint64_t A0 = g.A[t], st = ((const uint64_t*)base(r))[w];
+  const uint64_t A0 = g.A[t], st = ((const uint64_t*)base(t, r))[w];
   if (T == 0) return;
   uint64_t A = t < T ? A0 : 0ull;
   s.start[t][w] = t < T ? st : 0ull;
@@ -141,8 +153,9 @@ __device__ __forceinline__ void tile_reduce(const PanelTiles& p, PanelRecord& g,
   s.red[t][w] = v;
   ((uint64_t*)(p.po + ((size_t)tile * PSTEPS + t) * 2))[w] = v;
   if (!p.phases) return;
-  const uint32_t q = w == 0 && t < T ? q0(r) : 0u;
+  const uint32_t q = w == 0 && t < T ? q0(t, r) : 0u;
   __syncthreads();
+  if (w == 1 && t < T) red(t, s.red[t]);
   // G[t] bits 16 w .. 16 w + 15
   const uint64_t z0 = s.red[t][2], z1 = s.red[t][3];
   uint32_t bits = 0;
@@ -162,7 +175,8 @@ __device__ __forceinline__ void tile_reduce(const PanelTiles& p, PanelRecord& g,
 }
 
 // ---------------------------------------------------------------- phase data
-// The pivots' q and the lower triangle of G of one record, by a whole CTA.
+// The pivots' q and the lower triangle of G of one record, by a whole CTA;
+// own(t): the steps that multiplied pivot t before its own.
 struct PhaseSmem {
   uint64_t U[PSTEPS], A[PSTEPS], G[PSTEPS], GL[PSTEPS];
   uint32_t bal[8];
@@ -177,13 +191,13 @@ __device__ __forceinline__ uint64_t vote64(PhaseSmem& s, uint32_t slot, bool b) 
   return (uint64_t)s.bal[2 * slot] | ((uint64_t)s.bal[2 * slot + 1] << 32);
 }
 
-__device__ __forceinline__ void phase_data(const PanelTiles& p, const PanelRecord& g, PhaseSmem& s) {
+template <class Own>
+__device__ __forceinline__ void phase_data(const PanelRecord& g, PhaseSmem& s, Own own) {
   const uint32_t tid = threadIdx.x, T = g.T;
   uint32_t q0 = 0;
   if (tid < PSTEPS) {
     const bool in = tid < T;
-    // the steps that multiplied pivot t before its own
-    s.U[tid] = in ? p.U[g.stp[tid]] & ((1ull << tid) - 1ull) : 0ull;
+    s.U[tid] = in ? own(tid) : 0ull;
     s.A[tid] = in ? g.A[tid] : 0ull;
     s.G[tid] = in ? g.G[tid] : 0ull;
     s.GL[tid] = s.G[tid] & ((1ull << tid) - 1ull);

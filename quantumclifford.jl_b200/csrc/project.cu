@@ -22,6 +22,7 @@
 
 #include <algorithm>
 
+#include "panel.cuh"
 #include "qcb_internal.h"
 
 namespace cg = cooperative_groups;
@@ -757,6 +758,596 @@ __global__ void __launch_bounds__(PROJ_THREADS) project_grid_kernel(const ProjGr
   if (lead && tid == 0) { a.status[0] = PST_OK; a.status[1] = (int32_t)a.k; }
 }
 
+// ---------------------------------------------------------------- by panels
+// Runs of projections by panels of up to 64 Paulis over the whole GPU
+// (panel.cuh).  Projection j multiplies every row that anticommutes with P_j
+// by the first such stabilizer row (the pivot), copies the pivot into its
+// destabilizer row and puts P_j in its place.  Whether a row anticommutes with
+// the panel's Paulis is one word per row, and products act on these words as
+// on the rows, so the panel's steps run on them alone.  A row's start words
+// are its own, those of the last Pauli put into it (word CP[j], its
+// commutation bits with the other Paulis of the panel), or none (a copied
+// pivot: the set U is that step alone).  Per panel three launches:
+//   S   one CTA: the steps on the words;
+//   M   a CTA per tile: the reduced pivots and the tile's share of the phase
+//       data; CTAs over the rows: their sets U and start words;
+//   AF  a CTA per tile and range of rows: the panel applied, and on the new
+//       words the tile's share of the next panel's commutation words (32 byte
+//       lookups in tables over its Paulis); a few CTAs the rows' q.
+// A Pauli that commutes with the stabilizer (its result needs the rows), or
+// anticommutes with a logical row only, ends the run after the steps before
+// it; the host handles that one with the kernels above and goes on.
+// Bound by the chain of the three launches (their latencies; the rows' traffic
+// is a tenth of it).  1000 random Paulis, us each: Stabilizer n = 1000 / 2000 /
+// 4000 4.9 / 7.3 / 12.4 -> 0.60 / 0.61 / 0.70, Destabilizer n = 1000 / 2000
+// 5.4 / 11.3 -> 0.60 / 0.64 (one Pauli at a time, two cluster or grid barriers
+// each, before).
+struct ProjPanelArgs {
+  PanelTiles p;
+  uint64_t* xzs;
+  uint8_t* ph;
+  uint32_t nn;         // tableau row of the first stabilizer row; 0 without destabilizer rows
+  uint32_t rank;       // stabilizer rows
+  uint32_t plain;      // rows below it keep their phase in products (destabilizer rows)
+  int skip;            // a commuting Pauli does nothing (Stabilizer without a result)
+  const uint64_t* paulis;
+  const uint8_t* pph;
+  const uint8_t* rand_ph;
+  uint32_t j0, cnt;    // this panel's Paulis
+  uint32_t jn, cntn;   // the next panel's
+  PanelRecord* rec;
+  int32_t* state;      // [0] stopped, [1] the next Pauli
+  int32_t* anticom;
+  int32_t* result;
+  uint64_t *word, *wordn;   // [rows] commutation words of this and the next panel
+  unsigned long long *CP, *CPn;  // [PSTEPS] the Paulis' own
+  uint32_t *pq, *pqn;       // [PSTEPS] the Paulis' q
+  uint8_t* base;       // [rows] start words: BASE_ROW, BASE_NONE or the Pauli's index in the panel
+  uint32_t apply, nq, groups, per;
+};
+constexpr uint32_t BASE_ROW = 255, BASE_NONE = 254;
+constexpr uint32_t PP_SLOTS = 3, PP_WINDOW = 32 * PP_SLOTS, PP_REST = 31 * 32;
+
+// S: as canonicalize!'s steps, with the stabilizer rows in their fixed order.
+template <uint32_t RPT>
+__global__ void __launch_bounds__(1024) project_steps_kernel(const ProjPanelArgs a) {
+  constexpr uint32_t NONE = 0xFFFFFFFFu, KW = PP_SLOTS;
+  __shared__ uint4 recA[PSTEPS];  // pivot t: (word, mask)
+  __shared__ uint4 recB[PSTEPS];  // (stabilizer row, Pauli, src)
+  __shared__ uint2 sCP[PSTEPS];
+  __shared__ uint64_t rw[32], ra[32];
+  __shared__ uint32_t rs[32], rpos[32], shT, shB, rb, rT;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+  PanelRecord& g = *a.rec;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, R = a.rank;
+  if (tid < PSTEPS) {
+    g.G[tid] = 0;
+    g.q0[tid] = 0;
+    g.s[tid] = 0;
+    const uint64_t c = a.CP[tid];
+    sCP[tid] = make_uint2((uint32_t)c, (uint32_t)(c >> 32));
+  }
+  if (a.state[0]) {
+    if (tid == 0) g.T = 0;
+    return;
+  }
+  const uint64_t* word = a.word + a.nn;
+  uint32_t wd[KW][4], src[KW];
+  uint64_t w[RPT], A[RPT];
+  uint32_t ws[RPT];
+  if (warp == 0) {
+#pragma unroll
+    for (uint32_t k = 0; k < KW; k++) {
+      const uint32_t r = 32 * k + lane;
+      const uint64_t v = r < R ? word[r] : 0ull;
+      wd[k][0] = (uint32_t)v;
+      wd[k][1] = (uint32_t)(v >> 32);
+      wd[k][2] = wd[k][3] = 0;
+      src[k] = PSTEPS;
+    }
+  } else {
+#pragma unroll
+    for (uint32_t k = 0; k < RPT; k++) {
+      const uint32_t r = PP_WINDOW + PP_REST * k + tid - 32;
+      w[k] = r < R ? word[r] : 0ull;
+      A[k] = 0;
+      ws[k] = PSTEPS;
+    }
+  }
+  __syncthreads();
+  const uint32_t nrest = R > PP_WINDOW ? R - PP_WINDOW : 0u, nbw = min(31u, (nrest + 31) / 32), nbar = 32 * (nbw + 1);
+  if (warp == 0) {
+    uint32_t T = 0, t0 = 1, t1 = 0, stop = a.cnt;  // t1:t0: bit T
+    uint32_t ad = (uint32_t)__cvta_generic_to_shared(recA);
+    const uint32_t bd = (uint32_t)__cvta_generic_to_shared(recB) - ad;
+    const uint32_t cd = (uint32_t)__cvta_generic_to_shared(sCP);
+#pragma unroll
+    for (uint32_t h = 0; h < 2; h++) {
+      const uint32_t ce = a.cnt > 32 * h ? min(32u, a.cnt - 32 * h) : 0u;
+      for (uint32_t c = 0; c < ce && stop == a.cnt; c++) {
+        bool miss = false;
+        uint32_t cm = 1u << c;
+        // Paulis whose pivot is in the window
+#pragma unroll 1
+        for (; c < ce; c++, cm <<= 1) {
+          const uint32_t c0 = (wd[0][h] & cm) ? lane : NONE, c1 = (wd[1][h] & cm) ? 32 + lane : NONE,
+                         c2 = (wd[2][h] & cm) ? 64 + lane : NONE;
+          const uint32_t best = min(min(c0, c1), c2), m = __reduce_min_sync(0xFFFFFFFFu, best);
+          if (m == NONE) { miss = true; break; }
+          const bool y1 = c1 == best, y2 = c2 == best;
+          uint32_t s[4];
+#pragma unroll
+          for (uint32_t q = 0; q < 4; q++) s[q] = y2 ? wd[2][q] : (y1 ? wd[1][q] : wd[0][q]);
+          const uint32_t sr = y2 ? src[2] : (y1 ? src[1] : src[0]);
+          asm volatile("{.reg .pred p; setp.eq.u32 p, %0, %1; @p st.shared.v4.u32 [%2], {%3, %4, %5, %6};"
+                       "@p st.shared.v4.u32 [%7], {%1, %8, %9, %9};}" ::"r"(best), "r"(m), "r"(ad), "r"(s[0]), "r"(s[1]),
+                       "r"(s[2] | t0), "r"(s[3] | t1), "r"(ad + bd), "r"(32 * h + c), "r"(sr)
+                       : "memory");
+          __syncwarp();
+          uint32_t p[4], n0, n1;
+          asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(p[0]), "=r"(p[1]), "=r"(p[2]), "=r"(p[3]) : "r"(ad) : "memory");
+          asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(n0), "=r"(n1) : "r"(cd + 8 * (32 * h + c)) : "memory");
+          ad += 16;
+#pragma unroll
+          for (uint32_t k = 0; k < KW; k++) {
+            xor_if(wd[k], wd[k][h], cm, p);
+            if (32 * k + lane == m) {  // the Pauli takes the pivot's place
+              wd[k][0] = n0;
+              wd[k][1] = n1;
+              wd[k][2] = wd[k][3] = 0;
+              src[k] = T;
+            }
+          }
+          T++;
+          t1 = (t1 << 1) | (t0 >> 31);
+          t0 <<= 1;
+        }
+        if (!miss) break;
+        uint32_t m = NONE;
+        if (nrest) {
+          if (lane == 0) { rb = 32 * h + c; rT = T; }
+          __syncwarp();
+          asm volatile("bar.sync 1, %0;" ::"r"(nbar) : "memory");
+          asm volatile("bar.sync 2, %0;" ::"r"(nbar) : "memory");
+          const uint32_t v = lane >= 1 && lane <= nbw ? rpos[lane] : NONE;
+          m = __reduce_min_sync(0xFFFFFFFFu, v);
+          if (m != NONE && v == m) {
+            recA[T] = make_uint4((uint32_t)rw[lane], (uint32_t)(rw[lane] >> 32), (uint32_t)ra[lane] | t0,
+                                 (uint32_t)(ra[lane] >> 32) | t1);
+            recB[T] = make_uint4(m, 32 * h + c, rs[lane], 0);
+          }
+        }
+        if (m == NONE) {  // commutes with every stabilizer row
+          if (!a.skip) stop = 32 * h + c;
+          continue;
+        }
+        __syncwarp();  // no row of the window has the bit
+        ad += 16;
+        T++;
+        t1 = (t1 << 1) | (t0 >> 31);
+        t0 <<= 1;
+      }
+    }
+    if (lane == 0) { shT = T; shB = stop; rb = NONE; }
+    __syncwarp();
+    if (nrest) asm volatile("bar.sync 1, %0;" ::"r"(nbar) : "memory");
+  } else if (warp <= nbw) {
+    const uint32_t r0 = PP_WINDOW + tid - 32;
+    uint32_t t = 0;
+    while (true) {
+      asm volatile("bar.sync 1, %0;" ::"r"(nbar) : "memory");
+      const uint32_t b = rb, T = rT;
+      if (b == NONE) break;
+      for (; t < T; t++) {
+        const uint4 e = recA[t], f = recB[t];
+        const uint64_t pw = (uint64_t)e.x | ((uint64_t)e.y << 32), pA = (uint64_t)e.z | ((uint64_t)e.w << 32);
+        const uint2 n = sCP[f.y];
+#pragma unroll
+        for (uint32_t k = 0; k < RPT; k++) {
+          if (k && k * PP_REST >= nrest) break;
+          const uint64_t y = bitmask64(w[k], f.y);
+          w[k] ^= pw & y;
+          A[k] ^= pA & y;
+          if (f.x == r0 + k * PP_REST) {
+            w[k] = (uint64_t)n.x | ((uint64_t)n.y << 32);
+            A[k] = 0;
+            ws[k] = t;
+          }
+        }
+      }
+      uint32_t bp = NONE, bs = 0;
+      uint64_t bw = 0, bA = 0;
+#pragma unroll
+      for (uint32_t k = RPT; k-- > 0;)
+        if ((w[k] >> b) & 1ull) {
+          bp = r0 + k * PP_REST;
+          bw = w[k];
+          bA = A[k];
+          bs = ws[k];
+        }
+      const uint32_t m = __reduce_min_sync(0xFFFFFFFFu, bp);
+      if (lane == 0) rpos[warp] = m;
+      if (bp == m && m != NONE) { rw[warp] = bw; ra[warp] = bA; rs[warp] = bs; }
+      asm volatile("bar.sync 2, %0;" ::"r"(nbar) : "memory");
+    }
+  }
+  __syncthreads();
+  const uint32_t T = shT, done = shB;
+  if (tid < T) {
+    const uint4 e = recA[tid], f = recB[tid];
+    g.stp[tid] = a.nn + f.x;
+    g.bt[tid] = f.y;
+    g.src[tid] = f.z;
+    g.A[tid] = (uint64_t)e.z | ((uint64_t)e.w << 32);
+    g.PW[tid] = (uint64_t)e.x | ((uint64_t)e.y << 32);
+    a.anticom[a.j0 + f.y] = (int32_t)f.x + 1;
+    a.result[a.j0 + f.y] = a.rand_ph ? (int32_t)a.rand_ph[a.j0 + f.y] : -1;
+  }
+  if (tid == 0) {
+    g.T = T;
+    a.state[0] = done < a.cnt;
+    a.state[1] = (int32_t)(a.j0 + done);
+  }
+}
+
+// q of the stabilizer row that Pauli b of the panel becomes.
+__device__ __forceinline__ uint32_t new_row_q(const ProjPanelArgs& a, uint32_t b) {
+  return (a.pq[b] + (a.rand_ph ? a.rand_ph[a.j0 + b] - a.pph[a.j0 + b] : 0u)) & 3u;
+}
+
+// M: blocks 0 .. ntile - 1 a tile each, block ntile the pivots' own sets, the
+// others MID_THREADS rows each.
+__global__ void __launch_bounds__(MID_THREADS) project_mid_kernel(const ProjPanelArgs a) {
+  __shared__ union {
+    TileSmem t;
+    struct {
+      ulonglong2 P[PSTEPS];   // (pivot's word, the Pauli's word)
+      uint2 sb[PSTEPS];       // (pivot row, Pauli)
+    } r;
+  } s;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+  PanelRecord& g = *a.rec;
+  const PanelTiles& p = a.p;
+  const uint32_t tid = threadIdx.x, blk = blockIdx.x, T = g.T;
+  if (blk < p.ntile) {
+    const bool two = 2 * blk + 1 < p.len;
+    // a Pauli's words of the tile as the tiles keep them
+    __shared__ ulonglong2 pw[PSTEPS][2];
+    if (tid < PSTEPS) {
+      const uint32_t sr = g.src[tid];
+      if (tid < T && sr < PSTEPS) {
+        const uint64_t* P = a.paulis + (size_t)(a.j0 + g.bt[sr]) * p.W + 2 * blk;
+        pw[tid][0] = make_ulonglong2(P[0], two ? P[1] : 0ull);
+        pw[tid][1] = make_ulonglong2(P[p.len], two ? P[p.len + 1] : 0ull);
+      }
+    }
+    __syncthreads();
+    tile_reduce(
+        p, g, blk, s.t,
+        [&](uint32_t t, uint32_t r) -> const ulonglong2* {
+          return t < T && g.src[t] < PSTEPS ? pw[t] : p.t + ((size_t)blk * p.rows + r) * 2;
+        },
+        [&](uint32_t t, uint32_t r) -> uint32_t {
+          const uint32_t sr = g.src[t];
+          if (sr < PSTEPS) return blk == 0 ? new_row_q(a, g.bt[sr]) : 0u;
+          return 2u * p.par[(size_t)blk * p.rows + r] + (blk == 0 ? p.q[r] : 0u);
+        },
+        [&](uint32_t t, const uint64_t* v) {
+          const uint32_t c = (uint32_t)(__popcll(v[0] & v[2]) + __popcll(v[1] & v[3]));
+          if (c) atomicAdd(&g.s[t], c);
+        });
+    return;
+  }
+  if (tid < PSTEPS) {
+    const bool in = tid < T;
+    const uint32_t b = in ? g.bt[tid] : 0u;
+    s.r.P[tid] = make_ulonglong2(in ? g.PW[tid] : 0ull, a.CP[b]);
+    s.r.sb[tid] = make_uint2(in ? g.stp[tid] : 0xFFFFFFFFu, b);
+  }
+  __syncthreads();
+  if (blk == p.ntile) {
+    if (tid < PSTEPS) { a.CPn[tid] = 0; a.pqn[tid] = 0; }
+    // pivot t's start word replayed up to its step
+    if (tid < T) {
+      const uint32_t sr = g.src[tid];
+      uint64_t w = sr < PSTEPS ? s.r.P[sr].y : a.word[s.r.sb[tid].x], U = 0;
+      for (uint32_t t = sr < PSTEPS ? sr + 1 : 0; t < tid; t++) {
+        const uint64_t y = bitmask64(w, s.r.sb[t].y);
+        w ^= s.r.P[t].x & y;
+        U |= (1ull << t) & y;
+      }
+      g.own[tid] = U;
+    }
+    return;
+  }
+  const uint32_t r = (blk - p.ntile - 1) * MID_THREADS + tid;
+  if (r >= p.rows) return;
+  a.wordn[r] = 0;
+  uint64_t w = a.word[r], U = 0;
+  uint32_t base = BASE_ROW;
+  const uint32_t partner = r < a.nn ? r + a.nn : 0xFFFFFFFEu;  // its stabilizer row
+#pragma unroll 4
+  for (uint32_t t = 0; t < T; t++) {
+    const ulonglong2 P = s.r.P[t];
+    const uint2 sb = s.r.sb[t];
+    const uint64_t y = bitmask64(w, sb.y), tb = 1ull << t;
+    w ^= P.x & y;
+    U |= tb & y;
+    if (sb.x == r) {  // the Pauli takes its place
+      w = P.y;
+      U = 0;
+      base = sb.y;
+    } else if (sb.x == partner) {  // a copy of the pivot
+      w = P.x;
+      U = tb;
+      base = BASE_NONE;
+    }
+  }
+  p.U[r] = U;
+  a.base[r] = (uint8_t)base;
+}
+
+// The byte tables of the next panel's Paulis on one tile: tab[b][v] is the
+// XOR, over the bits of v, of the Paulis that anticommute with that bit of
+// byte b of a row's words (x, x, z, z).
+struct FlagSmem {
+  uint64_t col[256];
+  uint64_t tab4[64][16];
+  uint64_t tab[32][256];
+};
+
+__device__ __forceinline__ void flag_tables(const ProjPanelArgs& a, uint32_t tile, FlagSmem& s) {
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const PanelTiles& p = a.p;
+  {  // word k of the row (x0, x1, z0, z1) against word k ^ 2 of the Paulis; 32 warps, 8 bits each
+    const uint32_t k = warp >> 3, q = k ^ 2, c = 2 * tile + (q & 1);
+    const bool in = c < p.len;
+    const uint64_t* P = a.paulis + (size_t)a.jn * p.W + (q >= 2 ? p.len : 0) + c;
+    const uint64_t v0 = in && lane < a.cntn ? P[(size_t)lane * p.W] : 0ull;
+    const uint64_t v1 = in && lane + 32 < a.cntn ? P[(size_t)(lane + 32) * p.W] : 0ull;
+    for (uint32_t b = 8 * (warp & 7), e = b + 8; b < e; b++) {
+      const uint32_t lo = __ballot_sync(0xFFFFFFFFu, (v0 >> b) & 1ull), hi = __ballot_sync(0xFFFFFFFFu, (v1 >> b) & 1ull);
+      if (lane == 0) s.col[64 * k + b] = (uint64_t)lo | ((uint64_t)hi << 32);
+    }
+  }
+  __syncthreads();
+  {
+    const uint32_t k = tid >> 4, v = tid & 15;
+    uint64_t x = 0;
+#pragma unroll
+    for (uint32_t b = 0; b < 4; b++) x ^= s.col[4 * k + b] & bitmask64(v, b);
+    s.tab4[k][v] = x;
+  }
+  __syncthreads();
+#pragma unroll 4
+  for (uint32_t e = tid; e < 8192; e += 1024) {
+    const uint32_t k = e >> 8, v = e & 255;
+    s.tab[k][v] = s.tab4[2 * k][v & 15] ^ s.tab4[2 * k + 1][v >> 4];
+  }
+  __syncthreads();
+}
+
+__device__ __forceinline__ uint64_t flag_lookup(const FlagSmem& s, ulonglong2 x, ulonglong2 z) {
+  const uint64_t v[4] = {x.x, x.y, z.x, z.y};
+  uint64_t f = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < 4; k++)
+#pragma unroll
+    for (uint32_t b = 0; b < 8; b++) f ^= s.tab[8 * k + b][(uint32_t)(v[k] >> (8 * b)) & 255u];
+  return f;
+}
+
+struct ApplyFlagSmem {
+  ApplySmem a;
+  FlagSmem f;
+};
+
+// AF.
+__global__ void __launch_bounds__(1024) project_apply_kernel(const ProjPanelArgs a) {
+  extern __shared__ __align__(16) uint8_t dsm[];
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+  const PanelRecord& g = *a.rec;
+  const PanelTiles& p = a.p;
+  const uint32_t tid = threadIdx.x, blk = blockIdx.x, T = a.apply ? g.T : 0u;
+  if (blk < a.nq) {  // q of every row
+    if (!T) return;
+    PhaseSmem& s = *(PhaseSmem*)dsm;
+    phase_data(g, s, [&](uint32_t t) { return g.own[t]; });
+    for (uint32_t r = blk * blockDim.x + tid; r < p.rows; r += a.nq * blockDim.x) {
+      const uint64_t U = p.U[r];
+      const uint32_t base = a.base[r];
+      if (r < a.plain) {
+        // a destabilizer row: products keep its phase, a copy brings the pivot's
+        if (base == BASE_NONE) {
+          const uint32_t t = __ffsll((long long)U) - 1;
+          p.q[r] = (uint8_t)(((uint32_t)((s.Q1 >> t) & 1ull) + 2u * (uint32_t)((s.Q2 >> t) & 1ull) - g.s[t]) & 3u);
+        }
+      } else if (base != BASE_ROW || U) {
+        const uint32_t q = base != BASE_ROW ? new_row_q(a, base) : p.q[r];
+        p.q[r] = (uint8_t)((q + phase_of(s, U)) & 3u);
+      }
+    }
+    return;
+  }
+  const bool next = a.cntn && !a.state[0];
+  if (!T && !next) return;
+  const uint32_t u = blk - a.nq, tile = u / a.groups, grp = u - tile * a.groups;
+  ApplyFlagSmem& s = *(ApplyFlagSmem*)dsm;
+  if (T) apply_tables(p, tile, s.a);
+  if (next) flag_tables(a, tile, s.f);
+  const bool two = 2 * tile + 1 < p.len;
+  auto pauli = [&](uint32_t j, ulonglong2& x, ulonglong2& z) {
+    const uint64_t* P = a.paulis + (size_t)j * p.W + 2 * tile;
+    x = make_ulonglong2(P[0], two ? P[1] : 0ull);
+    z = make_ulonglong2(P[p.len], two ? P[p.len + 1] : 0ull);
+  };
+  const uint32_t r1 = min(p.rows, (grp + 1) * a.per);
+  for (uint32_t r = grp * a.per + tid; r < r1; r += blockDim.x) {
+    ulonglong2* d = p.t + ((size_t)tile * p.rows + r) * 2;
+    ulonglong2 x = d[0], z = d[1];
+    if (T) {
+      const uint64_t U = p.U[r];
+      const uint32_t base = a.base[r];
+      if (base == BASE_NONE) x = z = make_ulonglong2(0, 0);
+      else if (base != BASE_ROW) pauli(a.j0 + base, x, z);
+      if (U || base != BASE_ROW) {
+        ulonglong2 mx, mz;
+        apply_lookup(s.a, U, mx, mz);
+        const uint32_t odd = parity64((mz.x & x.x) ^ (mz.y & x.y));
+        x = xor128(x, mx);
+        z = xor128(z, mz);
+        d[0] = x;
+        d[1] = z;
+        if (r >= a.plain) {
+          uint8_t* par = p.par + (size_t)tile * p.rows + r;
+          if (base != BASE_ROW) *par = (uint8_t)odd;
+          else if (odd) *par ^= 1u;
+        }
+      }
+    }
+    if (next) {
+      const uint64_t f = flag_lookup(s.f, x, z);
+      if (f) atomicXor((unsigned long long*)a.wordn + r, (unsigned long long)f);
+    }
+  }
+  if (next && grp == 0 && tid < a.cntn) {  // the next Paulis' own words and q
+    ulonglong2 x, z;
+    pauli(a.jn + tid, x, z);
+    const uint64_t f = flag_lookup(s.f, x, z);
+    if (f) atomicXor(a.CPn + tid, (unsigned long long)f);
+    const uint32_t q = (uint32_t)(__popcll(x.x & z.x) + __popcll(x.y & z.y)) + (tile == 0 ? a.pph[a.jn + tid] : 0u);
+    if (q) atomicAdd(a.pqn + tid, q);
+  }
+}
+
+// The rows into the tiles, and back (a warp a row).
+__global__ void __launch_bounds__(256) project_load_kernel(const ProjPanelArgs a) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+  const uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (blockIdx.x == 0) {
+    for (uint32_t k = threadIdx.x; k < sizeof(PanelRecord) / 4; k += blockDim.x) ((uint32_t*)a.rec)[k] = 0;
+    if (threadIdx.x < PSTEPS) { a.CPn[threadIdx.x] = 0; a.pqn[threadIdx.x] = 0; }
+    if (threadIdx.x == 0) { a.state[0] = 0; a.state[1] = (int32_t)a.jn; }
+  }
+  if (r >= a.p.rows) return;
+  const uint32_t ph = a.ph[r];
+  tiles_load_row(a.p, a.xzs + (size_t)r * a.p.W, r, ph, lane);
+  if (lane == 0) {
+    a.wordn[r] = 0;
+    if (r < a.plain) a.p.q[r] = (uint8_t)ph;
+  }
+}
+
+__global__ void __launch_bounds__(256) project_store_kernel(const ProjPanelArgs a) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+  const uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (r >= a.p.rows) return;
+  const uint32_t ph = tiles_store_row(a.p, a.xzs + (size_t)r * a.p.W, r, lane);
+  if (lane == 0) a.ph[r] = r < a.plain ? a.p.q[r] : (uint8_t)ph;
+}
+
+// A launch as a programmatic dependent of the one before it on the stream.
+static cudaError_t launch_pp(void (*k)(const ProjPanelArgs), uint32_t grid, uint32_t block, size_t smem, cudaStream_t st,
+                             const ProjPanelArgs& a) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return cudaLaunchKernelEx(&cfg, k, a);
+}
+
+// Runs worth a panel (a panel costs about as much as 10 to 15 Paulis of the
+// other kernels; 32 Paulis on 100 / 1000 / 4000 qubits 205 / 241 / 486 -> 181 /
+// 177 / 136 us with the call), the most stabilizer rows its search holds in
+// registers, and the steps a run has to make before the next is tried at once.
+constexpr uint32_t PROJ_PANEL_MIN = 32, PROJ_PANEL_ROWS = PP_WINDOW + 9 * PP_REST, PROJ_PANEL_GOOD = 32;
+
+// Projections [*j, k) by panels until one that commutes with the stabilizer
+// (or all are done); *j gets the next.  The first panel's steps are waited
+// for: when they end at once nothing else is launched.
+static int project_panels(const qcb_tableau* t, int kind, uint32_t rank, const uint64_t* pxzs, const uint8_t* pph,
+                          const uint8_t* d_rand, uint32_t* j, uint32_t k, int skip, int32_t* d_anti, int32_t* d_res,
+                          cudaStream_t st) {
+  const bool destab = kind == QCB_DESTABILIZER || kind == QCB_MIXED_DESTABILIZER;
+  const uint32_t R = destab ? t->rows : rank, W = t->W, len = W / 2, ntile = (len + 1) / 2;
+  size_t bytes = 0;
+  auto place = [&](size_t n) { const size_t o = bytes; bytes += (n + 127) / 128 * 128; return o; };
+  const size_t o_t = place((size_t)ntile * R * 32), o_po = place((size_t)ntile * PSTEPS * 32),
+               o_w = place((size_t)2 * R * 8), o_u = place((size_t)R * 8), o_q = place(R), o_b = place(R),
+               o_par = place((size_t)ntile * R), o_rec = place(sizeof(PanelRecord)), o_cp = place(2 * PSTEPS * 8),
+               o_pq = place(2 * PSTEPS * 4), o_st = place(8);
+  uint8_t* m = nullptr;
+  QCB_CUDA(cudaMallocAsync(&m, bytes, st));
+  ProjPanelArgs a{};
+  a.p = PanelTiles{R, W, len, ntile, 1, (ulonglong2*)(m + o_t), (ulonglong2*)(m + o_po), nullptr, (uint64_t*)(m + o_u),
+                   m + o_q, m + o_par};
+  a.xzs = t->xzs; a.ph = t->phases; a.nn = destab ? t->rows / 2 : 0; a.rank = rank; a.plain = destab ? rank : 0;
+  a.skip = skip; a.paulis = pxzs; a.pph = pph; a.rand_ph = d_rand; a.rec = (PanelRecord*)(m + o_rec);
+  a.state = (int32_t*)(m + o_st); a.anticom = d_anti; a.result = d_res; a.base = m + o_b;
+  uint64_t* word = (uint64_t*)(m + o_w);
+  unsigned long long* CP = (unsigned long long*)(m + o_cp);
+  uint32_t* pq = (uint32_t*)(m + o_pq);
+  auto buffers = [&](uint32_t b) {  // panel b's words and Paulis, and the next one's
+    a.word = word + (size_t)(b & 1) * R; a.wordn = word + (size_t)((b + 1) & 1) * R;
+    a.CP = CP + (b & 1) * PSTEPS; a.CPn = CP + ((b + 1) & 1) * PSTEPS;
+    a.pq = pq + (b & 1) * PSTEPS; a.pqn = pq + ((b + 1) & 1) * PSTEPS;
+  };
+  const uint32_t rest = rank > PP_WINDOW ? rank - PP_WINDOW : 0;
+  void (*steps)(const ProjPanelArgs) = rest <= PP_REST ? project_steps_kernel<1>
+                                     : rest <= 2 * PP_REST ? project_steps_kernel<2>
+                                     : rest <= 5 * PP_REST ? project_steps_kernel<5> : project_steps_kernel<9>;
+  const size_t smem = std::max(sizeof(ApplyFlagSmem), sizeof(PhaseSmem));
+  QCB_CUDA(cudaFuncSetAttribute(project_apply_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const uint32_t nsm = (uint32_t)std::max(device_sm_count(), 1);
+  a.nq = (R + 1023) / 1024;
+  a.groups = std::max<uint32_t>(1, std::min<uint32_t>((nsm > a.nq ? nsm - a.nq : 1) / ntile, (R + 255) / 256));
+  a.per = (R + a.groups - 1) / a.groups;
+  const uint32_t row_blocks = (R + 7) / 8, first = *j;
+  int32_t h[2] = {0, 0};
+  int s = QCB_OK;
+  auto go = [&]() -> int {
+    buffers(1);  // the first panel's are panel 1's next
+    a.j0 = a.jn = first; a.cnt = 0; a.cntn = std::min(PSTEPS, k - first); a.apply = 0;
+    QCB_CUDA(launch_pp(project_load_kernel, row_blocks, 256, 0, st, a));
+    QCB_CUDA(launch_pp(project_apply_kernel, a.nq + ntile * a.groups, 1024, smem, st, a));
+    a.apply = 1;
+    for (uint32_t b = 0, j0 = first; j0 < k; b++, j0 += PSTEPS) {
+      buffers(b);
+      a.j0 = j0; a.cnt = std::min(PSTEPS, k - j0);
+      a.jn = j0 + a.cnt; a.cntn = std::min(PSTEPS, k - a.jn);
+      QCB_CUDA(launch_pp(steps, 1, 1024, 0, st, a));
+      if (b == 0) {
+        QCB_CUDA(cudaMemcpyAsync(h, a.state, 8, cudaMemcpyDeviceToHost, st));
+        QCB_CUDA(cudaStreamSynchronize(st));
+        if (h[0] && (uint32_t)h[1] == first) return QCB_OK;  // the tableau is as it was
+      }
+      QCB_CUDA(launch_pp(project_mid_kernel, ntile + 1 + (R + MID_THREADS - 1) / MID_THREADS, MID_THREADS, 0, st, a));
+      QCB_CUDA(launch_pp(project_apply_kernel, a.nq + ntile * a.groups, 1024, smem, st, a));
+      if (b == 0 && h[0]) break;
+    }
+    QCB_CUDA(launch_pp(project_store_kernel, row_blocks, 256, 0, st, a));
+    QCB_CUDA(cudaMemcpyAsync(h, a.state, 8, cudaMemcpyDeviceToHost, st));
+    QCB_CUDA(cudaStreamSynchronize(st));
+    return QCB_OK;
+  };
+  s = go();
+  cudaFreeAsync(m, st);
+  if (s == QCB_OK) *j = (uint32_t)h[1];
+  return s;
+}
+
 static uint32_t g_proj_cs = 0;  // tuner override (0 = automatic)
 static uint32_t g_proj_grid = 0;  // the whole-GPU kernel: 0 automatic, 1 always (where it applies), 2 never
 static uint32_t g_proj_withhold = 0;  // test knob, see ProjGridArgs::withhold
@@ -869,11 +1460,44 @@ static int project_impl(qcb_tableau* t, int kind, int32_t* rank_io, const uint64
   int status = QCB_OK;
   uint32_t j0 = 0;
   std::vector<int32_t> h_anti(k, 0), h_res(k, -1);
+  // runs of generic Paulis go by panels (the tuner's choices of the other
+  // kernels turn them off); a run that ends early leaves the next Paulis to
+  // the kernels below, more of them each time
+  const bool destab = kind == QCB_DESTABILIZER || kind == QCB_MIXED_DESTABILIZER;
+  const bool panels = !qubits && phases && len && !g_proj_grid && !g_proj_cs;
+  const int skip = !keep_result && (kind == QCB_STABILIZER || (kind == QCB_DESTABILIZER && t->rows / 2 == t->nqubits));
+  uint32_t next_try = 0, backoff = 32;
+  if (panels) {
+    QCB_CUDA(cudaMemsetAsync(d_anti, 0, (size_t)k * 4, st));
+    QCB_CUDA(cudaMemsetAsync(d_res, 0xFF, (size_t)k * 4, st));
+  }
   while (j0 < k) {
+    uint32_t kend = k;
+    if (panels && k - j0 >= PROJ_PANEL_MIN && j0 >= next_try) {
+      int32_t r_now = rank;
+      if (mixed && j0) {
+        QCB_CUDA(cudaMemcpyAsync(&r_now, d_rank, 4, cudaMemcpyDeviceToHost, st));
+        QCB_CUDA(cudaStreamSynchronize(st));
+      }
+      const uint32_t nr = kind == QCB_STABILIZER ? t->rows : kind == QCB_DESTABILIZER ? t->rows / 2 : (uint32_t)r_now;
+      if (nr && nr <= PROJ_PANEL_ROWS) {
+        const uint32_t at = j0;
+        if ((status = project_panels(t, kind, nr, pxzs, pph, d_rand, &j0, k, skip, d_anti, d_res, st))) break;
+        if (j0 >= k) break;
+        if (j0 - at >= PROJ_PANEL_GOOD) {
+          backoff = 32;
+          next_try = j0 + 1;
+        } else {
+          backoff = std::min<uint32_t>(backoff * 2, 1u << 20);
+          next_try = j0 + backoff;
+        }
+        if (destab || next_try > j0 + 1) kend = std::min(k, next_try);
+      }
+    }
     ProjArgs a{};
     a.xzs = t->xzs; a.ph = t->phases; a.rows = t->rows; a.n = t->nqubits; a.W = t->W;
     a.kind = kind; a.rank = d_rank; a.paulis = pxzs; a.pph = pph;
-    a.j0 = j0; a.k = k; a.keep_result = keep_result; a.phases = phases;
+    a.j0 = j0; a.k = kend; a.keep_result = keep_result; a.phases = phases;
     a.anticom = d_anti; a.result = d_res; a.status = d_stat; a.flags = d_flags;
     a.qubits = d_q; a.basis = basis; a.rand_ph = d_rand;
     cudaLaunchConfig_t cfg{};
@@ -913,7 +1537,10 @@ static int project_impl(qcb_tableau* t, int kind, int32_t* rank_io, const uint64
       status = fail(QCB_ETIMEOUT, "project!: a grid barrier wait of the whole-GPU kernel expired");
       break;
     }
-    if (hs[0] == PST_OK) break;
+    if (hs[0] == PST_OK) {
+      j0 = kend;
+      continue;
+    }
     const uint32_t j = (uint32_t)hs[1];
     if (hs[0] == PST_BADSTRUCT) {
       status = fail(QCB_EBADSTRUCT,

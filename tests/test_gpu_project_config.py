@@ -93,3 +93,73 @@ def test_project_after_a_commuting_pauli_in_the_cluster_kernel(qcb):
         outs.append((a, None if v < 0 else v))
     assert list(zip(anti, res)) == outs
     assert np.array_equal(st.tab.xzs, xz) and np.array_equal(st.tab.phases, ph)
+
+
+@pytest.mark.parametrize("kind", ["Stabilizer", "MixedStabilizer", "Destabilizer", "MixedDestabilizer"])
+@pytest.mark.parametrize("n,k,commuting", [(7, 64, ()), (64, 33, ()), (96, 130, (100,)), (97, 64, (63,)), (130, 200, (70, 71, 140)),
+                                           (1088, 65, ()), (1100, 130, (0, 64))])
+def test_project_by_panels(qcb, kind, n, k, commuting):
+    """Runs of Paulis by panels: ragged panels, views around the search's
+    window and rows per thread, Paulis that commute in between (repeats of the
+    one before, or a stabilizer row), low ranks with logical operators, and
+    without a result; against the oracle."""
+    rng = np.random.default_rng(n + k)
+    d = randoms.random_destabilizer(n, rng)
+    ps = randoms.random_paulis(k, n, rng, phases=True)
+    for j in commuting:
+        src = (ps.xzs[j - 1], ps.phases[j - 1]) if j else (d.tab.xzs[n], d.tab.phases[n])
+        ps.xzs[j], ps.phases[j] = src
+    rank = 0
+    if kind in ("Stabilizer", "MixedStabilizer"):
+        tab = Tableau(d.tab.phases[n:].copy(), n, d.tab.xzs[n:].copy())
+        if kind == "MixedStabilizer":
+            rank = max(1, n - n // 8)
+            tab.xzs[rank:], tab.phases[rank:] = 0, 0
+    else:
+        tab = d.tab
+        rank = n - n // 4 if kind == "MixedDestabilizer" else 0
+    for keep in (True, False):
+        st = getattr(qcb, kind)(tab.copy(), rank if kind.startswith("Mixed") else None).to_gpu()
+        _, anti, res = qcb.project_(st, ps.copy().to_gpu(), keep_result=keep)
+        st.to_cpu()
+        ph, xz, r, outs = tab.phases.copy(), tab.xzs.copy(), rank, []
+        for j in range(k):
+            code, ph, xz, r, a, v = oracle.project(kind, ph, xz, n, ps.xzs[j], ps.phases[j], r, keep, True)
+            assert code == 0
+            outs.append((a, None if v < 0 else v))
+        assert list(zip(anti, res)) == outs
+        assert np.array_equal(st.tab.xzs, xz) and np.array_equal(st.tab.phases, ph)
+        if kind.startswith("Mixed"):
+            assert st.rank == r
+
+
+@pytest.mark.parametrize("kind", ["Stabilizer", "Destabilizer", "MixedDestabilizer"])
+def test_projectrand_by_panels(qcb, kind):
+    """The random signs of projectrand! in a run by panels equal those of one
+    call per Pauli (the other kernels) with the same draws."""
+    n, k = 150, 100
+    rng = np.random.default_rng(11)
+    d = randoms.random_destabilizer(n, rng)
+    ps = randoms.random_paulis(k, n, rng, phases=True)
+    ps.xzs[80], ps.phases[80] = ps.xzs[79], ps.phases[79]
+    tab = d.tab if kind != "Stabilizer" else Tableau(d.tab.phases[n:].copy(), n, d.tab.xzs[n:].copy())
+    rank = n - 9 if kind == "MixedDestabilizer" else None
+    a = getattr(qcb, kind)(tab.copy(), rank).to_gpu()
+    b = getattr(qcb, kind)(tab.copy(), rank).to_gpu()
+    _, ra = qcb.projectrand_(a, ps.copy().to_gpu(), rng=np.random.default_rng(3))
+    draws = 2 * np.random.default_rng(3).integers(0, 2, size=k)
+
+    class Draw:
+        def __init__(self, v):
+            self.v = v
+
+        def integers(self, lo, hi, size):
+            return np.array([self.v // 2])
+
+    rb = []
+    for j in range(k):
+        p = qcb.PauliOperator(ps.phases[j:j + 1].copy(), n, ps.xzs[j:j + 1].copy()).to_gpu()
+        rb.append(qcb.projectrand_(b, p, rng=Draw(int(draws[j])))[1])
+    a.to_cpu()
+    b.to_cpu()
+    assert ra == rb and a == b
