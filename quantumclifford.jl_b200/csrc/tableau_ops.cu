@@ -460,156 +460,261 @@ __global__ void __launch_bounds__(512) apply_layers_kernel(uint64_t* xzs, uint8_
 }
 
 // ---------------------------------------------------------- dense apply!
-// One warp per state row.  The ordered product over qubits of the Clifford's
-// images (src/dense_cliffords.jl:152-169) is accumulated in registers; the
-// phase counters run across all the multiplications (each multiplication adds
-// +-1 per anticommuting lane, independent of the current counter value), so
-// one reduction at the end gives the exact total.
-template <int MAXW>
-__global__ void __launch_bounds__(256) apply_dense_kernel(uint64_t* xzs, uint8_t* ph, uint32_t rows,
-                                                          uint32_t W, uint32_t n,
-                                                          const uint64_t* __restrict__ c,
-                                                          const uint8_t* __restrict__ cph,
-                                                          int phases) {
+// Tableaux of fewer than DENSE_TABLES_MIN_N qubits (one word per half), a warp
+// per state row: the ordered product over qubits of the Clifford's images
+// (src/dense_cliffords.jl:152-169) in registers; the phase counters run across
+// all the multiplications (each adds +-1 per anticommuting lane, independent
+// of the current counter value), so one reduction gives the exact total.
+__global__ void __launch_bounds__(256) apply_dense_kernel(uint64_t* xzs, uint8_t* ph, uint32_t rows, uint32_t W,
+                                                          uint32_t n, const uint64_t* __restrict__ c,
+                                                          const uint8_t* __restrict__ cph, int phases) {
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= rows) return;
-  const uint32_t len = W / 2;
-  constexpr int PER = (MAXW / 2 + 31) / 32;  // words per lane per half
-  uint64_t bx[PER], bz[PER], c1[PER], c2[PER];
-#pragma unroll
-  for (int k = 0; k < PER; k++) { bx[k] = bz[k] = c1[k] = c2[k] = 0; }
+  uint64_t bx = 0, bz = 0, c1 = 0, c2 = 0;
   uint64_t* row = xzs + (uint64_t)warp * W;
+  const uint64_t xw = W ? row[0] : 0ull, zw = W ? row[1] : 0ull;  // broadcast loads
   uint32_t extra = 0;  // sum of Clifford-row phases and -1 corrections (mod 4)
-  for (uint32_t wq = 0; wq < len; wq++) {
-    const uint64_t xw = row[wq], zw = row[len + wq];  // broadcast loads
-    uint64_t both = xw | zw;
-    while (both) {
-      const uint32_t b = __ffsll((long long)both) - 1;
-      both &= both - 1;
-      const uint32_t q = wq * 64 + b;
-      if (q >= n) break;
-      const bool x = (xw >> b) & 1, z = (zw >> b) & 1;
-      if (x && z) extra += 3;  // phase -= 1
-      if (x) {
-        const uint64_t* cr = c + (uint64_t)q * W;
-#pragma unroll
-        for (int k = 0; k < PER; k++) {
-          const uint32_t w = lane + 32 * k;
-          if (w < len) mul_step<uint64_t>(__ldg(cr + w), __ldg(cr + len + w), bx[k], bz[k], c1[k], c2[k]);
-        }
-        extra += cph[q];
-      }
-      if (z) {
-        const uint64_t* cr = c + (uint64_t)(q + n) * W;
-#pragma unroll
-        for (int k = 0; k < PER; k++) {
-          const uint32_t w = lane + 32 * k;
-          if (w < len) mul_step<uint64_t>(__ldg(cr + w), __ldg(cr + len + w), bx[k], bz[k], c1[k], c2[k]);
-        }
-        extra += cph[q + n];
-      }
+  uint64_t both = xw | zw;
+  while (both) {
+    const uint32_t q = __ffsll((long long)both) - 1;
+    both &= both - 1;
+    if (q >= n) break;
+    const bool x = (xw >> q) & 1, z = (zw >> q) & 1;
+    if (x && z) extra += 3;  // phase -= 1
+    if (x) {
+      const uint64_t* cr = c + (uint64_t)q * W;
+      mul_step<uint64_t>(__ldg(cr), __ldg(cr + 1), bx, bz, c1, c2);
+      extra += cph[q];
+    }
+    if (z) {
+      const uint64_t* cr = c + (uint64_t)(q + n) * W;
+      mul_step<uint64_t>(__ldg(cr), __ldg(cr + 1), bx, bz, c1, c2);
+      extra += cph[q + n];
     }
   }
-  uint32_t s = 0;
-#pragma unroll
-  for (int k = 0; k < PER; k++) s += cnt_phase(c1[k], c2[k]);
-  s = __reduce_add_sync(0xFFFFFFFFu, s & 3u) & 3u;
   __syncwarp();
-#pragma unroll
-  for (int k = 0; k < PER; k++) {
-    const uint32_t w = lane + 32 * k;
-    if (w < len) { row[w] = bx[k]; row[len + w] = bz[k]; }
+  if (lane == 0) {
+    if (W) { row[0] = bx; row[1] = bz; }
+    ph[warp] = phases ? (uint8_t)((cnt_phase(c1, c2) + extra + ph[warp]) & 3u) : (uint8_t)0;
   }
-  if (lane == 0) ph[warp] = phases ? (uint8_t)((s + extra + ph[warp]) & 3u) : (uint8_t)0;
 }
 
-// The same product split over G warps per state row (one row per CTA): warp g
-// multiplies the Clifford rows of its share of the qubit words in order into
-// a partial product (bits, counters, phase), and warp 0 then left-multiplies
-// the partials in order.  The Pauli product is associative with exact phases,
-// so P_{G-1} ... P_1 P_0 is the ordered product of all the images, and the
-// row gets G times the warps of the one-warp kernel.
-template <int MAXW, int G>
-__global__ void __launch_bounds__(32 * G) apply_dense_split_kernel(uint64_t* xzs, uint8_t* ph, uint32_t rows,
-                                                                  uint32_t W, uint32_t n,
-                                                                  const uint64_t* __restrict__ c,
-                                                                  const uint8_t* __restrict__ cph, int phases) {
-  __shared__ uint64_t part[G][MAXW];
-  __shared__ uint32_t pph[G];
-  const uint32_t r = blockIdx.x, g = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (r >= rows) return;
-  const uint32_t len = W / 2;
-  constexpr int PER = (MAXW / 2 + 31) / 32;  // words per lane per half
-  uint64_t bx[PER], bz[PER], c1[PER], c2[PER];
+// Dense apply! by tables.  A state row selects up to four of the Clifford rows
+// of two qubits (x_q, z_q, x_q+1, z_q+1, in this order): 16 ordered products,
+// kept in shared memory for a run of qubits, so a row takes one table entry per
+// two qubits instead of up to four images.  Lanes hold the words of a row, so
+// an entry is read without bank conflicts.  With q = phase + |x & z| a product
+// L . R has q_L + q_R + 2 (z_L . x_R): the crossings of the entries with the
+// product so far are XOR-accumulated over all of them and counted once, and
+// the entries' own q (phases, crossings within an entry, -1 for each Y) are a
+// table of the Clifford alone (dense_q_kernel), summed over the row's entries
+// at the end.  The qubits are split into KG runs over CTAs; their partial
+// products are multiplied in order by dense_join_kernel.
+// Bound by shared memory (an entry is len x 16 bytes; about half its rate) and
+// by the instructions around each read.  Rows x qubits, us, against a product
+// of one image at a time with eight warps per row: 500 x 500 36 -> 18.5, 1000 x
+// 1000 122 -> 22, 2000 x 2000 392 -> 94, 4000 x 4000 2150 -> 759, 8000 x 8000
+// 12645 -> 6100, 20000 x 100 190 -> 53.
+struct DenseArgs {
+  uint64_t* xzs;
+  uint8_t* ph;
+  uint32_t rows, W, n;
+  const uint64_t* c;
+  const uint8_t* cph;
+  uint8_t* qt;         // [32 len][16] q of the entries of every two qubits
+  ulonglong2* part;    // [KG][rows][len] partial products (x, z)
+  uint8_t* odd;        // [KG][rows] parity of their crossings
+  uint32_t KG, wpg;    // runs, qubit words per run
+  uint32_t NT;         // tables in shared memory at a time
+  int phases;
+};
+
+// The Clifford row of bit b of an entry (b & 1: second qubit, b & 2: z), or
+// null past the qubits.
+__device__ __forceinline__ const uint64_t* dense_image(const DenseArgs& a, uint32_t pair, uint32_t b, uint32_t& row) {
+  const uint32_t q = 2 * pair + (b & 1);
+  row = q + ((b & 2) ? a.n : 0);
+  return q < a.n ? a.c + (uint64_t)row * a.W : nullptr;
+}
+
+// A warp per two qubits: the q of their 16 entries.
+__global__ void __launch_bounds__(256) dense_q_kernel(const DenseArgs a) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+  const uint32_t pair = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31, len = a.W / 2;
+  if (pair >= 32 * len) return;
+  const uint32_t order[4] = {0, 2, 1, 3};  // entry bits in the order of the product
+  const uint64_t* row[4];
+  uint32_t q[4];
 #pragma unroll
-  for (int k = 0; k < PER; k++) { bx[k] = bz[k] = c1[k] = c2[k] = 0; }
-  uint64_t* row = xzs + (uint64_t)r * W;
-  uint32_t extra = 0;  // Clifford-row phases and the -1 of every Y (mod 4)
-  const uint32_t wq0 = g * len / G, wq1 = (g + 1) * len / G;
-  for (uint32_t wq = wq0; wq < wq1; wq++) {
-    const uint64_t xw = row[wq], zw = row[len + wq];  // broadcast loads
-    uint64_t both = xw | zw;
-    while (both) {
-      const uint32_t b = __ffsll((long long)both) - 1;
-      both &= both - 1;
-      const uint32_t q = wq * 64 + b;
-      if (q >= n) break;
-      const bool x = (xw >> b) & 1, z = (zw >> b) & 1;
-      if (x && z) extra += 3;
-      if (x) {
-        const uint64_t* cr = c + (uint64_t)q * W;
-#pragma unroll
-        for (int k = 0; k < PER; k++) {
-          const uint32_t w = lane + 32 * k;
-          if (w < len) mul_step<uint64_t>(__ldg(cr + w), __ldg(cr + len + w), bx[k], bz[k], c1[k], c2[k]);
-        }
-        extra += cph[q];
-      }
-      if (z) {
-        const uint64_t* cr = c + (uint64_t)(q + n) * W;
-#pragma unroll
-        for (int k = 0; k < PER; k++) {
-          const uint32_t w = lane + 32 * k;
-          if (w < len) mul_step<uint64_t>(__ldg(cr + w), __ldg(cr + len + w), bx[k], bz[k], c1[k], c2[k]);
-        }
-        extra += cph[q + n];
-      }
-    }
+  for (uint32_t i = 0; i < 4; i++) {
+    uint32_t r;
+    row[i] = dense_image(a, pair, order[i], r);
+    q[i] = lane == 0 && row[i] ? a.cph[r] : 0u;
   }
+  uint64_t cr[6] = {0, 0, 0, 0, 0, 0};
+  for (uint32_t w = lane; w < len; w += 32) {
+    uint64_t x[4], z[4];
+#pragma unroll
+    for (uint32_t i = 0; i < 4; i++) {
+      x[i] = row[i] ? __ldg(row[i] + w) : 0ull;
+      z[i] = row[i] ? __ldg(row[i] + len + w) : 0ull;
+      q[i] += __popcll(x[i] & z[i]);
+    }
+    uint32_t k = 0;
+#pragma unroll
+    for (uint32_t i = 1; i < 4; i++)
+#pragma unroll
+      for (uint32_t j = 0; j < i; j++) cr[k++] ^= z[i] & x[j];
+  }
+  uint32_t odd = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < 6; k++) odd |= ((uint32_t)__popcll(cr[k]) & 1u) << k;
+  odd = __reduce_xor_sync(0xFFFFFFFFu, odd);
   uint32_t s = 0;
 #pragma unroll
-  for (int k = 0; k < PER; k++) s += cnt_phase(c1[k], c2[k]);
-  s = __reduce_add_sync(0xFFFFFFFFu, s & 3u) & 3u;
-#pragma unroll
-  for (int k = 0; k < PER; k++) {
-    const uint32_t w = lane + 32 * k;
-    if (w < len) { part[g][w] = bx[k]; part[g][len + w] = bz[k]; }
+  for (uint32_t i = 0; i < 4; i++) {
+    q[i] = __reduce_add_sync(0xFFFFFFFFu, q[i]);
+    if ((lane >> order[i]) & 1u) s += q[i];
   }
-  if (lane == 0) pph[g] = (s + extra) & 3u;
-  __syncthreads();
-  if (g != 0) return;
-  // warp 0: acc = P_0, then acc <- P_g * acc for g = 1 .. G-1
+  uint32_t k = 0;
 #pragma unroll
-  for (int k = 0; k < PER; k++) { c1[k] = c2[k] = 0; }
-  uint32_t tot = pph[0];
-  for (uint32_t h = 1; h < G; h++) {
+  for (uint32_t i = 1; i < 4; i++)
 #pragma unroll
-    for (int k = 0; k < PER; k++) {
-      const uint32_t w = lane + 32 * k;
-      if (w < len) mul_step<uint64_t>(part[h][w], part[h][len + w], bx[k], bz[k], c1[k], c2[k]);
+    for (uint32_t j = 0; j < i; j++, k++)
+      if (((lane >> order[i]) & 1u) && ((lane >> order[j]) & 1u)) s += 2u * ((odd >> k) & 1u);
+  if ((lane & 5) == 5 && row[0]) s += 3;  // Y on the first / second qubit
+  if ((lane & 10) == 10 && row[2]) s += 3;
+  if (lane < 16) a.qt[(size_t)pair * 16 + lane] = (uint8_t)(s & 3u);
+}
+
+// THREADS / 32 warps with 32 / LPR row slots each (LPR lanes), KPL words per
+// lane, RPW rows per slot (their products stay in registers while the tables
+// change).  NT divides 16, so a set of tables lies within half a qubit word;
+// a thread makes the 16 entries of at most one (table, word), its images
+// loaded while the rows take the previous tables.
+template <int THREADS, int LPR, int KPL, int RPW>
+__global__ void __launch_bounds__(THREADS, 1) dense_tables_kernel(const DenseArgs a) {
+  extern __shared__ __align__(16) ulonglong2 tab[];  // [NT][16][len]
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+  const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, len = a.W / 2;
+  const uint32_t kg = blockIdx.x, w0 = kg * a.wpg, w1 = min(len, w0 + a.wpg);
+  const uint32_t sl = lane & (LPR - 1);
+  const uint32_t r0 = ((blockIdx.y * (THREADS / 32) + warp) * (32 / LPR) + lane / LPR) * RPW;
+  const uint32_t mt = tid / len, mw = tid - mt * len;  // the thread's table and word
+  ulonglong2 v[4];
+  auto load = [&](uint32_t p0) {
+#pragma unroll
+    for (uint32_t b = 0; b < 4; b++) {
+      uint32_t r;
+      const uint64_t* im = mt < a.NT ? dense_image(a, p0 + mt, b, r) : nullptr;
+      v[b] = im ? make_ulonglong2(__ldg(im + mw), __ldg(im + len + mw)) : make_ulonglong2(0, 0);
     }
-    tot += pph[h];
-  }
-  s = 0;
+  };
+  uint64_t x[RPW][KPL], z[RPW][KPL], P[RPW];
 #pragma unroll
-  for (int k = 0; k < PER; k++) s += cnt_phase(c1[k], c2[k]);
-  s = __reduce_add_sync(0xFFFFFFFFu, s & 3u) & 3u;
+  for (int i = 0; i < RPW; i++) {
+    P[i] = 0;
 #pragma unroll
-  for (int k = 0; k < PER; k++) {
-    const uint32_t w = lane + 32 * k;
-    if (w < len) { row[w] = bx[k]; row[len + w] = bz[k]; }
+    for (int k = 0; k < KPL; k++) x[i][k] = z[i][k] = 0;
   }
-  if (lane == 0) ph[r] = phases ? (uint8_t)((s + tot + ph[r]) & 3u) : (uint8_t)0;
+  load(32 * w0);
+  for (uint32_t p0 = 32 * w0; p0 < 32 * w1; p0 += a.NT) {
+    // the rows' selector bits: two of the x word and two of the z word per entry
+    uint32_t xs[RPW], zs[RPW];
+#pragma unroll
+    for (int i = 0; i < RPW; i++) {
+      const uint64_t* row = a.xzs + (uint64_t)min(r0 + i, a.rows - 1) * a.W + (p0 >> 5);
+      xs[i] = (uint32_t)(row[0] >> (2 * (p0 & 31)));
+      zs[i] = (uint32_t)(row[len] >> (2 * (p0 & 31)));
+    }
+    __syncthreads();  // the previous tables are read until here
+    if (mt < a.NT) {
+      ulonglong2* d = tab + (size_t)mt * 16 * len + mw;
+#pragma unroll
+      for (uint32_t m = 0; m < 16; m++) {
+        ulonglong2 o = make_ulonglong2(0, 0);
+#pragma unroll
+        for (uint32_t b = 0; b < 4; b++)
+          if ((m >> b) & 1u) { o.x ^= v[b].x; o.y ^= v[b].y; }
+        d[m * len] = o;
+      }
+    }
+    __syncthreads();
+    if (p0 + a.NT < 32 * w1) load(p0 + a.NT);
+    if (r0 < a.rows) {
+#pragma unroll 1
+      for (uint32_t t = 0; t < a.NT; t++) {
+        const ulonglong2* tt = tab + (size_t)t * 16 * len + sl;
+#pragma unroll
+        for (int i = 0; i < RPW; i++) {
+          const uint32_t e = (xs[i] & 3u) | ((zs[i] & 3u) << 2);
+          xs[i] >>= 2;
+          zs[i] >>= 2;
+#pragma unroll
+          for (int k = 0; k < KPL; k++) {
+            if (sl + LPR * k < len) {
+              const ulonglong2 o = tt[e * len + LPR * k];
+              P[i] ^= o.y & x[i][k];
+              x[i][k] ^= o.x;
+              z[i][k] ^= o.y;
+            }
+          }
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < RPW; i++) {
+    uint32_t odd = (uint32_t)__popcll(P[i]);
+#pragma unroll
+    for (int d = LPR / 2; d; d >>= 1) odd += __shfl_xor_sync(0xFFFFFFFFu, odd, d);
+    if (r0 + i >= a.rows) continue;
+    ulonglong2* d = a.part + ((size_t)kg * a.rows + r0 + i) * len;
+#pragma unroll
+    for (int k = 0; k < KPL; k++) {
+      const uint32_t w = sl + LPR * k;
+      if (w < len) d[w] = make_ulonglong2(x[i][k], z[i][k]);
+    }
+    if (sl == 0) a.odd[(size_t)kg * a.rows + r0 + i] = (uint8_t)(odd & 1u);
+  }
+}
+
+// A warp per row: the runs' products multiplied in order, the row's phase.
+__global__ void __launch_bounds__(256) dense_join_kernel(const DenseArgs a) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+  const uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31, len = a.W / 2;
+  if (r >= a.rows) return;
+  uint64_t* row = a.xzs + (uint64_t)r * a.W;
+  uint32_t q = 0;
+  if (a.phases) {
+    // the entries' q: lane = two qubits of each word
+    for (uint32_t w = 0; w < len; w++) {
+      const uint32_t e = ((uint32_t)(row[w] >> (2 * lane)) & 3u) | (((uint32_t)(row[len + w] >> (2 * lane)) & 3u) << 2);
+      q += a.qt[((size_t)w * 32 + lane) * 16 + e];
+    }
+    for (uint32_t g = lane; g < a.KG; g += 32) q += 2u * a.odd[(size_t)g * a.rows + r];
+  }
+  __syncwarp();
+  uint64_t P = 0;
+  for (uint32_t w = lane; w < len; w += 32) {
+    uint64_t x = 0, z = 0;
+#pragma unroll 4
+    for (uint32_t g = 0; g < a.KG; g++) {
+      const ulonglong2 v = a.part[((size_t)g * a.rows + r) * len + w];
+      P ^= v.y & x;
+      x ^= v.x;
+      z ^= v.y;
+    }
+    row[w] = x;
+    row[len + w] = z;
+    q -= (uint32_t)__popcll(x & z);
+  }
+  q += 2u * ((uint32_t)__popcll(P) & 1u);
+  q = __reduce_add_sync(0xFFFFFFFFu, q);
+  if (lane == 0) a.ph[r] = a.phases ? (uint8_t)((q + a.ph[r]) & 3u) : (uint8_t)0;
 }
 
 // rowswap!(state, i, j; phases) (src/QuantumClifford.jl:899-927): rows i and
@@ -783,6 +888,62 @@ static int apply_layers(const qcb_tableau* t, const std::vector<GateOp>& g, int 
       return s;
     k0 = k;
   }
+  return QCB_OK;
+}
+
+// Qubits from which dense apply! goes by tables: its three launches take 14 us
+// for any small tableau, a warp per row 5 us + 0.2 us a qubit (us, tables /
+// warp: n = 32 14 / 11, 64 15 / 19, 100 16 / 28, 300 18 / 77); many rows cross
+// earlier (30 qubits x 100000 rows 101 / 278).
+constexpr uint32_t DENSE_TABLES_MIN_N = 48;
+
+template <class... P, class... A>
+static cudaError_t launch_dependent(void (*k)(P...), dim3 grid, uint32_t block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return cudaLaunchKernelEx(&cfg, k, args...);
+}
+
+static int apply_dense_tables(qcb_tableau* t, const qcb_tableau* c, int phases, cudaStream_t st) {
+  const uint32_t R = t->rows, len = t->W / 2;
+  // threads; lanes per row (half a warp up to 16 words), words per lane and
+  // rows per slot, whose products fill the registers
+  struct Form { void (*k)(const DenseArgs); uint32_t threads, rows; };
+  const Form f = len <= 16 ? Form{dense_tables_kernel<1024, 16, 1, 2>, 1024, 128}
+               : len <= 32 ? Form{dense_tables_kernel<1024, 32, 1, 4>, 1024, 128}
+               : len <= 64 ? Form{dense_tables_kernel<512, 32, 2, 6>, 512, 96}
+                           : Form{dense_tables_kernel<512, 32, 4, 4>, 512, 64};
+  const uint32_t RG = (R + f.rows - 1) / f.rows;
+  DenseArgs a{};
+  a.xzs = t->xzs; a.ph = t->phases; a.rows = R; a.W = t->W; a.n = t->nqubits; a.c = c->xzs; a.cph = c->phases; a.phases = phases;
+  // runs of whole qubit words, as many as give every SM a CTA
+  a.KG = std::max<uint32_t>(1, std::min<uint32_t>({len, 16u, (uint32_t)device_sm_count() / RG}));
+  a.wpg = (len + a.KG - 1) / a.KG;
+  a.KG = (len + a.wpg - 1) / a.wpg;
+  const size_t table = (size_t)16 * len * sizeof(ulonglong2);
+  a.NT = 16;
+  while (a.NT * len > f.threads || a.NT * table > (size_t)200 * 1024) a.NT /= 2;
+  const size_t smem = a.NT * table;
+  size_t bytes = 0;
+  auto place = [&](size_t n) { const size_t o = bytes; bytes += (n + 127) / 128 * 128; return o; };
+  const size_t o_qt = place((size_t)32 * len * 16), o_part = place((size_t)a.KG * R * len * 16), o_odd = place((size_t)a.KG * R);
+  uint8_t* m = nullptr;
+  QCB_CUDA(cudaMallocAsync(&m, bytes, st));
+  a.qt = m + o_qt; a.part = (ulonglong2*)(m + o_part); a.odd = m + o_odd;
+  QCB_CUDA(cudaFuncSetAttribute(f.k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (phases) QCB_CUDA(launch_dependent(dense_q_kernel, dim3((32 * len + 7) / 8), 256, 0, st, a));
+  QCB_CUDA(launch_dependent(f.k, dim3(a.KG, RG), f.threads, smem, st, a));
+  QCB_CUDA(launch_dependent(dense_join_kernel, dim3((R + 7) / 8), 256, 0, st, a));
+  QCB_CUDA(cudaFreeAsync(m, st));
   return QCB_OK;
 }
 
@@ -999,29 +1160,10 @@ int qcb_apply_dense(qcb_tableau* t, const qcb_tableau* c, int phases, void* stre
   if (!t->rows) return QCB_OK;
   cudaStream_t st = S(stream);
   const uint32_t W = t->W;
-  // 8 warps per row (one row per CTA) unless the rows alone fill the GPU
-  const bool split = (uint64_t)t->rows < 8ull * 148 * 8 && W >= 16;
-  if (split) {
-    if (W <= 64)
-      apply_dense_split_kernel<64, 8><<<t->rows, 256, 0, st>>>(t->xzs, t->phases, t->rows, W, t->nqubits, c->xzs, c->phases, phases);
-    else if (W <= 128)
-      apply_dense_split_kernel<128, 8><<<t->rows, 256, 0, st>>>(t->xzs, t->phases, t->rows, W, t->nqubits, c->xzs, c->phases, phases);
-    else if (W <= 256)
-      apply_dense_split_kernel<256, 8><<<t->rows, 256, 0, st>>>(t->xzs, t->phases, t->rows, W, t->nqubits, c->xzs, c->phases, phases);
-    else
-      return fail(QCB_EUNSUPPORTED, "qcb_apply_dense: at most 8192 qubits");
-    QCB_LAUNCHED();
-    return QCB_OK;
-  }
-  const uint32_t threads = 256, blocks = (t->rows * 32 + threads - 1) / threads;
-  if (W <= 64)
-    apply_dense_kernel<64><<<blocks, threads, 0, st>>>(t->xzs, t->phases, t->rows, W, t->nqubits, c->xzs, c->phases, phases);
-  else if (W <= 128)
-    apply_dense_kernel<128><<<blocks, threads, 0, st>>>(t->xzs, t->phases, t->rows, W, t->nqubits, c->xzs, c->phases, phases);
-  else if (W <= 256)
-    apply_dense_kernel<256><<<blocks, threads, 0, st>>>(t->xzs, t->phases, t->rows, W, t->nqubits, c->xzs, c->phases, phases);
-  else
-    return fail(QCB_EUNSUPPORTED, "qcb_apply_dense: at most 8192 qubits");
+  if (W > 256) return fail(QCB_EUNSUPPORTED, "qcb_apply_dense: at most 8192 qubits");
+  if (t->nqubits >= DENSE_TABLES_MIN_N || (t->nqubits >= 16 && t->rows >= 16384)) return apply_dense_tables(t, c, phases, st);
+  const uint32_t threads = 256, blocks = (uint32_t)(((uint64_t)t->rows * 32 + threads - 1) / threads);
+  apply_dense_kernel<<<blocks, threads, 0, st>>>(t->xzs, t->phases, t->rows, W, t->nqubits, c->xzs, c->phases, phases);
   QCB_LAUNCHED();
   return QCB_OK;
 }

@@ -419,3 +419,21 @@ def test_canonicalize_panel_windows(qcb, rows, n, density, phases):
     ph, xz, orx, orz = oracle.canonicalize(t.phases, t.xzs, n, phases)
     assert (rx, rz) == (orx, orz)
     assert np.array_equal(s.tab.xzs, xz) and np.array_equal(s.tab.phases, ph)
+
+
+@pytest.mark.parametrize("n,rows", [(47, 5), (48, 129), (16, 16384), (65, 1), (130, 64), (1024, 127), (1025, 33), (2049, 97),
+                                    (4097, 65)])
+def test_dense_apply_table_edges(qcb, n, rows):
+    """Dense apply! by tables at the edges of its forms: lanes and words per
+    row, rows per warp, runs of qubits; any rows and phases."""
+    rng = np.random.default_rng(n)
+    state = rand_tab(rows, n, rng)
+    c = qcb.CliffordOperator(qcb.random_destabilizer(n, rng).tab)
+    c.tab.phases[:] = rng.integers(0, 4, 2 * n)
+    c.to_gpu()
+    for phases in (True, False):
+        s = qcb.Stabilizer(state.copy()).to_gpu()
+        qcb.apply_(s, c, phases=phases)
+        s.to_cpu()
+        ph, xz = oracle.apply_dense(state.phases, state.xzs, n, c.tab.phases, c.tab.xzs, phases)
+        assert np.array_equal(s.tab.xzs, xz) and np.array_equal(s.tab.phases, ph)
