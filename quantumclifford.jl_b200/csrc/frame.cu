@@ -1055,29 +1055,27 @@ int qcb_frame_create(uint64_t frames, uint32_t qubits, uint32_t nbits, qcb_frame
   f->ncols = (frames + 31) / 32;
   f->pitch = std::max<uint64_t>(32, (f->ncols + 31) / 32 * 32);
   f->pre_own = true;
-  size_t pbytes = (size_t)2 * (f->nq1 + 1) * f->pitch * 4;
-  size_t rbytes = (size_t)std::max<uint32_t>(nbits, 1) * f->pitch * 4;
-  cudaError_t e = cudaMalloc(&f->planes, pbytes);
-  if (e == cudaSuccess) e = cudaMalloc(&f->record, rbytes);
-  if (e == cudaSuccess) e = cudaMalloc(&f->err, 16);
-  if (e == cudaSuccess) e = cudaMemset(f->err, 0, 16);
-  if (e == cudaSuccess) e = cudaMemset(f->planes, 0, pbytes);
-  if (e == cudaSuccess) e = cudaMemset(f->record, 0, rbytes);
+  // one block: planes, record, status word (plane rows are 128-byte aligned)
+  const size_t pbytes = (size_t)2 * (f->nq1 + 1) * f->pitch * 4;
+  const size_t rbytes = (size_t)std::max<uint32_t>(nbits, 1) * f->pitch * 4;
+  f->dev_bytes = pbytes + rbytes + 16;
+  void* base = nullptr;
+  const cudaError_t e = dev_alloc(&base, f->dev_bytes, true);
   if (e != cudaSuccess) {
-    cudaFree(f->planes); cudaFree(f->record); cudaFree(f->err);
     delete f;
     return cuda_fail(e, "qcb_frame_create");
   }
+  f->planes = (uint32_t*)base;
+  f->record = (uint32_t*)((uint8_t*)base + pbytes);
+  f->err = (int32_t*)((uint8_t*)base + pbytes + rbytes);
   *out = f;
   return QCB_OK;
 }
 
 int qcb_frame_destroy(qcb_frame* f) {
   if (!f) return QCB_OK;
-  cudaFree(f->planes);
-  cudaFree(f->record);
-  cudaFree(f->err);
-  cudaFree(f->pre);
+  dev_free(f->planes, f->dev_bytes);
+  dev_free(f->pre, f->pre_bytes);
   delete f;
   return QCB_OK;
 }
@@ -1271,10 +1269,10 @@ static uint64_t presample_bytes(const qcb_frame* f, const qcb_program* p) {
 static int ensure_presample_scratch(qcb_frame* f, const qcb_program* p) {
   const uint64_t need = presample_bytes(f, p);
   if (!need || f->pre_bytes >= need || !f->pre_own) return QCB_OK;
-  if (f->pre) QCB_CUDA(cudaFree(f->pre));
+  dev_free(f->pre, f->pre_bytes);
   f->pre = nullptr;
   f->pre_bytes = 0;
-  QCB_CUDA(cudaMalloc(&f->pre, need));
+  QCB_CUDA(dev_alloc((void**)&f->pre, need, false));
   f->pre_bytes = need;
   return QCB_OK;
 }
@@ -1364,10 +1362,10 @@ static int launch_walker_chunked(qcb_frame* f, const qcb_program* p, const WalkA
                                  cudaStream_t st, uint64_t cw) {
   const uint64_t half = (presample_need(p, cw) + 15) & ~15ull;
   if (f->pre_bytes < 2 * half) {
-    if (f->pre) QCB_CUDA(cudaFree(f->pre));
+    dev_free(f->pre, f->pre_bytes);
     f->pre = nullptr;
     f->pre_bytes = 0;
-    QCB_CUDA(cudaMalloc(&f->pre, 2 * half));
+    QCB_CUDA(dev_alloc((void**)&f->pre, 2 * half, false));
     f->pre_bytes = 2 * half;
   }
   cudaStream_t side = side_stream();

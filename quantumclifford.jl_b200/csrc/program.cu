@@ -524,39 +524,38 @@ int compile(const qcb_op* ops, size_t n_ops, Program& P) {
 }
 
 int upload(Program& P) {
-  // device copies
-  auto up = [&](auto** dptr, const auto& vec) -> cudaError_t {
-    size_t bytes = vec.size() * sizeof(vec[0]);
-    cudaError_t e = cudaMalloc((void**)dptr, bytes ? bytes : 16);
-    if (e != cudaSuccess) return e;
-    if (bytes) e = cudaMemcpy(*dptr, vec.data(), bytes, cudaMemcpyHostToDevice);
-    return e;
+  // the device copies in one block, each at a multiple of 256 bytes
+  std::vector<uint8_t> image;
+  std::vector<std::pair<void**, size_t>> at;
+  auto add = [&](auto** dptr, const auto& vec) {
+    const size_t bytes = vec.size() * sizeof(vec[0]), o = image.size();
+    image.resize(o + std::max<size_t>((bytes + 255) / 256 * 256, 256));
+    if (bytes) std::memcpy(image.data() + o, vec.data(), bytes);
+    at.push_back({(void**)dptr, o});
   };
-  cudaError_t e = up(&P.d_stream_slot, P.stream_slot);
-  if (e == cudaSuccess) e = up(&P.d_classes, P.classes);
-  if (e == cudaSuccess) e = up(&P.d_cdf, P.cdf);
-  if (e == cudaSuccess) e = up(&P.d_slot_qubit, P.slot_qubit);
   std::vector<uint32_t> qs(P.nq + 1, BIT_NONE);
   for (uint32_t s = 0; s < P.nslots; s++) qs[P.slot_qubit[s]] = s;
   P.qubit_slot_len = (uint32_t)qs.size();
-  if (e == cudaSuccess) e = up(&P.d_qubit_slot, qs);
   std::vector<uint32_t> sw(P.slot_swap.begin(), P.slot_swap.end());
-  if (e == cudaSuccess) e = up(&P.d_slot_swap, sw);
-  if (e == cudaSuccess) e = up(&P.d_pre_ent, P.pre_ent);
-  if (e == cudaSuccess) e = up(&P.d_pre_capoff, P.pre_capoff);
+  add(&P.d_stream_slot, P.stream_slot);
+  add(&P.d_classes, P.classes);
+  add(&P.d_cdf, P.cdf);
+  add(&P.d_slot_qubit, P.slot_qubit);
+  add(&P.d_qubit_slot, qs);
+  add(&P.d_slot_swap, sw);
+  add(&P.d_pre_ent, P.pre_ent);
+  add(&P.d_pre_capoff, P.pre_capoff);
+  void* base = nullptr;
+  const cudaError_t e = dev_alloc(&base, image.size(), false, image.data(), image.size());
   if (e != cudaSuccess) return cuda_fail(e, "qcb_program_compile upload");
+  P.dev_bytes = image.size();
+  for (auto& v : at) *v.first = (uint8_t*)base + v.second;
   return QCB_OK;
 }
 
 void release(Program& P) {
-  cudaFree(P.d_stream_slot);
-  cudaFree(P.d_classes);
-  cudaFree(P.d_cdf);
-  cudaFree(P.d_slot_qubit);
-  cudaFree(P.d_qubit_slot);
-  cudaFree(P.d_slot_swap);
-  cudaFree(P.d_pre_ent);
-  cudaFree(P.d_pre_capoff);
+  dev_free(P.d_stream_slot, P.dev_bytes);
+  P.dev_bytes = 0;
   P.d_pre_ent = nullptr;
   P.d_pre_capoff = nullptr;
   P.d_stream_slot = nullptr;

@@ -35,6 +35,17 @@ inline cudaStream_t S(void* s) { return (cudaStream_t)s; }
 int device_sm_count();
 int device_max_smem_optin();
 
+// Device memory of library objects (frames, programs and their scratch), ready
+// for any stream on return.  Blocks of up to DEV_POOL_MAX bytes come from the
+// device's stream-ordered pool, which keeps freed ones (a bounded amount, see
+// qcb_init); larger ones from cudaMalloc.  With `zero` the block is cleared,
+// with `init` its first init_bytes are copied from the host.  dev_free waits
+// for the device first, as cudaFree does: the block may be in use on any
+// stream.
+constexpr size_t DEV_POOL_MAX = 64ull << 20;
+cudaError_t dev_alloc(void** p, size_t bytes, bool zero, const void* init = nullptr, size_t init_bytes = 0);
+void dev_free(void* p, size_t bytes);
+
 // ------------------------------------------------------------ Philox
 enum : uint32_t { TAG_INITZ = 0x51A7u, TAG_RESET = 0x5E5Eu, TAG_NOISE = 0x4E01u };
 
@@ -167,6 +178,7 @@ struct Program {
   uint4* d_pre_ent = nullptr;
   uint32_t* d_pre_capoff = nullptr;
   uint32_t qubit_slot_len = 0;
+  size_t dev_bytes = 0;               // of the one block the device copies lie in (at d_stream_slot)
   uint64_t hash = 0;
 };
 
@@ -184,6 +196,7 @@ struct qcb_frame {
   uint32_t* planes;  // [(2*(nq1+1))][pitch]: plane 2q = x(q), 2q+1 = z(q); last pair = scratch
   uint32_t* record;  // [nbits][pitch]
   int32_t* err;      // device status word of the walker (QCB_ETIMEOUT on a stuck wait)
+  size_t dev_bytes = 0;  // of the one block planes, record and err lie in (at planes)
   // scratch of the noise pre-sampler (event buckets and counters), grown on
   // demand; only frames made by qcb_frame_create own one (pre_own)
   uint32_t* pre = nullptr;

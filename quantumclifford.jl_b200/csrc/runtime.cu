@@ -41,6 +41,51 @@ int device_max_smem_optin() {
   return v > 0 ? v : 48 * 1024;
 }
 
+// A stream per device for the allocations of dev_alloc.
+static cudaStream_t alloc_stream() {
+  static std::mutex mu;
+  static cudaStream_t streams[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return nullptr;
+  std::lock_guard<std::mutex> lk(mu);
+  if (!streams[dev]) cudaStreamCreateWithFlags(&streams[dev], cudaStreamNonBlocking);
+  return streams[dev];
+}
+
+cudaError_t dev_alloc(void** p, size_t bytes, bool zero, const void* init, size_t init_bytes) {
+  *p = nullptr;
+  if (!bytes) bytes = 16;
+  cudaStream_t st = alloc_stream();
+  cudaError_t e = bytes <= DEV_POOL_MAX ? cudaMallocAsync(p, bytes, st) : cudaMalloc(p, bytes);
+  if (e != cudaSuccess) return e;
+  if (zero) e = cudaMemsetAsync(*p, 0, bytes, st);
+  if (e == cudaSuccess && init_bytes) e = cudaMemcpyAsync(*p, init, init_bytes, cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) {
+    dev_free(*p, bytes);
+    *p = nullptr;
+  }
+  return e;
+}
+
+void dev_free(void* p, size_t bytes) {
+  if (!p) return;
+  if ((bytes ? bytes : 16) > DEV_POOL_MAX) {
+    cudaFree(p);
+    return;
+  }
+  // on the block's device, whichever is current
+  int dev = 0;
+  cudaPointerAttributes at{};
+  cudaGetDevice(&dev);
+  const bool other = cudaPointerGetAttributes(&at, p) == cudaSuccess && at.device != dev;
+  if (other) cudaSetDevice(at.device);
+  cudaDeviceSynchronize();
+  cudaFreeAsync(p, alloc_stream());
+  if (other) cudaSetDevice(dev);
+}
+
 __global__ void philox_probe_kernel(uint4 ctr, uint2 key, uint32_t* out) {
   uint32_t o[4];
   philox4x32_10(ctr.x, ctr.y, ctr.z, ctr.w, key.x, key.y, o);

@@ -173,7 +173,7 @@ class PauliFrame:
         out = np.empty((self.nbits, self.frames), dtype=np.uint8)  # column-major frames x nbits
         if out.size:
             check(lib().qcb_frame_download_measurements(self.handle, ptr(out), None))
-        return out.T.astype(bool)
+        return out.T.view(bool)  # the bytes are 0 or 1
 
     def set_measurements(self, meas: np.ndarray):
         """Load a Bool record matrix (frames x nbits) into the device record."""

@@ -48,9 +48,17 @@ class DeviceTableau:
         assert ph.shape == (self.rows,) and xz.shape == (self.rows, self.W)
         check(lib().qcb_tableau_upload(self.handle, ptr(ph) if ph.size else None, ptr(xz) if xz.size else None, None))
 
-    def download(self):
-        ph = np.empty(self.rows, dtype=np.uint8)
-        xz = np.empty((self.rows, self.W), dtype=np.uint64)
+    def download(self, ph=None, xz=None):
+        """(phases, xzs); into the given arrays where they fit (C-contiguous,
+        of the device tableau's shapes), else into new ones."""
+        def fits(a, dtype, shape):
+            return (isinstance(a, np.ndarray) and a.dtype == dtype and a.shape == shape and a.flags["C_CONTIGUOUS"]
+                    and a.flags["WRITEABLE"])
+
+        if not fits(ph, np.uint8, (self.rows,)):
+            ph = np.empty(self.rows, dtype=np.uint8)
+        if not fits(xz, np.uint64, (self.rows, self.W)):
+            xz = np.empty((self.rows, self.W), dtype=np.uint64)
         check(lib().qcb_tableau_download(self.handle, ptr(ph) if ph.size else None, ptr(xz) if xz.size else None, None))
         return ph, xz
 
@@ -126,7 +134,11 @@ class Tableau:
 
     def to_cpu(self) -> "Tableau":
         if self.dev is not None:
-            self.phases[:], self.xzs[:] = self.dev.download()
+            ph, xz = self.dev.download(self.phases, self.xzs)
+            if ph is not self.phases:
+                self.phases[:] = ph
+            if xz is not self.xzs:
+                self.xzs[:] = xz
         return self
 
     def _need_dev(self) -> DeviceTableau:
