@@ -223,8 +223,9 @@ int qcb_frame_download_planes(const qcb_frame* f, uint32_t* x_planes, uint32_t* 
  * is a fresh run (initZ! + circuit, Philox mode) of `program` on `frame`, so
  * its record equals that of qcb_pftrajectories_fresh with the same seed and
  * shot_offset.  The (job, shot-tile) items are queued longest first and taken
- * by one CTA per SM.  qcb_batch_run only clears the queue head and launches:
- * it can be captured in a CUDA graph.  Frames and programs must outlive the
+ * by one CTA per SM.  qcb_batch_run only clears counters and launches: it can
+ * be captured in a CUDA graph.  The batch holds up to 1 GB of device memory for
+ * its jobs' pre-sampled noise; jobs past that draw theirs in the walk.  Frames and programs must outlive the
  * batch; the frame tile of every job must fit one CTA's shared memory.      */
 typedef struct qcb_batch_job {
   qcb_frame* frame;

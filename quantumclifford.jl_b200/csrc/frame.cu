@@ -394,12 +394,10 @@ struct PresampleArgs {
   uint32_t force_overflow;  // test knob: every non-empty bucket reports more than its capacity
 };
 
-__global__ void __launch_bounds__(256) presample_kernel(const PresampleArgs p) {
-  // the walker that reads these buckets is a programmatic dependent: let it
-  // launch once every sampler CTA is resident, so that its CTAs take the SMs
-  // of the sampler's last wave as they free up (it waits before its first read)
-  asm volatile("griddepcontrol.launch_dependents;");
-  const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+// Entry e on groups g0, g0 + gstep, ... below g1.
+__device__ __forceinline__ void presample_entries(const PresampleArgs& p, uint32_t e, uint64_t g0, uint64_t g1,
+                                                  uint64_t gstep) {
+  const uint32_t lane = threadIdx.x & 31;
   const bool valid = e < p.nent;
   const uint4 pe = valid ? p.ent[e] : make_uint4(0u, 0u, 0xFFFFFFFFu, 0u);
   NoiseClass c{};
@@ -413,7 +411,7 @@ __global__ void __launch_bounds__(256) presample_kernel(const PresampleArgs p) {
   const uint32_t peers = __match_any_sync(0xFFFFFFFFu, j);
   const uint32_t first = __ffs(peers) - 1, last = 31 - __clz(peers);
   const uint32_t tag = pe.w << 16;
-  for (uint64_t g = blockIdx.y; g < p.ngroups; g += gridDim.y) {
+  for (uint64_t g = g0; g < g1; g += gstep) {
     const uint32_t glo = (uint32_t)(p.g0 + g);
     uint32_t o[4];
     const uint32_t k = valid ? sparse_count(c, p.cdf, pe.x, glo, k0, k1, o) : 0u;
@@ -437,6 +435,28 @@ __global__ void __launch_bounds__(256) presample_kernel(const PresampleArgs p) {
     if (k <= 3) sparse_emit<3>(c, kind, pe.x, glo, k0, k1, k, o, put);
     else sparse_emit<NOISE_KREG>(c, kind, pe.x, glo, k0, k1, k, o, put);
   }
+}
+
+__global__ void __launch_bounds__(256) presample_kernel(const PresampleArgs p) {
+  // the walker that reads these buckets is a programmatic dependent: let it
+  // launch once every sampler CTA is resident, so that its CTAs take the SMs
+  // of the sampler's last wave as they free up (it waits before its first read)
+  asm volatile("griddepcontrol.launch_dependents;");
+  presample_entries(p, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y, p.ngroups, gridDim.y);
+}
+
+// The jobs of a batch in one launch: block b takes item b, 256 entries of one
+// job on up to PRESAMPLE_ITEM_GROUPS groups.
+struct PresampleItem {
+  uint32_t job, e0, g0, pad;
+};
+constexpr uint32_t PRESAMPLE_ITEM_GROUPS = 16;
+
+__global__ void __launch_bounds__(256) presample_batch_kernel(const PresampleArgs* jobs, const PresampleItem* items) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  const PresampleItem it = items[blockIdx.x];
+  const PresampleArgs p = jobs[it.job];
+  presample_entries(p, it.e0 + threadIdx.x, it.g0, min((uint64_t)it.g0 + PRESAMPLE_ITEM_GROUPS, p.ngroups), 1);
 }
 
 // ---------------------------------------------------------------- walker
@@ -870,7 +890,7 @@ struct BatchArgs {
 constexpr uint32_t ITEM_NONE = 0xFFFFFFFFu;
 static_assert(sizeof(WalkArgs) % 8 == 0, "WalkArgs is copied in 8-byte words");
 
-__global__ void __launch_bounds__(768, 1) batch_walker_kernel(const BatchArgs b) {
+__global__ void __launch_bounds__(WALKER_THREADS, 1) batch_walker_kernel(const BatchArgs b) {
   extern __shared__ __align__(128) uint32_t sm[];
   __shared__ uint32_t itemq[8];
   __shared__ __align__(16) WalkArgs ja;
@@ -918,7 +938,7 @@ __global__ void __launch_bounds__(768, 1) batch_walker_kernel(const BatchArgs b)
     for (uint32_t w = tid; w < sizeof(WalkArgs) / 8; w += blockDim.x)
       ((uint64_t*)&ja)[w] = ((const uint64_t*)(b.jobs + bi.job))[w];
     __syncthreads();
-    if (!walk_tile<true, true, false>(ja, sm, win0, win1, bars, kwin, issue, bi.tile)) {
+    if (!walk_tile<true, true, true>(ja, sm, win0, win1, bars, kwin, issue, bi.tile)) {
       failed = true;
       break;
     }
@@ -1277,6 +1297,33 @@ static int ensure_presample_scratch(qcb_frame* f, const qcb_program* p) {
   return QCB_OK;
 }
 
+static uint64_t presample_cnt_words(const qcb_program* p, uint64_t ncols) { return (ncols + 31) / 32 * p->pre_nparts; }
+
+// The pre-sampler's arguments for the run `a` of program p with its counters
+// and buckets at cnt and buf; `a` is pointed at them.
+static PresampleArgs presample_args(const qcb_program* p, uint64_t ncols, WalkArgs& a, uint32_t* cnt, uint32_t* buf) {
+  PresampleArgs q{};
+  q.ent = p->d_pre_ent;
+  q.nent = (uint32_t)p->pre_ent.size();
+  q.nparts = p->pre_nparts;
+  q.g0 = a.col0 / 32;
+  q.ngroups = (ncols + 31) / 32;
+  q.classes = p->d_classes;
+  q.cdf = p->d_cdf;
+  q.seed = a.seed;
+  q.cnt = cnt;
+  q.buf = buf;
+  q.capoff = p->d_pre_capoff;
+  q.capg = p->pre_capoff.back();
+  q.force_overflow = g_presample == 2 ? 1u : 0u;
+  a.pre_buf = q.buf;
+  a.pre_cnt = q.cnt;
+  a.pre_capoff = p->d_pre_capoff;
+  a.pre_nparts = p->pre_nparts;
+  a.pre_capg = q.capg;
+  return q;
+}
+
 // Pre-sample the run's sparse noise into the frame's scratch (counts zeroed,
 // then one presample_kernel launch) and point the walk at it; nothing when
 // the scratch is absent or too small (the walk then draws the noise).
@@ -1285,34 +1332,15 @@ static int launch_presample(qcb_frame* f, const qcb_program* p, WalkArgs& a, cud
   if (!need) return QCB_OK;
   if (int s = ensure_presample_scratch(f, p)) return s;
   if (f->pre_bytes < need) return QCB_OK;
-  const uint64_t ngroups = (f->ncols + 31) / 32;
-  const uint64_t cnt_words = ngroups * p->pre_nparts;
-  PresampleArgs q{};
-  q.ent = p->d_pre_ent;
-  q.nent = (uint32_t)p->pre_ent.size();
-  q.nparts = p->pre_nparts;
-  q.g0 = a.col0 / 32;
-  q.ngroups = ngroups;
-  q.classes = p->d_classes;
-  q.cdf = p->d_cdf;
-  q.seed = a.seed;
-  q.cnt = f->pre;
-  q.buf = f->pre + cnt_words;
-  q.capoff = p->d_pre_capoff;
-  q.capg = p->pre_capoff.back();
-  q.force_overflow = g_presample == 2 ? 1u : 0u;
+  const uint64_t cnt_words = presample_cnt_words(p, f->ncols);
+  const PresampleArgs q = presample_args(p, f->ncols, a, f->pre, f->pre + cnt_words);
   QCB_CUDA(cudaMemsetAsync(q.cnt, 0, cnt_words * 4, st));
   // each thread walks groups g, g + grid.y, ...: about 8 CTAs per SM in all
   const uint32_t gx = (q.nent + 255) / 256;
   const uint64_t gy = std::max<uint64_t>(1, ((uint64_t)device_sm_count() * 8 + gx - 1) / gx);
-  const dim3 grid(gx, (uint32_t)std::min<uint64_t>(std::min<uint64_t>(ngroups, gy), 65535));
+  const dim3 grid(gx, (uint32_t)std::min<uint64_t>(std::min<uint64_t>(q.ngroups, gy), 65535));
   presample_kernel<<<grid, 256, 0, st>>>(q);
   QCB_LAUNCHED();
-  a.pre_buf = q.buf;
-  a.pre_cnt = q.cnt;
-  a.pre_capoff = p->d_pre_capoff;
-  a.pre_nparts = p->pre_nparts;
-  a.pre_capg = q.capg;
   return QCB_OK;
 }
 
@@ -1859,7 +1887,58 @@ struct qcb_batch {
   uint32_t win_words = 0;
   size_t smem_bytes = 0;
   uint32_t grid = 0;
+  // pre-sampled noise: every job's counters, then every job's buckets
+  uint32_t* pre = nullptr;
+  size_t pre_bytes = 0, pre_cnt_bytes = 0;
+  qcb::PresampleArgs* d_pre_jobs = nullptr;
+  qcb::PresampleItem* d_pre_items = nullptr;
+  uint32_t n_pre_items = 0;
 };
+
+// Event buckets of a batch's jobs at most; jobs past it draw their noise in
+// the walk, where a flush's (site, group) chains are exposed at its barrier.
+// 24 surface-code circuits (d <= 13, p log-U[1e-4, 1e-2]): one launch drawing in
+// the walk 1590 us; sampler 141 + walker 702 us.
+constexpr uint64_t BATCH_PRESAMPLE_MAX = 1ull << 30;
+
+// The scratch and the sampler's work list of a batch; the jobs' walks are
+// pointed at it.
+static int batch_presample(qcb_batch& b, const qcb_batch_job* jobs, size_t n_jobs, std::vector<qcb::WalkArgs>& wa) {
+  using namespace qcb;
+  std::vector<size_t> ids;
+  uint64_t cnt = 0, buf = 0;  // words
+  for (size_t j = 0; j < n_jobs; j++) {
+    const uint64_t ncols = jobs[j].frame->ncols, need = presample_need(jobs[j].program, ncols);
+    if (!need || (cnt + buf) * 4 + need > BATCH_PRESAMPLE_MAX) continue;
+    const uint64_t c = presample_cnt_words(jobs[j].program, ncols);
+    cnt += c;
+    buf += need / 4 - c;
+    ids.push_back(j);
+  }
+  if (ids.empty()) return QCB_OK;
+  b.pre_cnt_bytes = cnt * 4;
+  b.pre_bytes = (cnt + buf) * 4;
+  QCB_CUDA(dev_alloc((void**)&b.pre, b.pre_bytes, false));
+  std::vector<PresampleArgs> args;
+  std::vector<PresampleItem> items;
+  uint32_t *pc = b.pre, *pb = b.pre + cnt;
+  for (size_t j : ids) {
+    const qcb_program* p = jobs[j].program;
+    const uint64_t ncols = jobs[j].frame->ncols, c = presample_cnt_words(p, ncols);
+    args.push_back(presample_args(p, ncols, wa[j], pc, pb));
+    const PresampleArgs& q = args.back();
+    pc += c;
+    pb += presample_need(p, ncols) / 4 - c;
+    for (uint64_t g = 0; g < q.ngroups; g += PRESAMPLE_ITEM_GROUPS)
+      for (uint32_t e = 0; e < q.nent; e += 256) items.push_back({(uint32_t)args.size() - 1, e, (uint32_t)g, 0u});
+  }
+  b.n_pre_items = (uint32_t)items.size();
+  QCB_CUDA(cudaMalloc(&b.d_pre_jobs, args.size() * sizeof(PresampleArgs)));
+  QCB_CUDA(cudaMalloc(&b.d_pre_items, items.size() * sizeof(PresampleItem)));
+  QCB_CUDA(cudaMemcpy(b.d_pre_jobs, args.data(), args.size() * sizeof(PresampleArgs), cudaMemcpyHostToDevice));
+  QCB_CUDA(cudaMemcpy(b.d_pre_items, items.data(), items.size() * sizeof(PresampleItem), cudaMemcpyHostToDevice));
+  return QCB_OK;
+}
 
 extern "C" {
 
@@ -1913,13 +1992,22 @@ int qcb_batch_create(const qcb_batch_job* jobs, size_t n_jobs, qcb_batch** out) 
   b->tile_words = tile_words;
   b->win_words = win_words;
   b->smem_bytes = (size_t)((tile_words + 31) & ~31u) * 4 + (size_t)2 * win_words * 4 + 16;
+  if (int s = batch_presample(*b, jobs, n_jobs, wa)) {
+    dev_free(b->pre, b->pre_bytes);
+    cudaFree(b->d_pre_jobs);
+    cudaFree(b->d_pre_items);
+    return s;
+  }
   b->grid = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(b->nitems, 1), (uint64_t)device_sm_count());
   QCB_CUDA(cudaMalloc(&b->d_jobs, std::max<size_t>(wa.size(), 1) * sizeof(WalkArgs)));
   QCB_CUDA(cudaMalloc(&b->d_items, std::max<size_t>(it.size(), 1) * sizeof(BatchItem)));
   QCB_CUDA(cudaMalloc(&b->d_head, 4));
   if (!wa.empty()) QCB_CUDA(cudaMemcpy(b->d_jobs, wa.data(), wa.size() * sizeof(WalkArgs), cudaMemcpyHostToDevice));
   if (!it.empty()) QCB_CUDA(cudaMemcpy(b->d_items, it.data(), it.size() * sizeof(BatchItem), cudaMemcpyHostToDevice));
-  QCB_CUDA(cudaFuncSetAttribute(batch_walker_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, device_max_smem_optin() - 1024));
+  cudaFuncAttributes fa{};
+  QCB_CUDA(cudaFuncGetAttributes(&fa, batch_walker_kernel));
+  QCB_CUDA(cudaFuncSetAttribute(batch_walker_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                device_max_smem_optin() - (int)fa.sharedSizeBytes));
   *out = b.release();
   return QCB_OK;
 }
@@ -1930,8 +2018,24 @@ int qcb_batch_run(qcb_batch* b, void* stream) {
   if (!b->nitems) return QCB_OK;
   cudaStream_t st = S(stream);
   QCB_CUDA(cudaMemsetAsync(b->d_head, 0, 4, st));
+  if (b->n_pre_items) {
+    QCB_CUDA(cudaMemsetAsync(b->pre, 0, b->pre_cnt_bytes, st));
+    presample_batch_kernel<<<b->n_pre_items, 256, 0, st>>>(b->d_pre_jobs, b->d_pre_items);
+    QCB_LAUNCHED();
+  }
+  // the walker as the sampler's programmatic dependent, as in a plain run
   BatchArgs a{b->d_jobs, b->d_items, b->nitems, b->tile_words, b->d_head, b->win_words, 0u};
-  batch_walker_kernel<<<b->grid, 768, b->smem_bytes, st>>>(a);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(b->grid);
+  cfg.blockDim = dim3(WALKER_THREADS);
+  cfg.dynamicSmemBytes = b->smem_bytes;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = (b->n_pre_items && g_walker_pdl) ? 1 : 0;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  QCB_CUDA(cudaLaunchKernelEx(&cfg, batch_walker_kernel, (const BatchArgs)a));
   QCB_LAUNCHED();
   return QCB_OK;
 }
@@ -1948,6 +2052,9 @@ int qcb_batch_destroy(qcb_batch* b) {
   cudaFree(b->d_jobs);
   cudaFree(b->d_items);
   cudaFree(b->d_head);
+  cudaFree(b->d_pre_jobs);
+  cudaFree(b->d_pre_items);
+  dev_free(b->pre, b->pre_bytes);
   delete b;
   return QCB_OK;
 }

@@ -141,3 +141,33 @@ def test_batch_with_a_tall_program_in_16k_windows(qcb):
     frames, b = batched_frames(qcb, jobs)
     b.run().status()
     assert_same(qcb, frames, jobs)
+
+
+@pytest.mark.parametrize("presample", [0, 1, 2])
+def test_batch_noise_pre_sampled_or_in_the_walk(qcb, presample):
+    """The noise of a batch's jobs drawn ahead by one launch over all jobs, in
+    the walk, and with every bucket overflowing: the records of plain runs, for
+    uneven programs, shot counts and offsets, run twice."""
+    specs = [(3, 3, 0.02, 2000, 0), (5, 2, 0.004, 40_000, 1024), (15, 1, 0.001, 33_000, 0), (3, 1, 0.0, 100, 0),
+             (7, 7, 0.3, 5000, 2048)]
+    lib = qcb.lib()
+    qcb.check(lib.qcb_tune_set(b"presample", presample))
+    try:
+        jobs, want = [], []
+        for k, (d, rounds, p, shots, off) in enumerate(specs):
+            arr = O.to_array(circuits.rotated_surface_code_memory(d, rounds, p))
+            qmax, bmax = O.affected_counts(arr)
+            prog = qcb.Program(arr)
+            f = qcb.PauliFrame(shots, qmax, bmax, init=False, shot_offset=off)
+            jobs.append((f, prog, 90 + k, off))
+            g = qcb.PauliFrame(shots, qmax, bmax, init=False)
+            qcb.check(lib.qcb_pftrajectories_fresh(g.handle, prog.handle, 90 + k, off, None))
+            want.append((g.record_planes(), g.planes()))
+        b = qcb.Batch(jobs)
+        for _ in range(2):
+            b.run().status()
+            for (f, *_), (rec, pl) in zip(jobs, want):
+                assert np.array_equal(f.record_planes(), rec)
+                assert all(np.array_equal(u, v) for u, v in zip(f.planes(), pl))
+    finally:
+        qcb.check(lib.qcb_tune_set(b"presample", 0))
