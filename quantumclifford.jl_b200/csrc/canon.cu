@@ -1462,6 +1462,7 @@ struct ElimSpec {
   uint32_t ncols;
   int32_t* d_pivcols;
   int32_t* d_out;
+  bool waits;  // the caller waits for the stream anyway (it returns host values)
 };
 
 static uint32_t g_canon_blocked = 0;  // 0: automatic, 1: always, 2: never
@@ -1556,6 +1557,10 @@ static cudaError_t launch_panel(void (*k)(const CanonPanelArgs), uint32_t grid, 
   return cudaLaunchKernelEx(&cfg, k, a);
 }
 
+// Panels (both stages) from which a call that may wait looks whether all
+// pivots are found.
+constexpr uint32_t CANON_LOOK_PANELS = 16;
+
 // canonicalize! by panels over the whole GPU; scratch (the tiles: the tableau
 // rounded up to two word columns, and small arrays) from the stream-ordered
 // pool in one piece.
@@ -1595,8 +1600,19 @@ static int launch_grid(const ElimSpec& e, cudaStream_t st) {
   std::vector<std::pair<uint32_t, uint32_t>> panels;  // (stage, first column)
   for (uint32_t stage = 0; stage < 2; stage++)
     for (uint32_t c0 = 0; c0 < e.n; c0 += PSTEPS) panels.push_back({stage, c0});
-  const uint32_t P = (uint32_t)panels.size();
+  // A generic full-rank state has all its pivots after the X stage and the
+  // first Z panel (its X block lacks a rank or two); the rest of the Z stage
+  // (launches of 2 us with nothing to do) is left out where the call may look.
+  // The wait costs about 10 us.
+  uint32_t P = (uint32_t)panels.size();
+  const uint32_t look = e.waits && P >= CANON_LOOK_PANELS ? P / 2 + 1 : WORD_NONE;
   for (uint32_t k = 0; k <= P; k++) {
+    if (k == look) {
+      uint32_t done = 0;
+      QCB_CUDA(cudaMemcpyAsync(&done, &rec[(k - 1) & 1].done, 4, cudaMemcpyDeviceToHost, st));
+      QCB_CUDA(cudaStreamSynchronize(st));
+      if (done) P = k;
+    }
     a.steps = k < P;
     a.apply = k > 0;
     if (k < P) { a.stage = panels[k].first; a.c0 = panels[k].second; }
@@ -1673,8 +1689,9 @@ static int eliminate(const ElimSpec& e, cudaStream_t st) {
 }
 
 int canonicalize_view(uint64_t* xzs, uint8_t* ph, uint32_t rows, uint32_t n, uint32_t W, int phases,
-                      int32_t* d_out, cudaStream_t st) {
+                      int32_t* d_out, cudaStream_t st, bool waits) {
   ElimSpec e{};
+  e.waits = waits;
   e.xzs = xzs; e.ph = ph; e.rows = rows; e.n = n; e.W = W; e.phases = phases;
   e.mode = ELIM_BOTH; e.d_out = d_out;
   return eliminate(e, st);
@@ -1752,7 +1769,7 @@ int qcb_canonicalize(qcb_tableau* t, uint32_t row0, uint32_t nrows, int phases, 
   cudaStream_t st = S(stream);
   int32_t* d_out = (int32_t*)t->scratch + 16;
   if (int s = canonicalize_view(t->xzs + (size_t)(row0 - 1) * t->W, t->phases + (row0 - 1), nrows,
-                                t->nqubits, t->W, phases, d_out, st))
+                                t->nqubits, t->W, phases, d_out, st, rx || rz))
     return s;
   if (rx || rz) {
     int32_t h[2];
@@ -1775,7 +1792,7 @@ int qcb_canonicalize_state(qcb_tableau* t, int kind, int32_t rank, int phases, i
   e.xzs = t->xzs + (size_t)off * t->W; e.ph = t->phases + off;
   if (destab) { e.dxzs = t->xzs; e.dph = t->phases; }
   e.rows = rows; e.n = t->nqubits; e.W = t->W; e.phases = phases;
-  e.mode = ELIM_BOTH; e.d_out = (int32_t*)t->scratch + 16;
+  e.mode = ELIM_BOTH; e.d_out = (int32_t*)t->scratch + 16; e.waits = rx || rz;
   if (int s = eliminate(e, st)) return s;
   if (rx || rz) {
     int32_t h[2];

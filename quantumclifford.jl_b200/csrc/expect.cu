@@ -24,7 +24,7 @@
 namespace qcb {
 
 int canonicalize_view(uint64_t* xzs, uint8_t* ph, uint32_t rows, uint32_t n, uint32_t W, int phases,
-                      int32_t* d_out, cudaStream_t st);
+                      int32_t* d_out, cudaStream_t st, bool waits);
 
 __device__ __forceinline__ void mul_step_e(uint64_t x1, uint64_t z1, uint64_t& x2, uint64_t& z2, uint64_t& c1,
                                            uint64_t& c2) {
@@ -207,7 +207,7 @@ int qcb_expect(const qcb_tableau* t, int kind, int32_t rank, const qcb_tableau* 
     if (r) {
       QCB_CUDA(cudaMemcpyAsync(tmp, t->xzs, (size_t)r * W * 8, cudaMemcpyDeviceToDevice, st));
       QCB_CUDA(cudaMemcpyAsync(tph, t->phases, r, cudaMemcpyDeviceToDevice, st));
-      status = canonicalize_view(tmp, tph, r, n, W, 1, (int32_t*)t->scratch + 48, st);
+      status = canonicalize_view(tmp, tph, r, n, W, 1, (int32_t*)t->scratch + 48, st, true);
     }
     if (status == QCB_OK) {
       if (sm > 48 * 1024) QCB_CUDA(cudaFuncSetAttribute(expect_stab_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));

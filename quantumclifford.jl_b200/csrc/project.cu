@@ -30,7 +30,7 @@ namespace cg = cooperative_groups;
 namespace qcb {
 
 int canonicalize_view(uint64_t* xzs, uint8_t* ph, uint32_t rows, uint32_t n, uint32_t W, int phases,
-                      int32_t* d_out, cudaStream_t st);
+                      int32_t* d_out, cudaStream_t st, bool waits);
 int generate_dev(uint64_t* pauli, uint8_t* pph, const uint64_t* xzs, const uint8_t* ph, uint32_t rows,
                  uint32_t W, int phases, int32_t* d_ok, int32_t* d_used, uint32_t cap, uint32_t* d_nused,
                  cudaStream_t st);
@@ -1554,7 +1554,7 @@ static int project_impl(qcb_tableau* t, int kind, int32_t* rank_io, const uint64
     int32_t r_now = rank;
     if (kind == QCB_MIXED_STABILIZER) QCB_CUDA(cudaMemcpy(&r_now, d_rank, 4, cudaMemcpyDeviceToHost));
     const uint32_t nr = kind == QCB_STABILIZER ? t->rows : (uint32_t)r_now;
-    if (int s = canonicalize_view(t->xzs, t->phases, nr, t->nqubits, t->W, phases, d_cout, st)) { status = s; break; }
+    if (int s = canonicalize_view(t->xzs, t->phases, nr, t->nqubits, t->W, phases, d_cout, st, true)) { status = s; break; }
     std::vector<uint64_t> hp;
     const uint8_t zero = 0;
     if (qubits) {
