@@ -507,8 +507,8 @@ __device__ __forceinline__ bool walk_tile(const WalkArgs& a, uint32_t* sm, uint3
         if (q >= a.nq1) break;
         const uint32_t s = (SMEM && q < a.qubit_slot_len) ? __ldg(a.qubit_slot + q) : BIT_NONE;
         if (SMEM && s != BIT_NONE) {
-          *F.at2(2 * s, cw, cg) = make_uint2(0u, 0u);
-          *F.at2(2 * s + 1, cw, cg) = make_uint2(o[j], u[j]);
+          *F.at2(2 * s + slot_flip(s), cw, cg) = make_uint2(0u, 0u);
+          *F.at2(2 * s + 1 - slot_flip(s), cw, cg) = make_uint2(o[j], u[j]);
         } else {
           *(uint2*)(a.planes + (uint64_t)(2 * q) * pitch + cg) = make_uint2(0u, 0u);
           *(uint2*)(a.planes + (uint64_t)(2 * q + 1) * pitch + cg) = make_uint2(o[j], u[j]);
@@ -519,8 +519,8 @@ __device__ __forceinline__ bool walk_tile(const WalkArgs& a, uint32_t* sm, uint3
     for (uint32_t s = rr; s < a.nslots; s += R) {
       if (!act) break;
       const uint32_t q = __ldg(a.slot_qubit + s);
-      *F.at2(2 * s, cw, cg) = *(const uint2*)(a.planes + (uint64_t)(2 * q) * pitch + cg);
-      *F.at2(2 * s + 1, cw, cg) = *(const uint2*)(a.planes + (uint64_t)(2 * q + 1) * pitch + cg);
+      *F.at2(2 * s + slot_flip(s), cw, cg) = *(const uint2*)(a.planes + (uint64_t)(2 * q) * pitch + cg);
+      *F.at2(2 * s + 1 - slot_flip(s), cw, cg) = *(const uint2*)(a.planes + (uint64_t)(2 * q + 1) * pitch + cg);
     }
   }
   // mask mode: the events of the pair's columns, [ep[h], ep[h + 1]) for column h
@@ -822,7 +822,7 @@ __device__ __forceinline__ bool walk_tile(const WalkArgs& a, uint32_t* sm, uint3
     if (SMEM) {
       *gx = *F.at2(2 * s + sw, cw, cg);
       *gz = *F.at2(2 * s + 1 - sw, cw, cg);
-    } else if (sw) {
+    } else if (sw != slot_flip(s)) {
       const uint2 x = *gx, z = *gz;
       *gx = z;
       *gz = x;
@@ -849,7 +849,7 @@ __global__ void __launch_bounds__(WALKER_THREADS, 1) walker_kernel(const WalkArg
   uint32_t* win1 = win0 + a.win_words;
   uint64_t* bars = (uint64_t*)(win1 + a.win_words);
   if (!SMEM)
-    for (uint32_t p = tid; p < 2 * a.nslots; p += blockDim.x) sm[p] = 2 * a.slot_qubit[p >> 1] + (p & 1);
+    for (uint32_t p = tid; p < 2 * a.nslots; p += blockDim.x) sm[p] = 2 * a.slot_qubit[p >> 1] + ((p & 1) ^ slot_flip(p >> 1));
   const uint64_t ntiles = (a.ncols + T - 1) / T;
   const uint64_t my_tiles = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
   const uint64_t total_win = my_tiles * a.nwin;  // windows this CTA walks
@@ -1213,7 +1213,9 @@ static uint32_t balanced_tile(uint64_t ncols, uint32_t tmax) {
 // fit (a fixed part worth about 25 columns, the program's walk, and a part
 // per column), with k = 0.75 for power-of-two widths, whose warps' column
 // pairs cover whole rows of the tile and so meet no shared-memory bank
-// conflicts, 1.1 for 18 columns (nine pairs a row) and 1 otherwise; ties go
+// conflicts (0.6 for 16 columns, two rows at a time in opposite banks: d = 23,
+// 2^20 shots: 16 columns 7.06 ms, 22 7.52; d = 21: 5.63, 28 columns 5.03),
+// 1.1 for 18 columns (nine pairs a row) and 1 otherwise; ties go
 // to the wider tile.  Measured on surface-code memory circuits (2^21 shots,
 // ms): d = 17: 32 columns 4.53, 42 (fewest waves) 5.29; d = 19: 32 5.98, 34
 // 8.02; d = 21: 28 14.36, 16 16.75; d = 23: 22 20.21, 16 20.73; d = 25: 16
@@ -1226,7 +1228,7 @@ static uint32_t smem_tile(uint64_t ncols, uint32_t tmax, uint32_t tmin = 16) {
   uint64_t best_cost = UINT64_MAX;
   for (uint32_t t = tmin; t <= tmax; t += 2) {
     const uint64_t waves = ((ncols + t - 1) / t + nsm - 1) / nsm;
-    const uint64_t k = (t & (t - 1)) == 0 ? 75 : t == 18 ? 110 : 100;
+    const uint64_t k = t == 16 ? 60 : (t & (t - 1)) == 0 ? 75 : t == 18 ? 110 : 100;
     const uint64_t cost = waves * (2500 + k * t);
     if (cost <= best_cost) { best = t; best_cost = cost; }
   }

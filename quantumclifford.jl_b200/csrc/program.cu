@@ -136,7 +136,7 @@ static void binomial_count_table(double p, std::vector<uint32_t>& out) {
   }
 }
 
-int compile(const qcb_op* ops, size_t n_ops, Program& P) {
+int compile(const qcb_op* ops, size_t n_ops, Program& P, bool flip) {
   std::memset(&P.info, 0, sizeof(P.info));
   P.info.n_ops = (uint32_t)n_ops;
   std::vector<LOp> low;
@@ -252,6 +252,7 @@ int compile(const qcb_op* ops, size_t n_ops, Program& P) {
   }
   P.nslots = (uint32_t)P.slot_qubit.size();
   std::vector<uint8_t> swp(P.nslots, 0);
+  for (uint32_t k = 0; flip && k < P.nslots; k++) swp[k] = slot_flip(k);
   Emitter E{P.stream_slot, swp, qslot};
   P.stream_slot.clear();
   P.sites_slot.assign(nsites, Site{});
@@ -291,8 +292,29 @@ int compile(const qcb_op* ops, size_t n_ops, Program& P) {
   struct Rec { uint32_t kind, entry_words; std::vector<uint32_t> w; };
   std::vector<Rec> recs;
   auto pk = [](uint32_t a, uint32_t b) { return a | (b << 16); };
+  // Two-qubit entries in the order of the tile's banks: in a 16-column tile a
+  // half-warp works on two neighbouring entries, whose words of an even and
+  // an odd plane lie in different halves of the 32 banks, so entries are
+  // paired with ones whose planes have the other parity (both operands, or
+  // else one).  The entries of a segment commute.
+  auto pair_parities = [&](std::vector<LOp>& seg) {
+    std::vector<LOp> by[4], out;
+    for (auto it = seg.rbegin(); it != seg.rend(); ++it) by[(it->xa & 1) | (it->xb & 1) << 1].push_back(*it);
+    out.reserve(seg.size());
+    auto take = [&](int a, int b) {
+      while (!by[a].empty() && !by[b].empty()) {
+        for (int c : {a, b}) { out.push_back(std::move(by[c].back())); by[c].pop_back(); }
+      }
+    };
+    take(0, 3); take(1, 2);
+    take(0, 1); take(0, 2); take(3, 1); take(3, 2);
+    for (auto& v : by)
+      for (; !v.empty(); v.pop_back()) out.push_back(std::move(v.back()));
+    seg.swap(out);
+  };
   auto emit_seg = [&](uint32_t kind, std::vector<LOp>& seg) {
     if (seg.empty()) return;
+    if (kind == SEG_CNOT || kind == SEG_CZ || kind == SEG_G2) pair_parities(seg);
     Rec r{kind, 2, {}};
     switch (kind) {
       case SEG_CNOT:
@@ -575,7 +597,7 @@ int qcb_program_compile(const qcb_op* ops, size_t n_ops, qcb_program** out) {
   *out = nullptr;
   if (n_ops && !ops) return fail(QCB_EARG, "qcb_program_compile: null ops");
   qcb_program* p = new qcb_program();
-  int st = compile(ops, n_ops, *p);
+  int st = compile(ops, n_ops, *p, true);
   if (st == QCB_OK) st = upload(*p);
   if (st != QCB_OK) { release(*p); delete p; return st; }
   *out = p;
@@ -587,7 +609,7 @@ int qcb_debug_program_dump(const qcb_op* ops, size_t n_ops, uint32_t* stream, si
                            uint32_t* slot_qubit, uint32_t* slot_swap, size_t slots_cap, size_t* n_slots,
                            qcb_program_info* info) {
   Program P;
-  int st = compile(ops, n_ops, P);
+  int st = compile(ops, n_ops, P, false);  // x planes first in every slot
   if (st != QCB_OK) return st;
   if (stream_len) *stream_len = P.stream_slot.size();
   if (n_sites) *n_sites = P.sites_slot.size();

@@ -147,6 +147,14 @@ struct Site {
   double peff, q0, r;
 };
 
+// The tile's planes 2s and 2s + 1 hold the x and z bits of slot s, in the
+// other order for odd slots: the x planes of two slots (and their z planes)
+// then lie in different halves of the shared-memory banks as often as not,
+// where a 16-column tile's x planes in the even rows all met in one half.
+// With two-qubit entries paired by parity: d = 21, 150001 shots, p = 1e-3
+// 894 -> 813 us; d = 25, 2^17 shots 1342 -> 1204 us.
+__host__ __device__ inline uint32_t slot_flip(uint32_t s) { return s & 1u; }
+
 struct Program {
   qcb_program_info info;
   uint32_t nq;         // qubits referenced (max index)
@@ -157,7 +165,7 @@ struct Program {
   std::vector<Site> sites_slot;
   std::vector<int64_t> site_of_op;    // op index -> site (or -1)
   std::vector<uint32_t> site_arity;
-  std::vector<uint8_t> slot_swap;     // final x<->z relabel per slot
+  std::vector<uint8_t> slot_swap;     // plane (2s or 2s + 1) that slot's x bits end in
   std::vector<NoiseClass> classes;
   std::vector<uint32_t> cdf;          // Binomial count thresholds of the sparse classes
   double pmax = 0;

@@ -413,6 +413,26 @@ def test_presampled_noise_bit_exact(qcb, mode, which):
     assert np.array_equal(qcb.unpack_record(planes, frames), om)
 
 
+@pytest.mark.parametrize("tile", [0, 16])
+@pytest.mark.parametrize("p", [5e-4, 3e-3, 7e-3, 1.3e-2])
+def test_presampler_paths_by_event_count(qcb, p, tile):
+    """Event counts around the sampler's 3-, 6- and 12-event paths and above
+    them (means 0.5 to 13 a site and group), in 16-column tiles and the
+    chosen one: bit for bit the oracle's noise."""
+    circ, frames = circuits.rotated_surface_code_memory(7, 3, p), 5 * 1024 + 33
+    arr = O.to_array(circ)
+    qmax, bmax = O.affected_counts(arr)
+    qcb.check(qcb.lib().qcb_tune_set(b"walker_tile", tile))
+    try:
+        f = qcb.pftrajectories(arr, trajectories=frames, seed=77)
+        rec, xzs = f.measurements(), f.xzs()
+    finally:
+        qcb.check(qcb.lib().qcb_tune_set(b"walker_tile", 0))
+    ox, om = oracle.pftrajectories_philox(arr, frames, qmax, bmax, 77)
+    assert np.array_equal(rec, om)
+    assert np.array_equal(coding(xzs, qmax + 1), coding(ox, qmax + 1))
+
+
 @pytest.mark.parametrize("frames", [1, 31, 4097, 300_001])
 def test_measurements_download_chunks(qcb, frames):
     """measurements(frame) through the staged download: 32 MB chunks that
