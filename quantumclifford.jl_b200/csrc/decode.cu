@@ -36,9 +36,10 @@ __device__ __forceinline__ void swap_bits(uint32_t v[32], uint32_t m) {
 #pragma unroll
   for (uint32_t i = 0; i < 32; i++) {
     if (i & J) continue;
-    const uint32_t t = ((v[i] >> J) ^ v[i + J]) & m;
-    v[i + J] ^= t;
-    v[i] ^= t << J;
+    // two shifts and two selects; the exchange by XORs takes five
+    const uint32_t a = v[i], b = v[i + J];
+    v[i] = (a & m) | ((b << J) & ~m);
+    v[i + J] = ((a >> J) & m) | (b & ~m);
   }
 }
 
@@ -69,12 +70,17 @@ __device__ __forceinline__ void transpose32(uint32_t v[32]) {
 // words (blockIdx.x; 64 record rows each).  Half-warp h of warp w loads the 32
 // rows of 32-bit group 2w + h, a lane per column (64 contiguous bytes a row),
 // and each lane transposes its 32 x 32 bits in registers; the CTA's words are
-// staged in shared memory (a column's shots at an odd stride, so neither the
-// stores nor the loads meet bank conflicts) and leave as contiguous runs of
-// `pairs` words per shot.  Bound by DRAM (the record in, the matrix out).
-// 1e6 shots x 1441 bits: 93 us (364 MB, 3.9 TB/s); 519 us with a column per
-// CTA (4-byte reads a plane apart, 32 ballots per 32 x 32 block), 262 us with
-// the loads behind branches instead of predicates (one in flight at a time).
+// staged in shared memory, a column's shots at a stride of 2 mod 32 words (the
+// stores of a warp then hit 32 banks and the 64-bit loads are aligned), and
+// leave as contiguous runs of `pairs` words per shot, a column of 32 shots per
+// step of the CTA.  Bound by DRAM (the record in, the matrix out).
+// 1e6 shots x 1441 bits 85 us (364 MB, 4.3 TB/s), 150001 x 9681 73 us (5.0);
+// output steps of two shots a warp with an odd column stride, and exchanges by
+// five instructions: 92 and 93 us.  A persistent CTA with the next tile's
+// loads on their way while one leaves spills at 64 registers: 110 us.
+// With a column per CTA (4-byte reads a plane apart, 32 ballots per 32 x 32
+// block) 519 us, with the loads behind branches instead of predicates (one in
+// flight at a time) 262 us.
 constexpr uint32_t SYN_COLS = 16;
 constexpr uint32_t SYN_PAIRS = 16;  // output words of a CTA at most (512 threads)
 
@@ -83,9 +89,9 @@ __global__ void __launch_bounds__(32 * SYN_PAIRS, 2)
 syndrome_rows_kernel(const uint32_t* __restrict__ rec, uint64_t pitch, uint64_t ncols, uint64_t S,
                      const uint32_t* __restrict__ rows, uint32_t row0, uint32_t nsel, uint32_t Wsyn,
                      uint32_t pairs, uint64_t* __restrict__ out) {
-  extern __shared__ __align__(16) uint32_t tile[];  // [SYN_COLS][32 * RS + 1]
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const uint32_t RS = 2 * pairs, CS = 32 * RS + 1;  // words of a shot, of a column
+  extern __shared__ __align__(16) uint32_t tile[];  // [SYN_COLS][32 * RS + 2]
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;  // `pairs` warps
+  const uint32_t RS = 2 * pairs, CS = 32 * RS + 2;  // words of a shot, of a column
   const uint32_t w0 = blockIdx.x * pairs;           // the CTA's first output word
   const uint32_t words = min(pairs, Wsyn - w0);
   const uint64_t c0 = (uint64_t)blockIdx.y * SYN_COLS;
@@ -96,25 +102,31 @@ syndrome_rows_kernel(const uint32_t* __restrict__ rec, uint64_t pitch, uint64_t 
     // all 32 loads in flight: predicates, no branches
     const uint32_t lim = c < ncols ? min(32u, nsel - min(nsel, k0)) : 0u;
     uint32_t v[32];
+    if (LIST) {
 #pragma unroll
-    for (uint32_t i = 0; i < 32; i++) v[i] = LIST && i < lim ? __ldg(rows + k0 + i) : row0 + k0 + i;
+      for (uint32_t i = 0; i < 32; i++) v[i] = i < lim ? __ldg(rows + k0 + i) : 0u;
 #pragma unroll
-    for (uint32_t i = 0; i < 32; i++) v[i] = i < lim ? __ldcs(rec + (uint64_t)v[i] * pitch + c) : 0u;
+      for (uint32_t i = 0; i < 32; i++) v[i] = i < lim ? __ldcs(rec + (uint64_t)v[i] * pitch + c) : 0u;
+    } else {
+      const uint32_t* src = rec + (uint64_t)(row0 + k0) * pitch + c;  // read below lim only
+#pragma unroll
+      for (uint32_t i = 0; i < 32; i++, src += pitch) v[i] = i < lim ? __ldcs(src) : 0u;
+    }
     transpose32(v);
     uint32_t* t = tile + (size_t)cl * CS + 2 * warp + h;
 #pragma unroll
     for (uint32_t s = 0; s < 32; s++) t[s * RS] = v[s];
   }
   __syncthreads();
-  // half a warp per shot: its words are contiguous in out
-  const uint32_t wl = lane & 15;
+  // 32 * pairs threads: word wl of shot r of each column in turn
+  const uint32_t r = threadIdx.x / pairs, wl = threadIdx.x - r * pairs;
   if (wl >= words) return;
-  for (uint32_t s = 2 * warp + (lane >> 4); s < 32 * SYN_COLS; s += 2 * nw) {
-    const uint64_t shot = c0 * 32 + s;
-    if (shot >= S) break;
-    const uint32_t* t = tile + (size_t)(s >> 5) * CS + (s & 31) * RS + 2 * wl;
-    out[shot * Wsyn + w0 + wl] = (uint64_t)t[0] | ((uint64_t)t[1] << 32);
-  }
+  const uint32_t* t = tile + r * RS + 2 * wl;
+  uint64_t* o = out + (c0 * 32 + r) * Wsyn + w0 + wl;
+  const uint64_t step = (uint64_t)32 * Wsyn, left = S - c0 * 32;  // c0 < ncols: at least one shot
+#pragma unroll
+  for (uint32_t k = 0; k < SYN_COLS; k++, t += CS, o += step)
+    if (k * 32 + r < left) *o = *(const uint64_t*)t;
 }
 
 // guesses (column-major Bool S x k) -> planes [k][ncols] u32.
@@ -232,12 +244,16 @@ int qcb_frame_syndrome_rows(const qcb_frame* f, const uint32_t* bits, size_t nse
     QCB_CUDA(cudaMemcpyAsync(d_rows, rows.data(), nsel * 4, cudaMemcpyHostToDevice, st));
   }
   if (!out_on_device) QCB_CUDA(cudaMallocAsync(&d_out, out_bytes, st));
-  // words per CTA: the blocks of a shot's words as even as they divide
-  const uint32_t blocks = (Wsyn + SYN_PAIRS - 1) / SYN_PAIRS, pairs = (Wsyn + blocks - 1) / blocks;
-  const size_t sm = (size_t)SYN_COLS * (64 * pairs + 1) * 4;
+  // words per CTA: the blocks of a shot's words as even as they divide; 8 where
+  // the runs then start and end on 64 bytes of the output (150001 x 9681 73 us
+  // against 78 with 16, 2^20 x 2048 104 against 110; with Wsyn = 23 or 21
+  // shorter runs lose, 1e6 x 1320 89 against 81)
+  const uint32_t most = Wsyn % 8 ? SYN_PAIRS : 8;
+  const uint32_t blocks = (Wsyn + most - 1) / most, pairs = (Wsyn + blocks - 1) / blocks;
+  const size_t sm = (size_t)SYN_COLS * (64 * pairs + 2) * 4;
   auto kern = d_rows ? syndrome_rows_kernel<true> : syndrome_rows_kernel<false>;
   QCB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(SYN_COLS * (64 * SYN_PAIRS + 1) * 4)));
+                                (int)(SYN_COLS * (64 * SYN_PAIRS + 2) * 4)));
   // column blocks in slices of the grid's y limit (33.5e6 shots each)
   const uint64_t nblk = (f->ncols + SYN_COLS - 1) / SYN_COLS;
   for (uint64_t b0 = 0; b0 < nblk; b0 += 65535) {
