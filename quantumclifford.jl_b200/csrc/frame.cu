@@ -394,61 +394,141 @@ struct PresampleArgs {
   uint32_t force_overflow;  // test knob: every non-empty bucket reports more than its capacity
 };
 
-// Entry e on groups g0, g0 + gstep, ... below g1.
-__device__ __forceinline__ void presample_entries(const PresampleArgs& p, uint32_t e, uint64_t g0, uint64_t g1,
-                                                  uint64_t gstep) {
+// Sampler warps: the events of 32 (entry, group) pairs, drawn by their lanes
+// into shared memory, are finished by all lanes together, one event a lane.
+constexpr uint32_t SAMPLER_THREADS = 256;
+constexpr uint32_t SAMPLER_BLOCKS = 6;                      // Philox blocks of a pair at most
+constexpr uint32_t SAMPLER_EVENTS = 4 * SAMPLER_BLOCKS - 1;  // events of a pair at most (word 0 is the count's)
+struct SamplerWarp {
+  uint4 word[SAMPLER_BLOCKS][32];      // the pairs' noise words: block b of lane l
+  uint4 entry[32];                     // (entry index << 16 | Pauli noise << 8 | kinds, thr0, thr1, -)
+  uint16_t owner[32 * SAMPLER_EVENTS];  // event x: lane | event << 5
+  // word j of lane l's pair
+  __device__ __forceinline__ uint32_t& at(uint32_t l, uint32_t j) { return ((uint32_t*)&word[j >> 2][l])[j & 3]; }
+};
+
+// Words 1..k (k < 4 B) of the lane's pair (block 0 given), positions made
+// distinct: the procedure of sparse_emit, which runs only where the first
+// words have a position twice.
+template <uint32_t B>
+__device__ __forceinline__ void sampler_words(SamplerWarp& w, uint32_t lane, uint32_t site, uint32_t glo, uint32_t k0,
+                                              uint32_t k1, uint32_t k, const uint32_t o[4]) {
+  constexpr uint32_t PMASK = NOISE_GROUP - 1;
+  uint32_t v[4 * B];
+#pragma unroll
+  for (uint32_t i = 0; i < 4; i++) v[i] = o[i];
+#pragma unroll
+  for (uint32_t b = 1; b < B; b++) philox4x32_10(site, glo, b, TAG_NOISE, k0, k1, v + 4 * b);
+#pragma unroll
+  for (uint32_t b = 0; b < B; b++)
+    w.word[b][lane] = make_uint4(v[4 * b], v[4 * b + 1], v[4 * b + 2], v[4 * b + 3]);
+  bool dup = false;
+#pragma unroll
+  for (uint32_t e = 1; e < 4 * B; e++) {
+    v[e] = e <= k ? v[e] & PMASK : NOISE_GROUP + e;  // words not used: like no position and no other word
+#pragma unroll
+    for (uint32_t j = 1; j < e; j++) dup |= v[e] == v[j];
+  }
+  if (!dup) return;
+  uint32_t next = k + 1;  // next unused word
+  for (uint32_t e = 2; e <= k; e++) {
+    uint32_t x = w.at(lane, e);
+    for (uint32_t r = 0; r < NOISE_REDRAWS; r++) {
+      bool d = false;
+      for (uint32_t j = 1; j < e; j++) d |= ((x ^ w.at(lane, j)) & PMASK) == 0;
+      if (!d) break;
+      x = noise_word(site, glo, next++, k0, k1);
+    }
+    w.at(lane, e) = x;
+  }
+}
+
+// Entry e on groups g0, g0 + gstep, ... below g1 (the warp's lanes on
+// consecutive entries; the same groups for all).  Lanes whose count is small
+// wait for the largest, so only the words are drawn lane by lane; position,
+// kind and bucket slot of an event take one lane each.  Bound by instruction
+// issue (72%; a third of it Philox rounds).  d = 11, 1e6 shots, p = 1e-3: 139
+// -> 119 us; d = 21, 150001 shots, p = 4e-3: 302 -> 278 us against a lane for
+// all of a pair's events.
+__device__ __forceinline__ void presample_entries(const PresampleArgs& p, SamplerWarp& w, uint32_t e, uint64_t g0,
+                                                  uint64_t g1, uint64_t gstep) {
+  constexpr uint32_t FULL = 0xFFFFFFFFu;
   const uint32_t lane = threadIdx.x & 31;
   const bool valid = e < p.nent;
   const uint4 pe = valid ? p.ent[e] : make_uint4(0u, 0u, 0xFFFFFFFFu, 0u);
   NoiseClass c{};
   if (valid) c = p.classes[pe.y >> 8];
-  const uint32_t kind = pe.y & 0xFFu, j = pe.z;
+  const uint32_t kind = pe.y & 0xFFu, j = pe.z, tag = pe.w << 16;
   const uint32_t k0 = (uint32_t)p.seed, k1 = (uint32_t)(p.seed >> 32);
   const uint32_t off = valid ? p.capoff[j] : 0u, cap = valid ? p.capoff[j + 1] - off : 0u;
+  w.entry[lane] = make_uint4(tag | (kind == QCB_OP_PAULI_NOISE ? 256u : 0u) | c.np, (uint32_t)c.thr0, (uint32_t)c.thr1, 0u);
   // The entries are sorted by part, so the lanes of one part form a run
   // [first, last]: its events take one atomic on the bucket count (by the
   // run's last lane) and consecutive slots.
-  const uint32_t peers = __match_any_sync(0xFFFFFFFFu, j);
+  const uint32_t peers = __match_any_sync(FULL, j);
   const uint32_t first = __ffs(peers) - 1, last = 31 - __clz(peers);
-  const uint32_t tag = pe.w << 16;
   for (uint64_t g = g0; g < g1; g += gstep) {
     const uint32_t glo = (uint32_t)(p.g0 + g);
-    uint32_t o[4];
+    uint32_t o[4] = {0, 0, 0, 0};
     const uint32_t k = valid ? sparse_count(c, p.cdf, pe.x, glo, k0, k1, o) : 0u;
-    uint32_t inc = k;  // inclusive prefix of k over the run
+    const uint32_t top = __reduce_max_sync(FULL, k);
+    if (top == 0) continue;
+    uint32_t end = k;  // events of the lanes up to this one
 #pragma unroll
     for (uint32_t d = 1; d < 32; d <<= 1) {
-      const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, inc, d);
-      if (lane >= first + d) inc += v;
+      const uint32_t v = __shfl_up_sync(FULL, end, d);
+      if (lane >= d) end += v;
     }
+    const uint32_t total = __shfl_sync(FULL, end, 31);
+    uint32_t start = __shfl_sync(FULL, end, first ? first - 1 : 0u);  // of the run
+    if (first == 0) start = 0;
     uint32_t base = 0;
-    if (lane == last && inc) base = atomicAdd(p.cnt + g * p.nparts + j, inc + (p.force_overflow ? cap + 1 : 0u));
-    base = __shfl_sync(0xFFFFFFFFu, base, last);
-    const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, k);
-    if (k == 0) continue;
-    uint32_t* bk = p.buf + g * p.capg + off;
-    uint32_t t = base + inc - k;
-    auto put = [&](uint32_t pos, uint32_t code) {
-      if (t < cap) bk[t] = tag | (code << 10) | pos;
-      t++;
-    };
-    // the register path by the warp's largest count: its lanes then run one
-    // path (two cost the sum of their lengths), and the bitmap, whose
-    // positions go through local memory one by one, is left to counts above
-    // 12 (mean 4, d = 21 at p = 4e-3: sampler and walk 1520 -> 1292 us with
-    // the walk's batched event loads)
-    if (top <= 3) sparse_emit<3>(c, kind, pe.x, glo, k0, k1, k, o, put);
-    else if (top <= 6) sparse_emit<6>(c, kind, pe.x, glo, k0, k1, k, o, put);
-    else sparse_emit<12>(c, kind, pe.x, glo, k0, k1, k, o, put);
+    if (lane == last && end != start)
+      base = atomicAdd(p.cnt + g * p.nparts + j, end - start + (p.force_overflow ? cap + 1 : 0u));
+    uint32_t* bk = p.buf + g * p.capg;
+    if (top > SAMPLER_EVENTS) {  // longer lists: a lane a pair
+      base = __shfl_sync(FULL, base, last);
+      uint32_t t = base + end - k - start;
+      if (k)
+        sparse_emit(c, kind, pe.x, glo, k0, k1, k, o, [&](uint32_t pos, uint32_t code) {
+          if (t < cap) bk[off + t] = tag | (code << 10) | pos;
+          t++;
+        });
+      continue;
+    }
+    __syncwarp();  // the events of the previous group are read
+    if (top <= 3) sampler_words<1>(w, lane, pe.x, glo, k0, k1, k, o);
+    else if (top <= 7) sampler_words<2>(w, lane, pe.x, glo, k0, k1, k, o);
+    else if (top <= 11) sampler_words<3>(w, lane, pe.x, glo, k0, k1, k, o);
+    else if (top <= 15) sampler_words<4>(w, lane, pe.x, glo, k0, k1, k, o);
+    else sampler_words<SAMPLER_BLOCKS>(w, lane, pe.x, glo, k0, k1, k, o);
+    for (uint32_t i = 0; i < k; i++) w.owner[end - k + i] = (uint16_t)(lane | i << 5);
+    base = __shfl_sync(FULL, base, last);
+    // event x of the warp: slot base - start + x of its run's bucket
+    const uint32_t slot = off + base - start;
+    const int32_t lim = (int32_t)cap - (int32_t)(base - start);  // x < lim: inside the bucket
+    __syncwarp();
+    for (uint32_t x0 = 0; x0 < total; x0 += 32) {
+      const uint32_t x = x0 + lane, ow = w.owner[min(x, total - 1)];
+      const uint32_t l = ow & 31u, wd = w.at(l, 1 + (ow >> 5)), v = wd >> 10;
+      const uint4 en = w.entry[l];
+      const uint32_t to = __shfl_sync(FULL, slot, l);
+      const int32_t lm = __shfl_sync(FULL, lim, l);
+      const uint32_t uni = 1u + ((v * (en.x & 255u)) >> NOISE_KIND_BITS);  // sparse_code
+      const uint32_t xzy = v < en.y ? 1u : v < en.z ? 2u : 3u;
+      const uint32_t code = (en.x & 256u) ? xzy : uni;
+      if (x < total && (int32_t)x < lm) bk[to + x] = (en.x & 0xFFFF0000u) | (code << 10) | (wd & (NOISE_GROUP - 1));
+    }
   }
 }
 
-__global__ void __launch_bounds__(256) presample_kernel(const PresampleArgs p) {
+__global__ void __launch_bounds__(SAMPLER_THREADS, 4) presample_kernel(const PresampleArgs p) {
+  __shared__ SamplerWarp ws[SAMPLER_THREADS / 32];
   // the walker that reads these buckets is a programmatic dependent: let it
   // launch once every sampler CTA is resident, so that its CTAs take the SMs
   // of the sampler's last wave as they free up (it waits before its first read)
   asm volatile("griddepcontrol.launch_dependents;");
-  presample_entries(p, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y, p.ngroups, gridDim.y);
+  presample_entries(p, ws[threadIdx.x >> 5], blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y, p.ngroups, gridDim.y);
 }
 
 // The jobs of a batch in one launch: block b takes item b, 256 entries of one
@@ -458,11 +538,13 @@ struct PresampleItem {
 };
 constexpr uint32_t PRESAMPLE_ITEM_GROUPS = 16;
 
-__global__ void __launch_bounds__(256) presample_batch_kernel(const PresampleArgs* jobs, const PresampleItem* items) {
+__global__ void __launch_bounds__(SAMPLER_THREADS, 4)
+presample_batch_kernel(const PresampleArgs* jobs, const PresampleItem* items) {
+  __shared__ SamplerWarp ws[SAMPLER_THREADS / 32];
   asm volatile("griddepcontrol.launch_dependents;");
   const PresampleItem it = items[blockIdx.x];
   const PresampleArgs p = jobs[it.job];
-  presample_entries(p, it.e0 + threadIdx.x, it.g0, min((uint64_t)it.g0 + PRESAMPLE_ITEM_GROUPS, p.ngroups), 1);
+  presample_entries(p, ws[threadIdx.x >> 5], it.e0 + threadIdx.x, it.g0, min((uint64_t)it.g0 + PRESAMPLE_ITEM_GROUPS, p.ngroups), 1);
 }
 
 // ---------------------------------------------------------------- walker
@@ -1360,7 +1442,7 @@ static int launch_presample(qcb_frame* f, const qcb_program* p, WalkArgs& a, cud
   const uint32_t gx = (q.nent + 255) / 256;
   const uint64_t gy = std::max<uint64_t>(1, ((uint64_t)device_sm_count() * 8 + gx - 1) / gx);
   const dim3 grid(gx, (uint32_t)std::min<uint64_t>(std::min<uint64_t>(q.ngroups, gy), 65535));
-  presample_kernel<<<grid, 256, 0, st>>>(q);
+  presample_kernel<<<grid, SAMPLER_THREADS, 0, st>>>(q);
   QCB_LAUNCHED();
   return QCB_OK;
 }
@@ -2041,7 +2123,7 @@ int qcb_batch_run(qcb_batch* b, void* stream) {
   QCB_CUDA(cudaMemsetAsync(b->d_head, 0, 4, st));
   if (b->n_pre_items) {
     QCB_CUDA(cudaMemsetAsync(b->pre, 0, b->pre_cnt_bytes, st));
-    presample_batch_kernel<<<b->n_pre_items, 256, 0, st>>>(b->d_pre_jobs, b->d_pre_items);
+    presample_batch_kernel<<<b->n_pre_items, SAMPLER_THREADS, 0, st>>>(b->d_pre_jobs, b->d_pre_items);
     QCB_LAUNCHED();
   }
   // the walker as the sampler's programmatic dependent, as in a plain run
