@@ -133,7 +133,7 @@ struct Tile {
   uint32_t* planes;
   const uint32_t* pmap;
   uint64_t pitch;
-  uint32_t T;
+  uint32_t T, cols;  // width; columns inside the frame
   // word of plane p at tile column cl (frame column cg)
   __device__ __forceinline__ uint32_t* at32(uint32_t p, uint32_t cl, uint64_t cg) const {
     if (SMEM) return sm + p * T + cl;
@@ -220,25 +220,29 @@ __device__ __forceinline__ uint32_t sparse_code(uint32_t kind, const NoiseClass&
   return 1u + ((v * c.np) >> NOISE_KIND_BITS);
 }
 
-// Flip the event's Pauli into the tile at group shot `pos`; lc0 is the tile
-// column of the group's first column (a group may straddle tiles: columns
-// outside [0, T) belong to a neighbouring tile, which draws the same events).
+// Flip an event's Pauli into the tile at bit `pos` of tile column cl, a column
+// inside the frame.  Codes of one-qubit sites are below 4 (higher bits of
+// `code` than these four are not looked at).
 // e = (site, kind | class<<8, x_a | z_a<<16, x_b | z_b<<16).
 template <bool SMEM>
-__device__ __forceinline__ void apply_code(const Tile<SMEM>& F, const uint4& e, uint32_t code, int32_t lc0,
-                                           uint32_t pos, uint64_t c0, uint64_t ncols) {
-  const int32_t lc = lc0 + (int32_t)(pos >> 5);
-  if (lc < 0 || lc >= (int32_t)F.T) return;
-  const uint32_t cl = (uint32_t)lc;
+__device__ __forceinline__ void flip_code(const Tile<SMEM>& F, const uint4& e, uint32_t code, uint32_t cl,
+                                          uint32_t pos, uint64_t c0) {
   const uint64_t cg = c0 + cl;
-  if (cg >= ncols) return;
   const uint32_t bit = 1u << (pos & 31);
   if (code & 1) atomicXor(F.at32(e.z & 0xFFFFu, cl, cg), bit);
   if (code & 2) atomicXor(F.at32(e.z >> 16, cl, cg), bit);
-  if ((e.y & 0xFFu) == QCB_OP_DEPOL2) {
-    if (code & 4) atomicXor(F.at32(e.w & 0xFFFFu, cl, cg), bit);
-    if (code & 8) atomicXor(F.at32(e.w >> 16, cl, cg), bit);
-  }
+  if (code & 4) atomicXor(F.at32(e.w & 0xFFFFu, cl, cg), bit);
+  if (code & 8) atomicXor(F.at32(e.w >> 16, cl, cg), bit);
+}
+
+// The same at group shot `pos`; lc0 is the tile column of the group's first
+// column (a group may straddle tiles: columns outside [0, F.cols) belong to a
+// neighbouring tile, which draws the same events, or lie past the frame).
+template <bool SMEM>
+__device__ __forceinline__ void apply_code(const Tile<SMEM>& F, const uint4& e, uint32_t code, int32_t lc0,
+                                           uint32_t pos, uint64_t c0) {
+  const uint32_t cl = (uint32_t)(lc0 + (int32_t)(pos >> 5));
+  if (cl < F.cols) flip_code<SMEM>(F, e, code, cl, pos, c0);
 }
 
 // Word i of the noise stream of (site, group G): lane i % 4 of Philox block
@@ -358,7 +362,7 @@ __device__ __forceinline__ void sample_site_group(const WalkArgs& a, const Tile<
 #pragma unroll
       for (uint32_t j = 0; j < 4; j++) {
         const uint32_t code = dense_code(kind, c, o[j]);
-        if (code) apply_code<SMEM>(F, e, code, lc0, blk * 4 + j, c0, a.ncols);
+        if (code) apply_code<SMEM>(F, e, code, lc0, blk * 4 + j, c0);
       }
     }
     return;
@@ -366,7 +370,7 @@ __device__ __forceinline__ void sample_site_group(const WalkArgs& a, const Tile<
   const uint32_t k = sparse_count(c, a.cdf, site, glo, k0, k1, o);
   if (k == 0) return;
   sparse_emit(c, kind, site, glo, k0, k1, k, o,
-              [&](uint32_t pos, uint32_t code) { apply_code<SMEM>(F, e, code, lc0, pos, c0, a.ncols); });
+              [&](uint32_t pos, uint32_t code) { apply_code<SMEM>(F, e, code, lc0, pos, c0); });
 }
 
 // ---------------------------------------------------------------- pre-sampling
@@ -574,7 +578,7 @@ __device__ __forceinline__ bool walk_tile(const WalkArgs& a, uint32_t* sm, uint3
   const uint64_t col = a.col0 + cg, col1 = col + 1;
   const uint32_t clo = (uint32_t)col, chi = (uint32_t)(col >> 32);
   const uint32_t clo1 = (uint32_t)col1, chi1 = (uint32_t)(col1 >> 32);
-  const Tile<SMEM> F{sm, a.planes, sm, pitch, T};
+  const Tile<SMEM> F{sm, a.planes, sm, pitch, T, (uint32_t)min((uint64_t)T, a.ncols - c0)};
 
   // ---- initial frame
   if (a.fresh) {
@@ -619,6 +623,7 @@ __device__ __forceinline__ bool walk_tile(const WalkArgs& a, uint32_t* sm, uint3
   // flush, they arrive while the following records run)
   const uint64_t pG0 = (a.col0 + c0) / 32;
   const uint32_t png = (uint32_t)((a.col0 + min(c0 + T, a.ncols) - 1) / 32 - pG0 + 1);
+  const int32_t lcol0 = -(int32_t)((a.col0 + c0) & 31u);  // tile column of group pG0's first column
   const uint32_t pS = blockDim.x / png, pgl = tid / pS, pl = tid - pgl * pS;
   const bool pre = PRE && PHILOX && a.pre_buf != nullptr && pgl < png;
   const uint32_t* pbase = pre ? a.pre_buf + (pG0 + pgl - a.col0 / 32) * a.pre_capg : nullptr;
@@ -795,14 +800,17 @@ __device__ __forceinline__ bool walk_tile(const WalkArgs& a, uint32_t* sm, uint3
           if (a.pmax > 0.0) {
             // (site, shot group) tasks over all threads of the CTA; a group
             // is 32 run columns and may straddle the tile's edges
-            const uint64_t gc0 = a.col0 + c0;
-            const uint64_t gc1 = a.col0 + min(c0 + T, a.ncols);
-            const uint64_t G0 = gc0 / 32;
-            const uint32_t ng = (uint32_t)((gc1 - 1) / 32 - G0 + 1);
-            const uint32_t ntask = cnt * ng;
-            // t / ng as a multiply-high for ng >= 2: ng <= 10 and t < 2^13 (a
-            // record part fits one window), far inside t * (mg * ng - 2^32) < 2^32
-            const uint32_t mg = ng > 1 ? 0xFFFFFFFFu / ng + 1u : 0u;
+            auto draw = [&](bool dense_only) {
+              const uint32_t ntask = cnt * png;
+              // t / png as a multiply-high for png >= 2: png <= 10 and t < 2^13 (a
+              // record part fits one window), far inside t * (mg * png - 2^32) < 2^32
+              const uint32_t mg = png > 1 ? 0xFFFFFFFFu / png + 1u : 0u;
+              for (uint32_t t = tid; t < ntask; t += blockDim.x) {
+                const uint32_t i = png > 1 ? __umulhi(t, mg) : t, gt = t - i * png;
+                if (dense_only && !a.classes[en[i].y >> 8].dense) continue;
+                sample_site_group<SMEM>(a, F, en[i], pG0 + gt, lcol0 + 32 * (int32_t)gt, c0);
+              }
+            };
             if (PRE && a.pre_buf) {
               // pre-sampled: bucket (group G0 + pgl, part j), the count and
               // first events loaded at the previous flush part
@@ -811,12 +819,11 @@ __device__ __forceinline__ bool walk_tile(const WalkArgs& a, uint32_t* sm, uint3
               prefetch(j + 1, off + cap);
               if (pre && cap) {
                 const uint32_t* bk = pbase + off;
-                const int32_t lc0 = (int32_t)((int64_t)((pG0 + pgl) * 32) - (int64_t)gc0);
+                const int32_t lc0 = lcol0 + 32 * (int32_t)pgl;
                 if (total <= cap) {
                   auto put = [&](uint32_t ev) {
-                    const int32_t lc = lc0 + (int32_t)((ev & (NOISE_GROUP - 1)) >> 5);
-                    if (lc < 0 || lc >= (int32_t)T) return;  // a neighbouring tile's
-                    apply_code<SMEM>(F, en[ev >> 16], (ev >> 10) & 15u, lc0, ev & (NOISE_GROUP - 1), c0, a.ncols);
+                    const uint32_t cl = (uint32_t)(lc0 + (int32_t)((ev & (NOISE_GROUP - 1)) >> 5));
+                    if (cl < F.cols) flip_code<SMEM>(F, en[ev >> 16], ev >> 10, cl, ev, c0);
                   };
                   if (pl < total) put(ev0);
                   if (pl + pS < total) put(ev1);
@@ -835,20 +842,9 @@ __device__ __forceinline__ bool walk_tile(const WalkArgs& a, uint32_t* sm, uint3
                     if (!a.classes[en[i].y >> 8].dense) sample_site_group<SMEM>(a, F, en[i], pG0 + pgl, lc0, c0);
                 }
               }
-              if (h.y & FLAG_DENSE_SITES) {  // dense sites are drawn in the walk
-                for (uint32_t t = tid; t < ntask; t += blockDim.x) {
-                  const uint32_t i = ng > 1 ? __umulhi(t, mg) : t, gt = t - i * ng;
-                  if (!a.classes[en[i].y >> 8].dense) continue;
-                  const int32_t lc0 = (int32_t)((int64_t)((G0 + gt) * 32) - (int64_t)gc0);
-                  sample_site_group<SMEM>(a, F, en[i], G0 + gt, lc0, c0);
-                }
-              }
+              if (h.y & FLAG_DENSE_SITES) draw(true);  // dense sites are drawn in the walk
             } else {
-              for (uint32_t t = tid; t < ntask; t += blockDim.x) {
-                const uint32_t i = ng > 1 ? __umulhi(t, mg) : t, gl = t - i * ng;
-                const int32_t lc0 = (int32_t)((int64_t)((G0 + gl) * 32) - (int64_t)gc0);
-                sample_site_group<SMEM>(a, F, en[i], G0 + gl, lc0, c0);
-              }
+              draw(false);
             }
           }
         } else if (rr == 0 && act) {

@@ -298,28 +298,23 @@ int compile(const qcb_op* ops, size_t n_ops, Program& P, bool flip) {
   // paired with ones whose planes have the other parity (both operands, or
   // else one).  The entries of a segment commute.
   auto pair_parities = [&](std::vector<LOp>& seg) {
-    std::vector<LOp> by[4], out;
-    for (auto it = seg.rbegin(); it != seg.rend(); ++it) by[(it->xa & 1) | (it->xb & 1) << 1].push_back(*it);
-    out.reserve(seg.size());
-    auto take = [&](int a, int b) {
-      while (!by[a].empty() && !by[b].empty()) {
-        for (int c : {a, b}) { out.push_back(std::move(by[c].back())); by[c].pop_back(); }
-      }
-    };
-    take(0, 3); take(1, 2);
-    take(0, 1); take(0, 2); take(3, 1); take(3, 2);
-    for (auto& v : by)
-      for (; !v.empty(); v.pop_back()) out.push_back(std::move(v.back()));
-    seg.swap(out);
+    std::vector<uint32_t> by[4], order;
+    for (uint32_t i = (uint32_t)seg.size(); i-- > 0;) by[(seg[i].xa & 1) | (seg[i].xb & 1) << 1].push_back(i);
+    order.reserve(seg.size());
+    auto pop = [&](int c) { order.push_back(by[c].back()); by[c].pop_back(); };
+    for (auto [a, b] : {std::pair{0, 3}, {1, 2}, {0, 1}, {0, 2}, {3, 1}, {3, 2}})
+      while (!by[a].empty() && !by[b].empty()) { pop(a); pop(b); }
+    for (int c = 0; c < 4; c++)
+      while (!by[c].empty()) pop(c);
+    return order;
   };
   auto emit_seg = [&](uint32_t kind, std::vector<LOp>& seg) {
     if (seg.empty()) return;
-    if (kind == SEG_CNOT || kind == SEG_CZ || kind == SEG_G2) pair_parities(seg);
     Rec r{kind, 2, {}};
     switch (kind) {
       case SEG_CNOT:
       case SEG_CZ:  // (x_a | z_a << 16, x_b | z_b << 16)
-        for (auto& o : seg) { r.w.push_back(pk(o.xa, o.za)); r.w.push_back(pk(o.xb, o.zb)); }
+        for (uint32_t i : pair_parities(seg)) { const LOp& o = seg[i]; r.w.push_back(pk(o.xa, o.za)); r.w.push_back(pk(o.xb, o.zb)); }
         break;
       case SEG_S:
       case SEG_G1:  // (x | z << 16, opcode)
@@ -327,7 +322,7 @@ int compile(const qcb_op* ops, size_t n_ops, Program& P, bool flip) {
         break;
       case SEG_G2:  // (x_a | z_a << 16, x_b | z_b << 16, opcode, 0)
         r.entry_words = 4;
-        for (auto& o : seg) { r.w.push_back(pk(o.xa, o.za)); r.w.push_back(pk(o.xb, o.zb)); r.w.push_back(o.opcode); r.w.push_back(0); }
+        for (uint32_t i : pair_parities(seg)) { const LOp& o = seg[i]; r.w.push_back(pk(o.xa, o.za)); r.w.push_back(pk(o.xb, o.zb)); r.w.push_back(o.opcode); r.w.push_back(0); }
         break;
       case SEG_MZ:  // (x, bit)
         for (auto& o : seg) { r.w.push_back(o.xa); r.w.push_back(o.bit); }

@@ -414,11 +414,11 @@ def test_presampled_noise_bit_exact(qcb, mode, which):
 
 
 @pytest.mark.parametrize("tile", [0, 16])
-@pytest.mark.parametrize("p", [5e-4, 3e-3, 7e-3, 1.3e-2])
+@pytest.mark.parametrize("p", [5e-4, 3e-3, 7e-3, 1.1e-2, 1.5e-2])
 def test_presampler_paths_by_event_count(qcb, p, tile):
-    """Event counts around the sampler's 3-, 6- and 12-event paths and above
-    them (means 0.5 to 13 a site and group), in 16-column tiles and the
-    chosen one: bit for bit the oracle's noise."""
+    """Event counts on every path of the sampler (3 to 23 events of a site and
+    group, and more; means 0.5 to 15), in 16-column tiles and the chosen one:
+    bit for bit the oracle's noise."""
     circ, frames = circuits.rotated_surface_code_memory(7, 3, p), 5 * 1024 + 33
     arr = O.to_array(circ)
     qmax, bmax = O.affected_counts(arr)
