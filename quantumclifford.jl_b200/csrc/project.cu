@@ -1006,28 +1006,31 @@ __global__ void __launch_bounds__(MID_THREADS) project_mid_kernel(const ProjPane
       uint2 sb[PSTEPS];       // (pivot row, Pauli)
     } r;
   } s;
+  const PanelTiles& p = a.p;
+  const uint32_t tid = threadIdx.x, blk = blockIdx.x;
+  // While S runs: the Paulis' words of the tile as the tiles keep them, or the
+  // rows' panel words (S was launched behind the apply that wrote them).
+  __shared__ ulonglong2 pw[PSTEPS][2];
+  const uint32_t r = blk > p.ntile ? (blk - p.ntile - 1) * MID_THREADS + tid : p.rows;
+  uint64_t w = 0;
+  if (blk < p.ntile) {
+    const uint32_t b = tid >> 2, c = 2 * blk + (tid & 1);
+    ((uint64_t*)pw[b])[tid & 3] =
+        b < a.cnt && c < p.len ? a.paulis[(size_t)(a.j0 + b) * p.W + (tid & 2 ? p.len : 0) + c] : 0ull;
+  } else if (r < p.rows) {
+    w = a.word[r];
+  }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;");
   PanelRecord& g = *a.rec;
-  const PanelTiles& p = a.p;
-  const uint32_t tid = threadIdx.x, blk = blockIdx.x, T = g.T;
+  const uint32_t T = g.T;
   if (blk < p.ntile) {
-    const bool two = 2 * blk + 1 < p.len;
-    // a Pauli's words of the tile as the tiles keep them
-    __shared__ ulonglong2 pw[PSTEPS][2];
-    if (tid < PSTEPS) {
-      const uint32_t sr = g.src[tid];
-      if (tid < T && sr < PSTEPS) {
-        const uint64_t* P = a.paulis + (size_t)(a.j0 + g.bt[sr]) * p.W + 2 * blk;
-        pw[tid][0] = make_ulonglong2(P[0], two ? P[1] : 0ull);
-        pw[tid][1] = make_ulonglong2(P[p.len], two ? P[p.len + 1] : 0ull);
-      }
-    }
     __syncthreads();
     tile_reduce(
         p, g, blk, s.t,
         [&](uint32_t t, uint32_t r) -> const ulonglong2* {
-          return t < T && g.src[t] < PSTEPS ? pw[t] : p.t + ((size_t)blk * p.rows + r) * 2;
+          const uint32_t sr = t < T ? g.src[t] : PSTEPS;
+          return sr < PSTEPS ? pw[g.bt[sr]] : p.t + ((size_t)blk * p.rows + r) * 2;
         },
         [&](uint32_t t, uint32_t r) -> uint32_t {
           const uint32_t sr = g.src[t];
@@ -1062,10 +1065,9 @@ __global__ void __launch_bounds__(MID_THREADS) project_mid_kernel(const ProjPane
     }
     return;
   }
-  const uint32_t r = (blk - p.ntile - 1) * MID_THREADS + tid;
   if (r >= p.rows) return;
   a.wordn[r] = 0;
-  uint64_t w = a.word[r], U = 0;
+  uint64_t U = 0;
   uint32_t base = BASE_ROW;
   const uint32_t partner = r < a.nn ? r + a.nn : 0xFFFFFFFEu;  // its stabilizer row
 #pragma unroll 4
@@ -1147,11 +1149,26 @@ struct ApplyFlagSmem {
 // AF.
 __global__ void __launch_bounds__(1024) project_apply_kernel(const ProjPanelArgs a) {
   extern __shared__ __align__(16) uint8_t dsm[];
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;");
   const PanelRecord& g = *a.rec;
   const PanelTiles& p = a.p;
-  const uint32_t tid = threadIdx.x, blk = blockIdx.x, T = a.apply ? g.T : 0u;
+  const uint32_t tid = threadIdx.x, blk = blockIdx.x;
+  // While M runs: the next Paulis' tables, and the thread's first row (the
+  // previous apply wrote it, and S waited for that).
+  const uint32_t u = blk < a.nq ? 0u : blk - a.nq, tile = u / a.groups, grp = u - tile * a.groups;
+  const uint32_t r0 = grp * a.per + tid, r1 = min(p.rows, (grp + 1) * a.per);
+  ApplyFlagSmem& s = *(ApplyFlagSmem*)dsm;
+  ulonglong2 x0 = make_ulonglong2(0, 0), z0 = x0;
+  if (blk >= a.nq) {
+    if (a.apply && r0 < r1) {
+      const ulonglong2* d = p.t + ((size_t)tile * p.rows + r0) * 2;
+      x0 = d[0];
+      z0 = d[1];
+    }
+    if (a.cntn) flag_tables(a, tile, s.f);
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+  const uint32_t T = a.apply ? g.T : 0u;
   if (blk < a.nq) {  // q of every row
     if (!T) return;
     PhaseSmem& s = *(PhaseSmem*)dsm;
@@ -1174,20 +1191,17 @@ __global__ void __launch_bounds__(1024) project_apply_kernel(const ProjPanelArgs
   }
   const bool next = a.cntn && !a.state[0];
   if (!T && !next) return;
-  const uint32_t u = blk - a.nq, tile = u / a.groups, grp = u - tile * a.groups;
-  ApplyFlagSmem& s = *(ApplyFlagSmem*)dsm;
   if (T) apply_tables(p, tile, s.a);
-  if (next) flag_tables(a, tile, s.f);
   const bool two = 2 * tile + 1 < p.len;
   auto pauli = [&](uint32_t j, ulonglong2& x, ulonglong2& z) {
     const uint64_t* P = a.paulis + (size_t)j * p.W + 2 * tile;
     x = make_ulonglong2(P[0], two ? P[1] : 0ull);
     z = make_ulonglong2(P[p.len], two ? P[p.len + 1] : 0ull);
   };
-  const uint32_t r1 = min(p.rows, (grp + 1) * a.per);
-  for (uint32_t r = grp * a.per + tid; r < r1; r += blockDim.x) {
+  for (uint32_t r = r0; r < r1; r += blockDim.x) {
     ulonglong2* d = p.t + ((size_t)tile * p.rows + r) * 2;
-    ulonglong2 x = d[0], z = d[1];
+    const bool have = a.apply && r == r0;
+    ulonglong2 x = have ? x0 : d[0], z = have ? z0 : d[1];
     if (T) {
       const uint64_t U = p.U[r];
       const uint32_t base = a.base[r];
