@@ -1009,16 +1009,17 @@ __global__ void __launch_bounds__(MID_THREADS) project_mid_kernel(const ProjPane
   const PanelTiles& p = a.p;
   const uint32_t tid = threadIdx.x, blk = blockIdx.x;
   // While S runs: the Paulis' words of the tile as the tiles keep them, or the
-  // rows' panel words (S was launched behind the apply that wrote them).
+  // rows' panel words.  S waited for the apply that wrote them before it let
+  // this kernel start, so they are in L2; loads before the wait pass L1 by.
   __shared__ ulonglong2 pw[PSTEPS][2];
   const uint32_t r = blk > p.ntile ? (blk - p.ntile - 1) * MID_THREADS + tid : p.rows;
   uint64_t w = 0;
   if (blk < p.ntile) {
     const uint32_t b = tid >> 2, c = 2 * blk + (tid & 1);
     ((uint64_t*)pw[b])[tid & 3] =
-        b < a.cnt && c < p.len ? a.paulis[(size_t)(a.j0 + b) * p.W + (tid & 2 ? p.len : 0) + c] : 0ull;
+        b < a.cnt && c < p.len ? __ldcg(a.paulis + (size_t)(a.j0 + b) * p.W + (tid & 2 ? p.len : 0) + c) : 0ull;
   } else if (r < p.rows) {
-    w = a.word[r];
+    w = __ldcg(a.word + r);
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;");
@@ -1107,8 +1108,8 @@ __device__ __forceinline__ void flag_tables(const ProjPanelArgs& a, uint32_t til
     const uint32_t k = warp >> 3, q = k ^ 2, c = 2 * tile + (q & 1);
     const bool in = c < p.len;
     const uint64_t* P = a.paulis + (size_t)a.jn * p.W + (q >= 2 ? p.len : 0) + c;
-    const uint64_t v0 = in && lane < a.cntn ? P[(size_t)lane * p.W] : 0ull;
-    const uint64_t v1 = in && lane + 32 < a.cntn ? P[(size_t)(lane + 32) * p.W] : 0ull;
+    const uint64_t v0 = in && lane < a.cntn ? __ldcg(P + (size_t)lane * p.W) : 0ull;
+    const uint64_t v1 = in && lane + 32 < a.cntn ? __ldcg(P + (size_t)(lane + 32) * p.W) : 0ull;
     for (uint32_t b = 8 * (warp & 7), e = b + 8; b < e; b++) {
       const uint32_t lo = __ballot_sync(0xFFFFFFFFu, (v0 >> b) & 1ull), hi = __ballot_sync(0xFFFFFFFFu, (v1 >> b) & 1ull);
       if (lane == 0) s.col[64 * k + b] = (uint64_t)lo | ((uint64_t)hi << 32);
@@ -1153,7 +1154,8 @@ __global__ void __launch_bounds__(1024) project_apply_kernel(const ProjPanelArgs
   const PanelTiles& p = a.p;
   const uint32_t tid = threadIdx.x, blk = blockIdx.x;
   // While M runs: the next Paulis' tables, and the thread's first row (the
-  // previous apply wrote it, and S waited for that).
+  // previous apply wrote it, and S waited for that; loads past L1 as in M).
+  // 1000 Paulis, n = 1000 with destabilizers: 587 -> 530 us.
   const uint32_t u = blk < a.nq ? 0u : blk - a.nq, tile = u / a.groups, grp = u - tile * a.groups;
   const uint32_t r0 = grp * a.per + tid, r1 = min(p.rows, (grp + 1) * a.per);
   ApplyFlagSmem& s = *(ApplyFlagSmem*)dsm;
@@ -1161,8 +1163,8 @@ __global__ void __launch_bounds__(1024) project_apply_kernel(const ProjPanelArgs
   if (blk >= a.nq) {
     if (a.apply && r0 < r1) {
       const ulonglong2* d = p.t + ((size_t)tile * p.rows + r0) * 2;
-      x0 = d[0];
-      z0 = d[1];
+      x0 = __ldcg(d);
+      z0 = __ldcg(d + 1);
     }
     if (a.cntn) flag_tables(a, tile, s.f);
   }
