@@ -512,9 +512,11 @@ __global__ void __launch_bounds__(256) apply_dense_kernel(uint64_t* xzs, uint8_t
 // products are multiplied in order by dense_join_kernel.
 // Bound by shared memory (an entry is len x 16 bytes; about half its rate) and
 // by the instructions around each read.  Rows x qubits, us, against a product
-// of one image at a time with eight warps per row: 500 x 500 36 -> 18.5, 1000 x
-// 1000 122 -> 22, 2000 x 2000 392 -> 94, 4000 x 4000 2150 -> 759, 8000 x 8000
-// 12645 -> 6100, 20000 x 100 190 -> 53.
+// of one image at a time with eight warps per row: 500 x 500 36 -> 17.5, 1000 x
+// 1000 122 -> 19.7, 2000 x 2000 392 -> 94, 4000 x 4000 2150 -> 442, 8000 x 8000
+// 12645 -> 6160, 20000 x 100 190 -> 53.  (The tables waiting for dense_q_kernel,
+// loads through L1, the join's loads four at a time: 1000 22, 4000 759.)
+constexpr uint32_t DENSE_RUNS = 16;
 struct DenseArgs {
   uint64_t* xzs;
   uint8_t* ph;
@@ -524,7 +526,7 @@ struct DenseArgs {
   uint8_t* qt;         // [32 len][16] q of the entries of every two qubits
   ulonglong2* part;    // [KG][rows][len] partial products (x, z)
   uint8_t* odd;        // [KG][rows] parity of their crossings
-  uint32_t KG, wpg;    // runs, qubit words per run
+  uint32_t KG, wpg;    // runs (at most DENSE_RUNS), qubit words per run
   uint32_t NT;         // tables in shared memory at a time
   int phases;
 };
@@ -596,8 +598,9 @@ __global__ void __launch_bounds__(256) dense_q_kernel(const DenseArgs a) {
 template <int THREADS, int LPR, int KPL, int RPW>
 __global__ void __launch_bounds__(THREADS, 1) dense_tables_kernel(const DenseArgs a) {
   extern __shared__ __align__(16) ulonglong2 tab[];  // [NT][16][len]
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;");
+  // Behind dense_q_kernel, which waited for all before it, this kernel runs
+  // beside it and waits at its end (the join needs both); its loads pass L1 by.
+  if (!a.phases) asm volatile("griddepcontrol.wait;" ::: "memory");
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, len = a.W / 2;
   const uint32_t kg = blockIdx.x, w0 = kg * a.wpg, w1 = min(len, w0 + a.wpg);
   const uint32_t sl = lane & (LPR - 1);
@@ -609,7 +612,7 @@ __global__ void __launch_bounds__(THREADS, 1) dense_tables_kernel(const DenseArg
     for (uint32_t b = 0; b < 4; b++) {
       uint32_t r;
       const uint64_t* im = mt < a.NT ? dense_image(a, p0 + mt, b, r) : nullptr;
-      v[b] = im ? make_ulonglong2(__ldg(im + mw), __ldg(im + len + mw)) : make_ulonglong2(0, 0);
+      v[b] = im ? make_ulonglong2(__ldcg(im + mw), __ldcg(im + len + mw)) : make_ulonglong2(0, 0);
     }
   };
   uint64_t x[RPW][KPL], z[RPW][KPL], P[RPW];
@@ -626,8 +629,8 @@ __global__ void __launch_bounds__(THREADS, 1) dense_tables_kernel(const DenseArg
 #pragma unroll
     for (int i = 0; i < RPW; i++) {
       const uint64_t* row = a.xzs + (uint64_t)min(r0 + i, a.rows - 1) * a.W + (p0 >> 5);
-      xs[i] = (uint32_t)(row[0] >> (2 * (p0 & 31)));
-      zs[i] = (uint32_t)(row[len] >> (2 * (p0 & 31)));
+      xs[i] = (uint32_t)(__ldcg(row) >> (2 * (p0 & 31)));
+      zs[i] = (uint32_t)(__ldcg(row + len) >> (2 * (p0 & 31)));
     }
     __syncthreads();  // the previous tables are read until here
     if (mt < a.NT) {
@@ -679,6 +682,8 @@ __global__ void __launch_bounds__(THREADS, 1) dense_tables_kernel(const DenseArg
     }
     if (sl == 0) a.odd[(size_t)kg * a.rows + r0 + i] = (uint8_t)(odd & 1u);
   }
+  if (a.phases) asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
 }
 
 // A warp per row: the runs' products multiplied in order, the row's phase.
@@ -690,23 +695,33 @@ __global__ void __launch_bounds__(256) dense_join_kernel(const DenseArgs a) {
   uint64_t* row = a.xzs + (uint64_t)r * a.W;
   uint32_t q = 0;
   if (a.phases) {
-    // the entries' q: lane = two qubits of each word
-    for (uint32_t w = 0; w < len; w++) {
-      const uint32_t e = ((uint32_t)(row[w] >> (2 * lane)) & 3u) | (((uint32_t)(row[len + w] >> (2 * lane)) & 3u) << 2);
-      q += a.qt[((size_t)w * 32 + lane) * 16 + e];
+    // the entries' q: lane = two qubits of each word, eight words' loads in flight
+    for (uint32_t w0 = 0; w0 < len; w0 += 8) {
+      uint32_t e[8];
+#pragma unroll
+      for (uint32_t i = 0; i < 8; i++) {
+        const uint32_t w = min(w0 + i, len - 1);
+        e[i] = ((uint32_t)(row[w] >> (2 * lane)) & 3u) | (((uint32_t)(row[len + w] >> (2 * lane)) & 3u) << 2);
+      }
+#pragma unroll
+      for (uint32_t i = 0; i < 8; i++)
+        if (w0 + i < len) q += a.qt[((size_t)(w0 + i) * 32 + lane) * 16 + e[i]];
     }
     for (uint32_t g = lane; g < a.KG; g += 32) q += 2u * a.odd[(size_t)g * a.rows + r];
   }
   __syncwarp();
   uint64_t P = 0;
   for (uint32_t w = lane; w < len; w += 32) {
+    ulonglong2 v[DENSE_RUNS];
+#pragma unroll
+    for (uint32_t g = 0; g < DENSE_RUNS; g++)
+      v[g] = g < a.KG ? a.part[((size_t)g * a.rows + r) * len + w] : make_ulonglong2(0, 0);
     uint64_t x = 0, z = 0;
-#pragma unroll 4
-    for (uint32_t g = 0; g < a.KG; g++) {
-      const ulonglong2 v = a.part[((size_t)g * a.rows + r) * len + w];
-      P ^= v.y & x;
-      x ^= v.x;
-      z ^= v.y;
+#pragma unroll
+    for (uint32_t g = 0; g < DENSE_RUNS; g++) {
+      P ^= v[g].y & x;
+      x ^= v[g].x;
+      z ^= v[g].y;
     }
     row[w] = x;
     row[len + w] = z;
@@ -926,7 +941,7 @@ static int apply_dense_tables(qcb_tableau* t, const qcb_tableau* c, int phases, 
   DenseArgs a{};
   a.xzs = t->xzs; a.ph = t->phases; a.rows = R; a.W = t->W; a.n = t->nqubits; a.c = c->xzs; a.cph = c->phases; a.phases = phases;
   // runs of whole qubit words, as many as give every SM a CTA
-  a.KG = std::max<uint32_t>(1, std::min<uint32_t>({len, 16u, (uint32_t)device_sm_count() / RG}));
+  a.KG = std::max<uint32_t>(1, std::min<uint32_t>({len, DENSE_RUNS, (uint32_t)device_sm_count() / RG}));
   a.wpg = (len + a.KG - 1) / a.KG;
   a.KG = (len + a.wpg - 1) / a.wpg;
   const size_t table = (size_t)16 * len * sizeof(ulonglong2);
