@@ -2017,7 +2017,13 @@ static int batch_presample(qcb_batch& b, const qcb_batch_job* jobs, size_t n_job
   if (ids.empty()) return QCB_OK;
   b.pre_cnt_bytes = cnt * 4;
   b.pre_bytes = (cnt + buf) * 4;
-  QCB_CUDA(dev_alloc((void**)&b.pre, b.pre_bytes, false));
+  const cudaError_t e = dev_alloc((void**)&b.pre, b.pre_bytes, false);
+  if (e == cudaErrorMemoryAllocation) {  // no room: the walk draws the noise
+    cudaGetLastError();
+    b.pre_cnt_bytes = b.pre_bytes = 0;
+    return QCB_OK;
+  }
+  QCB_CUDA(e);
   std::vector<PresampleArgs> args;
   std::vector<PresampleItem> items;
   uint32_t *pc = b.pre, *pb = b.pre + cnt;

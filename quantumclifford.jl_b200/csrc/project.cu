@@ -1305,7 +1305,12 @@ static int project_panels(const qcb_tableau* t, int kind, uint32_t rank, const u
                o_par = place((size_t)ntile * R), o_rec = place(sizeof(PanelRecord)), o_cp = place(2 * PSTEPS * 8),
                o_pq = place(2 * PSTEPS * 4), o_st = place(8);
   uint8_t* m = nullptr;
-  QCB_CUDA(cudaMallocAsync(&m, bytes, st));
+  const cudaError_t e = cudaMallocAsync(&m, bytes, st);
+  if (e == cudaErrorMemoryAllocation) {  // no room for a copy of the rows: none done here
+    cudaGetLastError();
+    return QCB_OK;
+  }
+  QCB_CUDA(e);
   ProjPanelArgs a{};
   a.p = PanelTiles{R, W, len, ntile, 1, (ulonglong2*)(m + o_t), (ulonglong2*)(m + o_po), nullptr, (uint64_t*)(m + o_u),
                    m + o_q, m + o_par};
