@@ -517,6 +517,7 @@ __global__ void __launch_bounds__(256) apply_dense_kernel(uint64_t* xzs, uint8_t
 // 12645 -> 6160, 20000 x 100 190 -> 53.  (The tables waiting for dense_q_kernel,
 // loads through L1, the join's loads four at a time: 1000 22, 4000 759.)
 constexpr uint32_t DENSE_RUNS = 16;
+constexpr size_t DENSE_SCRATCH = 64ull << 20;
 struct DenseArgs {
   uint64_t* xzs;
   uint8_t* ph;
@@ -528,6 +529,7 @@ struct DenseArgs {
   uint8_t* odd;        // [KG][rows] parity of their crossings
   uint32_t KG, wpg;    // runs (at most DENSE_RUNS), qubit words per run
   uint32_t NT;         // tables in shared memory at a time
+  uint32_t beside;     // the tables run beside dense_q_kernel
   int phases;
 };
 
@@ -600,7 +602,7 @@ __global__ void __launch_bounds__(THREADS, 1) dense_tables_kernel(const DenseArg
   extern __shared__ __align__(16) ulonglong2 tab[];  // [NT][16][len]
   // Behind dense_q_kernel, which waited for all before it, this kernel runs
   // beside it and waits at its end (the join needs both); its loads pass L1 by.
-  if (!a.phases) asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (!a.beside) asm volatile("griddepcontrol.wait;" ::: "memory");
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, len = a.W / 2;
   const uint32_t kg = blockIdx.x, w0 = kg * a.wpg, w1 = min(len, w0 + a.wpg);
   const uint32_t sl = lane & (LPR - 1);
@@ -682,7 +684,7 @@ __global__ void __launch_bounds__(THREADS, 1) dense_tables_kernel(const DenseArg
     }
     if (sl == 0) a.odd[(size_t)kg * a.rows + r0 + i] = (uint8_t)(odd & 1u);
   }
-  if (a.phases) asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (a.beside) asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;");
 }
 
@@ -937,27 +939,49 @@ static int apply_dense_tables(qcb_tableau* t, const qcb_tableau* c, int phases, 
                : len <= 32 ? Form{dense_tables_kernel<1024, 32, 1, 4>, 1024, 128}
                : len <= 64 ? Form{dense_tables_kernel<512, 32, 2, 6>, 512, 96}
                            : Form{dense_tables_kernel<512, 32, 4, 4>, 512, 64};
-  const uint32_t RG = (R + f.rows - 1) / f.rows;
   DenseArgs a{};
-  a.xzs = t->xzs; a.ph = t->phases; a.rows = R; a.W = t->W; a.n = t->nqubits; a.c = c->xzs; a.cph = c->phases; a.phases = phases;
-  // runs of whole qubit words, as many as give every SM a CTA
-  a.KG = std::max<uint32_t>(1, std::min<uint32_t>({len, DENSE_RUNS, (uint32_t)device_sm_count() / RG}));
-  a.wpg = (len + a.KG - 1) / a.KG;
-  a.KG = (len + a.wpg - 1) / a.wpg;
+  a.W = t->W; a.n = t->nqubits; a.c = c->xzs; a.cph = c->phases; a.phases = phases;
   const size_t table = (size_t)16 * len * sizeof(ulonglong2);
   a.NT = 16;
   while (a.NT * len > f.threads || a.NT * table > (size_t)200 * 1024) a.NT /= 2;
   const size_t smem = a.NT * table;
-  size_t bytes = 0;
-  auto place = [&](size_t n) { const size_t o = bytes; bytes += (n + 127) / 128 * 128; return o; };
-  const size_t o_qt = place((size_t)32 * len * 16), o_part = place((size_t)a.KG * R * len * 16), o_odd = place((size_t)a.KG * R);
+  // runs of whole qubit words, as many as give every SM a CTA
+  const uint32_t nsm = (uint32_t)std::max(device_sm_count(), 1);
+  auto runs = [&](uint32_t rows) {
+    a.KG = std::max<uint32_t>(1, std::min<uint32_t>({len, DENSE_RUNS, nsm / ((rows + f.rows - 1) / f.rows)}));
+    a.wpg = (len + a.KG - 1) / a.KG;
+    a.KG = (len + a.wpg - 1) / a.wpg;
+  };
+  // Rows at a time: the partial products take 16 len bytes a row and run, at
+  // most DENSE_SCRATCH (more rows than fill the GPU many times over), and
+  // less where that much memory is not there.
+  uint32_t slab = std::min<uint64_t>(R, std::max<uint64_t>(f.rows, DENSE_SCRATCH / ((size_t)16 * len) / f.rows * f.rows));
   uint8_t* m = nullptr;
-  QCB_CUDA(cudaMallocAsync(&m, bytes, st));
-  a.qt = m + o_qt; a.part = (ulonglong2*)(m + o_part); a.odd = m + o_odd;
+  size_t o_part = 0, o_odd = 0;
+  while (true) {
+    runs(slab);
+    size_t bytes = 0;
+    auto place = [&](size_t n) { const size_t o = bytes; bytes += (n + 127) / 128 * 128; return o; };
+    place((size_t)32 * len * 16);
+    o_part = place((size_t)a.KG * slab * len * 16);
+    o_odd = place((size_t)a.KG * slab);
+    const cudaError_t e = cudaMallocAsync(&m, bytes, st);
+    if (e == cudaSuccess) break;
+    if (e != cudaErrorMemoryAllocation || slab <= f.rows) return cuda_fail(e, "qcb_apply_dense scratch");
+    cudaGetLastError();
+    slab = std::max(f.rows, slab / 2 / f.rows * f.rows);
+  }
+  a.qt = m; a.part = (ulonglong2*)(m + o_part); a.odd = m + o_odd;
   QCB_CUDA(cudaFuncSetAttribute(f.k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   if (phases) QCB_CUDA(launch_dependent(dense_q_kernel, dim3((32 * len + 7) / 8), 256, 0, st, a));
-  QCB_CUDA(launch_dependent(f.k, dim3(a.KG, RG), f.threads, smem, st, a));
-  QCB_CUDA(launch_dependent(dense_join_kernel, dim3((R + 7) / 8), 256, 0, st, a));
+  for (uint32_t r0 = 0; r0 < R; r0 += slab) {
+    a.xzs = t->xzs + (size_t)r0 * t->W;
+    a.ph = t->phases + r0;
+    a.rows = std::min(slab, R - r0);
+    a.beside = phases && r0 == 0;  // later slabs wait for the join before them
+    QCB_CUDA(launch_dependent(f.k, dim3(a.KG, (a.rows + f.rows - 1) / f.rows), f.threads, smem, st, a));
+    QCB_CUDA(launch_dependent(dense_join_kernel, dim3((a.rows + 7) / 8), 256, 0, st, a));
+  }
   QCB_CUDA(cudaFreeAsync(m, st));
   return QCB_OK;
 }

@@ -437,3 +437,19 @@ def test_dense_apply_table_edges(qcb, n, rows):
         s.to_cpu()
         ph, xz = oracle.apply_dense(state.phases, state.xzs, n, c.tab.phases, c.tab.xzs, phases)
         assert np.array_equal(s.tab.xzs, xz) and np.array_equal(s.tab.phases, ph)
+
+
+def test_dense_apply_more_rows_than_one_scratch(qcb):
+    """Rows beyond the scratch of one pass (64 MB of partial products) go slab
+    by slab: a tall stack of copies equals the copies one by one."""
+    rng = np.random.default_rng(64)
+    n, small, copies = 64, 1000, 4300  # 4.3e6 rows of one word
+    base = qcb.random_paulis(small, n, rng)
+    op = qcb.random_clifford(n, rng).to_gpu()
+    tall = qcb.Tableau(np.tile(base.phases, copies), n, np.tile(base.xzs, (copies, 1))).to_gpu()
+    one = base.copy().to_gpu()
+    for t in (one, tall):
+        qcb.check(qcb.lib().qcb_apply_dense(t.dev.handle, op.tab.dev.handle, 1, None))
+    one.to_cpu(), tall.to_cpu()
+    assert np.array_equal(tall.xzs.reshape(copies, small, -1), np.broadcast_to(one.xzs, (copies,) + one.xzs.shape))
+    assert np.array_equal(tall.phases.reshape(copies, small), np.broadcast_to(one.phases, (copies, small)))
