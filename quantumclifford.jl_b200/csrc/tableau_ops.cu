@@ -513,8 +513,8 @@ __global__ void __launch_bounds__(256) apply_dense_kernel(uint64_t* xzs, uint8_t
 // Bound by shared memory (an entry is len x 16 bytes; about half its rate) and
 // by the instructions around each read.  Rows x qubits, us, against a product
 // of one image at a time with eight warps per row: 500 x 500 36 -> 17.5, 1000 x
-// 1000 122 -> 19.7, 2000 x 2000 392 -> 94, 4000 x 4000 2150 -> 442, 8000 x 8000
-// 12645 -> 6160, 20000 x 100 190 -> 53.  (The tables waiting for dense_q_kernel,
+// 1000 122 -> 19.7, 2000 x 2000 392 -> 93, 4000 x 4000 2150 -> 385, 8000 x 8000
+// 12645 -> 5365, 20000 x 100 190 -> 53.  (The tables waiting for dense_q_kernel,
 // loads through L1, the join's loads four at a time: 1000 22, 4000 759.)
 constexpr uint32_t DENSE_RUNS = 16;
 constexpr size_t DENSE_SCRATCH = 64ull << 20;
@@ -945,12 +945,21 @@ static int apply_dense_tables(qcb_tableau* t, const qcb_tableau* c, int phases, 
   a.NT = 16;
   while (a.NT * len > f.threads || a.NT * table > (size_t)200 * 1024) a.NT /= 2;
   const size_t smem = a.NT * table;
-  // runs of whole qubit words, as many as give every SM a CTA
+  // Runs of whole qubit words: the least waves x (words of a run x the time of
+  // a word's tables, with 3 us for a CTA) and the partial products' traffic.  As
+  // many runs as fill one wave leaves large ones a
+  // half-empty last wave (rows x qubits, us: 20000 x 2000 1304 -> 779,
+  // 8000 x 4000 1269 -> 752, 4000 x 4000 441 -> 385, 8000 x 8000 6148 -> 5365).
   const uint32_t nsm = (uint32_t)std::max(device_sm_count(), 1);
   auto runs = [&](uint32_t rows) {
-    a.KG = std::max<uint32_t>(1, std::min<uint32_t>({len, DENSE_RUNS, nsm / ((rows + f.rows - 1) / f.rows)}));
-    a.wpg = (len + a.KG - 1) / a.KG;
-    a.KG = (len + a.wpg - 1) / a.wpg;
+    const uint32_t RG = (rows + f.rows - 1) / f.rows;
+    const double word_us = 0.005 * f.rows * len, run_us = (double)rows * len * 32 / 5e6;
+    double best = 0;
+    for (uint32_t g = 1; g <= std::min(len, DENSE_RUNS); g++) {
+      const uint32_t wpg = (len + g - 1) / g, kg = (len + wpg - 1) / wpg;
+      const double us = (RG * kg + nsm - 1) / nsm * (wpg * word_us + 3.0) + kg * run_us;
+      if (g == 1 || us < best) { best = us; a.KG = kg; a.wpg = wpg; }
+    }
   };
   // Rows at a time: the partial products take 16 len bytes a row and run, at
   // most DENSE_SCRATCH (more rows than fill the GPU many times over), and
