@@ -46,6 +46,7 @@ struct PanelRecord {
   uint64_t A[PSTEPS];         // start rows in the reduced pivot t
   uint64_t PW[PSTEPS];        // the pivot's panel word at its step
   uint32_t src[PSTEPS];       // project!: the step whose Pauli is pivot t's start row (PSTEPS: row stp)
+  uint32_t sbt[PSTEPS];       // project!: that Pauli (PSTEPS: none)
   uint64_t own[PSTEPS];       // project!: the steps that multiplied pivot t before its own
   uint32_t s[PSTEPS];         // project!: |x & z| of the reduced pivot, summed over the tiles
   unsigned long long G[PSTEPS];  // z_{P_t} . x_{P_s} (bit s), summed over the tiles

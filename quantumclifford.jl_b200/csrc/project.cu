@@ -1,7 +1,8 @@
 // project.cu -- project! for Stabilizer, MixedStabilizer, Destabilizer and
 // MixedDestabilizer tableaux (src/project_trace_reset.jl:231-439).
 //
-// One thread-block cluster projects a list of Paulis in order on one state.
+// Runs of 32 Paulis and more go by panels over the whole GPU (below).  Else
+// one thread-block cluster projects a list of Paulis in order on one state.
 // The tableau stays in global memory (it is L2 resident at these sizes).  Per
 // Pauli:
 //   1. every CTA computes comm(pauli, row) for its share of the rows (warp per
@@ -767,21 +768,26 @@ __global__ void __launch_bounds__(PROJ_THREADS) project_grid_kernel(const ProjGr
 // on the rows, so the panel's steps run on them alone.  A row's start words
 // are its own, those of the last Pauli put into it (word CP[j], its
 // commutation bits with the other Paulis of the panel), or none (a copied
-// pivot: the set U is that step alone).  Per panel three launches:
-//   S   one CTA: the steps on the words;
-//   M   a CTA per tile: the reduced pivots and the tile's share of the phase
-//       data; CTAs over the rows: their sets U and start words;
-//   AF  a CTA per tile and range of rows: the panel applied, and on the new
-//       words the tile's share of the next panel's commutation words (32 byte
-//       lookups in tables over its Paulis); a few CTAs the rows' q.
+// pivot: the set U is that step alone).  Per panel k two launches:
+//   SA(k)  CTA 0 (S): panel k's steps on the words; the other CTAs (AF): panel
+//          k - 1 applied, a CTA per tile and range of rows, and on the new
+//          words the tile's share of the rows' commutation words with panel k +
+//          1's Paulis (32 byte lookups in tables over them); a few CTAs the
+//          rows' q;
+//   M(k)   a CTA per tile: the reduced pivots and the tile's share of the phase
+//          data; CTAs over the rows: their sets U and start words, and their
+//          words of panel k + 1: the word AF(k - 1) found and the reduced
+//          pivots' for the steps in U.
+// So the apply is off the chain S, M of a panel.
 // A Pauli that commutes with the stabilizer (its result needs the rows), or
 // anticommutes with a logical row only, ends the run after the steps before
 // it; the host handles that one with the kernels above and goes on.
-// Bound by the chain of the three launches (their latencies; the rows' traffic
-// is a tenth of it).  1000 random Paulis, us each: Stabilizer n = 1000 / 2000 /
-// 4000 4.9 / 7.3 / 12.4 -> 0.60 / 0.61 / 0.70, Destabilizer n = 1000 / 2000
-// 5.4 / 11.3 -> 0.60 / 0.64 (one Pauli at a time, two cluster or grid barriers
-// each, before).
+// Bound by that chain: SA 10.4 + M 8.7 us a panel (n = 1000; 15.0 + 8.3 at
+// 4000, where the lookups set SA's length) and 1.6 us a launch.  1000 random
+// Paulis, us each with the call: Stabilizer n = 1000 / 4000 4.9 / 12.4 -> 0.48 /
+// 0.59, Destabilizer n = 1000 / 2000 5.4 / 11.3 -> 0.48 / 0.53 (one Pauli at a
+// time, two cluster or grid barriers each, before; with S, M and the apply as
+// three launches in turn 0.54 / 0.64, 0.53 / 0.58).
 struct ProjPanelArgs {
   PanelTiles p;
   uint64_t* xzs;
@@ -795,30 +801,33 @@ struct ProjPanelArgs {
   const uint8_t* rand_ph;
   uint32_t j0, cnt;    // this panel's Paulis
   uint32_t jn, cntn;   // the next panel's
-  PanelRecord* rec;
+  uint32_t jp;         // the first of the previous panel's
+  PanelRecord *rec, *prev;  // of this panel and the previous one
   int32_t* state;      // [0] stopped, [1] the next Pauli
   int32_t* anticom;
   int32_t* result;
   uint64_t *word, *wordn;   // [rows] commutation words of this and the next panel
-  unsigned long long *CP, *CPn;  // [PSTEPS] the Paulis' own
-  uint32_t *pq, *pqn;       // [PSTEPS] the Paulis' q
+  // [rows] words with the next panel's Paulis before this panel (AF writes,
+  // M reads), and the buffer of the SA after the next one, which M clears;
+  // likewise [PSTEPS] this panel's Paulis with the next panel's
+  unsigned long long *F, *Fz, *CPX, *CPXz;
+  unsigned long long *CP, *CPn, *CPz;  // [PSTEPS] the Paulis' own words
+  uint32_t *pq, *pqn, *pqz, *pqp;      // [PSTEPS] the Paulis' q; pqp: the previous panel's
   uint8_t* base;       // [rows] start words: BASE_ROW, BASE_NONE or the Pauli's index in the panel
-  uint32_t apply, nq, groups, per;
+  uint32_t steps, apply, nq, groups, per;
 };
 constexpr uint32_t BASE_ROW = 255, BASE_NONE = 254;
 constexpr uint32_t PP_SLOTS = 3, PP_WINDOW = 32 * PP_SLOTS, PP_REST = 31 * 32;
 
 // S: as canonicalize!'s steps, with the stabilizer rows in their fixed order.
 template <uint32_t RPT>
-__global__ void __launch_bounds__(1024) project_steps_kernel(const ProjPanelArgs a) {
+__device__ __forceinline__ void project_steps(const ProjPanelArgs& a) {
   constexpr uint32_t NONE = 0xFFFFFFFFu, KW = PP_SLOTS;
   __shared__ uint4 recA[PSTEPS];  // pivot t: (word, mask)
   __shared__ uint4 recB[PSTEPS];  // (stabilizer row, Pauli, src)
   __shared__ uint2 sCP[PSTEPS];
   __shared__ uint64_t rw[32], ra[32];
   __shared__ uint32_t rs[32], rpos[32], shT, shB, rb, rT;
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;");
   PanelRecord& g = *a.rec;
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, R = a.rank;
   if (tid < PSTEPS) {
@@ -829,7 +838,10 @@ __global__ void __launch_bounds__(1024) project_steps_kernel(const ProjPanelArgs
     sCP[tid] = make_uint2((uint32_t)c, (uint32_t)(c >> 32));
   }
   if (a.state[0]) {
-    if (tid == 0) g.T = 0;
+    if (tid == 0) {
+      g.T = 0;
+      g.done = 1;
+    }
     return;
   }
   const uint64_t* word = a.word + a.nn;
@@ -979,6 +991,7 @@ __global__ void __launch_bounds__(1024) project_steps_kernel(const ProjPanelArgs
     g.stp[tid] = a.nn + f.x;
     g.bt[tid] = f.y;
     g.src[tid] = f.z;
+    g.sbt[tid] = f.z < PSTEPS ? recB[f.z].y : PSTEPS;
     g.A[tid] = (uint64_t)e.z | ((uint64_t)e.w << 32);
     g.PW[tid] = (uint64_t)e.x | ((uint64_t)e.y << 32);
     a.anticom[a.j0 + f.y] = (int32_t)f.x + 1;
@@ -986,14 +999,15 @@ __global__ void __launch_bounds__(1024) project_steps_kernel(const ProjPanelArgs
   }
   if (tid == 0) {
     g.T = T;
+    g.done = done < a.cnt;
     a.state[0] = done < a.cnt;
     a.state[1] = (int32_t)(a.j0 + done);
   }
 }
 
-// q of the stabilizer row that Pauli b of the panel becomes.
-__device__ __forceinline__ uint32_t new_row_q(const ProjPanelArgs& a, uint32_t b) {
-  return (a.pq[b] + (a.rand_ph ? a.rand_ph[a.j0 + b] - a.pph[a.j0 + b] : 0u)) & 3u;
+// q of the stabilizer row that Pauli b of the panel from j0 on becomes.
+__device__ __forceinline__ uint32_t new_row_q(const ProjPanelArgs& a, const uint32_t* pq, uint32_t j0, uint32_t b) {
+  return (__ldcg(pq + b) + (a.rand_ph ? __ldcg(a.rand_ph + j0 + b) - __ldcg(a.pph + j0 + b) : 0u)) & 3u;
 }
 
 // M: blocks 0 .. ntile - 1 a tile each, block ntile the pivots' own sets, the
@@ -1003,17 +1017,23 @@ __global__ void __launch_bounds__(MID_THREADS) project_mid_kernel(const ProjPane
     TileSmem t;
     struct {
       ulonglong2 P[PSTEPS];   // (pivot's word, the Pauli's word)
-      uint2 sb[PSTEPS];       // (pivot row, Pauli)
+      ulonglong2 N[PSTEPS];   // the same with the next panel's Paulis
+      ulonglong2 C[PSTEPS];   // the Paulis' words with this panel's and the next one's
+      uint64_t start[PSTEPS];  // the pivots' start rows' words with the next one's
+      uint2 sb[PSTEPS];       // (pivot row, 31 - bit within its half word | Pauli << 8)
+      uint32_t bt[PSTEPS];
     } r;
   } s;
   const PanelTiles& p = a.p;
   const uint32_t tid = threadIdx.x, blk = blockIdx.x;
-  // While S runs: the Paulis' words of the tile as the tiles keep them, or the
-  // rows' panel words.  S waited for the apply that wrote them before it let
+  // While SA runs: the Paulis' words of the tile as the tiles keep them, or the
+  // rows' panel words.  SA waited for the launch that wrote them before it let
   // this kernel start, so they are in L2; loads before the wait pass L1 by.
   __shared__ ulonglong2 pw[PSTEPS][2];
+  __shared__ uint32_t sq[PSTEPS];  // tile 0: q of the rows the Paulis become
   const uint32_t r = blk > p.ntile ? (blk - p.ntile - 1) * MID_THREADS + tid : p.rows;
   uint64_t w = 0;
+  if (blk == 0 && tid < a.cnt) sq[tid] = new_row_q(a, a.pq, a.j0, tid);
   if (blk < p.ntile) {
     const uint32_t b = tid >> 2, c = 2 * blk + (tid & 1);
     ((uint64_t*)pw[b])[tid & 3] =
@@ -1030,12 +1050,12 @@ __global__ void __launch_bounds__(MID_THREADS) project_mid_kernel(const ProjPane
     tile_reduce(
         p, g, blk, s.t,
         [&](uint32_t t, uint32_t r) -> const ulonglong2* {
-          const uint32_t sr = t < T ? g.src[t] : PSTEPS;
-          return sr < PSTEPS ? pw[g.bt[sr]] : p.t + ((size_t)blk * p.rows + r) * 2;
+          const uint32_t b = g.sbt[t];  // of the record's T steps, or stale
+          return b < PSTEPS ? pw[b] : p.t + ((size_t)blk * p.rows + r) * 2;
         },
         [&](uint32_t t, uint32_t r) -> uint32_t {
-          const uint32_t sr = g.src[t];
-          if (sr < PSTEPS) return blk == 0 ? new_row_q(a, g.bt[sr]) : 0u;
+          const uint32_t b = g.sbt[t];
+          if (b < PSTEPS) return blk == 0 ? sq[b] : 0u;
           return 2u * p.par[(size_t)blk * p.rows + r] + (blk == 0 ? p.q[r] : 0u);
         },
         [&](uint32_t t, const uint64_t* v) {
@@ -1044,21 +1064,54 @@ __global__ void __launch_bounds__(MID_THREADS) project_mid_kernel(const ProjPane
         });
     return;
   }
+  // The record's fields beyond its T steps are stale but readable (zero at the
+  // start): nothing here waits for T, or for an index, before loading what it can.
+  const bool next = a.cntn != 0;
+  const uint32_t t4 = tid >> 2, x0 = (tid & 3) * 16;
+  const uint64_t A = g.A[t4] >> x0;
+  uint32_t b = 0, sp = 0, sr = PSTEPS, sbt = PSTEPS;
+  uint64_t PW = 0, F = 0, v = 0, w_own = 0;
   if (tid < PSTEPS) {
+    b = g.bt[tid];
+    sp = g.stp[tid];
+    sr = g.src[tid];
+    sbt = g.sbt[tid];
+    PW = g.PW[tid];
+    s.r.bt[tid] = b;
+    if (blk == p.ntile && sr >= PSTEPS) w_own = a.word[sp];
+    s.r.C[tid] = make_ulonglong2(a.CP[tid], next ? a.CPX[tid] : 0ull);
+    if (next) F = a.F[sp];
+  }
+  if (r < p.rows) {
+    a.Fz[r] = 0;
+    if (next) v = a.F[r];
+  }
+  const uint32_t T0 = __syncthreads_count(tid < T && b < 32);  // steps in the words' low halves
+  if (tid < PSTEPS) {
+    const ulonglong2 c = s.r.C[b];
     const bool in = tid < T;
-    const uint32_t b = in ? g.bt[tid] : 0u;
-    s.r.P[tid] = make_ulonglong2(in ? g.PW[tid] : 0ull, a.CP[b]);
-    s.r.sb[tid] = make_uint2(in ? g.stp[tid] : 0xFFFFFFFFu, b);
+    s.r.P[tid] = make_ulonglong2(PW, c.x);
+    s.r.N[tid].y = c.y;
+    s.r.sb[tid] = make_uint2(sp, (31u - (b & 31u)) | b << 8);
+    s.r.start[tid] = !in ? 0ull : sbt < PSTEPS ? s.r.C[sbt].y : F;
+  }
+  __syncthreads();
+  {  // the reduced pivots' next words: a thread per pivot and 16 start rows
+    uint64_t n = 0;
+#pragma unroll
+    for (uint32_t x = 0; x < 16; x++) n ^= s.r.start[x0 + x] & bitmask64(A, x);
+    n ^= __shfl_xor_sync(0xFFFFFFFFu, n, 1);
+    n ^= __shfl_xor_sync(0xFFFFFFFFu, n, 2);
+    if ((tid & 3) == 0) s.r.N[t4].x = n;
   }
   __syncthreads();
   if (blk == p.ntile) {
-    if (tid < PSTEPS) { a.CPn[tid] = 0; a.pqn[tid] = 0; }
+    if (tid < PSTEPS) { a.CPz[tid] = 0; a.pqz[tid] = 0; a.CPXz[tid] = 0; }
     // pivot t's start word replayed up to its step
     if (tid < T) {
-      const uint32_t sr = g.src[tid];
-      uint64_t w = sr < PSTEPS ? s.r.P[sr].y : a.word[s.r.sb[tid].x], U = 0;
+      uint64_t w = sr < PSTEPS ? s.r.P[sr].y : w_own, U = 0;
       for (uint32_t t = sr < PSTEPS ? sr + 1 : 0; t < tid; t++) {
-        const uint64_t y = bitmask64(w, s.r.sb[t].y);
+        const uint64_t y = bitmask64(w, s.r.bt[t]);
         w ^= s.r.P[t].x & y;
         U |= (1ull << t) & y;
       }
@@ -1067,28 +1120,38 @@ __global__ void __launch_bounds__(MID_THREADS) project_mid_kernel(const ProjPane
     return;
   }
   if (r >= p.rows) return;
-  a.wordn[r] = 0;
-  uint64_t U = 0;
+  uint32_t p0 = (uint32_t)w, p1 = (uint32_t)(w >> 32), v0 = (uint32_t)v, v1 = (uint32_t)(v >> 32), u0 = 0, u1 = 0;
   uint32_t base = BASE_ROW;
   const uint32_t partner = r < a.nn ? r + a.nn : 0xFFFFFFFEu;  // its stabilizer row
-#pragma unroll 4
-  for (uint32_t t = 0; t < T; t++) {
-    const ulonglong2 P = s.r.P[t];
+  auto replay = [&](uint32_t t, uint32_t& half) {
+    const ulonglong2 P = s.r.P[t], N = s.r.N[t];
     const uint2 sb = s.r.sb[t];
-    const uint64_t y = bitmask64(w, sb.y), tb = 1ull << t;
-    w ^= P.x & y;
-    U |= tb & y;
-    if (sb.x == r) {  // the Pauli takes its place
-      w = P.y;
-      U = 0;
-      base = sb.y;
-    } else if (sb.x == partner) {  // a copy of the pivot
-      w = P.x;
-      U = tb;
-      base = BASE_NONE;
+    const uint32_t m = (uint32_t)((int32_t)__funnelshift_l(0u, half, sb.y) >> 31);  // by 31 - bit
+    const uint32_t tb = 1u << (t & 31), b0 = t < 32 ? tb : 0u, b1 = t < 32 ? 0u : tb;
+    p0 ^= (uint32_t)P.x & m;
+    p1 ^= (uint32_t)(P.x >> 32) & m;
+    v0 ^= (uint32_t)N.x & m;
+    v1 ^= (uint32_t)(N.x >> 32) & m;
+    u0 |= b0 & m;
+    u1 |= b1 & m;
+    const bool pivot = sb.x == r;
+    if (pivot || sb.x == partner) {  // the Pauli takes its place; a copy of the pivot
+      const uint64_t nw = pivot ? P.y : P.x, nv = pivot ? N.y : N.x;
+      p0 = (uint32_t)nw;
+      p1 = (uint32_t)(nw >> 32);
+      v0 = (uint32_t)nv;
+      v1 = (uint32_t)(nv >> 32);
+      u0 = pivot ? 0u : b0;
+      u1 = pivot ? 0u : b1;
+      base = pivot ? sb.y >> 8 : BASE_NONE;
     }
-  }
-  p.U[r] = U;
+  };
+#pragma unroll 4
+  for (uint32_t t = 0; t < T0; t++) replay(t, p0);
+#pragma unroll 4
+  for (uint32_t t = T0; t < T; t++) replay(t, p1);
+  a.wordn[r] = (uint64_t)v0 | ((uint64_t)v1 << 32);
+  p.U[r] = (uint64_t)u0 | ((uint64_t)u1 << 32);
   a.base[r] = (uint8_t)base;
 }
 
@@ -1147,15 +1210,21 @@ struct ApplyFlagSmem {
   FlagSmem f;
 };
 
-// AF.
-__global__ void __launch_bounds__(1024) project_apply_kernel(const ProjPanelArgs a) {
+// SA.
+template <uint32_t RPT>
+__global__ void __launch_bounds__(1024) project_steps_apply_kernel(const ProjPanelArgs a) {
   extern __shared__ __align__(16) uint8_t dsm[];
-  const PanelRecord& g = *a.rec;
+  if (blockIdx.x == 0) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
+    if (a.steps) project_steps<RPT>(a);
+    return;
+  }
+  const PanelRecord& g = *a.prev;
   const PanelTiles& p = a.p;
-  const uint32_t tid = threadIdx.x, blk = blockIdx.x;
+  const uint32_t tid = threadIdx.x, blk = blockIdx.x - 1;
   // While M runs: the next Paulis' tables, and the thread's first row (the
-  // previous apply wrote it, and S waited for that; loads past L1 as in M).
-  // 1000 Paulis, n = 1000 with destabilizers: 587 -> 530 us.
+  // previous apply wrote it, and M waited for that; loads past L1 as in M).
   const uint32_t u = blk < a.nq ? 0u : blk - a.nq, tile = u / a.groups, grp = u - tile * a.groups;
   const uint32_t r0 = grp * a.per + tid, r1 = min(p.rows, (grp + 1) * a.per);
   ApplyFlagSmem& s = *(ApplyFlagSmem*)dsm;
@@ -1185,13 +1254,13 @@ __global__ void __launch_bounds__(1024) project_apply_kernel(const ProjPanelArgs
           p.q[r] = (uint8_t)(((uint32_t)((s.Q1 >> t) & 1ull) + 2u * (uint32_t)((s.Q2 >> t) & 1ull) - g.s[t]) & 3u);
         }
       } else if (base != BASE_ROW || U) {
-        const uint32_t q = base != BASE_ROW ? new_row_q(a, base) : p.q[r];
+        const uint32_t q = base != BASE_ROW ? new_row_q(a, a.pqp, a.jp, base) : p.q[r];
         p.q[r] = (uint8_t)((q + phase_of(s, U)) & 3u);
       }
     }
     return;
   }
-  const bool next = a.cntn && !a.state[0];
+  const bool next = a.cntn && !(a.apply && g.done);
   if (!T && !next) return;
   if (T) apply_tables(p, tile, s.a);
   const bool two = 2 * tile + 1 < p.len;
@@ -1208,7 +1277,7 @@ __global__ void __launch_bounds__(1024) project_apply_kernel(const ProjPanelArgs
       const uint64_t U = p.U[r];
       const uint32_t base = a.base[r];
       if (base == BASE_NONE) x = z = make_ulonglong2(0, 0);
-      else if (base != BASE_ROW) pauli(a.j0 + base, x, z);
+      else if (base != BASE_ROW) pauli(a.jp + base, x, z);
       if (U || base != BASE_ROW) {
         ulonglong2 mx, mz;
         apply_lookup(s.a, U, mx, mz);
@@ -1226,7 +1295,7 @@ __global__ void __launch_bounds__(1024) project_apply_kernel(const ProjPanelArgs
     }
     if (next) {
       const uint64_t f = flag_lookup(s.f, x, z);
-      if (f) atomicXor((unsigned long long*)a.wordn + r, (unsigned long long)f);
+      if (f) atomicXor(a.F + r, (unsigned long long)f);
     }
   }
   if (next && grp == 0 && tid < a.cntn) {  // the next Paulis' own words and q
@@ -1237,6 +1306,12 @@ __global__ void __launch_bounds__(1024) project_apply_kernel(const ProjPanelArgs
     const uint32_t q = (uint32_t)(__popcll(x.x & z.x) + __popcll(x.y & z.y)) + (tile == 0 ? a.pph[a.jn + tid] : 0u);
     if (q) atomicAdd(a.pqn + tid, q);
   }
+  if (next && grp == 0 && tid >= 512 && tid - 512 < a.cnt) {  // this panel's Paulis with them
+    ulonglong2 x, z;
+    pauli(a.j0 + tid - 512, x, z);
+    const uint64_t f = flag_lookup(s.f, x, z);
+    if (f) atomicXor(a.CPX + tid - 512, (unsigned long long)f);
+  }
 }
 
 // The rows into the tiles, and back (a warp a row).
@@ -1245,15 +1320,18 @@ __global__ void __launch_bounds__(256) project_load_kernel(const ProjPanelArgs a
   asm volatile("griddepcontrol.launch_dependents;");
   const uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (blockIdx.x == 0) {
-    for (uint32_t k = threadIdx.x; k < sizeof(PanelRecord) / 4; k += blockDim.x) ((uint32_t*)a.rec)[k] = 0;
-    if (threadIdx.x < PSTEPS) { a.CPn[threadIdx.x] = 0; a.pqn[threadIdx.x] = 0; }
-    if (threadIdx.x == 0) { a.state[0] = 0; a.state[1] = (int32_t)a.jn; }
+    // both records, and the Paulis' words and q of three panels
+    for (uint32_t k = threadIdx.x; k < 2 * sizeof(PanelRecord) / 4; k += blockDim.x) ((uint32_t*)a.rec)[k] = 0;
+    for (uint32_t k = threadIdx.x; k < 3 * PSTEPS; k += blockDim.x) { a.CP[k] = 0; a.pq[k] = 0; }
+    for (uint32_t k = threadIdx.x; k < 2 * PSTEPS; k += blockDim.x) a.CPX[k] = 0;
+    if (threadIdx.x == 0) { a.state[0] = 0; a.state[1] = (int32_t)a.j0; }
   }
   if (r >= a.p.rows) return;
   const uint32_t ph = a.ph[r];
   tiles_load_row(a.p, a.xzs + (size_t)r * a.p.W, r, ph, lane);
   if (lane == 0) {
-    a.wordn[r] = 0;
+    a.word[r] = 0;
+    a.F[r] = a.Fz[r] = 0;
     if (r < a.plain) a.p.q[r] = (uint8_t)ph;
   }
 }
@@ -1301,9 +1379,9 @@ static int project_panels(const qcb_tableau* t, int kind, uint32_t rank, const u
   size_t bytes = 0;
   auto place = [&](size_t n) { const size_t o = bytes; bytes += (n + 127) / 128 * 128; return o; };
   const size_t o_t = place((size_t)ntile * R * 32), o_po = place((size_t)ntile * PSTEPS * 32),
-               o_w = place((size_t)2 * R * 8), o_u = place((size_t)R * 8), o_q = place(R), o_b = place(R),
-               o_par = place((size_t)ntile * R), o_rec = place(sizeof(PanelRecord)), o_cp = place(2 * PSTEPS * 8),
-               o_pq = place(2 * PSTEPS * 4), o_st = place(8);
+               o_w = place((size_t)4 * R * 8), o_u = place((size_t)R * 8), o_q = place(R), o_b = place(R),
+               o_par = place((size_t)ntile * R), o_rec = place(2 * sizeof(PanelRecord)), o_cp = place(5 * PSTEPS * 8),
+               o_pq = place(3 * PSTEPS * 4), o_st = place(8);
   uint8_t* m = nullptr;
   const cudaError_t e = cudaMallocAsync(&m, bytes, st);
   if (e == cudaErrorMemoryAllocation) {  // no room for a copy of the rows: none done here
@@ -1315,48 +1393,60 @@ static int project_panels(const qcb_tableau* t, int kind, uint32_t rank, const u
   a.p = PanelTiles{R, W, len, ntile, 1, (ulonglong2*)(m + o_t), (ulonglong2*)(m + o_po), nullptr, (uint64_t*)(m + o_u),
                    m + o_q, m + o_par};
   a.xzs = t->xzs; a.ph = t->phases; a.nn = destab ? t->rows / 2 : 0; a.rank = rank; a.plain = destab ? rank : 0;
-  a.skip = skip; a.paulis = pxzs; a.pph = pph; a.rand_ph = d_rand; a.rec = (PanelRecord*)(m + o_rec);
+  a.skip = skip; a.paulis = pxzs; a.pph = pph; a.rand_ph = d_rand;
   a.state = (int32_t*)(m + o_st); a.anticom = d_anti; a.result = d_res; a.base = m + o_b;
   uint64_t* word = (uint64_t*)(m + o_w);
-  unsigned long long* CP = (unsigned long long*)(m + o_cp);
+  unsigned long long *F = (unsigned long long*)word + (size_t)2 * R, *CP = (unsigned long long*)(m + o_cp);
   uint32_t* pq = (uint32_t*)(m + o_pq);
-  auto buffers = [&](uint32_t b) {  // panel b's words and Paulis, and the next one's
-    a.word = word + (size_t)(b & 1) * R; a.wordn = word + (size_t)((b + 1) & 1) * R;
-    a.CP = CP + (b & 1) * PSTEPS; a.CPn = CP + ((b + 1) & 1) * PSTEPS;
-    a.pq = pq + (b & 1) * PSTEPS; a.pqn = pq + ((b + 1) & 1) * PSTEPS;
+  PanelRecord* rec = (PanelRecord*)(m + o_rec);
+  auto buffers = [&](uint32_t b) {  // of panel b
+    const uint32_t e = b & 1, o = e ^ 1, i0 = b % 3, i1 = (b + 1) % 3, i2 = (b + 2) % 3;
+    a.rec = rec + e; a.prev = rec + o;
+    a.word = word + (size_t)e * R; a.wordn = word + (size_t)o * R;
+    a.F = F + (size_t)o * R; a.Fz = F + (size_t)e * R;
+    a.CP = CP + i0 * PSTEPS; a.CPn = CP + i1 * PSTEPS; a.CPz = CP + i2 * PSTEPS;
+    a.pq = pq + i0 * PSTEPS; a.pqn = pq + i1 * PSTEPS; a.pqz = a.pqp = pq + i2 * PSTEPS;
+    a.CPX = CP + (3 + e) * PSTEPS; a.CPXz = CP + (3 + o) * PSTEPS;
   };
   const uint32_t rest = rank > PP_WINDOW ? rank - PP_WINDOW : 0;
-  void (*steps)(const ProjPanelArgs) = rest <= PP_REST ? project_steps_kernel<1>
-                                     : rest <= 2 * PP_REST ? project_steps_kernel<2>
-                                     : rest <= 5 * PP_REST ? project_steps_kernel<5> : project_steps_kernel<9>;
+  void (*sa)(const ProjPanelArgs) = rest <= PP_REST ? project_steps_apply_kernel<1>
+                                  : rest <= 2 * PP_REST ? project_steps_apply_kernel<2>
+                                  : rest <= 5 * PP_REST ? project_steps_apply_kernel<5> : project_steps_apply_kernel<9>;
   const size_t smem = std::max(sizeof(ApplyFlagSmem), sizeof(PhaseSmem));
-  QCB_CUDA(cudaFuncSetAttribute(project_apply_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  QCB_CUDA(cudaFuncSetAttribute(sa, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const uint32_t nsm = (uint32_t)std::max(device_sm_count(), 1);
   a.nq = (R + 1023) / 1024;
-  a.groups = std::max<uint32_t>(1, std::min<uint32_t>((nsm > a.nq ? nsm - a.nq : 1) / ntile, (R + 255) / 256));
+  a.groups = std::max<uint32_t>(1, std::min<uint32_t>((nsm > a.nq + 1 ? nsm - 1 - a.nq : 1) / ntile, (R + 255) / 256));
   a.per = (R + a.groups - 1) / a.groups;
   const uint32_t row_blocks = (R + 7) / 8, first = *j;
   int32_t h[2] = {0, 0};
   int s = QCB_OK;
   auto go = [&]() -> int {
-    buffers(1);  // the first panel's are panel 1's next
-    a.j0 = a.jn = first; a.cnt = 0; a.cntn = std::min(PSTEPS, k - first); a.apply = 0;
+    const uint32_t grid = 1 + a.nq + ntile * a.groups;
+    uint32_t nb = (k - first + PSTEPS - 1) / PSTEPS;  // panels
+    auto span = [&](uint32_t b) { return b < nb ? std::min(PSTEPS, k - first - b * PSTEPS) : 0u; };
+    buffers(0);
+    a.j0 = first;
     QCB_CUDA(launch_pp(project_load_kernel, row_blocks, 256, 0, st, a));
-    QCB_CUDA(launch_pp(project_apply_kernel, a.nq + ntile * a.groups, 1024, smem, st, a));
-    a.apply = 1;
-    for (uint32_t b = 0, j0 = first; j0 < k; b++, j0 += PSTEPS) {
+    // panel 0's words, as the next words of a panel before it without steps
+    a.jn = first; a.cntn = span(0);
+    a.F = (unsigned long long*)a.word; a.CPn = a.CP; a.pqn = a.pq;
+    QCB_CUDA(launch_pp(sa, grid, 1024, smem, st, a));
+    for (uint32_t b = 0; b <= nb; b++) {
       buffers(b);
-      a.j0 = j0; a.cnt = std::min(PSTEPS, k - j0);
-      a.jn = j0 + a.cnt; a.cntn = std::min(PSTEPS, k - a.jn);
-      QCB_CUDA(launch_pp(steps, 1, 1024, 0, st, a));
+      a.jp = a.j0;
+      a.j0 = first + b * PSTEPS; a.cnt = span(b);
+      a.jn = a.j0 + a.cnt; a.cntn = span(b + 1);
+      a.steps = b < nb; a.apply = b > 0;
+      QCB_CUDA(launch_pp(sa, a.apply || a.cntn ? grid : 1u, 1024, smem, st, a));
+      if (b == nb) break;
       if (b == 0) {
         QCB_CUDA(cudaMemcpyAsync(h, a.state, 8, cudaMemcpyDeviceToHost, st));
         QCB_CUDA(cudaStreamSynchronize(st));
         if (h[0] && (uint32_t)h[1] == first) return QCB_OK;  // the tableau is as it was
+        if (h[0]) nb = 1;  // no second panel
       }
       QCB_CUDA(launch_pp(project_mid_kernel, ntile + 1 + (R + MID_THREADS - 1) / MID_THREADS, MID_THREADS, 0, st, a));
-      QCB_CUDA(launch_pp(project_apply_kernel, a.nq + ntile * a.groups, 1024, smem, st, a));
-      if (b == 0 && h[0]) break;
     }
     QCB_CUDA(launch_pp(project_store_kernel, row_blocks, 256, 0, st, a));
     QCB_CUDA(cudaMemcpyAsync(h, a.state, 8, cudaMemcpyDeviceToHost, st));
