@@ -10,17 +10,19 @@
 // planes packed along shots: plane 2q holds the x bits of qubit q, plane 2q+1
 // its z bits, one uint32 word per 32 shots ("column").  The record is one
 // plane per measurement bit.  A column is independent of every other column
-// under every frame operation, so one thread owns one column for the whole
-// circuit: it walks the compiled program, keeping its column of every touched
-// qubit in shared memory (or in the HBM planes when the frame is too tall),
-// and only the record and the final frame go to HBM.
+// under every frame operation, so a CTA takes a tile of columns through the
+// whole circuit: it walks the compiled program, keeping its columns of every
+// touched qubit in shared memory (or in the HBM planes when the frame is too
+// tall), and only the record and the final frame go to HBM.
 //
 // Noise (Philox mode).  Counter-based streams (key = seed): initZ! and reset
 // draws per (index, shot column); noise per (site, group of 1024 shots), where
 // one word gives the group's Binomial event count and one word per event its
-// shot and kind, in integer fixed point (sample_site_group).  The sites of a
-// FLUSH record are sampled there, as (site, group) tasks spread over the
-// whole CTA, and flipped into the tile with shared-memory atomics.
+// shot and kind, in integer fixed point (sample_site_group).  A kernel before
+// the walk draws the events of every sparse site (presample_kernel) where its
+// scratch fits, else the sites of a FLUSH record are sampled there, as (site,
+// group) tasks spread over the whole CTA; either way a FLUSH flips them into
+// the tile with shared-memory atomics.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
