@@ -90,6 +90,8 @@ syndrome_rows_kernel(const uint32_t* __restrict__ rec, uint64_t pitch, uint64_t 
                      const uint32_t* __restrict__ rows, uint32_t row0, uint32_t nsel, uint32_t Wsyn,
                      uint32_t pairs, uint64_t* __restrict__ out) {
   extern __shared__ __align__(16) uint32_t tile[];  // [SYN_COLS][32 * RS + 2]
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;  // `pairs` warps
   const uint32_t RS = 2 * pairs, CS = 32 * RS + 2;  // words of a shot, of a column
   const uint32_t w0 = blockIdx.x * pairs;           // the CTA's first output word
@@ -259,8 +261,22 @@ int qcb_frame_syndrome_rows(const qcb_frame* f, const uint32_t* bits, size_t nse
   for (uint64_t b0 = 0; b0 < nblk; b0 += 65535) {
     const uint32_t nb = (uint32_t)std::min<uint64_t>(65535, nblk - b0);
     const uint64_t cb = b0 * SYN_COLS;
-    kern<<<dim3(blocks, nb), 32 * pairs, sm, st>>>(f->record + cb, f->pitch, f->ncols - cb, f->frames - cb * 32, d_rows,
-                                                   rows[0], (uint32_t)nsel, Wsyn, pairs, d_out + cb * 32 * Wsyn);
+    // a programmatic dependent of the launch before it, so that a row of these
+    // (the jobs of a batch) and the walk before them leave no launch gaps: 24
+    // jobs with their walk 811 -> 778 us
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks, nb);
+    cfg.blockDim = dim3(32 * pairs);
+    cfg.dynamicSmemBytes = sm;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    QCB_CUDA(cudaLaunchKernelEx(&cfg, kern, (const uint32_t*)(f->record + cb), f->pitch, f->ncols - cb,
+                                f->frames - cb * 32, (const uint32_t*)d_rows, rows[0], (uint32_t)nsel, Wsyn, pairs,
+                                d_out + cb * 32 * Wsyn));
     QCB_LAUNCHED();
   }
   if (!out_on_device) {
