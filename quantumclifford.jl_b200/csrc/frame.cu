@@ -29,6 +29,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <queue>
 #include <unordered_map>
 
 #include "qcb_internal.h"
@@ -2002,6 +2003,72 @@ struct qcb_batch {
 // the walk 1590 us; sampler 141 + walker 702 us.
 constexpr uint64_t BATCH_PRESAMPLE_MAX = 1ull << 30;
 
+// A batch job for the choice of its tile width: program length, columns, the
+// widest tile that fits, and the width (0: to be chosen).
+struct BatchShape {
+  double length;
+  uint64_t ncols;
+  uint32_t tmax, T;
+};
+
+// Time of a tile as in smem_tile, in units of a record word and column.
+static double batch_tile_cost(const BatchShape& b, uint32_t T) {
+  return b.length * (25.0 + ((T & (T - 1)) == 0 ? 0.75 : 1.0) * T);
+}
+
+// The widths of the jobs that have none: powers of two, the widest whose tile
+// takes no longer than a limit common to all jobs, with the limit (a tile of
+// the longest program at one of its widths) that gives the shortest longest
+// SM when the tiles go longest first to the next free one.  Batches of few
+// tiles gain from narrow ones, and long programs before short ones; many
+// tiles an SM need no search.  Surface codes (jobs, largest d and shots), us, the
+// widest tiles for all before: 12, 13, 30000 371 -> 181; 8, 11, 300000 186 -> 114;
+// 20, 7, 8210 106 -> 73; 24, 13, 300000 619 -> 609; 24, 7, 300000 237 -> 238; one
+// power of two for all is no better in any of them.
+static void batch_widths(std::vector<BatchShape>& jobs) {
+  constexpr uint64_t MANY = 64;  // tiles an SM: the last ones hardly count
+  const uint64_t nsm = (uint64_t)std::max(device_sm_count(), 1);
+  const BatchShape* longest = nullptr;
+  for (auto& b : jobs)
+    if (!b.T && (!longest || b.length > longest->length)) longest = &b;
+  if (!longest) return;
+  auto width = [](const BatchShape& b, double limit) {
+    uint32_t T = 256;
+    while (T > 16 && (T > b.tmax || T / 2 >= b.ncols || batch_tile_cost(b, T) > limit)) T /= 2;
+    return T;
+  };
+  double best = 0, best_limit = 0;
+  for (uint32_t w = 256; w >= 16; w /= 2) {
+    if (w > 16 && w > longest->tmax) continue;
+    const double limit = batch_tile_cost(*longest, w);
+    std::vector<std::pair<double, uint64_t>> tiles;  // (time, number) of each job
+    uint64_t n = 0;
+    for (auto& b : jobs) {
+      const uint32_t T = b.T ? b.T : width(b, limit);
+      tiles.push_back({batch_tile_cost(b, T), (b.ncols + T - 1) / T});
+      n += tiles.back().second;
+    }
+    double end = 0;
+    if (n > MANY * nsm) {
+      for (auto& t : tiles) end += t.first * (double)t.second / (double)nsm;
+    } else {
+      std::sort(tiles.begin(), tiles.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
+      std::priority_queue<double, std::vector<double>, std::greater<double>> sm;  // when each SM is free
+      for (uint64_t k = 0; k < nsm; k++) sm.push(0.0);
+      for (auto& t : tiles)
+        for (uint64_t k = 0; k < t.second; k++) {
+          const double e = sm.top() + t.first;
+          sm.pop();
+          sm.push(e);
+          end = std::max(end, e);
+        }
+    }
+    if (best_limit == 0 || end < best) { best = end; best_limit = limit; }
+  }
+  for (auto& b : jobs)
+    if (!b.T) b.T = width(b, best_limit);
+}
+
 // The scratch and the sampler's work list of a batch; the jobs' walks are
 // pointed at it.
 static int batch_presample(qcb_batch& b, const qcb_batch_job* jobs, size_t n_jobs, std::vector<qcb::WalkArgs>& wa) {
@@ -2062,6 +2129,7 @@ int qcb_batch_create(const qcb_batch_job* jobs, size_t n_jobs, qcb_batch** out) 
   uint32_t win_words = PROG_WINDOW_WORDS;
   for (size_t j = 0; j < n_jobs; j++)
     if (jobs[j].program) win_words = std::max(win_words, jobs[j].program->win_words);
+  std::vector<BatchShape> shape(n_jobs);
   for (size_t j = 0; j < n_jobs; j++) {
     const qcb_batch_job& J = jobs[j];
     qcb_noise_source n{};
@@ -2075,10 +2143,15 @@ int qcb_batch_create(const qcb_batch_job* jobs, size_t n_jobs, qcb_batch** out) 
     if (T && (T % 2 || T < 16 || T > tmax)) return fail(QCB_EARG, "batch job " + std::to_string(j) + ": bad tile width");
     if (!T) {
       auto it = g_tuned_tile.find(J.program->nslots);
-      T = it != g_tuned_tile.end() ? std::min(it->second, tmax) : tmax;
+      if (it != g_tuned_tile.end()) T = std::min(it->second, tmax);
     }
+    shape[j] = {(double)J.program->stream_slot.size(), J.frame->ncols, tmax, T};
+  }
+  batch_widths(shape);
+  for (size_t j = 0; j < n_jobs; j++) {
+    const qcb_batch_job& J = jobs[j];
     const uint64_t ncols = J.frame->ncols;
-    T = (uint32_t)std::min<uint64_t>(T, std::max<uint64_t>(16, (ncols + 1) & ~1ull));
+    const uint32_t T = (uint32_t)std::min<uint64_t>(shape[j].T, std::max<uint64_t>(16, (ncols + 1) & ~1ull));
     WalkArgs& a = wa[j];
     fill_common(a, J.frame, J.program);
     a.seed = J.seed;
@@ -2088,7 +2161,7 @@ int qcb_batch_create(const qcb_batch_job* jobs, size_t n_jobs, qcb_batch** out) 
     tile_words = std::max(tile_words, 2 * J.program->nslots * T);
     b->frames.push_back(J.frame);
     // longest first: a tile walks every record once, its ops over T columns
-    const double cost = (double)J.program->stream_slot.size() * (1.0 + T / 64.0);
+    const double cost = batch_tile_cost(shape[j], T);
     for (uint64_t t = 0; t * T < ncols; t++) items.push_back({cost, (uint32_t)j, t});
   }
   std::stable_sort(items.begin(), items.end(), [](const Cost& x, const Cost& y) { return x.c > y.c; });
