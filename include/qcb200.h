@@ -225,7 +225,8 @@ int qcb_frame_download_planes(const qcb_frame* f, uint32_t* x_planes, uint32_t* 
  * shot_offset.  The (job, shot-tile) items are queued longest first and taken
  * by one CTA per SM.  qcb_batch_run only clears counters and launches: it can
  * be captured in a CUDA graph.  The batch holds up to 1 GB of device memory for
- * its jobs' pre-sampled noise; jobs past that draw theirs in the walk.  Frames and programs must outlive the
+ * its jobs' pre-sampled noise; jobs past that draw theirs in the walk, as all
+ * do where that memory is not there.  Frames and programs must outlive the
  * batch; the frame tile of every job must fit one CTA's shared memory.      */
 typedef struct qcb_batch_job {
   qcb_frame* frame;
@@ -233,7 +234,8 @@ typedef struct qcb_batch_job {
   uint64_t seed;
   uint64_t shot_offset;   /* a multiple of 1024                                */
   uint32_t tile;          /* shot columns per tile (even, 16..256); 0 = tuned
-                             width of the job's size class, else the widest  */
+                             width of the job's size class, else chosen for
+                             the batch as a whole                            */
   uint32_t reserved;
 } qcb_batch_job;
 typedef struct qcb_batch qcb_batch;

@@ -621,7 +621,7 @@ __device__ __forceinline__ bool walk_tile(const WalkArgs& a, uint32_t* sm, uint3
   }
 
   // ---- pre-sampled noise: thread (pgl, pl) takes events pl, pl + pS, ... of
-  // the buckets of its group G0 + pgl of the tile; the count and the first
+  // the buckets of its group pG0 + pgl of the tile; the count and the first
   // two events of the next flush part are loaded one part ahead (issued at a
   // flush, they arrive while the following records run)
   const uint64_t pG0 = (a.col0 + c0) / 32;
@@ -815,7 +815,7 @@ __device__ __forceinline__ bool walk_tile(const WalkArgs& a, uint32_t* sm, uint3
               }
             };
             if (PRE && a.pre_buf) {
-              // pre-sampled: bucket (group G0 + pgl, part j), the count and
+              // pre-sampled: bucket (group pG0 + pgl, part j), the count and
               // first events loaded at the previous flush part
               const uint32_t j = h.z, off = h.w, cap = h.y >> 8;
               const uint32_t total = pf_tot, ev0 = pf_e0, ev1 = pf_e1;
