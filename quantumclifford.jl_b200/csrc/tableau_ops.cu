@@ -517,6 +517,9 @@ __global__ void __launch_bounds__(256) apply_dense_kernel(uint64_t* xzs, uint8_t
 // 12645 -> 5365, 20000 x 100 190 -> 53.  (The tables waiting for dense_q_kernel,
 // loads through L1, the join's loads four at a time: 1000 22, 4000 759.)
 constexpr uint32_t DENSE_RUNS = 16;
+// Shared memory of the tables at most: the limit of every launch of a form, so
+// that calls of other sizes on other threads never lower it in between.
+constexpr size_t DENSE_TABLE_SMEM = 200 * 1024;
 constexpr size_t DENSE_SCRATCH = 64ull << 20;
 struct DenseArgs {
   uint64_t* xzs;
@@ -943,7 +946,7 @@ static int apply_dense_tables(qcb_tableau* t, const qcb_tableau* c, int phases, 
   a.W = t->W; a.n = t->nqubits; a.c = c->xzs; a.cph = c->phases; a.phases = phases;
   const size_t table = (size_t)16 * len * sizeof(ulonglong2);
   a.NT = 16;
-  while (a.NT * len > f.threads || a.NT * table > (size_t)200 * 1024) a.NT /= 2;
+  while (a.NT * len > f.threads || a.NT * table > DENSE_TABLE_SMEM) a.NT /= 2;
   const size_t smem = a.NT * table;
   // Runs of whole qubit words: the least waves x (words of a run x the time of
   // a word's tables, with 3 us for a CTA) and the partial products' traffic.  As
@@ -981,7 +984,7 @@ static int apply_dense_tables(qcb_tableau* t, const qcb_tableau* c, int phases, 
     slab = std::max(f.rows, slab / 2 / f.rows * f.rows);
   }
   a.qt = m; a.part = (ulonglong2*)(m + o_part); a.odd = m + o_odd;
-  QCB_CUDA(cudaFuncSetAttribute(f.k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  QCB_CUDA(cudaFuncSetAttribute(f.k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DENSE_TABLE_SMEM));
   if (phases) QCB_CUDA(launch_dependent(dense_q_kernel, dim3((32 * len + 7) / 8), 256, 0, st, a));
   for (uint32_t r0 = 0; r0 < R; r0 += slab) {
     a.xzs = t->xzs + (size_t)r0 * t->W;

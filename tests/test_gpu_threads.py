@@ -1,0 +1,65 @@
+"""Host threads with a handle and a stream of their own: calls on tableaux of
+different sizes at the same time, which share the kernels' launch attributes."""
+import ctypes
+import threading
+
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from qcb200 import Tableau
+from qcb200._lib import check
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def qcb():
+    import qcb200
+
+    qcb200.ensure_init(0)
+    return qcb200
+
+
+def run_threads(jobs, times):
+    """jobs: functions of a stream pointer, each called `times` times by a
+    thread of its own, all at once; the first error of each."""
+    errors, gate = [None] * len(jobs), threading.Barrier(len(jobs))
+
+    def body(k):
+        st = torch.cuda.Stream()
+        try:
+            gate.wait()
+            for _ in range(times):
+                jobs[k](ctypes.c_void_p(st.cuda_stream))
+        except Exception as e:  # noqa: BLE001
+            errors[k] = e
+        st.synchronize()
+
+    threads = [threading.Thread(target=body, args=(k,)) for k in range(len(jobs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    return errors
+
+
+def random_rows(rows, n, rng):
+    return Tableau.from_bits(rng.integers(0, 4, rows), rng.random((rows, n)) < 0.5, rng.random((rows, n)) < 0.5)
+
+
+def test_dense_apply_of_two_sizes_at_once(qcb):
+    """Operators on 1000 and on 800 qubits (64 and 52 KB of tables)."""
+    rng = np.random.default_rng(1)
+    jobs, tabs, times = [], [], 400
+    for n in (1000, 800):
+        op = qcb.CliffordOperator(qcb.tensor_pow(qcb.tCNOT(), n // 2).tab).to_gpu()
+        t = random_rows(40, n, rng)
+        g = t.copy().to_gpu()
+        tabs.append((t, g, op))
+        jobs.append(lambda st, g=g, op=op: check(qcb.lib().qcb_apply_dense(g.dev.handle, op.tab.dev.handle, 1, st)))
+    assert run_threads(jobs, times) == [None, None]
+    for t, g, op in tabs:  # tCNOT twice is the identity
+        g.to_cpu()
+        assert np.array_equal(g.xzs, t.xzs) and np.array_equal(g.phases, t.phases)
