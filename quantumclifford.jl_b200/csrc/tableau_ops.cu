@@ -847,6 +847,10 @@ static size_t layer_min_gates(const qcb_tableau* t) { return 8 + (((size_t)t->ro
 
 static size_t layer_smem(const qcb_tableau* t) { return (size_t)LAYER_SLICE * (2 * t->W + 1) * 4; }
 
+// The most a slice may take, and the limit of every launch above the default
+// one: a call on a smaller tableau on another thread does not lower it.
+static size_t layer_smem_max() { return (size_t)device_max_smem_optin() - 1024; }
+
 template <uint32_t CAP>
 static int launch_layers(const qcb_tableau* t, const std::vector<uint64_t>& list, uint32_t threads, int phases,
                          cudaStream_t st) {
@@ -854,7 +858,7 @@ static int launch_layers(const qcb_tableau* t, const std::vector<uint64_t>& list
   std::copy(list.begin(), list.end(), l.e);
   const size_t sm = layer_smem(t);
   if (sm > 40 * 1024)
-    QCB_CUDA(cudaFuncSetAttribute(apply_layers_kernel<CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    QCB_CUDA(cudaFuncSetAttribute(apply_layers_kernel<CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)layer_smem_max()));
   QCB_CUDA(launch_gates(apply_layers_kernel<CAP>, (t->rows + LAYER_SLICE - 1) / LAYER_SLICE, threads, sm, st, t->xzs,
                         t->phases, t->rows, t->W, (const LayerList<CAP>&)l, (uint32_t)list.size(), phases));
   QCB_LAUNCHED();
@@ -1191,7 +1195,7 @@ int qcb_apply_gates(qcb_tableau* t, const qcb_op* ops, size_t n_ops, int phases,
   }
   if (g.empty() || !t->rows) return QCB_OK;
   cudaStream_t st = S(stream);
-  if (g.size() >= layer_min_gates(t) && layer_smem(t) <= (size_t)device_max_smem_optin() - 1024)
+  if (g.size() >= layer_min_gates(t) && layer_smem(t) <= layer_smem_max())
     return apply_layers(t, g, phases, st);
   for (size_t k0 = 0; k0 < g.size(); k0 += GATE_BATCH) {
     const uint32_t n = (uint32_t)std::min<size_t>(GATE_BATCH, g.size() - k0);
