@@ -1588,7 +1588,10 @@ static int launch_grid(const ElimSpec& e, cudaStream_t st) {
                                    : rest <= 5 * STEP_REST ? canon_steps_apply_kernel<5> : canon_steps_apply_kernel<9>;
   static_assert(STEP_WINDOW + 9 * STEP_REST >= CANON_GRID_MAX_ROWS, "every row has a thread");
   const size_t smem = std::max({sizeof(ApplySmem), sizeof(PhaseSmem), (size_t)R * 16});
-  QCB_CUDA(cudaFuncSetAttribute(l1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // the limit for the most rows, whatever this call's: calls on other threads
+  // may be between their limit and their launches
+  constexpr size_t smem_max = std::max({sizeof(ApplySmem), sizeof(PhaseSmem), (size_t)CANON_GRID_MAX_ROWS * 16});
+  QCB_CUDA(cudaFuncSetAttribute(l1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max));
   // L1: the steps' CTA has an SM of its own (1024 threads of up to 64
   // registers fill its register file), the apply the other SMs: a CTA per
   // tile and range of at least 256 rows (a CTA's tables cost about as much

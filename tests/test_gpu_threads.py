@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 import torch
 
+import oracle
 from qcb200 import Tableau, ops as O
 from qcb200._lib import check, ptr
 
@@ -78,3 +79,19 @@ def test_gate_lists_on_two_widths_at_once(qcb):
     for t, g in tabs:  # CNOTs twice are the identity
         g.to_cpu()
         assert np.array_equal(g.xzs, t.xzs) and np.array_equal(g.phases, t.phases)
+
+
+def test_canonicalize_of_two_heights_at_once(qcb):
+    """Views of 8192 and 5100 rows (128 and 80 KB of row lists)."""
+    rng = np.random.default_rng(3)
+    jobs, tabs = [], []
+    for rows in (8192, 5100):
+        t = random_rows(rows, 130, rng)
+        g = qcb.Stabilizer(t.copy()).to_gpu()
+        tabs.append((t, g))
+        jobs.append(lambda st, g=g, rows=rows: check(qcb.lib().qcb_canonicalize(g.tab.dev.handle, 1, rows, 0, None, None, st)))
+    assert run_threads(jobs, 100) == [None, None]
+    for t, g in tabs:  # without phases, the canonical form is its own
+        _, xz, _, _ = oracle.canonicalize(t.phases, t.xzs, 130, False)
+        g.to_cpu()
+        assert np.array_equal(g.tab.xzs, xz)
