@@ -372,7 +372,9 @@ int qcb_pftrajectories_fresh(qcb_frame* f, const qcb_program* prog, uint64_t see
  * "walker_narrow" 1 (default) / 0: programs too tall for a 16-column
  * shared-memory tile run in 8..14-column tiles, or on the HBM planes.
  * "gates_pdl" 1 (default) / 0: qcb_apply_gates launches as programmatic
- * dependents of the launch before them on the stream, or plain.            */
+ * dependents of the launch before them on the stream, or plain.  Test knob
+ * "scratch_limit" k > 0: device scratch of more than k KB counts as not there,
+ * in the calls that go another way without it (canonicalize!).             */
 int qcb_tune_set(const char* key, int64_t value);
 
 /* ------------------------------------------------------------ tableaux    */

@@ -1564,16 +1564,20 @@ constexpr uint32_t CANON_LOOK_PANELS = 16;
 
 // canonicalize! by panels over the whole GPU; scratch (the tiles: the tableau
 // rounded up to two word columns, and small arrays) from the stream-ordered
-// pool in one piece.
-static int launch_grid(const ElimSpec& e, cudaStream_t st) {
+// pool in one piece.  Without room for it *none is set and nothing done.
+static int launch_grid(const ElimSpec& e, cudaStream_t st, bool* none) {
   const uint32_t R = e.rows, W = e.W, len = W / 2, ntile = (len + 1) / 2;
   CanonPanelArgs a{};
   size_t bytes = 0;
   auto place = [&](size_t n) { const size_t o = bytes; bytes += (n + 127) / 128 * 128; return o; };
   const size_t o_t = place((size_t)ntile * R * 32), o_po = place((size_t)ntile * PSTEPS * 32), o_w = place((size_t)R * 8),
                o_u = place((size_t)R * 8), o_q = place(R), o_par = place((size_t)ntile * R), o_inv = place((size_t)R * 4), o_rec = place(2 * sizeof(PanelRecord));
-  uint8_t* m = nullptr;
-  QCB_CUDA(cudaMallocAsync(&m, bytes, st));
+  Scratch scratch(st);
+  const cudaError_t got = scratch.alloc(bytes);
+  *none = got == cudaErrorMemoryAllocation;
+  if (*none) return QCB_OK;
+  QCB_CUDA(got);
+  uint8_t* m = scratch.p;
   PanelRecord* rec = (PanelRecord*)(m + o_rec);
   a.p = PanelTiles{R, W, len, ntile, e.phases, (ulonglong2*)(m + o_t), (ulonglong2*)(m + o_po), (uint64_t*)(m + o_w),
                    (uint64_t*)(m + o_u), m + o_q, m + o_par};
@@ -1628,7 +1632,6 @@ static int launch_grid(const ElimSpec& e, cudaStream_t st) {
     QCB_CUDA(launch_panel(canon_mid_kernel, ntile + 1 + (R + MID_THREADS - 1) / MID_THREADS, MID_THREADS, 0, st, a));
   }
   QCB_CUDA(launch_panel(canon_tiles_store_kernel, row_blocks, 32 * warps, 0, st, a));
-  QCB_CUDA(cudaFreeAsync(m, st));
   return QCB_OK;
 }
 
@@ -1641,8 +1644,11 @@ static int eliminate(const ElimSpec& e, cudaStream_t st) {
   }
   const bool D = e.dxzs != nullptr;
   if (e.mode == ELIM_BOTH && !D && e.n > 0 && g_canon_blocked != 2 && g_canon_grid != 2 && e.rows <= CANON_GRID_MAX_ROWS &&
-      (g_canon_grid == 1 || canon_grid_pays(e.rows, e.n)))
-    return launch_grid(e, st);
+      (g_canon_grid == 1 || canon_grid_pays(e.rows, e.n))) {
+    bool none = false;  // no room for a copy of the rows: the cluster kernels
+    const int s = launch_grid(e, st, &none);
+    if (!none) return s;
+  }
   if (e.mode == ELIM_BOTH && !D && e.rows <= 8192 && g_canon_blocked != 2 && (g_canon_blocked == 1 || e.rows >= 64))
     return launch_blocked(e, st);
   CanonPlan p = canon_plan(e.rows, e.W, D);

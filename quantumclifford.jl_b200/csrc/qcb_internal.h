@@ -46,6 +46,24 @@ constexpr size_t DEV_POOL_MAX = 64ull << 20;
 cudaError_t dev_alloc(void** p, size_t bytes, bool zero, const void* init = nullptr, size_t init_bytes = 0);
 void dev_free(void* p, size_t bytes);
 
+// Scratch of one call from the stream-ordered pool, given back in stream order
+// when it goes out of scope.  cudaErrorMemoryAllocation (memory not there, or
+// the test knob "scratch_limit") leaves no error behind: the caller goes
+// another way.
+struct Scratch {
+  uint8_t* p = nullptr;
+  cudaStream_t st;
+  explicit Scratch(cudaStream_t s) : st(s) {}
+  Scratch(const Scratch&) = delete;
+  Scratch& operator=(const Scratch&) = delete;
+  ~Scratch() {
+    if (p) cudaFreeAsync(p, st);
+  }
+  cudaError_t alloc(size_t bytes);
+};
+// Whether scratch of this size is to count as not there ("scratch_limit").
+bool scratch_refused(size_t bytes);
+
 // ------------------------------------------------------------ Philox
 enum : uint32_t { TAG_INITZ = 0x51A7u, TAG_RESET = 0x5E5Eu, TAG_NOISE = 0x4E01u };
 

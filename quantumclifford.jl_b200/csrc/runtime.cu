@@ -86,6 +86,20 @@ void dev_free(void* p, size_t bytes) {
   if (other) cudaSetDevice(dev);
 }
 
+static std::atomic<uint32_t> g_scratch_limit{0};  // KB; test knob, 0: none
+
+bool scratch_refused(size_t bytes) {
+  const uint32_t kb = g_scratch_limit.load(std::memory_order_relaxed);
+  return kb && bytes > (size_t)kb << 10;
+}
+
+cudaError_t Scratch::alloc(size_t bytes) {
+  cudaError_t e = scratch_refused(bytes) ? cudaErrorMemoryAllocation : cudaMallocAsync(&p, bytes, st);
+  if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+  if (e != cudaSuccess) p = nullptr;
+  return e;
+}
+
 __global__ void philox_probe_kernel(uint4 ctr, uint2 key, uint32_t* out) {
   uint32_t o[4];
   philox4x32_10(ctr.x, ctr.y, ctr.z, ctr.w, key.x, key.y, o);
@@ -217,6 +231,9 @@ int qcb_tune_set(const char* key, int64_t value) {
     // canonicalize! by panels over the whole GPU: 0 from 64 rows, 1 always, 2 never
     if (value > 2) return fail(QCB_EARG, "canon_grid must be 0 (automatic), 1 (always) or 2 (never)");
     set_canon_grid((uint32_t)value);
+  } else if (k == "scratch_limit") {
+    // test knob: scratch of more than this many KB counts as not there (0: none does)
+    g_scratch_limit.store((uint32_t)value);
   } else if (k == "canon_rpt") {
     if (value && value != 1 && value != 2 && value != 4 && value != 8 && value != 16)
       return fail(QCB_EARG, "canon_rpt must be 0, 1, 2, 4, 8 or 16");
