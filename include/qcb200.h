@@ -570,14 +570,22 @@ int qcb_apply_dense(qcb_tableau* t, const qcb_tableau* c, int phases, void* stre
 /* ------------------------------------------------------------ diagnostics */
 /* Philox-4x32-10 block (counter, key) -> out, computed on the device.       */
 int qcb_debug_philox(const uint32_t ctr[4], const uint32_t key[2], uint32_t out[4]);
-/* Compile on the host only (no device needed) and copy out the device
- * program: the record stream (uint32 words), the noise-site table (80 bytes
- * per site), and per slot the frame qubit and the final x<->z relabel flag.
- * Buffers may be NULL or too small, in which case only the sizes are set.   */
+/* Compile on the host only (no device needed) and copy out the program: the
+ * record stream (uint32 words), the noise-site table (80 bytes per site), and
+ * per slot the frame qubit and which of the slot's two planes (2s or 2s + 1)
+ * its x bits end in.  Buffers may be NULL or too small, in which case only the
+ * sizes are set.  `_dump` numbers the planes with x first (x of slot s starts
+ * in plane 2s); `_device` gives the program as qcb_program_compile uploads it:
+ * x of an odd slot starts in plane 2s + 1, and the entries of a two-qubit
+ * record are ordered by their planes' parities.                             */
 int qcb_debug_program_dump(const qcb_op* ops, size_t n_ops, uint32_t* stream, size_t stream_cap,
                            size_t* stream_len, uint8_t* sites, size_t sites_cap, size_t* n_sites,
                            uint32_t* slot_qubit, uint32_t* slot_swap, size_t slots_cap, size_t* n_slots,
                            qcb_program_info* info);
+int qcb_debug_program_device(const qcb_op* ops, size_t n_ops, uint32_t* stream, size_t stream_cap,
+                             size_t* stream_len, uint8_t* sites, size_t sites_cap, size_t* n_sites,
+                             uint32_t* slot_qubit, uint32_t* slot_swap, size_t slots_cap, size_t* n_slots,
+                             qcb_program_info* info);
 
 #ifdef __cplusplus
 }

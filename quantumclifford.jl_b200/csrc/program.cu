@@ -599,12 +599,11 @@ int qcb_program_compile(const qcb_op* ops, size_t n_ops, qcb_program** out) {
   return QCB_OK;
 }
 
-int qcb_debug_program_dump(const qcb_op* ops, size_t n_ops, uint32_t* stream, size_t stream_cap,
-                           size_t* stream_len, uint8_t* sites, size_t sites_cap, size_t* n_sites,
-                           uint32_t* slot_qubit, uint32_t* slot_swap, size_t slots_cap, size_t* n_slots,
-                           qcb_program_info* info) {
+static int program_dump(const qcb_op* ops, size_t n_ops, bool flip, uint32_t* stream, size_t stream_cap,
+                        size_t* stream_len, uint8_t* sites, size_t sites_cap, size_t* n_sites, uint32_t* slot_qubit,
+                        uint32_t* slot_swap, size_t slots_cap, size_t* n_slots, qcb_program_info* info) {
   Program P;
-  int st = compile(ops, n_ops, P, false);  // x planes first in every slot
+  int st = compile(ops, n_ops, P, flip);
   if (st != QCB_OK) return st;
   if (stream_len) *stream_len = P.stream_slot.size();
   if (n_sites) *n_sites = P.sites_slot.size();
@@ -621,6 +620,22 @@ int qcb_debug_program_dump(const qcb_op* ops, size_t n_ops, uint32_t* stream, si
     }
   }
   return QCB_OK;
+}
+
+int qcb_debug_program_dump(const qcb_op* ops, size_t n_ops, uint32_t* stream, size_t stream_cap,
+                           size_t* stream_len, uint8_t* sites, size_t sites_cap, size_t* n_sites,
+                           uint32_t* slot_qubit, uint32_t* slot_swap, size_t slots_cap, size_t* n_slots,
+                           qcb_program_info* info) {
+  return program_dump(ops, n_ops, false, stream, stream_cap, stream_len, sites, sites_cap, n_sites, slot_qubit, slot_swap,
+                      slots_cap, n_slots, info);
+}
+
+int qcb_debug_program_device(const qcb_op* ops, size_t n_ops, uint32_t* stream, size_t stream_cap,
+                             size_t* stream_len, uint8_t* sites, size_t sites_cap, size_t* n_sites,
+                             uint32_t* slot_qubit, uint32_t* slot_swap, size_t slots_cap, size_t* n_slots,
+                             qcb_program_info* info) {
+  return program_dump(ops, n_ops, true, stream, stream_cap, stream_len, sites, sites_cap, n_sites, slot_qubit, slot_swap,
+                      slots_cap, n_slots, info);
 }
 
 int qcb_program_info_get(const qcb_program* prog, qcb_program_info* info) {
