@@ -1989,12 +1989,23 @@ struct qcb_batch {
   uint32_t win_words = 0;
   size_t smem_bytes = 0;
   uint32_t grid = 0;
-  // pre-sampled noise: every job's counters, then every job's buckets
+  // pre-sampled noise, one block: every job's counters, every job's buckets,
+  // the sampler's jobs and items
   uint32_t* pre = nullptr;
   size_t pre_bytes = 0, pre_cnt_bytes = 0;
   qcb::PresampleArgs* d_pre_jobs = nullptr;
   qcb::PresampleItem* d_pre_items = nullptr;
   uint32_t n_pre_items = 0;
+
+  qcb_batch() = default;
+  qcb_batch(const qcb_batch&) = delete;
+  qcb_batch& operator=(const qcb_batch&) = delete;
+  ~qcb_batch() {
+    cudaFree(d_jobs);
+    cudaFree(d_items);
+    cudaFree(d_head);
+    qcb::dev_free(pre, pre_bytes);
+  }
 };
 
 // Event buckets of a batch's jobs at most; jobs past it draw their noise in
@@ -2084,17 +2095,26 @@ static int batch_presample(qcb_batch& b, const qcb_batch_job* jobs, size_t n_job
     ids.push_back(j);
   }
   if (ids.empty()) return QCB_OK;
-  b.pre_cnt_bytes = cnt * 4;
-  b.pre_bytes = (cnt + buf) * 4;
-  const cudaError_t e = dev_alloc((void**)&b.pre, b.pre_bytes, false);
+  uint64_t nitems = 0;
+  auto item_count = [&](size_t j) {
+    const uint64_t ngroups = (jobs[j].frame->ncols + 31) / 32;
+    return (ngroups + PRESAMPLE_ITEM_GROUPS - 1) / PRESAMPLE_ITEM_GROUPS * ((jobs[j].program->pre_ent.size() + 255) / 256);
+  };
+  for (size_t j : ids) nitems += item_count(j);
+  const size_t o_jobs = ((size_t)(cnt + buf) * 4 + 255) / 256 * 256;
+  const size_t o_items = o_jobs + (ids.size() * sizeof(PresampleArgs) + 255) / 256 * 256;
+  const size_t bytes = o_items + nitems * sizeof(PresampleItem);
+  const cudaError_t e = scratch_refused(bytes) ? cudaErrorMemoryAllocation : dev_alloc((void**)&b.pre, bytes, false);
   if (e == cudaErrorMemoryAllocation) {  // no room: the walk draws the noise
     cudaGetLastError();
-    b.pre_cnt_bytes = b.pre_bytes = 0;
     return QCB_OK;
   }
+  b.pre_bytes = bytes;
   QCB_CUDA(e);
+  b.pre_cnt_bytes = cnt * 4;
   std::vector<PresampleArgs> args;
   std::vector<PresampleItem> items;
+  items.reserve(nitems);
   uint32_t *pc = b.pre, *pb = b.pre + cnt;
   for (size_t j : ids) {
     const qcb_program* p = jobs[j].program;
@@ -2107,8 +2127,8 @@ static int batch_presample(qcb_batch& b, const qcb_batch_job* jobs, size_t n_job
       for (uint32_t e = 0; e < q.nent; e += 256) items.push_back({(uint32_t)args.size() - 1, e, (uint32_t)g, 0u});
   }
   b.n_pre_items = (uint32_t)items.size();
-  QCB_CUDA(cudaMalloc(&b.d_pre_jobs, args.size() * sizeof(PresampleArgs)));
-  QCB_CUDA(cudaMalloc(&b.d_pre_items, items.size() * sizeof(PresampleItem)));
+  b.d_pre_jobs = (PresampleArgs*)((uint8_t*)b.pre + o_jobs);
+  b.d_pre_items = (PresampleItem*)((uint8_t*)b.pre + o_items);
   QCB_CUDA(cudaMemcpy(b.d_pre_jobs, args.data(), args.size() * sizeof(PresampleArgs), cudaMemcpyHostToDevice));
   QCB_CUDA(cudaMemcpy(b.d_pre_items, items.data(), items.size() * sizeof(PresampleItem), cudaMemcpyHostToDevice));
   return QCB_OK;
@@ -2172,16 +2192,12 @@ int qcb_batch_create(const qcb_batch_job* jobs, size_t n_jobs, qcb_batch** out) 
   b->tile_words = tile_words;
   b->win_words = win_words;
   b->smem_bytes = (size_t)((tile_words + 31) & ~31u) * 4 + (size_t)2 * win_words * 4 + 16;
-  if (int s = batch_presample(*b, jobs, n_jobs, wa)) {
-    dev_free(b->pre, b->pre_bytes);
-    cudaFree(b->d_pre_jobs);
-    cudaFree(b->d_pre_items);
-    return s;
-  }
   b->grid = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(b->nitems, 1), (uint64_t)device_sm_count());
+  // what the batch cannot do without first: the noise scratch takes what is left
   QCB_CUDA(cudaMalloc(&b->d_jobs, std::max<size_t>(wa.size(), 1) * sizeof(WalkArgs)));
   QCB_CUDA(cudaMalloc(&b->d_items, std::max<size_t>(it.size(), 1) * sizeof(BatchItem)));
   QCB_CUDA(cudaMalloc(&b->d_head, 4));
+  if (int s = batch_presample(*b, jobs, n_jobs, wa)) return s;
   if (!wa.empty()) QCB_CUDA(cudaMemcpy(b->d_jobs, wa.data(), wa.size() * sizeof(WalkArgs), cudaMemcpyHostToDevice));
   if (!it.empty()) QCB_CUDA(cudaMemcpy(b->d_items, it.data(), it.size() * sizeof(BatchItem), cudaMemcpyHostToDevice));
   cudaFuncAttributes fa{};
@@ -2228,13 +2244,6 @@ int qcb_batch_status(const qcb_batch* b) {
 }
 
 int qcb_batch_destroy(qcb_batch* b) {
-  if (!b) return QCB_OK;
-  cudaFree(b->d_jobs);
-  cudaFree(b->d_items);
-  cudaFree(b->d_head);
-  cudaFree(b->d_pre_jobs);
-  cudaFree(b->d_pre_items);
-  dev_free(b->pre, b->pre_bytes);
   delete b;
   return QCB_OK;
 }

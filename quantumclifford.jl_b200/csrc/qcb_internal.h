@@ -16,10 +16,17 @@ int fail(int status, const std::string& msg);
 int cuda_fail(cudaError_t e, const char* what);
 extern std::atomic<uint64_t> g_launches;
 
-#define QCB_CUDA(call)                                        \
-  do {                                                        \
-    cudaError_t e_ = (call);                                  \
-    if (e_ != cudaSuccess) return ::qcb::cuda_fail(e_, #call); \
+// Test knob "fail_call": the k-th checked call from now on is not made and
+// counts as failed.
+extern std::atomic<uint32_t> g_fail_call;
+inline bool call_withheld() {
+  return g_fail_call.load(std::memory_order_relaxed) && g_fail_call.fetch_sub(1) == 1;
+}
+
+#define QCB_CUDA(call)                                                                \
+  do {                                                                                \
+    cudaError_t e_ = ::qcb::call_withheld() ? cudaErrorUnknown : (cudaError_t)(call); \
+    if (e_ != cudaSuccess) return ::qcb::cuda_fail(e_, #call);                        \
   } while (0)
 
 // Check the launch that was just issued and count it.

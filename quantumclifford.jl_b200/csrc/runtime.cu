@@ -8,6 +8,7 @@
 namespace qcb {
 
 std::atomic<uint64_t> g_launches{0};
+std::atomic<uint32_t> g_fail_call{0};
 static thread_local int t_status = QCB_OK;
 static thread_local std::string t_msg;
 
@@ -234,6 +235,9 @@ int qcb_tune_set(const char* key, int64_t value) {
   } else if (k == "scratch_limit") {
     // test knob: scratch of more than this many KB counts as not there (0: none does)
     g_scratch_limit.store((uint32_t)value);
+  } else if (k == "fail_call") {
+    // test knob: the value-th checked CUDA call from now on fails without being made (0: none)
+    g_fail_call.store((uint32_t)value);
   } else if (k == "canon_rpt") {
     if (value && value != 1 && value != 2 && value != 4 && value != 8 && value != 16)
       return fail(QCB_EARG, "canon_rpt must be 0, 1, 2, 4, 8 or 16");

@@ -1,9 +1,13 @@
-"""Calls whose device scratch is not there (test knob "scratch_limit")."""
+"""Calls whose device scratch is not there (test knob "scratch_limit") or that
+end in the middle (test knob "fail_call")."""
+import ctypes
+
 import numpy as np
 import pytest
+import torch
 
 import oracle
-from qcb200 import randoms
+from qcb200 import circuits, ops as O, randoms
 from test_gpu_tableau import rand_tab
 
 pytestmark = pytest.mark.gpu
@@ -33,3 +37,74 @@ def test_canonicalize_without_scratch(qcb, no_scratch, rows, n, phases):
     ph, xz, orx, orz = oracle.canonicalize(t.phases, t.xzs, n, phases)
     assert (rx, rz) == (orx, orz)
     assert np.array_equal(s.tab.xzs, xz) and np.array_equal(s.tab.phases, ph)
+
+
+def pool_used():
+    """Bytes in use of device 0's stream-ordered pool."""
+    cu = ctypes.CDLL("libcuda.so.1")
+    pool, used = ctypes.c_void_p(), ctypes.c_uint64()
+    assert cu.cuDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+    assert cu.cuMemPoolGetAttribute(pool, 7, ctypes.byref(used)) == 0  # CU_MEMPOOL_ATTR_USED_MEM_CURRENT
+    return used.value
+
+
+def memory_in_use():
+    """(bytes of the pool in use, bytes of the device in use outside the pool's reserve)"""
+    cu = ctypes.CDLL("libcuda.so.1")
+    torch.cuda.synchronize()
+    pool, res = ctypes.c_void_p(), ctypes.c_uint64()
+    assert cu.cuDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+    assert cu.cuMemPoolGetAttribute(pool, 5, ctypes.byref(res)) == 0  # CU_MEMPOOL_ATTR_RESERVED_MEM_CURRENT
+    free, total = torch.cuda.mem_get_info()
+    return pool_used(), total - free - res.value
+
+
+def failing_calls(qcb, call, most=200):
+    """`call` with its first, second, ... checked CUDA call failing, until it
+    makes them all; how many failed."""
+    for k in range(1, most):
+        qcb.check(qcb.lib().qcb_tune_set(b"fail_call", k))
+        try:
+            call()
+            failed = False
+        except qcb.QCBError:
+            failed = True
+        finally:
+            qcb.check(qcb.lib().qcb_tune_set(b"fail_call", 0))
+        if not failed:
+            return k - 1
+    raise AssertionError("the call never succeeds")
+
+
+def batch_jobs(qcb, specs):
+    jobs = []
+    for d, rounds, p, shots in specs:
+        arr = O.to_array(circuits.rotated_surface_code_memory(d, rounds, p))
+        qmax, bmax = O.affected_counts(arr)
+        jobs.append((qcb.PauliFrame(shots, qmax, bmax, init=False), qcb.Program(arr), 5))
+    return jobs
+
+
+@pytest.mark.parametrize("specs", [[(3, 3, 1e-3, 2000)], [(9, 9, 5e-3, 400_000), (3, 1, 1e-3, 100)]])
+def test_failing_batch_create_gives_its_memory_back(qcb, specs):
+    """qcb_batch_create with every one of its CUDA calls failing in turn; the
+    second batch's noise scratch lies outside the pool (above 64 MB)."""
+    jobs = batch_jobs(qcb, specs)
+    qcb.Batch(jobs).run().status()  # warm: modules, pools
+    before = memory_in_use()
+    assert failing_calls(qcb, lambda: qcb.Batch(jobs)) >= 5
+    after = memory_in_use()
+    assert after[0] == before[0] and abs(after[1] - before[1]) < 16 << 20
+
+
+def test_batch_without_noise_scratch(qcb, no_scratch):
+    """Without room for the noise scratch the jobs' noise is drawn in the walk."""
+    jobs = batch_jobs(qcb, [(5, 3, 4e-3, 20_000), (3, 2, 1e-2, 3000)])
+    records = []
+    for kb in (0, 1):
+        no_scratch(kb)
+        b = qcb.Batch(jobs)
+        no_scratch(0)
+        b.run().status()
+        records.append([f.record_planes() for f, *_ in jobs])
+    assert all(np.array_equal(a, b) for a, b in zip(*records))
