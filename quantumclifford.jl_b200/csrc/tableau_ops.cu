@@ -972,7 +972,7 @@ static int apply_dense_tables(qcb_tableau* t, const qcb_tableau* c, int phases, 
   // most DENSE_SCRATCH (more rows than fill the GPU many times over), and
   // less where that much memory is not there.
   uint32_t slab = std::min<uint64_t>(R, std::max<uint64_t>(f.rows, DENSE_SCRATCH / ((size_t)16 * len) / f.rows * f.rows));
-  uint8_t* m = nullptr;
+  Scratch scratch(st);
   size_t o_part = 0, o_odd = 0;
   while (true) {
     runs(slab);
@@ -981,12 +981,12 @@ static int apply_dense_tables(qcb_tableau* t, const qcb_tableau* c, int phases, 
     place((size_t)32 * len * 16);
     o_part = place((size_t)a.KG * slab * len * 16);
     o_odd = place((size_t)a.KG * slab);
-    const cudaError_t e = cudaMallocAsync(&m, bytes, st);
+    const cudaError_t e = scratch.alloc(bytes);
     if (e == cudaSuccess) break;
     if (e != cudaErrorMemoryAllocation || slab <= f.rows) return cuda_fail(e, "qcb_apply_dense scratch");
-    cudaGetLastError();
     slab = std::max(f.rows, slab / 2 / f.rows * f.rows);
   }
+  uint8_t* m = scratch.p;
   a.qt = m; a.part = (ulonglong2*)(m + o_part); a.odd = m + o_odd;
   QCB_CUDA(cudaFuncSetAttribute(f.k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DENSE_TABLE_SMEM));
   if (phases) QCB_CUDA(launch_dependent(dense_q_kernel, dim3((32 * len + 7) / 8), 256, 0, st, a));
@@ -998,7 +998,6 @@ static int apply_dense_tables(qcb_tableau* t, const qcb_tableau* c, int phases, 
     QCB_CUDA(launch_dependent(f.k, dim3(a.KG, (a.rows + f.rows - 1) / f.rows), f.threads, smem, st, a));
     QCB_CUDA(launch_dependent(dense_join_kernel, dim3((a.rows + 7) / 8), 256, 0, st, a));
   }
-  QCB_CUDA(cudaFreeAsync(m, st));
   return QCB_OK;
 }
 

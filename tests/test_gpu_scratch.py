@@ -108,3 +108,34 @@ def test_batch_without_noise_scratch(qcb, no_scratch):
         b.run().status()
         records.append([f.record_planes() for f, *_ in jobs])
     assert all(np.array_equal(a, b) for a, b in zip(*records))
+
+
+@pytest.mark.parametrize("what", ["dense", "canonicalize", "canonicalize_ranks"])
+def test_failing_calls_give_their_scratch_back(qcb, what):
+    """apply! of a dense operator and canonicalize! by panels with every one of
+    their CUDA calls failing in turn; the last one, which makes them all, is
+    right."""
+    n, rng = 130, np.random.default_rng(8)
+    t = rand_tab(90, n, rng)
+    op = qcb.random_clifford(n, rng)
+    op.to_gpu()
+    s = qcb.Stabilizer(t.copy()).to_gpu()
+
+    def call():
+        if what == "dense":
+            qcb.check(qcb.lib().qcb_apply_dense(s.tab.dev.handle, op.tab.dev.handle, 1, None))
+        else:
+            qcb.canonicalize_(s, ranks=what != "canonicalize")
+
+    call()  # warm
+    torch.cuda.synchronize()
+    before = pool_used()
+    assert failing_calls(qcb, lambda: (s.tab.dev.upload(t.phases, t.xzs), call())) >= 5
+    torch.cuda.synchronize()
+    assert pool_used() == before
+    s.to_cpu()
+    if what == "dense":
+        ph, xz = oracle.apply_dense(t.phases, t.xzs, n, op.tab.phases, op.tab.xzs, True)
+    else:
+        ph, xz, _, _ = oracle.canonicalize(t.phases, t.xzs, n, True)
+    assert np.array_equal(s.tab.xzs, xz) and np.array_equal(s.tab.phases, ph)
