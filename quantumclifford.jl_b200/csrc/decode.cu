@@ -65,7 +65,9 @@ __device__ __forceinline__ void transpose32(uint32_t v[32]) {
 }
 
 // Shot-major syndrome matrix: out[s * Wsyn + w] bit b = record[rows[64w + b], s]
-// (bits past nsel are zero; rows == null: record row row0 + k for bit k).
+// (bits past nsel are zero; without LIST: record row rows[0] + k for bit k).
+// The rows come by value, up to SYN_LIST to a launch: nothing is allocated or
+// copied, and the call need not wait.
 // A CTA takes SYN_COLS word columns (512 shots) and a block of `pairs` output
 // words (blockIdx.x; 64 record rows each).  Half-warp h of warp w loads the 32
 // rows of 32-bit group 2w + h, a lane per column (64 contiguous bytes a row),
@@ -84,10 +86,17 @@ __device__ __forceinline__ void transpose32(uint32_t v[32]) {
 constexpr uint32_t SYN_COLS = 16;
 constexpr uint32_t SYN_PAIRS = 16;  // output words of a CTA at most (512 threads)
 
+constexpr uint32_t SYN_LIST = 4096;  // 16 KB of parameters
+
+template <bool LIST>
+struct SynRows {
+  uint32_t row[LIST ? SYN_LIST : 1];
+};
+
 template <bool LIST>
 __global__ void __launch_bounds__(32 * SYN_PAIRS, 2)
 syndrome_rows_kernel(const uint32_t* __restrict__ rec, uint64_t pitch, uint64_t ncols, uint64_t S,
-                     const uint32_t* __restrict__ rows, uint32_t row0, uint32_t nsel, uint32_t Wsyn,
+                     const __grid_constant__ SynRows<LIST> rows, uint32_t nsel, uint32_t nwords, uint32_t Wsyn,
                      uint32_t pairs, uint64_t* __restrict__ out) {
   extern __shared__ __align__(16) uint32_t tile[];  // [SYN_COLS][32 * RS + 2]
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -95,7 +104,7 @@ syndrome_rows_kernel(const uint32_t* __restrict__ rec, uint64_t pitch, uint64_t 
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;  // `pairs` warps
   const uint32_t RS = 2 * pairs, CS = 32 * RS + 2;  // words of a shot, of a column
   const uint32_t w0 = blockIdx.x * pairs;           // the CTA's first output word
-  const uint32_t words = min(pairs, Wsyn - w0);
+  const uint32_t words = min(pairs, nwords - w0);
   const uint64_t c0 = (uint64_t)blockIdx.y * SYN_COLS;
   const uint32_t cl = lane & (SYN_COLS - 1), h = lane / SYN_COLS;
   const uint64_t c = c0 + cl;
@@ -106,11 +115,11 @@ syndrome_rows_kernel(const uint32_t* __restrict__ rec, uint64_t pitch, uint64_t 
     uint32_t v[32];
     if (LIST) {
 #pragma unroll
-      for (uint32_t i = 0; i < 32; i++) v[i] = i < lim ? __ldg(rows + k0 + i) : 0u;
+      for (uint32_t i = 0; i < 32; i++) v[i] = i < lim ? rows.row[k0 + i] : 0u;
 #pragma unroll
       for (uint32_t i = 0; i < 32; i++) v[i] = i < lim ? __ldcs(rec + (uint64_t)v[i] * pitch + c) : 0u;
     } else {
-      const uint32_t* src = rec + (uint64_t)(row0 + k0) * pitch + c;  // read below lim only
+      const uint32_t* src = rec + (uint64_t)(rows.row[0] + k0) * pitch + c;  // read below lim only
 #pragma unroll
       for (uint32_t i = 0; i < 32; i++, src += pitch) v[i] = i < lim ? __ldcs(src) : 0u;
     }
@@ -176,6 +185,46 @@ __global__ void evaluate_guesses_kernel(const uint32_t* rec, uint64_t pitch, uin
   if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(fails, (unsigned long long)cnt);
 }
 
+// The syndrome words of nsel selected bits: words out[s * Wsyn ..] of every shot s.
+template <bool LIST>
+static int launch_syndrome(const qcb_frame* f, const SynRows<LIST>& rows, uint32_t nsel, uint32_t Wsyn, uint64_t* out,
+                           cudaStream_t st) {
+  const uint32_t nwords = (nsel + 63) / 64;
+  // words per CTA: the blocks of a shot's words as even as they divide; 8 where
+  // the runs then start and end on 64 bytes of the output (150001 x 9681 73 us
+  // against 78 with 16, 2^20 x 2048 104 against 110; with Wsyn = 23 or 21
+  // shorter runs lose, 1e6 x 1320 89 against 81)
+  const uint32_t most = Wsyn % 8 ? SYN_PAIRS : 8;
+  const uint32_t blocks = (nwords + most - 1) / most, pairs = (nwords + blocks - 1) / blocks;
+  const size_t sm = (size_t)SYN_COLS * (64 * pairs + 2) * 4;
+  auto kern = syndrome_rows_kernel<LIST>;
+  QCB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(SYN_COLS * (64 * SYN_PAIRS + 2) * 4)));
+  // column blocks in slices of the grid's y limit (33.5e6 shots each)
+  const uint64_t nblk = (f->ncols + SYN_COLS - 1) / SYN_COLS;
+  for (uint64_t b0 = 0; b0 < nblk; b0 += 65535) {
+    const uint32_t nb = (uint32_t)std::min<uint64_t>(65535, nblk - b0);
+    const uint64_t cb = b0 * SYN_COLS;
+    // a programmatic dependent of the launch before it, so that a row of these
+    // (the jobs of a batch) and the walk before them leave no launch gaps: 24
+    // jobs with their walk 811 -> 778 us
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks, nb);
+    cfg.blockDim = dim3(32 * pairs);
+    cfg.dynamicSmemBytes = sm;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    QCB_CUDA(cudaLaunchKernelEx(&cfg, kern, (const uint32_t*)(f->record + cb), f->pitch, f->ncols - cb,
+                                f->frames - cb * 32, rows, nsel, nwords, Wsyn, pairs, out + cb * 32 * Wsyn));
+    QCB_LAUNCHED();
+  }
+  return QCB_OK;
+}
+
 }  // namespace qcb
 
 using namespace qcb;
@@ -235,56 +284,31 @@ int qcb_frame_syndrome_rows(const qcb_frame* f, const uint32_t* bits, size_t nse
   cudaStream_t st = S(stream);
   const uint32_t Wsyn = (uint32_t)((nsel + 63) / 64);
   const size_t out_bytes = (size_t)f->frames * Wsyn * 8;
+  Scratch host_out(st);
+  uint64_t* d_out = out;
+  if (!out_on_device) {
+    QCB_CUDA(host_out.alloc(out_bytes));
+    d_out = (uint64_t*)host_out.p;
+  }
   // a run of consecutive record bits (the whole record, the syndrome of a
-  // round) needs no index list on the device
+  // round) in one launch, other selections SYN_LIST bits to a launch
   bool run = true;
   for (size_t k = 1; k < nsel && run; k++) run = rows[k] == rows[0] + k;
-  uint32_t* d_rows = nullptr;
-  uint64_t* d_out = out;
-  if (!run) {
-    QCB_CUDA(cudaMallocAsync(&d_rows, nsel * 4, st));
-    QCB_CUDA(cudaMemcpyAsync(d_rows, rows.data(), nsel * 4, cudaMemcpyHostToDevice, st));
-  }
-  if (!out_on_device) QCB_CUDA(cudaMallocAsync(&d_out, out_bytes, st));
-  // words per CTA: the blocks of a shot's words as even as they divide; 8 where
-  // the runs then start and end on 64 bytes of the output (150001 x 9681 73 us
-  // against 78 with 16, 2^20 x 2048 104 against 110; with Wsyn = 23 or 21
-  // shorter runs lose, 1e6 x 1320 89 against 81)
-  const uint32_t most = Wsyn % 8 ? SYN_PAIRS : 8;
-  const uint32_t blocks = (Wsyn + most - 1) / most, pairs = (Wsyn + blocks - 1) / blocks;
-  const size_t sm = (size_t)SYN_COLS * (64 * pairs + 2) * 4;
-  auto kern = d_rows ? syndrome_rows_kernel<true> : syndrome_rows_kernel<false>;
-  QCB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(SYN_COLS * (64 * SYN_PAIRS + 2) * 4)));
-  // column blocks in slices of the grid's y limit (33.5e6 shots each)
-  const uint64_t nblk = (f->ncols + SYN_COLS - 1) / SYN_COLS;
-  for (uint64_t b0 = 0; b0 < nblk; b0 += 65535) {
-    const uint32_t nb = (uint32_t)std::min<uint64_t>(65535, nblk - b0);
-    const uint64_t cb = b0 * SYN_COLS;
-    // a programmatic dependent of the launch before it, so that a row of these
-    // (the jobs of a batch) and the walk before them leave no launch gaps: 24
-    // jobs with their walk 811 -> 778 us
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(blocks, nb);
-    cfg.blockDim = dim3(32 * pairs);
-    cfg.dynamicSmemBytes = sm;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    QCB_CUDA(cudaLaunchKernelEx(&cfg, kern, (const uint32_t*)(f->record + cb), f->pitch, f->ncols - cb,
-                                f->frames - cb * 32, (const uint32_t*)d_rows, rows[0], (uint32_t)nsel, Wsyn, pairs,
-                                d_out + cb * 32 * Wsyn));
-    QCB_LAUNCHED();
+  if (run) {
+    SynRows<false> r{{rows[0]}};
+    if (int s = launch_syndrome(f, r, (uint32_t)nsel, Wsyn, d_out, st)) return s;
+  } else {
+    for (size_t k = 0; k < nsel; k += SYN_LIST) {
+      SynRows<true> r;
+      const uint32_t n = (uint32_t)std::min<size_t>(SYN_LIST, nsel - k);
+      std::copy(rows.begin() + k, rows.begin() + k + n, r.row);
+      if (int s = launch_syndrome(f, r, n, Wsyn, d_out + k / 64, st)) return s;
+    }
   }
   if (!out_on_device) {
     QCB_CUDA(cudaMemcpyAsync(out, d_out, out_bytes, cudaMemcpyDeviceToHost, st));
-    cudaFreeAsync(d_out, st);
+    QCB_CUDA(cudaStreamSynchronize(st));
   }
-  if (d_rows) cudaFreeAsync(d_rows, st);
-  if (d_rows || !out_on_device) QCB_CUDA(cudaStreamSynchronize(st));  // rows lives on this stack frame
   return QCB_OK;
 }
 

@@ -94,3 +94,51 @@ def test_syndrome_rows_tile_edges(qcb, frames, nsel, start):
         out = torch.full(want.shape, -1, dtype=torch.int64, device="cuda")
         qcb.check(qcb.lib().qcb_frame_syndrome_rows(f.handle, b.ctypes.data, len(b), out.data_ptr(), 1, None))
         assert np.array_equal(out.cpu().numpy().view(np.uint64), want)
+
+
+@pytest.mark.parametrize("frames,nsel", [(33, 4095), (515, 4096), (40, 4097), (1000, 9000), (20_000, 100)])
+def test_syndrome_rows_of_any_selection_do_not_wait(qcb, frames, nsel):
+    """A device matrix of bits in any order is written in the stream's order
+    without waiting for the stream (as of consecutive bits), also from a graph;
+    selections longer than one launch's list."""
+    import ctypes
+
+    import torch
+
+    rng = np.random.default_rng(nsel)
+    nb = 2200
+    meas = rng.random((frames, nb)) < 0.5
+    f = qcb.PauliFrame(frames, 1, nb, init=False).set_measurements(meas)
+    bits = rng.integers(1, nb + 1, nsel)
+    want = pack_rows(meas[:, bits - 1])
+    b = bits.astype(np.uint32)
+    out = torch.full(want.shape, -1, dtype=torch.int64, device="cuda")
+
+    def call(stream):
+        qcb.check(qcb.lib().qcb_frame_syndrome_rows(f.handle, b.ctypes.data, len(b), out.data_ptr(), 1,
+                                                    ctypes.c_void_p(stream.cuda_stream)))
+
+    st = torch.cuda.Stream()
+    call(st)
+    st.synchronize()
+    assert np.array_equal(out.cpu().numpy().view(np.uint64), want)
+    out.fill_(-1)
+    torch.cuda.synchronize()
+    done = torch.cuda.Event()
+    with torch.cuda.stream(st):
+        torch.cuda._sleep(200_000_000)  # about 0.1 s
+        call(st)
+        done.record()
+    assert not done.query()  # the call came back while the stream was busy
+    st.synchronize()
+    assert np.array_equal(out.cpu().numpy().view(np.uint64), want)
+    out.fill_(-1)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call(torch.cuda.current_stream())
+    b[:] = 1  # the selection is borrowed for the call only
+    graph.replay()
+    torch.cuda.synchronize()
+    del graph
+    assert np.array_equal(out.cpu().numpy().view(np.uint64), want)
