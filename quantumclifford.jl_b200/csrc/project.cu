@@ -519,7 +519,10 @@ __global__ void __launch_bounds__(PROJ_THREADS) project_smem_kernel(const ProjSm
           a.result[j] = a.phases ? (int32_t)((s + extra) & 3u) : (int32_t)(pphase & 3u);
         }
       }
-      cl.sync();  // the partial products and P are read until here
+      // CTA 0's other warps fill P for the next Pauli only now; the other CTAs
+      // reuse their partial products after its first cluster barrier, which
+      // CTA 0 enters when it has read them
+      __syncthreads();
       continue;
     }
     // 3. MixedDestabilizer logical branch: the row swaps (rare), by CTA 0
