@@ -22,6 +22,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <memory>
 
 #include "panel.cuh"
 #include "qcb_internal.h"
@@ -66,9 +67,20 @@ struct ProjArgs {
   const uint32_t* qubits;  // projectX!/Y!/Z!: Pauli j is the single-qubit Pauli on qubits[j] (0-based), or null
   uint32_t basis;          // with qubits: bit 0 = X component, bit 1 = Z component
   const uint8_t* rand_ph;  // projectrand!: phase (0 or 2) given to the new stabilizer row of Pauli j, or null
+  // a trial by panels from j0 on, launched before: [0] ended, [1] the next
+  // Pauli; unless it ended within PROJ_PANEL_SHORT Paulis this launch does
+  // nothing (null: always)
+  const int32_t* trial;
 };
 
 constexpr uint32_t PROJ_THREADS = 1024;
+
+// Steps of a run's first panel that are not worth the launches which bring the
+// rows up to date (about 30 us, 3 to 5 us a Pauli by the other kernels).
+constexpr uint32_t PROJ_PANEL_SHORT = 8;
+__host__ __device__ inline bool short_trial(const int32_t* state, uint32_t j0) {
+  return state[0] && (uint32_t)state[1] - j0 < PROJ_PANEL_SHORT;
+}
 
 // row m <- row i * row m (mul_left!(tab, m, i)), warp-cooperative.
 __device__ __forceinline__ void warp_rowmul(uint64_t* xzs, uint8_t* ph, uint32_t W, uint32_t m,
@@ -91,6 +103,7 @@ __device__ __forceinline__ void warp_rowmul(uint64_t* xzs, uint8_t* ph, uint32_t
 }
 
 __global__ void __launch_bounds__(PROJ_THREADS) project_kernel(const ProjArgs a) {
+  if (a.trial && !short_trial(a.trial, a.j0)) return;
   cg::cluster_group cl = cg::this_cluster();
   const uint32_t me = cl.block_rank(), CS = cl.num_blocks();
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
@@ -336,6 +349,7 @@ __device__ __forceinline__ uint32_t group_lanes(uint32_t len) {
 
 __global__ void __launch_bounds__(PROJ_THREADS) project_smem_kernel(const ProjSmemArgs pa) {
   const ProjArgs& a = pa.a;
+  if (a.trial && !short_trial(a.trial, a.j0)) return;
   cg::cluster_group cl = cg::this_cluster();
   const uint32_t me = cl.block_rank(), CS = cl.num_blocks();
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
@@ -817,6 +831,11 @@ struct ProjPanelArgs {
   unsigned long long *CP, *CPn, *CPz;  // [PSTEPS] the Paulis' own words
   uint32_t *pq, *pqn, *pqz, *pqp;      // [PSTEPS] the Paulis' q; pqp: the previous panel's
   uint8_t* base;       // [rows] start words: BASE_ROW, BASE_NONE or the Pauli's index in the panel
+  // up to the first panel's steps: set by the load when the run's first Pauli
+  // anticommutes with a stabilizer row; while it is not, these launches do
+  // nothing and the run ends before its first Pauli (null: always live)
+  uint32_t* live;
+  uint32_t first;      // the run's first Pauli
   uint32_t steps, apply, nq, groups, per;
 };
 constexpr uint32_t BASE_ROW = 255, BASE_NONE = 254;
@@ -840,10 +859,11 @@ __device__ __forceinline__ void project_steps(const ProjPanelArgs& a) {
     const uint64_t c = a.CP[tid];
     sCP[tid] = make_uint2((uint32_t)c, (uint32_t)(c >> 32));
   }
-  if (a.state[0]) {
+  if (a.state[0] || (a.live && !*a.live)) {
     if (tid == 0) {
       g.T = 0;
       g.done = 1;
+      a.state[0] = 1;
     }
     return;
   }
@@ -1242,6 +1262,7 @@ __global__ void __launch_bounds__(1024) project_steps_apply_kernel(const ProjPan
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;");
+  if (a.live && !*a.live) return;
   const uint32_t T = a.apply ? g.T : 0u;
   if (blk < a.nq) {  // q of every row
     if (!T) return;
@@ -1331,7 +1352,15 @@ __global__ void __launch_bounds__(256) project_load_kernel(const ProjPanelArgs a
   }
   if (r >= a.p.rows) return;
   const uint32_t ph = a.ph[r];
-  tiles_load_row(a.p, a.xzs + (size_t)r * a.p.W, r, ph, lane);
+  const uint64_t* row = a.xzs + (size_t)r * a.p.W;
+  tiles_load_row(a.p, row, r, ph, lane);
+  if (a.live && r >= a.nn && r < a.nn + a.rank) {
+    const uint64_t* P = a.paulis + (size_t)a.j0 * a.p.W;
+    uint64_t c = 0;
+    for (uint32_t k = lane; k < a.p.len; k += 32) c ^= (row[k] & P[a.p.len + k]) ^ (row[a.p.len + k] & P[k]);
+    const uint32_t odd = __reduce_xor_sync(0xFFFFFFFFu, parity64(c));
+    if (lane == 0 && odd) *a.live = 1;
+  }
   if (lane == 0) {
     a.word[r] = 0;
     a.F[r] = a.Fz[r] = 0;
@@ -1343,7 +1372,7 @@ __global__ void __launch_bounds__(256) project_store_kernel(const ProjPanelArgs 
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;");
   const uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (r >= a.p.rows) return;
+  if (r >= a.p.rows || short_trial(a.state, a.first)) return;
   const uint32_t ph = tiles_store_row(a.p, a.xzs + (size_t)r * a.p.W, r, lane);
   if (lane == 0) a.ph[r] = r < a.plain ? a.p.q[r] : (uint8_t)ph;
 }
@@ -1368,41 +1397,32 @@ static cudaError_t launch_pp(void (*k)(const ProjPanelArgs), uint32_t grid, uint
 // Runs worth a panel (a panel costs about as much as 10 to 15 Paulis of the
 // other kernels; 32 Paulis on 100 / 1000 / 4000 qubits 205 / 241 / 486 -> 181 /
 // 177 / 136 us with the call), the most stabilizer rows its search holds in
-// registers, and the steps a run has to make before the next is tried at once.
-constexpr uint32_t PROJ_PANEL_MIN = 32, PROJ_PANEL_ROWS = PP_WINDOW + 9 * PP_REST, PROJ_PANEL_GOOD = 32;
+// registers, the steps a run has to make before the next is tried at once, the
+// Paulis before the next trial after a first short one, and the panels queued
+// before anything is waited for.
+constexpr uint32_t PROJ_PANEL_MIN = 32, PROJ_PANEL_ROWS = PP_WINDOW + 9 * PP_REST, PROJ_PANEL_GOOD = 32,
+                   PROJ_PANEL_BACKOFF = 64, PROJ_TRIAL_PANELS = 4;
 
-// Projections [*j, k) by panels until one that commutes with the stabilizer
-// (or all are done); *j gets the next.  The first panel's steps are waited
-// for: when they end at once nothing else is launched.
-static int project_panels(const qcb_tableau* t, int kind, uint32_t rank, const uint64_t* pxzs, const uint8_t* pph,
-                          const uint8_t* d_rand, uint32_t* j, uint32_t k, int skip, int32_t* d_anti, int32_t* d_res,
-                          cudaStream_t st) {
-  const bool destab = kind == QCB_DESTABILIZER || kind == QCB_MIXED_DESTABILIZER;
-  const uint32_t R = destab ? t->rows : rank, W = t->W, len = W / 2, ntile = (len + 1) / 2;
-  size_t bytes = 0;
-  auto place = [&](size_t n) { const size_t o = bytes; bytes += (n + 127) / 128 * 128; return o; };
-  const size_t o_t = place((size_t)ntile * R * 32), o_po = place((size_t)ntile * PSTEPS * 32),
-               o_w = place((size_t)4 * R * 8), o_u = place((size_t)R * 8), o_q = place(R), o_b = place(R),
-               o_par = place((size_t)ntile * R), o_rec = place(2 * sizeof(PanelRecord)), o_cp = place(5 * PSTEPS * 8),
-               o_pq = place(3 * PSTEPS * 4), o_st = place(8);
-  uint8_t* m = nullptr;
-  const cudaError_t e = cudaMallocAsync(&m, bytes, st);
-  if (e == cudaErrorMemoryAllocation) {  // no room for a copy of the rows: none done here
-    cudaGetLastError();
-    return QCB_OK;
-  }
-  QCB_CUDA(e);
+// Projections [first, k) by panels until one that commutes with the stabilizer
+// (or all are done): begin(), queue() of the panels, store().  A run that ends
+// within PROJ_PANEL_SHORT Paulis (short_trial of `state`) is a failed trial: its
+// store() leaves the tableau as it was, for the other kernels.  Panels queued
+// past a run's end do nothing.  `live` is zero before.
+struct PanelRun {
+  Scratch scratch;
+  cudaStream_t st;
   ProjPanelArgs a{};
-  a.p = PanelTiles{R, W, len, ntile, 1, (ulonglong2*)(m + o_t), (ulonglong2*)(m + o_po), nullptr, (uint64_t*)(m + o_u),
-                   m + o_q, m + o_par};
-  a.xzs = t->xzs; a.ph = t->phases; a.nn = destab ? t->rows / 2 : 0; a.rank = rank; a.plain = destab ? rank : 0;
-  a.skip = skip; a.paulis = pxzs; a.pph = pph; a.rand_ph = d_rand;
-  a.state = (int32_t*)(m + o_st); a.anticom = d_anti; a.result = d_res; a.base = m + o_b;
-  uint64_t* word = (uint64_t*)(m + o_w);
-  unsigned long long *F = (unsigned long long*)word + (size_t)2 * R, *CP = (unsigned long long*)(m + o_cp);
-  uint32_t* pq = (uint32_t*)(m + o_pq);
-  PanelRecord* rec = (PanelRecord*)(m + o_rec);
-  auto buffers = [&](uint32_t b) {  // of panel b
+  uint32_t R = 0, k = 0, grid = 0, row_blocks = 0, next = 0;  // next: the panel to queue
+  uint64_t* word = nullptr;
+  unsigned long long *F = nullptr, *CP = nullptr;
+  uint32_t* pq = nullptr;
+  PanelRecord* rec = nullptr;
+  void (*sa)(const ProjPanelArgs) = nullptr;
+  static constexpr size_t SMEM = std::max(sizeof(ApplyFlagSmem), sizeof(PhaseSmem));
+
+  explicit PanelRun(cudaStream_t s) : scratch(s), st(s) {}
+
+  void buffers(uint32_t b) {  // of panel b
     const uint32_t e = b & 1, o = e ^ 1, i0 = b % 3, i1 = (b + 1) % 3, i2 = (b + 2) % 3;
     a.rec = rec + e; a.prev = rec + o;
     a.word = word + (size_t)e * R; a.wordn = word + (size_t)o * R;
@@ -1410,57 +1430,88 @@ static int project_panels(const qcb_tableau* t, int kind, uint32_t rank, const u
     a.CP = CP + i0 * PSTEPS; a.CPn = CP + i1 * PSTEPS; a.CPz = CP + i2 * PSTEPS;
     a.pq = pq + i0 * PSTEPS; a.pqn = pq + i1 * PSTEPS; a.pqz = a.pqp = pq + i2 * PSTEPS;
     a.CPX = CP + (3 + e) * PSTEPS; a.CPXz = CP + (3 + o) * PSTEPS;
-  };
-  const uint32_t rest = rank > PP_WINDOW ? rank - PP_WINDOW : 0;
-  void (*sa)(const ProjPanelArgs) = rest <= PP_REST ? project_steps_apply_kernel<1>
-                                  : rest <= 2 * PP_REST ? project_steps_apply_kernel<2>
-                                  : rest <= 5 * PP_REST ? project_steps_apply_kernel<5> : project_steps_apply_kernel<9>;
-  const size_t smem = std::max(sizeof(ApplyFlagSmem), sizeof(PhaseSmem));
-  QCB_CUDA(cudaFuncSetAttribute(sa, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const uint32_t nsm = (uint32_t)std::max(device_sm_count(), 1);
-  a.nq = (R + 1023) / 1024;
-  a.groups = std::max<uint32_t>(1, std::min<uint32_t>((nsm > a.nq + 1 ? nsm - 1 - a.nq : 1) / ntile, (R + 255) / 256));
-  a.per = (R + a.groups - 1) / a.groups;
-  const uint32_t row_blocks = (R + 7) / 8, first = *j;
-  int32_t h[2] = {0, 0};
-  int s = QCB_OK;
-  auto go = [&]() -> int {
-    const uint32_t grid = 1 + a.nq + ntile * a.groups;
-    uint32_t nb = (k - first + PSTEPS - 1) / PSTEPS;  // panels
-    auto span = [&](uint32_t b) { return b < nb ? std::min(PSTEPS, k - first - b * PSTEPS) : 0u; };
+  }
+  uint32_t panels() const { return (k - a.first + PSTEPS - 1) / PSTEPS; }
+  uint32_t span(uint32_t b) const { return b < panels() ? std::min(PSTEPS, k - a.first - b * PSTEPS) : 0u; }
+
+  // Launch SA of panel b.
+  int steps(uint32_t b) {
+    buffers(b);
+    a.jp = a.j0;
+    a.j0 = a.first + b * PSTEPS; a.cnt = span(b);
+    a.jn = a.j0 + a.cnt; a.cntn = span(b + 1);
+    a.steps = b < panels(); a.apply = b > 0;
+    QCB_CUDA(launch_pp(sa, a.apply || a.cntn ? grid : 1u, 1024, SMEM, st, a));
+    return QCB_OK;
+  }
+
+  // *none: no room for a copy of the rows, nothing launched.
+  int begin(const qcb_tableau* t, int kind, uint32_t rank, const uint64_t* pxzs, const uint8_t* pph,
+            const uint8_t* d_rand, uint32_t j0, uint32_t end, int skip, int32_t* d_anti, int32_t* d_res, uint32_t* live,
+            bool* none) {
+    const bool destab = kind == QCB_DESTABILIZER || kind == QCB_MIXED_DESTABILIZER;
+    const uint32_t W = t->W, len = W / 2, ntile = (len + 1) / 2;
+    R = destab ? t->rows : rank;
+    a.first = j0;
+    k = end;
+    size_t bytes = 0;
+    auto place = [&](size_t n) { const size_t o = bytes; bytes += (n + 127) / 128 * 128; return o; };
+    const size_t o_t = place((size_t)ntile * R * 32), o_po = place((size_t)ntile * PSTEPS * 32),
+                 o_w = place((size_t)4 * R * 8), o_u = place((size_t)R * 8), o_q = place(R), o_b = place(R),
+                 o_par = place((size_t)ntile * R), o_rec = place(2 * sizeof(PanelRecord)), o_cp = place(5 * PSTEPS * 8),
+                 o_pq = place(3 * PSTEPS * 4), o_st = place(8);
+    const cudaError_t e = scratch.alloc(bytes);
+    *none = e == cudaErrorMemoryAllocation;
+    if (*none) return QCB_OK;
+    QCB_CUDA(e);
+    uint8_t* m = scratch.p;
+    a.p = PanelTiles{R, W, len, ntile, 1, (ulonglong2*)(m + o_t), (ulonglong2*)(m + o_po), nullptr, (uint64_t*)(m + o_u),
+                     m + o_q, m + o_par};
+    a.xzs = t->xzs; a.ph = t->phases; a.nn = destab ? t->rows / 2 : 0; a.rank = rank; a.plain = destab ? rank : 0;
+    a.skip = skip; a.paulis = pxzs; a.pph = pph; a.rand_ph = d_rand;
+    a.state = (int32_t*)(m + o_st); a.anticom = d_anti; a.result = d_res; a.base = m + o_b;
+    word = (uint64_t*)(m + o_w);
+    F = (unsigned long long*)word + (size_t)2 * R;
+    CP = (unsigned long long*)(m + o_cp);
+    pq = (uint32_t*)(m + o_pq);
+    rec = (PanelRecord*)(m + o_rec);
+    const uint32_t rest = rank > PP_WINDOW ? rank - PP_WINDOW : 0;
+    sa = rest <= PP_REST ? project_steps_apply_kernel<1>
+       : rest <= 2 * PP_REST ? project_steps_apply_kernel<2>
+       : rest <= 5 * PP_REST ? project_steps_apply_kernel<5> : project_steps_apply_kernel<9>;
+    QCB_CUDA(cudaFuncSetAttribute(sa, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM));
+    const uint32_t nsm = (uint32_t)std::max(device_sm_count(), 1);
+    a.nq = (R + 1023) / 1024;
+    a.groups = std::max<uint32_t>(1, std::min<uint32_t>((nsm > a.nq + 1 ? nsm - 1 - a.nq : 1) / ntile, (R + 255) / 256));
+    a.per = (R + a.groups - 1) / a.groups;
+    grid = 1 + a.nq + ntile * a.groups;
+    row_blocks = (R + 7) / 8;
     buffers(0);
-    a.j0 = first;
+    a.j0 = a.first;
+    a.live = skip ? nullptr : live;  // skipped Paulis do not end the run
     QCB_CUDA(launch_pp(project_load_kernel, row_blocks, 256, 0, st, a));
     // panel 0's words, as the next words of a panel before it without steps
-    a.jn = first; a.cntn = span(0);
+    a.jn = a.first; a.cntn = span(0);
     a.F = (unsigned long long*)a.word; a.CPn = a.CP; a.pqn = a.pq;
-    QCB_CUDA(launch_pp(sa, grid, 1024, smem, st, a));
-    for (uint32_t b = 0; b <= nb; b++) {
-      buffers(b);
-      a.jp = a.j0;
-      a.j0 = first + b * PSTEPS; a.cnt = span(b);
-      a.jn = a.j0 + a.cnt; a.cntn = span(b + 1);
-      a.steps = b < nb; a.apply = b > 0;
-      QCB_CUDA(launch_pp(sa, a.apply || a.cntn ? grid : 1u, 1024, smem, st, a));
-      if (b == nb) break;
-      if (b == 0) {
-        QCB_CUDA(cudaMemcpyAsync(h, a.state, 8, cudaMemcpyDeviceToHost, st));
-        QCB_CUDA(cudaStreamSynchronize(st));
-        if (h[0] && (uint32_t)h[1] == first) return QCB_OK;  // the tableau is as it was
-        if (h[0]) nb = 1;  // no second panel
-      }
-      QCB_CUDA(launch_pp(project_mid_kernel, ntile + 1 + (R + MID_THREADS - 1) / MID_THREADS, MID_THREADS, 0, st, a));
-    }
-    QCB_CUDA(launch_pp(project_store_kernel, row_blocks, 256, 0, st, a));
-    QCB_CUDA(cudaMemcpyAsync(h, a.state, 8, cudaMemcpyDeviceToHost, st));
-    QCB_CUDA(cudaStreamSynchronize(st));
+    QCB_CUDA(launch_pp(sa, grid, 1024, SMEM, st, a));
+    if (int s = steps(0)) return s;
+    a.live = nullptr;
     return QCB_OK;
-  };
-  s = go();
-  cudaFreeAsync(m, st);
-  if (s == QCB_OK) *j = (uint32_t)h[1];
-  return s;
-}
+  }
+
+  // Launches up to and with the apply of panel `upto` - 1.
+  int queue(uint32_t upto) {
+    for (; next < upto; next++) {
+      QCB_CUDA(launch_pp(project_mid_kernel, a.p.ntile + 1 + (R + MID_THREADS - 1) / MID_THREADS, MID_THREADS, 0, st, a));
+      if (int s = steps(next + 1)) return s;
+    }
+    return QCB_OK;
+  }
+  int store() {
+    QCB_CUDA(launch_pp(project_store_kernel, row_blocks, 256, 0, st, a));
+    return QCB_OK;
+  }
+};
 
 static uint32_t g_proj_cs = 0;  // tuner override (0 = automatic)
 static uint32_t g_proj_grid = 0;  // the whole-GPU kernel: 0 automatic, 1 always (where it applies), 2 never
@@ -1515,7 +1566,8 @@ static int project_impl(qcb_tableau* t, int kind, int32_t* rank_io, const uint64
   uint8_t* d_flags = nullptr;
   uint64_t* d_tmp = nullptr;
   uint8_t* d_tmpph = nullptr;
-  QCB_CUDA(cudaMallocAsync(&d_anti, (size_t)k * 4, st));
+  const uint32_t tries = k / PROJ_PANEL_MIN + 1;  // by panels: each takes at least PROJ_PANEL_MIN Paulis of the run
+  QCB_CUDA(cudaMallocAsync(&d_anti, ((size_t)k + tries) * 4, st));
   QCB_CUDA(cudaMallocAsync(&d_res, (size_t)k * 4, st));
   QCB_CUDA(cudaMallocAsync(&d_stat, 64, st));
   QCB_CUDA(cudaMallocAsync(&d_rank, 4, st));
@@ -1575,18 +1627,21 @@ static int project_impl(qcb_tableau* t, int kind, int32_t* rank_io, const uint64
   uint32_t j0 = 0;
   std::vector<int32_t> h_anti(k, 0), h_res(k, -1);
   // runs of generic Paulis go by panels (the tuner's choices of the other
-  // kernels turn them off); a run that ends early leaves the next Paulis to
-  // the kernels below, more of them each time
+  // kernels turn them off).  The first panel's steps are a trial: the other
+  // kernels are launched behind it and take the run where it ends at once (a
+  // Pauli that commutes with the state), for more Paulis each time before the
+  // next trial
   const bool destab = kind == QCB_DESTABILIZER || kind == QCB_MIXED_DESTABILIZER;
   const bool panels = !qubits && phases && len && !g_proj_grid && !g_proj_cs;
   const int skip = !keep_result && (kind == QCB_STABILIZER || (kind == QCB_DESTABILIZER && t->rows / 2 == t->nqubits));
-  uint32_t next_try = 0, backoff = 32;
+  uint32_t next_try = 0, backoff = PROJ_PANEL_BACKOFF, tried = 0;
   if (panels) {
-    QCB_CUDA(cudaMemsetAsync(d_anti, 0, (size_t)k * 4, st));
+    QCB_CUDA(cudaMemsetAsync(d_anti, 0, ((size_t)k + tries) * 4, st));
     QCB_CUDA(cudaMemsetAsync(d_res, 0xFF, (size_t)k * 4, st));
   }
   while (j0 < k) {
     uint32_t kend = k;
+    std::unique_ptr<PanelRun> trial;
     if (panels && k - j0 >= PROJ_PANEL_MIN && j0 >= next_try) {
       int32_t r_now = rank;
       if (mixed && j0) {
@@ -1595,17 +1650,54 @@ static int project_impl(qcb_tableau* t, int kind, int32_t* rank_io, const uint64
       }
       const uint32_t nr = kind == QCB_STABILIZER ? t->rows : kind == QCB_DESTABILIZER ? t->rows / 2 : (uint32_t)r_now;
       if (nr && nr <= PROJ_PANEL_ROWS) {
-        const uint32_t at = j0;
-        if ((status = project_panels(t, kind, nr, pxzs, pph, d_rand, &j0, k, skip, d_anti, d_res, st))) break;
-        if (j0 >= k) break;
-        if (j0 - at >= PROJ_PANEL_GOOD) {
-          backoff = 32;
-          next_try = j0 + 1;
-        } else {
-          backoff = std::min<uint32_t>(backoff * 2, 1u << 20);
-          next_try = j0 + backoff;
+        uint32_t* live = (uint32_t*)d_anti + k + std::min(tried++, tries - 1);
+        trial = std::make_unique<PanelRun>(st);
+        bool none = false;
+        if ((status = trial->begin(t, kind, nr, pxzs, pph, d_rand, j0, k, skip, d_anti, d_res, live, &none))) break;
+        if (none) trial.reset();
+        next_try = j0 + backoff;
+        kend = std::min(k, next_try);
+      }
+    } else if (panels && next_try > j0 && (destab || next_try > j0 + 1)) {
+      kend = std::min(k, next_try);
+    }
+    // The first panels are queued at once.  A run of no more is stored, and the
+    // other kernels launched behind it for the case that it fails, with one
+    // wait for all; a longer one goes on when its first panels are known.
+    int32_t at[2] = {0, 0};  // the trial's state
+    auto read_trial = [&]() -> int {
+      QCB_CUDA(cudaMemcpyAsync(at, trial->a.state, 8, cudaMemcpyDeviceToHost, st));
+      return QCB_OK;
+    };
+    auto advance = [&]() {  // behind a run that did not fail; where the next may start
+      const uint32_t from = j0;
+      j0 = (uint32_t)at[1];
+      if (j0 - from >= PROJ_PANEL_GOOD) {
+        backoff = PROJ_PANEL_BACKOFF;
+        next_try = j0 + 1;
+      } else {
+        next_try = j0 + backoff;
+        backoff = std::min<uint32_t>(backoff * 4, 1u << 20);
+      }
+    };
+    const bool whole = trial && !grid && trial->panels() <= PROJ_TRIAL_PANELS;
+    if (trial) {
+      const uint32_t np = trial->panels();
+      if ((status = trial->queue(std::min(np, PROJ_TRIAL_PANELS)))) break;
+      if (whole) {
+        if ((status = trial->store())) break;
+      } else {
+        if ((status = read_trial())) break;
+        QCB_CUDA(cudaStreamSynchronize(st));
+        if (!short_trial(at, j0)) {
+          // ended: the steps of the panel after the queued ones are still to be applied
+          if ((status = trial->queue(at[0] ? std::min(np, trial->next + 1) : np))) break;
+          if ((status = trial->store()) || (status = read_trial())) break;
+          QCB_CUDA(cudaStreamSynchronize(st));
+          advance();
+          continue;
         }
-        if (destab || next_try > j0 + 1) kend = std::min(k, next_try);
+        backoff = std::min<uint32_t>(backoff * 4, 1u << 20);
       }
     }
     ProjArgs a{};
@@ -1614,6 +1706,7 @@ static int project_impl(qcb_tableau* t, int kind, int32_t* rank_io, const uint64
     a.j0 = j0; a.k = kend; a.keep_result = keep_result; a.phases = phases;
     a.anticom = d_anti; a.result = d_res; a.status = d_stat; a.flags = d_flags;
     a.qubits = d_q; a.basis = basis; a.rand_ph = d_rand;
+    a.trial = whole ? trial->a.state : nullptr;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(cs);
     cfg.blockDim = dim3(PROJ_THREADS);
@@ -1646,7 +1739,15 @@ static int project_impl(qcb_tableau* t, int kind, int32_t* rank_io, const uint64
     int32_t hs[2];
     QCB_CUDA(cudaMemcpyAsync(hs, d_stat, 8, cudaMemcpyDeviceToHost, st));
     if (grid) QCB_CUDA(cudaMemcpyAsync(&htimeout, d_bar + 5, 4, cudaMemcpyDeviceToHost, st));
+    if (whole && (status = read_trial())) break;
     QCB_CUDA(cudaStreamSynchronize(st));
+    if (whole) {
+      if (!short_trial(at, j0)) {
+        advance();
+        continue;
+      }
+      backoff = std::min<uint32_t>(backoff * 4, 1u << 20);
+    }
     if (htimeout) {
       status = fail(QCB_ETIMEOUT, "project!: a grid barrier wait of the whole-GPU kernel expired");
       break;
