@@ -66,16 +66,16 @@ def test_dense_apply_of_two_sizes_at_once(qcb):
 
 
 def test_gate_lists_on_two_widths_at_once(qcb):
-    """Slices of 160 and 48 KB (20000 and 6000 qubits)."""
+    """Slices of 160 and 48 KB (20000 and 6000 qubits), two threads of each."""
     rng = np.random.default_rng(2)
-    jobs, tabs, times = [], [], 400
-    for n in (20000, 6000):
-        arr = O.to_array([O.sCNOT(2 * k + 1, 2 * k + 2) for k in range(40)])
+    jobs, tabs, times = [], [], 4000
+    for n in (20000, 6000, 20000, 6000):
+        arr = O.to_array([O.sCNOT(2 * k + 1, 2 * k + 2) for k in range(60)])
         t = random_rows(20, n, rng)
         g = t.copy().to_gpu()
         tabs.append((t, g))
         jobs.append(lambda st, g=g, arr=arr: check(qcb.lib().qcb_apply_gates(g.dev.handle, ptr(arr), len(arr), 1, st)))
-    assert run_threads(jobs, times) == [None, None]
+    assert run_threads(jobs, times) == [None] * 4
     for t, g in tabs:  # CNOTs twice are the identity
         g.to_cpu()
         assert np.array_equal(g.xzs, t.xzs) and np.array_equal(g.phases, t.phases)
