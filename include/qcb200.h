@@ -589,6 +589,12 @@ int qcb_debug_program_device(const qcb_op* ops, size_t n_ops, uint32_t* stream, 
                              size_t* stream_len, uint8_t* sites, size_t sites_cap, size_t* n_sites,
                              uint32_t* slot_qubit, uint32_t* slot_swap, size_t slots_cap, size_t* n_slots,
                              qcb_program_info* info);
+/* The tile widths qcb_batch_create chooses on a device of `sms` SMs (host only):
+ * per job the program's length in words, the time of a tile apart from and per
+ * column (any unit), the frame's columns and the widest tile; widths[j] != 0 on
+ * entry is a given width, which stays.                                      */
+int qcb_debug_batch_widths(const double* lengths, const double* fixed, const double* per_col, const uint64_t* ncols,
+                           const uint32_t* tmax, size_t n_jobs, uint32_t sms, uint32_t* widths);
 
 #ifdef __cplusplus
 }

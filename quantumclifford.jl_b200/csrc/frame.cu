@@ -2014,70 +2014,124 @@ struct qcb_batch {
 // the walk 1590 us; sampler 141 + walker 702 us.
 constexpr uint64_t BATCH_PRESAMPLE_MAX = 1ull << 30;
 
-// A batch job for the choice of its tile width: program length, columns, the
-// widest tile that fits, and the width (0: to be chosen).
+// A batch job for the choice of its tile width: program length, the time of a
+// tile apart from and per column (us), columns, the widest tile that fits, and
+// the width (0: to be chosen).
 struct BatchShape {
-  double length;
+  double length, fixed, per_col;
   uint64_t ncols;
   uint32_t tmax, T;
 };
 
-// Time of a tile as in smem_tile, in units of a record word and column.
+// Time of a tile on an SM, sampler included: a barrier and its latencies per
+// record, the entries' decoding, and per column the entries' accesses and the
+// events.  Widths whose warps do not cover whole rows of the tile take longer.
+// Fitted to surface codes of d = 3..21 at p = 1e-4, 1e-3 and 4e-3 in 19 widths
+// (6 % rms): d = 5, p = 1e-3: 16 columns 32 us, 64 35, 256 74; d = 11: 16 97, 32
+// 124, 64 174, 96 237; d = 15: 16 203, 32 253, 48 331, 56 400; d = 21: 16 373, 20
+// 491, 28 620.
+static BatchShape batch_shape(const qcb_program* p, uint64_t ncols, uint32_t tmax, uint32_t T) {
+  const double records = (double)p->info.n_segments + p->info.n_flushes, length = (double)p->stream_slot.size();
+  double events = 0;  // of a shot
+  for (const Site& s : p->sites_slot) events += s.peff;
+  return {length, 0.45 * records + 2.3e-4 * length, 2.7e-5 * length + 0.048 * events, ncols, tmax, T};
+}
+
+static double batch_tile_us(const BatchShape& b, uint32_t T) {
+  const double odd = (T & (T - 1)) == 0 ? 1.0 : T % 16 == 0 ? 1.05 : T % 8 == 0 || T > 48 ? 1.15 : 1.25;
+  return (b.fixed + b.per_col * T) * odd;
+}
+
+// The same as program length x columns, by which the tiles are queued.
 static double batch_tile_cost(const BatchShape& b, uint32_t T) {
   return b.length * (25.0 + ((T & (T - 1)) == 0 ? 0.75 : 1.0) * T);
 }
 
-// The widths of the jobs that have none: powers of two, the widest whose tile
-// takes no longer than a limit common to all jobs, with the limit (a tile of
-// the longest program at one of its widths) that gives the shortest longest
-// SM when the tiles go longest first to the next free one.  Batches of few
-// tiles gain from narrow ones, and long programs before short ones; many
-// tiles an SM need no search.  Surface codes (jobs, largest d and shots), us, the
-// widest tiles for all before: 12, 13, 30000 371 -> 181; 8, 11, 300000 186 -> 114;
-// 20, 7, 8210 106 -> 73; 24, 13, 300000 619 -> 609; 24, 7, 300000 237 -> 238; one
-// power of two for all is no better in any of them.
-static void batch_widths(std::vector<BatchShape>& jobs) {
+// When the last SM is done with tiles of these widths that go longest first to
+// the next free SM.
+template <class Cost>
+static double batch_end(const std::vector<BatchShape>& jobs, const std::vector<uint32_t>& T, uint64_t nsm, Cost cost) {
   constexpr uint64_t MANY = 64;  // tiles an SM: the last ones hardly count
-  const uint64_t nsm = (uint64_t)std::max(device_sm_count(), 1);
+  std::vector<std::pair<double, uint64_t>> tiles;  // (time, number) of each job
+  uint64_t n = 0;
+  for (size_t k = 0; k < jobs.size(); k++) {
+    tiles.push_back({cost(jobs[k], T[k]), (jobs[k].ncols + T[k] - 1) / T[k]});
+    n += tiles.back().second;
+  }
+  double end = 0;
+  if (n > MANY * nsm) {
+    for (auto& t : tiles) end += t.first * (double)t.second / (double)nsm;
+    return end;
+  }
+  std::sort(tiles.begin(), tiles.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
+  std::priority_queue<double, std::vector<double>, std::greater<double>> sm;  // when each SM is free
+  for (uint64_t k = 0; k < nsm; k++) sm.push(0.0);
+  for (auto& t : tiles)
+    for (uint64_t k = 0; k < t.second; k++) {
+      const double e = sm.top() + t.first;
+      sm.pop();
+      sm.push(e);
+      end = std::max(end, e);
+    }
+  return end;
+}
+
+// The widths of the jobs that have none.  First powers of two, for each job the
+// widest whose tile takes no longer than a limit common to all jobs, with the
+// limit (a tile of the longest program at one of its widths) that gives the
+// shortest longest SM: batches of few tiles gain from narrow ones, and long
+// programs before short ones.  Then, by the times above, multiples of 16 and the
+// widest tile, for each job the one of least work within the limit or the widest
+// within it; these where they are 3 % shorter, which the times can tell.
+// Surface codes, p = 1e-3 (jobs, d, shots), us, powers of two / now: 4, 15, 200000
+// 1495 / 1268; 16, 15, 200000 5491 / 4966; 8, 15, 30000 506 / 431; 24 uneven ones
+// up to d = 13 with their matrices 769 / 694.  The widest tiles for all before
+// both: 12, 13, 30000 371 -> 181; 20, 7, 8210 106 -> 73.
+static void batch_widths(std::vector<BatchShape>& jobs, uint64_t nsm) {
+  std::vector<uint32_t> T(jobs.size()), two, other;
   const BatchShape* longest = nullptr;
   for (auto& b : jobs)
     if (!b.T && (!longest || b.length > longest->length)) longest = &b;
   if (!longest) return;
-  auto width = [](const BatchShape& b, double limit) {
-    uint32_t T = 256;
-    while (T > 16 && (T > b.tmax || T / 2 >= b.ncols || batch_tile_cost(b, T) > limit)) T /= 2;
-    return T;
-  };
-  double best = 0, best_limit = 0;
+  double best = 0;
   for (uint32_t w = 256; w >= 16; w /= 2) {
     if (w > 16 && w > longest->tmax) continue;
     const double limit = batch_tile_cost(*longest, w);
-    std::vector<std::pair<double, uint64_t>> tiles;  // (time, number) of each job
-    uint64_t n = 0;
-    for (auto& b : jobs) {
-      const uint32_t T = b.T ? b.T : width(b, limit);
-      tiles.push_back({batch_tile_cost(b, T), (b.ncols + T - 1) / T});
-      n += tiles.back().second;
+    for (size_t k = 0; k < jobs.size(); k++) {
+      const BatchShape& b = jobs[k];
+      uint32_t t = 256;
+      while (t > 16 && (t > b.tmax || t / 2 >= b.ncols || batch_tile_cost(b, t) > limit)) t /= 2;
+      T[k] = b.T ? b.T : t;
     }
-    double end = 0;
-    if (n > MANY * nsm) {
-      for (auto& t : tiles) end += t.first * (double)t.second / (double)nsm;
-    } else {
-      std::sort(tiles.begin(), tiles.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
-      std::priority_queue<double, std::vector<double>, std::greater<double>> sm;  // when each SM is free
-      for (uint64_t k = 0; k < nsm; k++) sm.push(0.0);
-      for (auto& t : tiles)
-        for (uint64_t k = 0; k < t.second; k++) {
-          const double e = sm.top() + t.first;
-          sm.pop();
-          sm.push(e);
-          end = std::max(end, e);
-        }
-    }
-    if (best_limit == 0 || end < best) { best = end; best_limit = limit; }
+    const double end = batch_end(jobs, T, nsm, batch_tile_cost);
+    if (two.empty() || end < best) { best = end; two = T; }
   }
+  // multiples of 16 below a job's widest tile, and that: other widths below 48
+  // columns never gained, and lost up to a quarter at strong noise
+  auto width = [](const BatchShape& b, uint32_t i) { return std::min(16 * (i + 1), b.tmax); };
   for (auto& b : jobs)
-    if (!b.T) b.T = width(b, best_limit);
+    if (!b.T && batch_tile_us(b, 16) > batch_tile_us(*longest, 16)) longest = &b;
+  best = 0;
+  for (uint32_t i = 16; i-- > 0;) {
+    if (i && width(*longest, i - 1) == longest->tmax) continue;
+    const double limit = batch_tile_us(*longest, width(*longest, i));
+    for (bool widest : {false, true}) {
+      for (size_t k = 0; k < jobs.size(); k++) {
+        const BatchShape& b = jobs[k];
+        double least = 0;
+        T[k] = b.T;
+        for (uint32_t j = 0, t = 0; !b.T && t < b.tmax && t < b.ncols && j < 16; j++) {
+          t = width(b, j);
+          const double us = batch_tile_us(b, t), work = us * (double)((b.ncols + t - 1) / t);
+          if (j == 0 || (us <= limit && (widest || work < least))) { T[k] = t; least = work; }
+        }
+      }
+      const double end = batch_end(jobs, T, nsm, batch_tile_us);
+      if (other.empty() || end < best) { best = end; other = T; }
+    }
+  }
+  const bool gains = best < 0.97 * batch_end(jobs, two, nsm, batch_tile_us);
+  for (size_t k = 0; k < jobs.size(); k++) jobs[k].T = gains ? other[k] : two[k];
 }
 
 // The scratch and the sampler's work list of a batch; the jobs' walks are
@@ -2165,9 +2219,9 @@ int qcb_batch_create(const qcb_batch_job* jobs, size_t n_jobs, qcb_batch** out) 
       auto it = g_tuned_tile.find(J.program->nslots);
       if (it != g_tuned_tile.end()) T = std::min(it->second, tmax);
     }
-    shape[j] = {(double)J.program->stream_slot.size(), J.frame->ncols, tmax, T};
+    shape[j] = batch_shape(J.program, J.frame->ncols, tmax, T);
   }
-  batch_widths(shape);
+  batch_widths(shape, (uint64_t)std::max(device_sm_count(), 1));
   for (size_t j = 0; j < n_jobs; j++) {
     const qcb_batch_job& J = jobs[j];
     const uint64_t ncols = J.frame->ncols;
@@ -2205,6 +2259,19 @@ int qcb_batch_create(const qcb_batch_job* jobs, size_t n_jobs, qcb_batch** out) 
   QCB_CUDA(cudaFuncSetAttribute(batch_walker_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 device_max_smem_optin() - (int)fa.sharedSizeBytes));
   *out = b.release();
+  return QCB_OK;
+}
+
+int qcb_debug_batch_widths(const double* lengths, const double* fixed, const double* per_col, const uint64_t* ncols,
+                           const uint32_t* tmax, size_t n_jobs, uint32_t sms, uint32_t* widths) {
+  if (n_jobs && (!lengths || !fixed || !per_col || !ncols || !tmax || !widths)) return qcb::fail(QCB_EARG, "null argument");
+  std::vector<BatchShape> shape(n_jobs);
+  for (size_t j = 0; j < n_jobs; j++) {
+    if (widths[j] > tmax[j] || tmax[j] < 16) return qcb::fail(QCB_EARG, "bad tile width");
+    shape[j] = {lengths[j], fixed[j], per_col[j], ncols[j], tmax[j], widths[j]};
+  }
+  batch_widths(shape, std::max(sms, 1u));
+  for (size_t j = 0; j < n_jobs; j++) widths[j] = shape[j].T;
   return QCB_OK;
 }
 

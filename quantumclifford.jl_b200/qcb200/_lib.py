@@ -209,6 +209,7 @@ def lib():
                                    ctypes.c_int),
         "qcb_debug_program_device": ([vp, sz, vp, sz, P(sz), vp, sz, P(sz), vp, vp, sz, P(sz), P(qcb_program_info)],
                                      ctypes.c_int),
+        "qcb_debug_batch_widths": ([vp, vp, vp, vp, vp, sz, u32, vp], ctypes.c_int),
     }
     for name, (args, res) in sig.items():
         fn = getattr(L, name)
