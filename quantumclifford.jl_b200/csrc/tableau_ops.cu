@@ -520,7 +520,7 @@ constexpr uint32_t DENSE_RUNS = 16;
 // Shared memory of the tables at most: the limit of every launch of a form, so
 // that calls of other sizes on other threads never lower it in between.
 constexpr size_t DENSE_TABLE_SMEM = 200 * 1024;
-constexpr size_t DENSE_SCRATCH = 64ull << 20;
+constexpr size_t DENSE_SCRATCH = 256ull << 20;  // of partial products at most
 struct DenseArgs {
   uint64_t* xzs;
   uint8_t* ph;
@@ -952,30 +952,36 @@ static int apply_dense_tables(qcb_tableau* t, const qcb_tableau* c, int phases, 
   a.NT = 16;
   while (a.NT * len > f.threads || a.NT * table > DENSE_TABLE_SMEM) a.NT /= 2;
   const size_t smem = a.NT * table;
-  // Runs of whole qubit words: the least waves x (words of a run x the time of
-  // a word's tables, with 3 us for a CTA) and the partial products' traffic.  As
-  // many runs as fill one wave leaves large ones a
-  // half-empty last wave (rows x qubits, us: 20000 x 2000 1304 -> 779,
-  // 8000 x 4000 1269 -> 752, 4000 x 4000 441 -> 385, 8000 x 8000 6148 -> 5365).
+  // Runs of whole qubit words and rows at a time (a slab): the least waves x
+  // (words of a run x the time of a word's tables, with 3 us for a CTA) and the
+  // partial products' traffic, among those whose partial products (16 len bytes
+  // a row and run) take at most `cap`.  As many runs as fill one wave leaves
+  // large ones a half-empty last wave (rows x qubits, us: 20000 x 2000 1304 ->
+  // 779, 8000 x 4000 1269 -> 752, 4000 x 4000 441 -> 385, 8000 x 8000 6148 -> 5365).
   const uint32_t nsm = (uint32_t)std::max(device_sm_count(), 1);
-  auto runs = [&](uint32_t rows) {
-    const uint32_t RG = (rows + f.rows - 1) / f.rows;
-    const double word_us = 0.005 * f.rows * len, run_us = (double)rows * len * 32 / 5e6;
+  uint32_t slab = 0;
+  auto split = [&](size_t cap) {
+    auto time = [&](uint32_t rows, uint32_t kg, uint32_t wpg) {
+      const uint32_t RG = (rows + f.rows - 1) / f.rows;
+      const double word_us = 0.005 * f.rows * len, run_us = (double)rows * len * 32 / 5e6;
+      return (RG * kg + nsm - 1) / nsm * (wpg * word_us + 3.0) + kg * run_us;
+    };
     double best = 0;
+    slab = 0;
     for (uint32_t g = 1; g <= std::min(len, DENSE_RUNS); g++) {
       const uint32_t wpg = (len + g - 1) / g, kg = (len + wpg - 1) / wpg;
-      const double us = (RG * kg + nsm - 1) / nsm * (wpg * word_us + 3.0) + kg * run_us;
-      if (g == 1 || us < best) { best = us; a.KG = kg; a.wpg = wpg; }
+      size_t fit = std::min<size_t>(R, cap / ((size_t)kg * (16 * len + 1)) / f.rows * f.rows);
+      if (!fit && kg == 1) fit = std::min(R, f.rows);  // the least
+      if (!fit) continue;
+      const uint32_t full = R / (uint32_t)fit, rest = R % (uint32_t)fit;
+      const double us = full * time((uint32_t)fit, kg, wpg) + (rest ? time(rest, kg, wpg) : 0.0);
+      if (!slab || us < best) { best = us; slab = (uint32_t)fit; a.KG = kg; a.wpg = wpg; }
     }
   };
-  // Rows at a time: the partial products take 16 len bytes a row and run, at
-  // most DENSE_SCRATCH (more rows than fill the GPU many times over), and
-  // less where that much memory is not there.
-  uint32_t slab = std::min<uint64_t>(R, std::max<uint64_t>(f.rows, DENSE_SCRATCH / ((size_t)16 * len) / f.rows * f.rows));
   Scratch scratch(st);
   size_t o_part = 0, o_odd = 0;
-  while (true) {
-    runs(slab);
+  for (size_t cap = DENSE_SCRATCH;; cap /= 2) {  // less where that much memory is not there
+    split(cap);
     size_t bytes = 0;
     auto place = [&](size_t n) { const size_t o = bytes; bytes += (n + 127) / 128 * 128; return o; };
     place((size_t)32 * len * 16);
@@ -983,8 +989,7 @@ static int apply_dense_tables(qcb_tableau* t, const qcb_tableau* c, int phases, 
     o_odd = place((size_t)a.KG * slab);
     const cudaError_t e = scratch.alloc(bytes);
     if (e == cudaSuccess) break;
-    if (e != cudaErrorMemoryAllocation || slab <= f.rows) return cuda_fail(e, "qcb_apply_dense scratch");
-    slab = std::max(f.rows, slab / 2 / f.rows * f.rows);
+    if (e != cudaErrorMemoryAllocation || (a.KG == 1 && slab <= f.rows)) return cuda_fail(e, "qcb_apply_dense scratch");
   }
   uint8_t* m = scratch.p;
   a.qt = m; a.part = (ulonglong2*)(m + o_part); a.odd = m + o_odd;

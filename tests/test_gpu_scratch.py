@@ -139,3 +139,50 @@ def test_failing_calls_give_their_scratch_back(qcb, what):
     else:
         ph, xz, _, _ = oracle.canonicalize(t.phases, t.xzs, n, True)
     assert np.array_equal(s.tab.xzs, xz) and np.array_equal(s.tab.phases, ph)
+
+
+def pool_peak(call):
+    """Bytes of the pool in use at most during `call`, beyond those before."""
+    cu = ctypes.CDLL("libcuda.so.1")
+    pool, zero, high = ctypes.c_void_p(), ctypes.c_uint64(0), ctypes.c_uint64()
+    assert cu.cuDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+    torch.cuda.synchronize()
+    before = pool_used()
+    assert cu.cuMemPoolSetAttribute(pool, 8, ctypes.byref(zero)) == 0  # CU_MEMPOOL_ATTR_USED_MEM_HIGH
+    call()
+    torch.cuda.synchronize()
+    assert cu.cuMemPoolGetAttribute(pool, 8, ctypes.byref(high)) == 0
+    return high.value - before
+
+
+@pytest.mark.parametrize("rows,n", [(36_000, 7424), (49_000, 4928), (900_000, 1000), (5_000_000, 64)])
+def test_dense_apply_scratch_is_bounded(qcb, rows, n):
+    """The partial products of all runs of qubits take at most 256 MB."""
+    rng = np.random.default_rng(rows)
+    W = 2 * ((n + 63) // 64)
+    t = qcb.DeviceTableau(rows, n)
+    t.upload(np.zeros(rows, np.uint8), np.repeat(rng.integers(0, 2**63, (1000, W), dtype=np.uint64), rows // 1000, axis=0))
+    op = qcb.DeviceTableau(2 * n, n)
+    op.upload(np.zeros(2 * n, np.uint8), rng.integers(0, 2**63, (2 * n, W), dtype=np.uint64))
+    peak = pool_peak(lambda: qcb.check(qcb.lib().qcb_apply_dense(t.handle, op.handle, 1, None)))
+    assert 0 < peak <= (256 << 20) + (1 << 20)
+
+
+@pytest.mark.parametrize("n,rows,kb", [(1000, 1000, 200), (1000, 777, 100), (300, 500, 30), (2100, 700, 400), (4097, 200, 400),
+                                       (64, 5000, 40)])
+@pytest.mark.parametrize("phases", [True, False])
+def test_dense_apply_in_slabs(qcb, no_scratch, n, rows, kb, phases):
+    """Several slabs of rows, the last one ragged, with one and more runs of
+    qubits each, where only kb KB of scratch are there."""
+    rng = np.random.default_rng(n + rows)
+    state = rand_tab(rows, n, rng)
+    c = rand_tab(2 * n, n, rng)
+    s, op = state.copy().to_gpu(), c.copy().to_gpu()
+    before = qcb.lib().qcb_launch_count()
+    no_scratch(kb)
+    qcb.check(qcb.lib().qcb_apply_dense(s.dev.handle, op.dev.handle, int(phases), None))
+    no_scratch(0)
+    assert qcb.lib().qcb_launch_count() - before >= 4 + phases  # two slabs at least
+    s.to_cpu()
+    ph, xz = oracle.apply_dense(state.phases, state.xzs, n, c.phases, c.xzs, phases)
+    assert np.array_equal(s.xzs, xz) and np.array_equal(s.phases, ph)
