@@ -375,7 +375,7 @@ int qcb_pftrajectories_fresh(qcb_frame* f, const qcb_program* prog, uint64_t see
  * dependents of the launch before them on the stream, or plain.  Test knob
  * "scratch_limit" k > 0: device scratch of more than k KB counts as not there,
  * in the calls that go another way without it (canonicalize!, project!,
- * batches) or in smaller pieces (dense apply!).
+ * dense apply!, batches).
  * Test knob "fail_call" k > 0: the k-th CUDA runtime call that the library
  * checks from then on is not made and counts as failed (QCB_ECUDA).         */
 int qcb_tune_set(const char* key, int64_t value);

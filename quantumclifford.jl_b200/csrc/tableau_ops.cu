@@ -499,6 +499,54 @@ __global__ void __launch_bounds__(256) apply_dense_kernel(uint64_t* xzs, uint8_t
   }
 }
 
+// The same for any width where the tables' scratch is not there: lane l holds
+// words l, l + 32, ... of the product.
+template <int PER>
+__global__ void __launch_bounds__(256) apply_dense_rows_kernel(uint64_t* xzs, uint8_t* ph, uint32_t rows, uint32_t W,
+                                                               uint32_t n, const uint64_t* __restrict__ c,
+                                                               const uint8_t* __restrict__ cph, int phases) {
+  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31, len = W / 2;
+  if (warp >= rows) return;
+  uint64_t* row = xzs + (uint64_t)warp * W;
+  uint64_t bx[PER], bz[PER], c1[PER], c2[PER];
+#pragma unroll
+  for (int k = 0; k < PER; k++) bx[k] = bz[k] = c1[k] = c2[k] = 0;
+  uint32_t extra = 0;  // sum of Clifford-row phases and -1 corrections (mod 4)
+  auto image = [&](uint32_t r) {
+    const uint64_t* cr = c + (uint64_t)r * W;
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+      const uint32_t w = lane + 32 * k;
+      if (w < len) mul_step<uint64_t>(__ldg(cr + w), __ldg(cr + len + w), bx[k], bz[k], c1[k], c2[k]);
+    }
+    extra += cph[r];
+  };
+  for (uint32_t wq = 0; wq < len; wq++) {
+    const uint64_t xw = row[wq], zw = row[len + wq];  // broadcast loads
+    uint64_t both = xw | zw;
+    while (both) {
+      const uint32_t b = __ffsll((long long)both) - 1, q = wq * 64 + b;
+      both &= both - 1;
+      if (q >= n) break;
+      const bool x = (xw >> b) & 1, z = (zw >> b) & 1;
+      if (x && z) extra += 3;  // phase -= 1
+      if (x) image(q);
+      if (z) image(q + n);
+    }
+  }
+  uint32_t s = 0;
+#pragma unroll
+  for (int k = 0; k < PER; k++) s += cnt_phase(c1[k], c2[k]);
+  s = __reduce_add_sync(0xFFFFFFFFu, s & 3u);
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < PER; k++) {
+    const uint32_t w = lane + 32 * k;
+    if (w < len) { row[w] = bx[k]; row[len + w] = bz[k]; }
+  }
+  if (lane == 0) ph[warp] = phases ? (uint8_t)((s + extra + ph[warp]) & 3u) : (uint8_t)0;
+}
+
 // Dense apply! by tables.  A state row selects up to four of the Clifford rows
 // of two qubits (x_q, z_q, x_q+1, z_q+1, in this order): 16 ordered products,
 // kept in shared memory for a run of qubits, so a row takes one table entry per
@@ -937,7 +985,8 @@ static cudaError_t launch_dependent(void (*k)(P...), dim3 grid, uint32_t block, 
   return cudaLaunchKernelEx(&cfg, k, args...);
 }
 
-static int apply_dense_tables(qcb_tableau* t, const qcb_tableau* c, int phases, cudaStream_t st) {
+// *none: no room for the partial products of one row group, nothing done.
+static int apply_dense_tables(qcb_tableau* t, const qcb_tableau* c, int phases, cudaStream_t st, bool* none) {
   const uint32_t R = t->rows, len = t->W / 2;
   // threads; lanes per row (half a warp up to 16 words), words per lane and
   // rows per slot, whose products fill the registers
@@ -989,7 +1038,9 @@ static int apply_dense_tables(qcb_tableau* t, const qcb_tableau* c, int phases, 
     o_odd = place((size_t)a.KG * slab);
     const cudaError_t e = scratch.alloc(bytes);
     if (e == cudaSuccess) break;
-    if (e != cudaErrorMemoryAllocation || (a.KG == 1 && slab <= f.rows)) return cuda_fail(e, "qcb_apply_dense scratch");
+    if (e != cudaErrorMemoryAllocation) return cuda_fail(e, "qcb_apply_dense scratch");
+    *none = a.KG == 1 && slab <= f.rows;
+    if (*none) return QCB_OK;
   }
   uint8_t* m = scratch.p;
   a.qt = m; a.part = (ulonglong2*)(m + o_part); a.odd = m + o_odd;
@@ -1220,9 +1271,15 @@ int qcb_apply_dense(qcb_tableau* t, const qcb_tableau* c, int phases, void* stre
   cudaStream_t st = S(stream);
   const uint32_t W = t->W;
   if (W > 256) return fail(QCB_EUNSUPPORTED, "qcb_apply_dense: at most 8192 qubits");
-  if (t->nqubits >= DENSE_TABLES_MIN_N || (t->nqubits >= 16 && t->rows >= 16384)) return apply_dense_tables(t, c, phases, st);
+  const bool tables = t->nqubits >= DENSE_TABLES_MIN_N || (t->nqubits >= 16 && t->rows >= 16384);
+  if (tables) {
+    bool none = false;
+    const int s = apply_dense_tables(t, c, phases, st, &none);
+    if (!none) return s;
+  }
   const uint32_t threads = 256, blocks = (uint32_t)(((uint64_t)t->rows * 32 + threads - 1) / threads);
-  apply_dense_kernel<<<blocks, threads, 0, st>>>(t->xzs, t->phases, t->rows, W, t->nqubits, c->xzs, c->phases, phases);
+  auto kern = W <= 2 ? apply_dense_kernel : W <= 64 ? apply_dense_rows_kernel<1> : apply_dense_rows_kernel<4>;
+  kern<<<blocks, threads, 0, st>>>(t->xzs, t->phases, t->rows, W, t->nqubits, c->xzs, c->phases, phases);
   QCB_LAUNCHED();
   return QCB_OK;
 }

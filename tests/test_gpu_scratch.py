@@ -186,3 +186,20 @@ def test_dense_apply_in_slabs(qcb, no_scratch, n, rows, kb, phases):
     s.to_cpu()
     ph, xz = oracle.apply_dense(state.phases, state.xzs, n, c.phases, c.xzs, phases)
     assert np.array_equal(s.xzs, xz) and np.array_equal(s.phases, ph)
+
+
+@pytest.mark.parametrize("n,rows", [(48, 70), (64, 9), (65, 100), (1000, 130), (2048, 33), (2049, 40), (4100, 20), (30, 20_000)])
+@pytest.mark.parametrize("phases", [True, False])
+def test_dense_apply_without_scratch(qcb, no_scratch, n, rows, phases):
+    """Without room for the partial products of one group of rows, a warp a row
+    multiplies its images."""
+    rng = np.random.default_rng(n + rows)
+    state = rand_tab(rows, n, rng)
+    c = rand_tab(2 * n, n, rng)
+    s, op = state.copy().to_gpu(), c.copy().to_gpu()
+    no_scratch(1)
+    qcb.check(qcb.lib().qcb_apply_dense(s.dev.handle, op.dev.handle, int(phases), None))
+    no_scratch(0)
+    s.to_cpu()
+    ph, xz = oracle.apply_dense(state.phases, state.xzs, n, c.phases, c.xzs, phases)
+    assert np.array_equal(s.xzs, xz) and np.array_equal(s.phases, ph)
