@@ -953,8 +953,11 @@ static int apply_layers(const qcb_tableau* t, const std::vector<GateOp>& g, int 
       const uint32_t l = lev[at[i]];
       list[start[l]++ + l + 1] = (uint64_t)o.op | ((uint64_t)o.q1 << 16) | ((uint64_t)o.q2 << 40);
     }
-    // threads for the widest level, and a warp per two transposes
-    const uint32_t threads = std::min<uint32_t>(512, std::max<uint32_t>(64, std::max((most + 31) / 32 * 32, 32 * t->W)));
+    // threads for the widest level and a warp per two transposes, at least 256:
+    // the slice's loads and stores take a warp a row (64 threads up to 64 qubits,
+    // us a call in a stream: 8 gates, 100 x 10 8.4 -> 4.4, 1000 x 64 8.8 -> 4.4; 128
+    // up to 128 qubits, 1000 x 100 6.7 -> 4.4)
+    const uint32_t threads = std::min<uint32_t>(512, std::max<uint32_t>(256, std::max((most + 31) / 32 * 32, 32 * t->W)));
     if (int s = list.size() <= LAYER_CAP_S ? launch_layers<LAYER_CAP_S>(t, list, threads, phases, st)
                                            : launch_layers<LAYER_CAP_L>(t, list, threads, phases, st))
       return s;
