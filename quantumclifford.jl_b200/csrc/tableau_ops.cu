@@ -886,12 +886,17 @@ static cudaError_t launch_gates(void (*k)(P...), uint32_t grid, uint32_t block, 
   return cudaLaunchKernelEx(&cfg, k, args...);
 }
 
-// Shortest gate list that runs bit-sliced.  The row-per-thread kernel takes
-// 1.6 us + 0.55..1.1 us a gate whatever the rows; the slices cost a read, two
-// transposes and a write of the tableau whatever the gates (2n rows, n = 100 /
-// 1000 / 4000: 5.5 / 4.4 / 17.5 us), so the lines cross at 8 gates for small
-// tableaux and one more per MB of a large one (8 MB: 16 gates, 17.5 us both).
-static size_t layer_min_gates(const qcb_tableau* t) { return 8 + (((size_t)t->rows * t->W * 8) >> 20); }
+// Shortest gate list that runs bit-sliced.  The row-per-thread kernel takes 4 us
+// a call in a stream up to 10 gates, then 0.3 to 1 us a gate; the slices cost a
+// read, two transposes and a write of the tableau whatever the gates: 4.5 us up
+// to 2000 qubits, where 8 gates are as fast either way, then a CTA's 32 rows of
+// all qubits take 1.9 us per 1000 qubits (20 rows or 1000; us, slices / rows of 12
+// gates: 5000 qubits 11 / 9.5, 10000 22 / 9.8, 20000 39 / 10.7; the lines cross at
+// 15, 29 and 50 gates), and many slices the tableau's traffic (a gate per MB).
+static size_t layer_min_gates(const qcb_tableau* t) {
+  const size_t mb = ((size_t)t->rows * t->W * 8) >> 20;
+  return std::max(8 + mb, t->W / 12 + (t->rows > 4096 ? mb : 0));
+}
 
 static size_t layer_smem(const qcb_tableau* t) { return (size_t)LAYER_SLICE * (2 * t->W + 1) * 4; }
 

@@ -128,3 +128,18 @@ def test_gate_list_replayed_from_a_graph(qcb):
     del graph
     g.to_cpu()
     assert np.array_equal(g.xzs, xz) and np.array_equal(g.phases, ph)
+
+
+@pytest.mark.parametrize("n,rows", [(5000, 70), (20_000, 33), (30_000, 5)])
+@pytest.mark.parametrize("count", [12, 13, 14, 51, 52, 53])
+def test_gate_lists_on_wide_tableaux(qcb, n, rows, count):
+    """Around the shortest list that runs bit-sliced on wide tableaux (13 gates
+    on 5000 qubits, 52 on 20000; above about 28000 none does)."""
+    rng = np.random.default_rng(n + count)
+    t = rand_tab(rows, n, rng)
+    arr = O.to_array(random_gates(n, count, rng))
+    g = t.copy().to_gpu()
+    qcb.apply_(g, arr)
+    g.to_cpu()
+    ph, xz = oracle.apply_gates(t.phases, t.xzs, n, arr, True)
+    assert np.array_equal(g.xzs, xz) and np.array_equal(g.phases, ph)
