@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(512) apply_layers_kernel(uint64_t* xzs, uint8_
 }
 
 // ---------------------------------------------------------- dense apply!
-// Tableaux of fewer than DENSE_TABLES_MIN_N qubits (one word per half), a warp
+// Tableaux of few qubits (one word per half, see dense_tables_pay), a warp
 // per state row: the ordered product over qubits of the Clifford's images
 // (src/dense_cliffords.jl:152-169) in registers; the phase counters run across
 // all the multiplications (each adds +-1 per anticommuting lane, independent
@@ -971,11 +971,17 @@ static int apply_layers(const qcb_tableau* t, const std::vector<GateOp>& g, int 
   return QCB_OK;
 }
 
-// Qubits from which dense apply! goes by tables: its three launches take 14 us
-// for any small tableau, a warp per row 5 us + 0.2 us a qubit (us, tables /
-// warp: n = 32 14 / 11, 64 15 / 19, 100 16 / 28, 300 18 / 77); many rows cross
-// earlier (30 qubits x 100000 rows 101 / 278).
-constexpr uint32_t DENSE_TABLES_MIN_N = 48;
+// Whether dense apply! goes by tables: its three launches take 11 to 16 us in a
+// stream of calls and 25 to 29 us alone for any small tableau, a warp per row 8 us
+// (16 alone) and 0.17 us a qubit.  us in a stream / alone, tables against warps:
+// 48 qubits x 1 row 11.6 / 25.6 and 16.7 / 24.8, x 200 rows 16.1 / 29.1 and 14.5 /
+// 23.1, x 4000 19.4 / 32.1 and 28.7 / 36.2; 56 x 200 16.1 / 28.9 and 16.6 / 25.0;
+// 64 x 200 16.1 / 29.1 and 18.6 / 26.8.  Many rows cross earlier (20000 rows: 16
+// qubits 42 / 55 and 36 / 44, 32 42 / 56 and 66 / 74).
+static bool dense_tables_pay(uint32_t rows, uint32_t n) {
+  if (rows >= 16384) return n >= 24;
+  return n >= (rows < 128 || rows >= 2048 ? 48u : 56u);
+}
 
 template <class... P, class... A>
 static cudaError_t launch_dependent(void (*k)(P...), dim3 grid, uint32_t block, size_t smem, cudaStream_t st, A... args) {
@@ -1279,8 +1285,7 @@ int qcb_apply_dense(qcb_tableau* t, const qcb_tableau* c, int phases, void* stre
   cudaStream_t st = S(stream);
   const uint32_t W = t->W;
   if (W > 256) return fail(QCB_EUNSUPPORTED, "qcb_apply_dense: at most 8192 qubits");
-  const bool tables = t->nqubits >= DENSE_TABLES_MIN_N || (t->nqubits >= 16 && t->rows >= 16384);
-  if (tables) {
+  if (dense_tables_pay(t->rows, t->nqubits)) {
     bool none = false;
     const int s = apply_dense_tables(t, c, phases, st, &none);
     if (!none) return s;

@@ -453,3 +453,17 @@ def test_dense_apply_more_rows_than_one_scratch(qcb):
     one.to_cpu(), tall.to_cpu()
     assert np.array_equal(tall.xzs.reshape(copies, small, -1), np.broadcast_to(one.xzs, (copies,) + one.xzs.shape))
     assert np.array_equal(tall.phases.reshape(copies, small), np.broadcast_to(one.phases, (copies, small)))
+
+
+@pytest.mark.parametrize("n", [23, 24, 47, 48, 55, 56])
+@pytest.mark.parametrize("rows", [1, 127, 128, 2047, 2048, 16383, 16384])
+def test_dense_apply_around_the_tables_lines(qcb, n, rows):
+    """Both sides of the rows and qubits from which dense apply! goes by tables."""
+    rng = np.random.default_rng(n + rows)
+    state = rand_tab(rows, n, rng)
+    c = qcb.random_clifford(n, rng).to_gpu()
+    s = state.copy().to_gpu()
+    qcb.check(qcb.lib().qcb_apply_dense(s.dev.handle, c.tab.dev.handle, 1, None))
+    s.to_cpu()
+    ph, xz = oracle.apply_dense(state.phases, state.xzs, n, c.tab.phases, c.tab.xzs, True)
+    assert np.array_equal(s.xzs, xz) and np.array_equal(s.phases, ph)
