@@ -358,8 +358,10 @@ int qcb_pftrajectories_fresh(qcb_frame* f, const qcb_program* prog, uint64_t see
  * canonicalize! by panels over the whole GPU: "canon_grid" 0 (automatic:
  * stabilizer views of 64..8192 rows) / 1 always / 2 never; "canon_pdl" 1
  * (default) / 0: the panel launches as programmatic dependent launches or
- * plain.  "canon_rpt" (0, 1, 2, 4, 8, 16), "canon_apply_rows" (0 or 8..32) and
- * "canon_lookahead" (1 default, 0) are accepted without effect.  project! on the whole GPU: "project_grid" 0 (automatic: runs
+ * plain; "canon_lookahead" 1 (default) / 0: a panel's pivot steps run beside
+ * the previous panel's apply, or in a launch of their own after it.
+ * "canon_rpt" (0, 1, 2, 4, 8, 16) and "canon_apply_rows" (0 or 8..32) are
+ * accepted without effect.  project! on the whole GPU: "project_grid" 0 (automatic: runs
  * of 32 or more generic Paulis by panels of 64, shorter ones on Stabilizer
  * kinds too tall for one cluster's shared memory one at a time on all SMs) /
  * 1 one at a time on all SMs where that applies / 2 one cluster.  Test knob "project_withhold" 1: one CTA

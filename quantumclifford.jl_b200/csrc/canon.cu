@@ -1523,6 +1523,7 @@ static int launch_blocked(const ElimSpec& e, cudaStream_t st) {
 
 static uint32_t g_canon_grid = 0;  // 0: automatic, 1: always, 2: never (panels over the whole GPU)
 static uint32_t g_canon_pdl = 1;   // panel launches as programmatic dependents (0: plain)
+static uint32_t g_canon_lookahead = 1;  // a panel's steps beside the previous panel's apply (0: after it)
 // Stabilizer views that run by panels over the whole GPU.
 constexpr uint32_t CANON_GRID_MIN_ROWS = 16, CANON_GRID_MAX_ROWS = 8192;
 
@@ -1626,7 +1627,16 @@ static int launch_grid(const ElimSpec& e, cudaStream_t st, bool* none) {
     if (k < P) { a.stage = panels[k].first; a.c0 = panels[k].second; }
     a.rec = rec + (k & 1);
     a.prev = rec + ((k + 1) & 1);
-    QCB_CUDA(launch_panel(l1, 1 + (a.apply ? a.nq + ntile * a.groups : 0), CANON_THREADS, smem, st, a));
+    const uint32_t apply_ctas = a.apply ? a.nq + ntile * a.groups : 0;
+    if (a.steps && a.apply && !g_canon_lookahead) {  // in turn
+      a.steps = 0;
+      QCB_CUDA(launch_panel(l1, 1 + apply_ctas, CANON_THREADS, smem, st, a));
+      a.steps = 1;
+      a.apply = 0;
+      QCB_CUDA(launch_panel(l1, 1, CANON_THREADS, smem, st, a));
+    } else {
+      QCB_CUDA(launch_panel(l1, 1 + apply_ctas, CANON_THREADS, smem, st, a));
+    }
     if (k == P) break;
     a.wn = k + 1 < P ? panel_word(panels[k + 1].first, panels[k + 1].second, len) : WORD_NONE;
     QCB_CUDA(launch_panel(canon_mid_kernel, ntile + 1 + (R + MID_THREADS - 1) / MID_THREADS, MID_THREADS, 0, st, a));
@@ -1765,6 +1775,7 @@ void set_canon_threads(uint32_t n) { g_canon_threads = n; }
 void set_canon_blocked(uint32_t v) { g_canon_blocked = v; }
 void set_canon_grid(uint32_t v) { g_canon_grid = v; }
 void set_canon_pdl(uint32_t v) { g_canon_pdl = v; }
+void set_canon_lookahead(uint32_t v) { g_canon_lookahead = v; }
 
 }  // namespace qcb
 

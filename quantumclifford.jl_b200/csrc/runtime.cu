@@ -121,6 +121,7 @@ void set_canon_blocked(uint32_t v);
 void set_canon_grid(uint32_t v);
 void set_server_fill(uint32_t v);
 void set_canon_pdl(uint32_t v);
+void set_canon_lookahead(uint32_t v);
 void set_gates_pdl(uint32_t v);
 void set_walker_pdl(uint32_t v);
 void set_walker_narrow(uint32_t v);
@@ -239,6 +240,7 @@ int qcb_tune_set(const char* key, int64_t value) {
     // test knob: the value-th checked CUDA call from now on fails without being made (0: none)
     g_fail_call.store((uint32_t)value);
   } else if (k == "canon_rpt") {
+    // accepted without effect, as canon_apply_rows
     if (value && value != 1 && value != 2 && value != 4 && value != 8 && value != 16)
       return fail(QCB_EARG, "canon_rpt must be 0, 1, 2, 4, 8 or 16");
   } else if (k == "walker_narrow") {
@@ -255,8 +257,10 @@ int qcb_tune_set(const char* key, int64_t value) {
     if (value > 1) return fail(QCB_EARG, "canon_pdl must be 0 or 1");
     set_canon_pdl((uint32_t)value);
   } else if (k == "canon_lookahead") {
-    // accepted without effect, as canon_rpt and canon_apply_rows
+    // canonicalize! by panels over the whole GPU: a panel's pivot steps beside
+    // the previous panel's apply (1, default) or in a launch after it (0)
     if (value > 1) return fail(QCB_EARG, "canon_lookahead must be 0 or 1");
+    set_canon_lookahead((uint32_t)value);
   } else if (k == "gates_pdl") {
     // symbolic apply! launches (qcb_apply_gates) as programmatic dependents (1, default) or plain (0)
     if (value > 1) return fail(QCB_EARG, "gates_pdl must be 0 or 1");

@@ -467,3 +467,28 @@ def test_dense_apply_around_the_tables_lines(qcb, n, rows):
     s.to_cpu()
     ph, xz = oracle.apply_dense(state.phases, state.xzs, n, c.tab.phases, c.tab.xzs, True)
     assert np.array_equal(s.xzs, xz) and np.array_equal(s.phases, ph)
+
+
+def test_canonicalize_in_turn_takes_a_launch_more_a_panel(qcb):
+    """canon_lookahead 0 runs each panel's steps in a launch after the previous
+    panel's apply: one launch more for every panel but the first, with the same
+    result as beside it; without ranks, so that no panel is left out."""
+    n, rng = 300, np.random.default_rng(9)
+    t = rand_tab(n, n, rng)
+    lib, out = qcb.lib(), []
+    for look in (1, 0):
+        qcb.check(lib.qcb_tune_set(b"canon_lookahead", look))
+        try:
+            s = qcb.Stabilizer(t.copy()).to_gpu()
+            before = lib.qcb_launch_count()
+            qcb.canonicalize_(s)
+            launches = lib.qcb_launch_count() - before
+        finally:
+            qcb.check(lib.qcb_tune_set(b"canon_lookahead", 1))
+        s.to_cpu()
+        out.append((launches, s.tab.phases.copy(), s.tab.xzs.copy()))
+    panels = 2 * ((n + 63) // 64)
+    assert out[1][0] - out[0][0] == panels - 1
+    ph, xz, _, _ = oracle.canonicalize(t.phases, t.xzs, n, True)
+    for _, p, x in out:
+        assert np.array_equal(p, ph) and np.array_equal(x, xz)
