@@ -25,6 +25,7 @@ int fail(int status, const std::string& msg) {
 int cuda_fail(cudaError_t e, const char* what) {
   std::string m = std::string("CUDA error in ") + what + ": " + cudaGetErrorString(e);
   int st = (e == cudaErrorMemoryAllocation) ? QCB_EOOM : QCB_ECUDA;
+  cudaGetLastError();  // reported here: not the next launch's error
   return fail(st, m);
 }
 

@@ -203,3 +203,17 @@ def test_dense_apply_without_scratch(qcb, no_scratch, n, rows, phases):
     s.to_cpu()
     ph, xz = oracle.apply_dense(state.phases, state.xzs, n, c.phases, c.xzs, phases)
     assert np.array_equal(s.xzs, xz) and np.array_equal(s.phases, ph)
+
+
+def test_a_refused_allocation_is_reported_once(qcb):
+    """A frame and a tableau larger than the device are refused with QCB_EOOM;
+    the call after it is not affected (its launch reported the same error)."""
+    t = rand_tab(10, 100, np.random.default_rng(3))
+    arr = O.to_array([O.sHadamard(1)])
+    g = t.copy().to_gpu()
+    for make in (lambda: qcb.PauliFrame(2**40, 100, 100, init=False), lambda: qcb.DeviceTableau(2**31 - 1, 10_000)):
+        with pytest.raises(qcb.QCBError, match="memory"):
+            make()
+        qcb.apply_(g, arr)
+    g.to_cpu()
+    assert np.array_equal(g.xzs, t.xzs) and np.array_equal(g.phases, t.phases)  # H twice
