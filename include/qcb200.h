@@ -356,7 +356,8 @@ int qcb_pftrajectories_fresh(qcb_frame* f, const qcb_program* prog, uint64_t see
  * hit keeps results right).  Knob "server_fill" (read by qcb_server_create):
  * 1 (default) admits onto idle SMs only, 0 whenever a slot is free.
  * canonicalize! by panels over the whole GPU: "canon_grid" 0 (automatic:
- * stabilizer views of 64..8192 rows) / 1 always / 2 never; "canon_pdl" 1
+ * stabilizer views of 640..8192 rows, and of 16..639 rows not much wider than
+ * tall: at most 7 qubit words per 64 rows) / 1 always / 2 never; "canon_pdl" 1
  * (default) / 0: the panel launches as programmatic dependent launches or
  * plain; "canon_lookahead" 1 (default) / 0: a panel's pivot steps run beside
  * the previous panel's apply, or in a launch of their own after it.

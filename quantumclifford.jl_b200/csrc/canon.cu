@@ -4,9 +4,10 @@
 // elimination: for every column j (X bits, then Z bits) find the first row at
 // or below the current pivot position i with the bit set, swap it to i, and
 // left-multiply every other row that has the bit by the pivot row.  Stabilizer
-// views of 64 rows and more go by panels of 64 columns (below: on one CTA or
-// cluster, or over the whole GPU); all other eliminations by column steps on
-// one thread-block cluster that stays resident throughout:
+// views go by panels of 64 columns, over the whole GPU (canon_grid_pays: 16 to
+// 8192 rows that are not much wider than tall, all from 640 on) or, from 64 rows,
+// on one CTA or cluster; all other eliminations by column steps on one
+// thread-block cluster that stays resident throughout:
 //   - the rows are split over the cluster's CTAs and held in shared memory
 //     (row stride W+1 words, so a thread-per-row column probe and a
 //     warp-per-row update are both bank-conflict free); tableaux too tall for
