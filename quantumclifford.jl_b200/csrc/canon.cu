@@ -1724,7 +1724,7 @@ static int permute_dev(uint64_t* xzs, uint32_t rows, uint32_t n, uint32_t W, con
   if (!rows || !n) return QCB_OK;
   const uint32_t threads = 256, wpb = threads / 32;
   const size_t sm = (size_t)wpb * W * 8;
-  if (sm > 48 * 1024) QCB_CUDA(cudaFuncSetAttribute(permute_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  if (sm > 48 * 1024) QCB_CUDA(allow_max_smem(permute_kernel));
   const uint32_t blocks = std::min<uint32_t>((rows + wpb - 1) / wpb, 4 * (uint32_t)device_sm_count());
   permute_kernel<<<blocks, threads, sm, st>>>(xzs, rows, n, W, d_perm);
   QCB_LAUNCHED();
@@ -1765,7 +1765,7 @@ int generate_dev(uint64_t* pauli, uint8_t* pph, const uint64_t* xzs, const uint8
                  uint32_t W, int phases, int32_t* d_ok, int32_t* d_used, uint32_t cap, uint32_t* d_nused,
                  cudaStream_t st) {
   const size_t sm = (size_t)W * 8;
-  if (sm > 48 * 1024) QCB_CUDA(cudaFuncSetAttribute(generate_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  if (sm > 48 * 1024) QCB_CUDA(allow_max_smem(generate_kernel));
   generate_kernel<<<1, 1024, sm, st>>>(pauli, pph, xzs, ph, rows, W, phases, d_ok, d_used, cap, d_nused);
   QCB_LAUNCHED();
   return QCB_OK;

@@ -347,7 +347,7 @@ int qcb_evaluate_guesses(const qcb_frame* f, const uint32_t* logical_bits, size_
     QCB_LAUNCHED();
   }
   if (smF > 48 * 1024)
-    QCB_CUDA(cudaFuncSetAttribute(evaluate_guesses_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smF));
+    QCB_CUDA(allow_max_smem(evaluate_guesses_kernel));
   const uint32_t blocks = (uint32_t)std::min<uint64_t>((f->ncols + 255) / 256, 4ull * device_sm_count());
   evaluate_guesses_kernel<<<std::max<uint32_t>(blocks, 1), 256, smF, st>>>(
       f->record, f->pitch, f->frames, d_rows, (uint32_t)nlog, d_planes, (uint32_t)k, f->ncols, d_F, Fw, d_fails);

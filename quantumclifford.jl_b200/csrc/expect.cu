@@ -192,7 +192,7 @@ int qcb_expect(const qcb_tableau* t, int kind, int32_t rank, const qcb_tableau* 
     const bool mixed = kind == QCB_MIXED_DESTABILIZER;
     if (mixed && (rank < 0 || (uint32_t)rank > nn)) { cudaFreeAsync(d_out, st); return fail(QCB_EBOUNDS, "rank out of range"); }
     const uint32_t r = mixed ? (uint32_t)rank : nn;
-    if (sm > 48 * 1024) QCB_CUDA(cudaFuncSetAttribute(expect_destab_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    if (sm > 48 * 1024) QCB_CUDA(allow_max_smem(expect_destab_kernel));
     expect_destab_kernel<<<blocks, threads, sm, st>>>(t->xzs, t->phases, nn, r, mixed ? 1 : 0, W, paulis->xzs,
                                                        paulis->phases, k, d_out);
     QCB_LAUNCHED();
@@ -210,7 +210,7 @@ int qcb_expect(const qcb_tableau* t, int kind, int32_t rank, const qcb_tableau* 
       status = canonicalize_view(tmp, tph, r, n, W, 1, (int32_t*)t->scratch + 48, st, true);
     }
     if (status == QCB_OK) {
-      if (sm > 48 * 1024) QCB_CUDA(cudaFuncSetAttribute(expect_stab_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+      if (sm > 48 * 1024) QCB_CUDA(allow_max_smem(expect_stab_kernel));
       expect_stab_kernel<<<blocks, threads, sm, st>>>(tmp, tph, r, W, paulis->xzs, paulis->phases, k, d_out);
       QCB_LAUNCHED();
     }

@@ -1617,7 +1617,7 @@ static int project_impl(qcb_tableau* t, int kind, int32_t* rank_io, const uint64
   uint32_t* d_bar = nullptr;  // [0..1] barrier, [2..4] first anticommuting rows, [5] timeout flag
   if (grid) {
     if (gsm > 48 * 1024)
-      QCB_CUDA(cudaFuncSetAttribute(project_grid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsm));
+      QCB_CUDA(allow_max_smem(project_grid_kernel));
     int nb = 0;
     QCB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, project_grid_kernel, PROJ_THREADS, gsm));
     G = (uint32_t)std::max(1, nb) * (uint32_t)std::max(device_sm_count(), 1);

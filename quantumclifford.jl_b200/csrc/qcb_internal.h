@@ -42,6 +42,18 @@ inline cudaStream_t S(void* s) { return (cudaStream_t)s; }
 int device_sm_count();
 int device_max_smem_optin();
 
+// The kernel's limit of dynamic shared memory to all that its static part
+// leaves.  The limit belongs to the kernel, not to a call: it is never set to
+// one call's size, which calls on other threads could lower before the launch.
+template <class F>
+inline cudaError_t allow_max_smem(F* kernel) {
+  cudaFuncAttributes fa{};
+  const cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              device_max_smem_optin() - (int)fa.sharedSizeBytes);
+}
+
 // Device memory of library objects (frames, programs and their scratch), ready
 // for any stream on return.  Blocks of up to DEV_POOL_MAX bytes come from the
 // device's stream-ordered pool, which keeps freed ones (a bounded amount, see

@@ -95,3 +95,18 @@ def test_canonicalize_of_two_heights_at_once(qcb):
         _, xz, _, _ = oracle.canonicalize(t.phases, t.xzs, 130, False)
         g.to_cpu()
         assert np.array_equal(g.tab.xzs, xz)
+
+
+def test_permutations_of_two_widths_at_once(qcb):
+    """Rows of 50000 and 26000 qubits (98 and 51 KB of staging), two threads of each."""
+    jobs, tabs, rng = [], [], np.random.default_rng(4)
+    for n in (50_000, 26_000, 50_000, 26_000):
+        perm = np.arange(n, 0, -1, dtype=np.uint32)
+        t = random_rows(3, n, rng)
+        g = t.copy().to_gpu()
+        tabs.append((t, g))
+        jobs.append(lambda st, g=g, perm=perm: check(qcb.lib().qcb_permutesystems(g.dev.handle, ptr(perm), st)))
+    assert run_threads(jobs, 2000) == [None] * 4
+    for t, g in tabs:  # an even number of reversals
+        g.to_cpu()
+        assert np.array_equal(g.xzs, t.xzs)
