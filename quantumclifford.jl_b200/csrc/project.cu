@@ -1398,10 +1398,12 @@ static cudaError_t launch_pp(void (*k)(const ProjPanelArgs), uint32_t grid, uint
 // other kernels; 32 Paulis on 100 / 1000 / 4000 qubits 205 / 241 / 486 -> 181 /
 // 177 / 136 us with the call), the most stabilizer rows its search holds in
 // registers, the steps a run has to make before the next is tried at once, the
-// Paulis before the next trial after a first short one, and the panels queued
-// before anything is waited for.
+// Paulis before the next trial after a first failed one and those that have to be
+// left for it (a trial costs 20 to 40 us), and the panels queued before anything is
+// waited for.
 constexpr uint32_t PROJ_PANEL_MIN = 32, PROJ_PANEL_ROWS = PP_WINDOW + 9 * PP_REST, PROJ_PANEL_GOOD = 32,
-                   PROJ_PANEL_BACKOFF = 64, PROJ_TRIAL_PANELS = 4;
+                   PROJ_PANEL_BACKOFF = 64, PROJ_PANEL_AGAIN = 128,
+                   PROJ_TRIAL_PANELS = 4;
 
 // Projections [first, k) by panels until one that commutes with the stabilizer
 // (or all are done): begin(), queue() of the panels, store().  A run that ends
@@ -1635,6 +1637,9 @@ static int project_impl(qcb_tableau* t, int kind, int32_t* rank_io, const uint64
   const bool panels = !qubits && phases && len && !g_proj_grid && !g_proj_cs;
   const int skip = !keep_result && (kind == QCB_STABILIZER || (kind == QCB_DESTABILIZER && t->rows / 2 == t->nqubits));
   uint32_t next_try = 0, backoff = PROJ_PANEL_BACKOFF, tried = 0;
+  auto after = [&](uint32_t j) {  // the next trial behind a failed one at j, or none
+    return k - j >= backoff + PROJ_PANEL_AGAIN ? j + backoff : k;
+  };
   if (panels) {
     QCB_CUDA(cudaMemsetAsync(d_anti, 0, ((size_t)k + tries) * 4, st));
     QCB_CUDA(cudaMemsetAsync(d_res, 0xFF, (size_t)k * 4, st));
@@ -1655,8 +1660,8 @@ static int project_impl(qcb_tableau* t, int kind, int32_t* rank_io, const uint64
         bool none = false;
         if ((status = trial->begin(t, kind, nr, pxzs, pph, d_rand, j0, k, skip, d_anti, d_res, live, &none))) break;
         if (none) trial.reset();
-        next_try = j0 + backoff;
-        kend = std::min(k, next_try);
+        next_try = after(j0);
+        kend = next_try;
       }
     } else if (panels && next_try > j0 && (destab || next_try > j0 + 1)) {
       kend = std::min(k, next_try);
@@ -1676,7 +1681,7 @@ static int project_impl(qcb_tableau* t, int kind, int32_t* rank_io, const uint64
         backoff = PROJ_PANEL_BACKOFF;
         next_try = j0 + 1;
       } else {
-        next_try = j0 + backoff;
+        next_try = after(j0);
         backoff = std::min<uint32_t>(backoff * 4, 1u << 20);
       }
     };
