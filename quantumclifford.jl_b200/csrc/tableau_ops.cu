@@ -895,7 +895,8 @@ static cudaError_t launch_gates(void (*k)(P...), uint32_t grid, uint32_t block, 
 // 15, 29 and 50 gates), and many slices the tableau's traffic (a gate per MB).
 static size_t layer_min_gates(const qcb_tableau* t) {
   const size_t mb = ((size_t)t->rows * t->W * 8) >> 20;
-  return std::max(8 + mb, t->W / 12 + (t->rows > 4096 ? mb : 0));
+  const size_t least = t->rows < 64 || t->W <= 2 ? 12 : 8;  // the sorting into levels, 0.8 us on the host
+  return std::max(least + mb, t->W / 12 + (t->rows > 4096 ? mb : 0));
 }
 
 static size_t layer_smem(const qcb_tableau* t) { return (size_t)LAYER_SLICE * (2 * t->W + 1) * 4; }
