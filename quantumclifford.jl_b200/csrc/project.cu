@@ -1394,9 +1394,8 @@ static cudaError_t launch_pp(void (*k)(const ProjPanelArgs), uint32_t grid, uint
   return cudaLaunchKernelEx(&cfg, k, a);
 }
 
-// Runs worth a panel (a panel costs about as much as 10 to 15 Paulis of the
-// other kernels; 32 Paulis on 100 / 1000 / 4000 qubits 205 / 241 / 486 -> 181 /
-// 177 / 136 us with the call), the most stabilizer rows its search holds in
+// Runs worth a panel (32 random Paulis on 100 / 1000 / 4000 qubits 186 / 244 / 486
+// -> 112 / 114 / 142 us with the call), the most stabilizer rows its search holds in
 // registers, the steps a run has to make before the next is tried at once, the
 // Paulis before the next trial after a first failed one and those that have to be
 // left for it (a trial costs 20 to 40 us), and the panels queued before anything is

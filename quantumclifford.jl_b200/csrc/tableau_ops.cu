@@ -365,7 +365,7 @@ __global__ void apply_gates_kernel(uint64_t* xzs, uint8_t* ph, uint32_t rows, ui
 // a graph capture of the call would have to keep alive.  Bound by a level's
 // latency (the parameter reads, the words, a barrier: 0.3-0.5 us) and, for few
 // gates, by the transposes.  400 gates on a 2000 x 1000-qubit tableau: 7.1 us;
-// a circuit of 2300 gates on 1000 x 500 qubits 25 us, with one row per thread
+// a circuit of 2300 gates on 1000 x 500 qubits 11 us, with one row per thread
 // (every gate a read and a write of global words) 1.5 ms.
 //  list: per level a header (the level's gate count), then its gates
 //  (opcode and flags | q1 << 16 | q2 << 40, 0-based qubits below 2^24).
