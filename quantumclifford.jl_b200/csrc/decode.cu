@@ -287,7 +287,7 @@ int qcb_frame_syndrome_rows(const qcb_frame* f, const uint32_t* bits, size_t nse
   Scratch host_out(st);
   uint64_t* d_out = out;
   if (!out_on_device) {
-    QCB_CUDA(host_out.alloc(out_bytes));
+    QCB_CUDA(host_out.alloc(out_bytes, false));
     d_out = (uint64_t*)host_out.p;
   }
   // a run of consecutive record bits (the whole record, the syndrome of a

@@ -2119,7 +2119,7 @@ static void batch_widths(std::vector<BatchShape>& jobs, uint64_t nsm) {
       for (size_t k = 0; k < jobs.size(); k++) {
         const BatchShape& b = jobs[k];
         double least = 0;
-        T[k] = b.T;
+        T[k] = b.T ? b.T : 16;  // a frame without shots has no tiles
         for (uint32_t j = 0, t = 0; !b.T && t < b.tmax && t < b.ncols && j < 16; j++) {
           t = width(b, j);
           const double us = batch_tile_us(b, t), work = us * (double)((b.ncols + t - 1) / t);

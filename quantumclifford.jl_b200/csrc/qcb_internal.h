@@ -67,8 +67,8 @@ void dev_free(void* p, size_t bytes);
 
 // Scratch of one call from the stream-ordered pool, given back in stream order
 // when it goes out of scope.  cudaErrorMemoryAllocation (memory not there, or
-// the test knob "scratch_limit") leaves no error behind: the caller goes
-// another way.
+// for `optional` scratch the test knob "scratch_limit") leaves no error behind:
+// the caller goes another way.
 struct Scratch {
   uint8_t* p = nullptr;
   cudaStream_t st;
@@ -78,7 +78,7 @@ struct Scratch {
   ~Scratch() {
     if (p) cudaFreeAsync(p, st);
   }
-  cudaError_t alloc(size_t bytes);
+  cudaError_t alloc(size_t bytes, bool optional = true);
 };
 // Whether scratch of this size is to count as not there ("scratch_limit").
 bool scratch_refused(size_t bytes);

@@ -95,8 +95,8 @@ bool scratch_refused(size_t bytes) {
   return kb && bytes > (size_t)kb << 10;
 }
 
-cudaError_t Scratch::alloc(size_t bytes) {
-  cudaError_t e = scratch_refused(bytes) ? cudaErrorMemoryAllocation : cudaMallocAsync(&p, bytes, st);
+cudaError_t Scratch::alloc(size_t bytes, bool optional) {
+  cudaError_t e = optional && scratch_refused(bytes) ? cudaErrorMemoryAllocation : cudaMallocAsync(&p, bytes, st);
   if (e == cudaErrorMemoryAllocation) cudaGetLastError();
   if (e != cudaSuccess) p = nullptr;
   return e;

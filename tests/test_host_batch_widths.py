@@ -79,6 +79,12 @@ def test_given_widths_stay():
     assert got[0] == 20 and got[2] == 64
 
 
+def test_frames_without_shots():
+    got = widths([job(15, 0), job(15, 200_000), job(3, 0)])
+    assert all(16 <= t <= 256 for t in got)
+    assert widths([job(7, 0)])[0] >= 16
+
+
 def test_bad_arguments():
     with pytest.raises(qcb200.ArgumentError):
         widths([(1.0, 1.0, 1.0, 10, 8)])
